@@ -240,7 +240,8 @@ class OpTimer:
             proj, normaliser, n_seqs, H, dim, vdim = a[0], a[9], a[14], a[15], a[16], a[17]
             T, vs = proj.shape[0], vdim + (1 if normaliser else 0)
             flops = 4.0 * T * H * dim * vs
-            byts = float(T * (2 * H * dim + H * vdim) * proj.element_size() + T * H * vs * 4 + 2 * n_seqs * H * dim * vs * 4)
+            of_values = (kw.get("values") if kw.get("values") is not None else proj).element_size()
+            byts = float(T * (2 * H * dim * proj.element_size() + H * vdim * of_values) + T * H * vs * 4 + 2 * n_seqs * H * dim * vs * 4)
         elif name == "attn_prefill_paged":
             qkv, nq, nkv, hd, window = a[0], a[1], a[2], a[3], a[13]
             T = qkv.shape[0]

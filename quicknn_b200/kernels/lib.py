@@ -116,6 +116,8 @@ _SIGNATURES: Dict[str, list] = {
                       c_vp, c_int, c_int, c_vp],
     "qnn_memory_scan": [c_vp, c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_ll, c_float, c_int, c_vp, c_vp, c_vp, c_vp,
                         c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp],
+    "qnn_memory_chunks": [c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_ll, c_int, c_vp, c_ll, c_float, c_int, c_int, c_vp, c_vp,
+                          c_vp, c_vp, c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp],
     "qnn_mlstm_gates": [c_vp, c_ll, c_vp, c_int, c_float, c_vp, c_vp, c_vp, c_vp, c_ll, c_vp, c_int, c_int, c_vp],
     "qnn_group_rmsnorm": [c_vp, c_int, c_vp, c_int, c_float, c_int, c_vp, c_int, c_int, c_int, c_vp],
     "qnn_add2_group_rmsnorm": [c_vp, c_vp, c_int, c_vp, c_int, c_vp, c_int, c_float, c_int, c_vp, c_int, c_int, c_int, c_vp],

@@ -1032,6 +1032,49 @@ GLA_SEGMENT = 256            # rows of a segment when long sequences are walked 
 GLA_SEGMENTS_FROM = 512      # the longest sequence of a step from which that is done
 
 
+MEMORY_CHUNK = 64            # rows of a chunk of qnn_memory_chunks
+# The longest sequence of a step from which prompts run in chunks on the tensor cores: one decay per head (or 64 key channels
+# with a decay each), and 128 channels with a decay each.  Measured (us, chunks / row by row; 12 heads of 64 x 128 and 9 of 128 x 256):
+# a gate per head, one sequence of 64 / 96 / 300 rows: 20.5 / 20.9, 20.5 / 29.9, 21.8 / 87.9 and 35.7 / 27.4, 35.8 / 38.8, 36.8 / 111;
+# eight sequences: 27 / 27, 35 / 39, 64 / 113 and 52 / 74, 54 / 106, 116 / 313.  A decay per channel, one sequence: 22.3 / 20.3,
+# 22.7 / 29.4, 23.4 / 87 and (128 rows: 56 / 49) 57 / 110; eight: 29 / 26, 41 / 38, 76 / 111 and (128 rows: 68 / 71) 144 / 160.
+# One prompt of 2048 rows, 9 heads of 128 x 256: 89 against 330 us (the walk in segments); 2813 rows in three prompts, 12 heads
+# of 64 x 128, a gate per head: 72 against 550 us.
+MEMORY_CHUNKS_FROM, MEMORY_CHUNKS_FROM_WIDE = 96, 160
+MEMORY_CHUNKS_SCRATCH = 80 << 20      # bytes of chunk states per round, which then stay in L2 between the three kernels
+
+
+def memory_chunks_fit(values_dtype: torch.dtype, dim: int, vdim: int, longest: int, *columns: int, per_channel: bool = False) -> bool:
+    """Whether prompts run in chunks of 64 rows on the tensor cores: bfloat16 values, heads of 64 or 128 key channels and up to
+    256 value columns, rows and first columns (``columns``) on 16 bytes, and a sequence that is long enough.  Everything
+    else (single tokens, short steps, float32 models, other sizes) walks the rows one by one."""
+    least = MEMORY_CHUNKS_FROM_WIDE if per_channel and dim > 64 else MEMORY_CHUNKS_FROM
+    return (values_dtype == torch.bfloat16 and longest >= least and dim in (64, 128) and vdim % 8 == 0
+            and 8 <= vdim <= 256 and all(c % 8 == 0 for c in columns))
+
+
+def _memory_chunks(qk: torch.Tensor, q_col: int, k_col: int, values: torch.Tensor, v_col: int, decay: torch.Tensor, decay_ld: int,
+                   per_channel: bool, key_weight: Optional[torch.Tensor], kw_col: int, q_scale: float, normaliser: bool,
+                   key_from_decay: bool, seq_row0: torch.Tensor, seq_len: torch.Tensor, slots: torch.Tensor, state: torch.Tensor,
+                   state_stride: int, out: torch.Tensor, n_seqs: int, n_heads: int, dim: int, vdim: int, longest: int) -> None:
+    chunks = -(-longest // MEMORY_CHUNK)
+    at_once = max(1, min(chunks, MEMORY_CHUNKS_SCRATCH // (4 * n_seqs * n_heads * dim * vdim)))
+    rounds = -(-chunks // at_once)
+    at_once = -(-chunks // rounds)
+    units = n_seqs * at_once * n_heads
+    n_local, n_norm, n_decay = units * dim * vdim, units * dim if normaliser else 0, 2 * units * (dim if per_channel else 1)
+    scratch = torch.empty(n_local + n_norm + n_decay, dtype=torch.float32, device=qk.device)
+    ldw = 0 if key_weight is None else key_weight.shape[1]
+    at = lambda n: ctypes.c_void_p(scratch.data_ptr() + 4 * n)  # noqa: E731
+    for r in range(rounds):
+        _lib.check(_lib.load().qnn_memory_chunks(
+            _col_ptr(qk, q_col), _col_ptr(qk, k_col), qk.shape[1], dt_code(qk), _col_ptr(values, v_col), values.shape[1],
+            _p(decay), int(decay_ld), int(per_channel), _col_ptr(key_weight, kw_col) if key_weight is not None else None, ldw,
+            float(q_scale), int(normaliser), int(key_from_decay), _p(seq_row0), _p(seq_len), _p(slots), _p(state),
+            int(state_stride), _p(out), out.shape[1], n_seqs, n_heads, dim, vdim, r * at_once * MEMORY_CHUNK, at_once,
+            at(0), at(n_local), at(n_local + n_norm), _stream()), "memory_chunks", 3)
+
+
 def gla_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, q_scale: float,
              seq_row0: Optional[torch.Tensor], seq_len: Optional[torch.Tensor], slots: torch.Tensor,
              state: torch.Tensor, n_seqs: int, n_heads: int, dim: int, vdim: int, longest: int = 0,
@@ -1040,8 +1083,8 @@ def gla_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torc
     state of the sequence's slot and back into it.  ``proj`` holds q and k ([*, heads*dim]) and v ([*, heads*vdim])
     from the given columns on; ``decay`` the decays a, float32 [rows, heads*dim]; returns o, float32 [rows, heads*vdim].
 
-    ``longest``: the most rows that one sequence brings (0: unknown).  From 512 rows on the sequences are cut into
-    segments of 256 rows that run side by side (the recurrence is linear in the state: each segment's own state and
+    ``longest``: the most rows that one sequence brings (0: unknown).  Where ``memory_chunks_fit`` the rows run in chunks
+    on the tensor cores.  Otherwise, from 512 rows on, the sequences are cut into segments of 256 rows that run side by side (the recurrence is linear in the state: each segment's own state and
     decay product first, a short pass over the segments in order, then the outputs); results differ from the walk
     in one piece by rounding only.  ``key_from_decay``: the keys are 1 - a, formed in float32 inside the scan (what the
     forget gate lets go is what is written); ``k_col`` is then not read."""
@@ -1059,6 +1102,12 @@ def gla_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torc
     if seq_row0 is None and T < n_seqs:
         raise ValueError("gla_scan: fewer rows than sequences")
     out = torch.empty((T, n_heads * vdim), dtype=torch.float32, device=proj.device)
+    if (seq_row0 is not None and memory_chunks_fit(proj.dtype, dim, vdim, longest, proj.shape[1], q_col, k_col, v_col,
+                                                         per_channel=True)
+            and (proj.data_ptr() | decay.data_ptr()) % 16 == 0):
+        _memory_chunks(proj, q_col, k_col, proj, v_col, decay, decay.shape[1], True, None, 0, q_scale, False, key_from_decay,
+                       seq_row0, seq_len, slots, state, n_heads * dim * vdim, out, n_seqs, n_heads, dim, vdim, longest)
+        return out
     if seq_row0 is not None and longest >= GLA_SEGMENTS_FROM and n_seqs * -(-longest // GLA_SEGMENT) <= 65535:
         nseg = -(-longest // GLA_SEGMENT)
         scratch = torch.zeros((n_seqs * nseg, n_heads, dim, vdim), dtype=torch.float32, device=proj.device)
@@ -1449,7 +1498,7 @@ def memory_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: t
                 key_weight: Optional[torch.Tensor], kw_col: int, q_scale: float, normaliser: bool,
                 seq_row0: Optional[torch.Tensor],
                 seq_len: Optional[torch.Tensor], slots: torch.Tensor, state: torch.Tensor, n_seqs: int, n_heads: int,
-                dim: int, vdim: int, longest: int = 0) -> torch.Tensor:
+                dim: int, vdim: int, longest: int = 0, values: Optional[torch.Tensor] = None) -> torch.Tensor:
     """S_t = d_t S_{t-1} + w_t k_t v_t^T, o_t = S_t^T (q_t q_scale) over the rows of every sequence in order, from
     the state of the sequence's slot and back into it; d and w are one float32 number per (row, head).
 
@@ -1457,7 +1506,9 @@ def memory_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: t
     per head); ``key_weight``: float32 rows with the weights of a row's heads from column ``kw_col`` on, or None for 1.  ``normaliser``: the state has a column more
     than v, fed 1 in every row (n_t = d_t n_{t-1} + w_t k_t); the result then has vdim + 1 columns per head, the last
     being n_t . q_t.  ``state``: float32 [slots, floats per slot], a slot's [heads, dim, vdim (+1)] first.  Returns
-    float32 [rows, heads * (vdim (+1))].  Long sequences run in segments side by side like ``gla_scan``."""
+    float32 [rows, heads * (vdim (+1))].  Long sequences run in chunks, or in segments side by side, like ``gla_scan``.
+    ``values``: the rows that hold v (from ``v_col`` on) where they are not ``proj``'s: bfloat16 beside float32 queries and
+    keys, for steps that ``memory_chunks_fit``."""
     _req(proj, "proj", None, 2)
     _req(decay, "decay", torch.float32)
     _req(slots, "slots", torch.int32, 1)
@@ -1474,6 +1525,17 @@ def memory_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: t
             raise ValueError("memory_scan: a key weight per (row, head)")
     ldw = 0 if key_weight is None else key_weight.shape[1]
     out = torch.empty((T, n_heads * vs), dtype=torch.float32, device=proj.device)
+    rows = proj if values is None else values
+    if (seq_row0 is not None and memory_chunks_fit(rows.dtype, dim, vdim, longest, rows.shape[1], v_col, proj.shape[1], q_col, k_col)
+            and (proj.data_ptr() | rows.data_ptr()) % 16 == 0):
+        _req(rows, "values", None, 2)
+        if rows.shape[0] != T:
+            raise ValueError("memory_scan: a row of values per row")
+        _memory_chunks(proj, q_col, k_col, rows, v_col, decay, decay_ld, False, key_weight, kw_col, q_scale, normaliser, False,
+                       seq_row0, seq_len, slots, state, state.shape[1], out, n_seqs, n_heads, dim, vdim, longest)
+        return out
+    if values is not None:
+        raise ValueError("memory_scan: values of their own need a step that runs in chunks")
     seg_len = nseg = 0
     scratch = seg_decay = None
     if seq_row0 is not None and longest >= GLA_SEGMENTS_FROM and n_seqs * -(-longest // GLA_SEGMENT) <= 65535:

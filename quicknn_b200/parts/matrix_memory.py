@@ -26,8 +26,8 @@ the read-out of all heads together is RMS-normed with a weight per column and mu
 
 The state lives in the cache's fixed-size state region, float32, zeroed when the slot is handed out: for ``mlstm`` a
 slot keeps [heads, dim, vdim + 1] (the last column is n: the normaliser is the state column of a value that is 1 in
-every row) and then m per head.  One scan walks every sequence's rows in order from the slot's state and back, so
-prompts, portions and single tokens are the same launches.  Gates, decays, rotation angles, the state and the norms
+every row) and then m per head.  One scan takes every sequence's rows in order from the slot's state and back: prompts,
+portions and single tokens, row by row or in chunks (``ops.memory_scan``).  Gates, decays, rotation angles, the state and the norms
 are float32 in both precisions; the rotated queries and keys of ``retention`` go into the scan as float32 rows (they are
 not rounded to bfloat16 again).  The scale of the keys (retention) is applied on the query's side of o = S^T q, which is
 linear in both.
@@ -104,13 +104,15 @@ class Retention(_MatrixMemory):
     def forward(self, x: torch.Tensor, step, line) -> torch.Tensor:
         H, d, vd = self.n_heads, self.dim, self.vdim
         p = project(x, self.w_in)                                         # q | k | v | gate
-        # rotated q and k, and v beside them, as float32 rows for the scan
-        rows = torch.empty((p.shape[0], H * (2 * d + vd)), dtype=torch.float32, device=p.device)
-        ops.head_prep(p, 0, H, H, H * vd, d, dst=rows, rot_dim=self.rot_dim, inv_freq=self.position.inv_freq,
-                      interleaved=getattr(self.position, "layout", "half") == "interleaved", tok_pos=step.tok_pos)
         row0, lens, longest = self._rows(step)
+        # rotated q and k as float32 rows for the scan; v stays where it is if the scan runs in chunks, and beside them if not
+        chunks = row0 is not None and ops.memory_chunks_fit(p.dtype, d, vd, longest, p.shape[1], 2 * H * d)
+        beside = 0 if chunks else H * vd
+        rows = torch.empty((p.shape[0], H * 2 * d + beside), dtype=torch.float32, device=p.device)
+        ops.head_prep(p, 0, H, H, beside, d, dst=rows, rot_dim=self.rot_dim, inv_freq=self.position.inv_freq,
+                      interleaved=getattr(self.position, "layout", "half") == "interleaved", tok_pos=step.tok_pos)
         o = ops.memory_scan(rows, 0, H * d, 2 * H * d, self.decay_dev, 0, None, 0, float(d) ** -0.5, False, row0, lens,
-                            step.slots, line.state, step.n_seqs, H, d, vd, longest=longest)
+                            step.slots, line.state, step.n_seqs, H, d, vd, longest=longest, values=p if chunks else None)
         g = ops.head_norm_gate(o, vd, H, vd, self.eps, p, 2 * H * d + H * vd, "silu")
         return project(g, self.w_o)
 
