@@ -9,7 +9,7 @@
 //   qnn_activation         out = act(x) elementwise (gelu_tanh, silu, squared relu)
 //
 // All sums are float32; a block per row; the order of a row's sums depends on the width only.
-#include "common.cuh"
+#include "rows.cuh"
 
 using namespace qnn;
 
@@ -38,6 +38,56 @@ __global__ void layernorm_kernel(const void* __restrict__ x, int x_dt, const voi
     const float inv = rsqrtf(block_sum(ss, red) / (float)H + eps);
     for (int i = threadIdx.x; i < H; i += blockDim.x)
         store_from_f(out, out_dt, base + i, (load_as_f(x, x_dt, base + i) - mean) * inv * load_as_f(w, w_dt, i));
+}
+
+__global__ void __launch_bounds__(ROW8_THREADS)
+layernorm_vec_kernel(const void* __restrict__ x, int x_dt, const void* __restrict__ w, int w_dt, float eps,
+                     void* __restrict__ out, int out_dt, int H) {
+    __shared__ float red[32];
+    const size_t base = (size_t)blockIdx.x * H;
+    float g[8], v[8];
+    row8_load(w, w_dt, 0, H, g);
+    pdl_wait();
+    row8_load(x, x_dt, base, H, v);
+    const float mean = block_sum(sum8(v), red) / (float)H;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = (int)threadIdx.x * 8 < H ? v[e] - mean : 0.f;
+    const float inv = rsqrtf(block_sum(squares8(v), red) / (float)H + eps);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * g[e];
+    row8_store(out, out_dt, base, H, v);
+}
+
+// resid += layernorm(v) * g of a row in registers (g and the stream's row r were asked for before)
+__device__ __forceinline__ void add_layernorm_of_row8(float (&v)[8], const float (&r)[8], const float (&g)[8], float* red,
+                                                      float* __restrict__ resid, float eps, void* __restrict__ copy, int copy_dt, int H) {
+    const size_t base = (size_t)blockIdx.x * H;
+    const float mean = block_sum(sum8(v), red) / (float)H;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = (int)threadIdx.x * 8 < H ? v[e] - mean : 0.f;
+    const float inv = rsqrtf(block_sum(squares8(v), red) / (float)H + eps);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = r[e] + v[e] * inv * g[e];
+    row8_store(resid, QNN_DT_F32, base, H, v);
+    if (copy != nullptr) row8_store(copy, copy_dt, base, H, v);
+}
+
+__global__ void __launch_bounds__(ROW8_THREADS)
+add_layernorm_vec_kernel(float* __restrict__ resid, const void* __restrict__ y, int y_dt,
+                         const void* __restrict__ bias, int b_dt, const void* __restrict__ w, int w_dt,
+                         float eps, void* __restrict__ copy, int copy_dt, int H) {
+    __shared__ float red[32];
+    const size_t base = (size_t)blockIdx.x * H;
+    float g[8], b[8], v[8], r[8];
+    row8_load(w, w_dt, 0, H, g);
+    if (bias != nullptr) row8_load(bias, b_dt, 0, H, b);
+    else zero8(b);
+    pdl_wait();
+    row8_load(y, y_dt, base, H, v);
+    row8_load(resid, QNN_DT_F32, base, H, r);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] += b[e];
+    add_layernorm_of_row8(v, r, g, red, resid, eps, copy, copy_dt, H);
 }
 
 // The row that is normed is held in shared memory as float32 (row[H]) once it has been formed.
@@ -121,6 +171,44 @@ __global__ void add_mean_layernorm_kernel(float* __restrict__ resid, Branches br
     add_layernorm_of_row(row, red, resid, w, w_dt, eps, copy, copy_dt, H);
 }
 
+// Up to 4096 columns: the branches' rows take more registers than a block of 1024 threads has
+constexpr int MEAN_ROW8_MAX = 4096;
+__global__ void __launch_bounds__(MEAN_ROW8_MAX / 8)
+add_mean_layernorm_vec_kernel(float* __restrict__ resid, Branches br, int y_dt, int bw_dt, float eps_branch,
+                              const void* __restrict__ w, int w_dt, float eps, void* __restrict__ copy,
+                              int copy_dt, int H) {
+    __shared__ float red[32];
+    const size_t base = (size_t)blockIdx.x * H;
+    float g[8], r[8], y[MAX_BRANCHES][8], mean[8];
+    row8_load(w, w_dt, 0, H, g);
+    pdl_wait();
+#pragma unroll
+    for (int b = 0; b < MAX_BRANCHES; ++b)
+        if (b < br.n) row8_load(br.y[b], y_dt, base, H, y[b]);
+    row8_load(resid, QNN_DT_F32, base, H, r);
+    zero8(mean);
+#pragma unroll
+    for (int b = 0; b < MAX_BRANCHES; ++b)
+        if (b < br.n) {
+            float bw[8];
+            row8_load(br.w[b], bw_dt, 0, H, bw);
+            const float inv = rsqrtf(block_sum(squares8(y[b]), red) / (float)H + eps_branch);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) mean[e] += y[b][e] * inv * bw[e];
+        }
+    const float share = 1.f / (float)br.n;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) mean[e] *= share;
+    add_layernorm_of_row8(mean, r, g, red, resid, eps, copy, copy_dt, H);
+}
+
+inline bool branches_fit(const Branches& br, int H, std::initializer_list<const void*> ps) {
+    if (!row8_fits(H, ps) || H > MEAN_ROW8_MAX) return false;
+    for (int b = 0; b < br.n; ++b)
+        if ((((uintptr_t)br.y[b] | (uintptr_t)br.w[b]) & 15) != 0) return false;
+    return true;
+}
+
 __global__ void add_bias_kernel(void* __restrict__ y, int dt, const void* __restrict__ bias, int b_dt, int N, size_t total) {
     pdl_wait();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -153,6 +241,10 @@ QNN_API int qnn_layernorm(const void* x, int x_dt, const void* w, int w_dt, floa
                           cudaStream_t st) {
     if (T <= 0) return 0;
     if (H <= 0) return QNN_ERR_ARGUMENT;
+    if (row8_fits(H, {x, w, out})) {
+        launch_pdl(layernorm_vec_kernel, dim3(T), dim3(row8_threads(H)), 0, st, x, x_dt, w, w_dt, eps, out, out_dt, H);
+        QNN_LAUNCH_CHECK();
+    }
     launch_pdl(layernorm_kernel, dim3(T), dim3(row_threads(H)), 0, st, x, x_dt, w, w_dt, eps, out, out_dt, H);
     QNN_LAUNCH_CHECK();
 }
@@ -163,6 +255,11 @@ QNN_API int qnn_add_layernorm(float* resid, const void* y, int y_dt, const void*
     if (T <= 0) return 0;
     if (H <= 0) return QNN_ERR_ARGUMENT;
     if ((size_t)H * sizeof(float) > 160 * 1024) return QNN_ERR_UNSUPPORTED;
+    if (row8_fits(H, {resid, y, bias, w, copy})) {
+        launch_pdl(add_layernorm_vec_kernel, dim3(T), dim3(row8_threads(H)), 0, st, resid, y, y_dt, bias, b_dt, w, w_dt, eps, copy,
+                   copy_dt, H);
+        QNN_LAUNCH_CHECK();
+    }
     const size_t smem = (size_t)H * sizeof(float);
     static bool set = false;
     if (smem > 40 * 1024 && !set) {      // beside the static shared memory
@@ -200,6 +297,11 @@ QNN_API int qnn_add_mean_layernorm(float* resid, const void* const* ys, const vo
     if ((size_t)H * sizeof(float) > 160 * 1024) return QNN_ERR_UNSUPPORTED;
     Branches br;
     if (int rc = fill(br, ys, ws, n)) return rc;
+    if (branches_fit(br, H, {resid, w, copy})) {
+        launch_pdl(add_mean_layernorm_vec_kernel, dim3(T), dim3(row8_threads(H)), 0, st, resid, br, y_dt, bw_dt, eps_branch, w, w_dt, eps,
+                   copy, copy_dt, H);
+        QNN_LAUNCH_CHECK();
+    }
     const size_t smem = (size_t)H * sizeof(float);
     static bool set = false;
     if (smem > 40 * 1024 && !set) {      // beside the static shared memory

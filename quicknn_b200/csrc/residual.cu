@@ -10,7 +10,7 @@
 //   qnn_gate_heads           the same with the gate's logits x . w_h formed in the kernel
 //   qnn_small_linear_f32     x w^T with float32 sums and float32 results, for the few outputs that feed
 //                            float32 math (gates, decay logits)
-#include "common.cuh"
+#include "rows.cuh"
 
 using namespace qnn;
 
@@ -33,6 +33,53 @@ __global__ void add_scaled_rmsnorm_kernel(float* __restrict__ resid, const void*
     const float inv = rsqrtf(ss / (float)H + eps);
     for (int i = threadIdx.x; i < H; i += blockDim.x)          // each thread re-reads what it wrote itself
         store_from_f(out, out_dt, base + i, resid[base + i] * inv * (load_as_f(w, w_dt, i) + offset));
+}
+
+__global__ void __launch_bounds__(ROW8_THREADS)
+add_scaled_rmsnorm_vec_kernel(float* __restrict__ resid, const void* __restrict__ y, int y_dt, float scale,
+                              const void* __restrict__ w, int w_dt, float eps, float offset,
+                              void* __restrict__ out, int out_dt, int H) {
+    __shared__ float red[32];
+    const size_t base = (size_t)blockIdx.x * H;
+    float g[8], v[8], r[8];
+    if (out != nullptr) row8_load(w, w_dt, 0, H, g);         // no kernel of a step writes weights
+    pdl_wait();
+    row8_load(y, y_dt, base, H, v);
+    row8_load(resid, QNN_DT_F32, base, H, r);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r[e] = r[e] + scale * v[e];
+    row8_store(resid, QNN_DT_F32, base, H, r);
+    if (out == nullptr) return;
+    const float inv = rsqrtf(block_sum(squares8(r), red) / (float)H + eps);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r[e] = r[e] * inv * (g[e] + offset);
+    row8_store(out, out_dt, base, H, r);
+}
+
+__global__ void __launch_bounds__(ROW8_THREADS)
+rmsnorm_strided_vec_kernel(const void* __restrict__ x, int x_dt, long long ldx, const void* __restrict__ w,
+                           int w_dt, float eps, void* __restrict__ out, int out_dt, long long ldo,
+                           void* __restrict__ out2, long long ldo2, int N) {
+    __shared__ float red[32];
+    float g[8], v[8];
+    row8_load(w, w_dt, 0, N, g);
+    pdl_wait();
+    row8_load(x, x_dt, (size_t)blockIdx.x * ldx, N, v);
+    const float inv = rsqrtf(block_sum(squares8(v), red) / (float)N + eps);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * g[e];
+    row8_store(out, out_dt, (size_t)blockIdx.x * ldo, N, v);
+    if (out2) row8_store(out2, out_dt, (size_t)blockIdx.x * ldo2, N, v);
+}
+
+// rows of 16-byte pieces, a block per 256 of them
+__global__ void __launch_bounds__(256) copy_rows_vec_kernel(const uint4* __restrict__ src, long long lds, uint4* __restrict__ dst,
+                                                            long long ldd, int per_row, unsigned total) {
+    pdl_wait();
+    const unsigned i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= total) return;
+    const unsigned t = i / per_row, c = i - t * per_row;
+    dst[(size_t)t * ldd + c] = src[(size_t)t * lds + c];
 }
 
 __global__ void rmsnorm_strided_kernel(const void* __restrict__ x, int x_dt, long long ldx, const void* __restrict__ w,
@@ -91,15 +138,68 @@ __global__ void small_linear_warp_kernel(const TX* __restrict__ x, const TW* __r
     const size_t t = i / N;
     const TX* xr = x + t * K;
     const TW* wr = w + (i - t * N) * K;
+    constexpr int VX = Vec16<TX>::N, VW = Vec16<TW>::N, V = VX > VW ? VX : VW;
     float d = 0.f;
-    for (int k = lane; k < K; k += 32) d += to_f(xr[k]) * to_f(wr[k]);
+    if (K % V == 0 && ((((uintptr_t)x | (uintptr_t)w) & 15) == 0)) {     // 16-byte loads where the rows allow
+        for (int k = lane * V; k < K; k += 32 * V) {
+            float xf[V], wf[V];
+#pragma unroll
+            for (int j = 0; j < V; j += VX) { Vec16<TX> v; v.load(xr + k + j); v.unpack(xf + j); }
+#pragma unroll
+            for (int j = 0; j < V; j += VW) { Vec16<TW> v; v.load(wr + k + j); v.unpack(wf + j); }
+#pragma unroll
+            for (int j = 0; j < V; ++j) d += xf[j] * wf[j];
+        }
+    } else {
+        for (int k = lane; k < K; k += 32) d += to_f(xr[k]) * to_f(wr[k]);
+    }
     d = warp_sum(d);
     if (lane == 0) out[i] = finish(d, bias, bias_dt, inv_tau, (int)(i - t * N));
 }
 // Short rows: a thread per output; a block owns 8 rows x 32 outputs and reads their inner elements through shared
 // memory (the weight rows of neighbouring outputs lie K elements apart: read directly, every load of a warp
 // would touch 32 lines).
+// With many rows a block owns 32 of them and a thread four: a weight's element then serves four sums and a row's elements come four
+// at a time (one row per thread reads shared memory twice for every product: 2048 rows, 1152 outputs of 64, 57 -> 35 us).  The order
+// of a sum is the same.
 constexpr int SL_ROWS = 8, SL_OUTS = 32, SL_MAXK = 128;
+template <typename TX, typename TW>
+__global__ void __launch_bounds__(SL_ROWS * SL_OUTS)
+small_linear_rows_kernel(const TX* __restrict__ x, const TW* __restrict__ w, float* __restrict__ out, int T, int N, int K,
+                         const void* __restrict__ bias, int bias_dt, float inv_tau) {
+    constexpr int R = 4;
+    __shared__ __align__(16) float xs[SL_ROWS * R][SL_MAXK];
+    __shared__ float ws[SL_OUTS][SL_MAXK + 1];
+    pdl_wait();
+    const int t0 = blockIdx.y * SL_ROWS * R, n0 = blockIdx.x * SL_OUTS, Kp = (K + 3) / 4 * 4;
+    for (int idx = threadIdx.x; idx < SL_ROWS * R * Kp; idx += blockDim.x) {
+        const int r = idx / Kp, kk = idx - r * Kp;
+        xs[r][kk] = t0 + r < T && kk < K ? to_f(x[(size_t)(t0 + r) * K + kk]) : 0.f;
+    }
+    for (int idx = threadIdx.x; idx < SL_OUTS * Kp; idx += blockDim.x) {
+        const int c = idx / Kp, kk = idx - c * Kp;
+        ws[c][kk] = n0 + c < N && kk < K ? to_f(w[(size_t)(n0 + c) * K + kk]) : 0.f;
+    }
+    __syncthreads();
+    const int r = threadIdx.x / SL_OUTS, c = threadIdx.x % SL_OUTS;
+    float d[R] = {};
+    for (int kk = 0; kk < Kp; kk += 4) {
+        const float w4[4] = {ws[c][kk], ws[c][kk + 1], ws[c][kk + 2], ws[c][kk + 3]};
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const float4 v = *reinterpret_cast<const float4*>(&xs[r + u * SL_ROWS][kk]);
+            d[u] += v.x * w4[0];
+            d[u] += v.y * w4[1];
+            d[u] += v.z * w4[2];
+            d[u] += v.w * w4[3];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+        const int t = t0 + r + u * SL_ROWS;
+        if (t < T && n0 + c < N) out[(size_t)t * N + n0 + c] = finish(d[u], bias, bias_dt, inv_tau, n0 + c);
+    }
+}
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(SL_ROWS * SL_OUTS)
 small_linear_thread_kernel(const TX* __restrict__ x, const TW* __restrict__ w, float* __restrict__ out, int T, int N, int K,
@@ -182,6 +282,11 @@ QNN_API int qnn_add_scaled_rmsnorm(float* resid, const void* y, int y_dt, float 
                                    int unit_offset, void* out, int out_dt, int T, int H, cudaStream_t st) {
     if (T <= 0) return 0;
     if (H <= 0 || (out != nullptr && w == nullptr)) return QNN_ERR_ARGUMENT;
+    if (row8_fits(H, {resid, y, w, out})) {
+        launch_pdl(add_scaled_rmsnorm_vec_kernel, dim3(T), dim3(row8_threads(H)), 0, st, resid, y, y_dt, scale, w, w_dt, eps,
+                   unit_offset ? 1.f : 0.f, out, out_dt, H);
+        QNN_LAUNCH_CHECK();
+    }
     launch_pdl(add_scaled_rmsnorm_kernel, dim3(T), dim3(row_threads(H)), 0, st, resid, y, y_dt, scale, w, w_dt, eps,
                unit_offset ? 1.f : 0.f, out, out_dt, H);
     QNN_LAUNCH_CHECK();
@@ -191,6 +296,11 @@ QNN_API int qnn_rmsnorm_strided(const void* x, int x_dt, long long ldx, const vo
                                 int out_dt, long long ldo, void* out2, long long ldo2, int T, int N, cudaStream_t st) {
     if (T <= 0) return 0;
     if (N <= 0 || ldx < N || ldo < N || (out2 && ldo2 < N)) return QNN_ERR_ARGUMENT;
+    if (row8_fits(N, {x, w, out, out2}, {ldx * dt_bytes(x_dt), ldo * dt_bytes(out_dt), out2 ? ldo2 * dt_bytes(out_dt) : 0})) {
+        launch_pdl(rmsnorm_strided_vec_kernel, dim3(T), dim3(row8_threads(N)), 0, st, x, x_dt, ldx, w, w_dt, eps, out, out_dt, ldo,
+                   out2, ldo2, N);
+        QNN_LAUNCH_CHECK();
+    }
     launch_pdl(rmsnorm_strided_kernel, dim3(T), dim3(row_threads(N)), 0, st, x, x_dt, ldx, w, w_dt, eps, out, out_dt, ldo,
                out2, ldo2, N);
     QNN_LAUNCH_CHECK();
@@ -199,6 +309,12 @@ QNN_API int qnn_rmsnorm_strided(const void* x, int x_dt, long long ldx, const vo
 QNN_API int qnn_copy_rows(const void* src, int dt, long long lds, void* dst, long long ldd, int T, int N, cudaStream_t st) {
     if (T <= 0) return 0;
     if (N <= 0 || lds < N || ldd < N) return QNN_ERR_ARGUMENT;
+    const long long es = dt_bytes(dt), total = (long long)T * (N * es / 16);
+    if (((((uintptr_t)src | (uintptr_t)dst) & 15) == 0) && N * es % 16 == 0 && lds * es % 16 == 0 && ldd * es % 16 == 0 && total < (1ll << 31)) {
+        launch_pdl(copy_rows_vec_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, (const uint4*)src, lds * es / 16,
+                   (uint4*)dst, ldd * es / 16, (int)(N * es / 16), (unsigned)total);
+        QNN_LAUNCH_CHECK();
+    }
     launch_pdl(copy_rows_kernel, dim3(T), dim3(row_threads(N)), 0, st, src, dt, lds, dst, ldd, N);
     QNN_LAUNCH_CHECK();
 }
@@ -222,6 +338,9 @@ QNN_API int qnn_small_linear_f32(const void* x, int x_dt, const void* w, int w_d
     if (K > SL_MAXK)                                                                                                 \
         launch_pdl(small_linear_warp_kernel<TX, TW>, dim3((unsigned)((total + 7) / 8)), dim3(256), 0, st,            \
                    (const TX*)x, (const TW*)w, out, N, K, total, bias, bias_dt, inv_tau);                            \
+    else if (T >= 128)                                                                                               \
+        launch_pdl(small_linear_rows_kernel<TX, TW>, dim3((N + SL_OUTS - 1) / SL_OUTS, (T + 4 * SL_ROWS - 1) / (4 * SL_ROWS)), \
+                   dim3(SL_ROWS * SL_OUTS), 0, st, (const TX*)x, (const TW*)w, out, T, N, K, bias, bias_dt, inv_tau); \
     else                                                                                                             \
         launch_pdl(small_linear_thread_kernel<TX, TW>, dim3((N + SL_OUTS - 1) / SL_OUTS, (T + SL_ROWS - 1) / SL_ROWS), \
                    dim3(SL_ROWS * SL_OUTS), 0, st, (const TX*)x, (const TW*)w, out, T, N, K, bias, bias_dt, inv_tau);

@@ -1,0 +1,81 @@
+"""Row kernels that take eight elements per thread, and those that walk a row, at the sizes where the way changes: the smallest
+rows, rows that are no whole number of warps, the largest, eight elements more, and rows that do not start on 16 bytes.
+
+Tolerance: sums of up to 8192 float32 terms by a tree (about 2^-24 sqrt(13)) and a few roundings: 2e-6 of the row's largest value;
+bfloat16 results one rounding of 2^-8."""
+import pytest
+import torch
+
+from quicknn_b200.kernels import ops
+from quicknn_b200.kernels.lib import NonFiniteLogits
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+WIDTHS = [8, 24, 256, 264, 2304, 4096, 4104, 8184, 8192, 8200, 100, 2305]
+
+
+def close(got, want, dtype=torch.float32):
+    tol = 2e-6 if dtype == torch.float32 else 2 ** -8
+    assert ((got.double() - want).abs().amax(-1) <= tol * want.abs().amax(-1).clamp(min=1e-30)).all()
+
+
+def rms(x, eps):
+    return x / (x.pow(2).mean(-1, keepdim=True) + eps).sqrt()
+
+
+def layernorm(x, eps):
+    d = x - x.mean(-1, keepdim=True)
+    return d / (d.pow(2).mean(-1, keepdim=True) + eps).sqrt()
+
+
+@pytest.mark.parametrize("W", WIDTHS)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 9])
+def test_norms_and_adds(W, dtype, T):
+    torch.manual_seed(W + T)
+    mk = lambda *s: torch.randn(s, device=DEV).to(dtype)  # noqa: E731
+    x, y, z, w, b = mk(T, W), mk(T, W), mk(T, W), mk(W), mk(W)
+    stream = torch.randn((T, W), device=DEV)
+    D = lambda t: t.double()  # noqa: E731
+    close(ops.rmsnorm(x, w, 1e-6, True, dtype), rms(D(x), 1e-6) * (1 + D(w)), dtype)
+    r = stream.clone()
+    want = D(stream) + 0.5 * D(y)
+    out = ops.add_scaled_rmsnorm(r, y, 0.5, w, 1e-6, False, dtype)
+    close(r, want)
+    close(out, rms(want, 1e-6) * D(w), dtype)
+    close(ops.layernorm(x, w, 1e-5, dtype), layernorm(D(x), 1e-5) * D(w), dtype)
+    r = stream.clone()
+    copy = ops.add_layernorm(r, y, w, 1e-5, bias=b, copy_dtype=dtype)
+    want = D(stream) + layernorm(D(y) + D(b), 1e-5) * D(w)
+    close(r, want)
+    close(copy, want, dtype)
+    r = stream.clone()
+    copy = ops.add_mean_layernorm(r, [y, z], [b, w], 1e-6, w, 1e-5, dtype)
+    want = D(stream) + layernorm((rms(D(y), 1e-6) * D(b) + rms(D(z), 1e-6) * D(w)) / 2, 1e-5) * D(w)
+    close(r, want)
+    close(copy, want, dtype)
+    table = mk(7, W)
+    ids = torch.arange(T, dtype=torch.int32, device=DEV) % 7
+    close(ops.embed(ids, table, 3.0), 3.0 * D(table)[ids.long()])
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 4095, 4096, 4097, 1 << 20])
+@pytest.mark.parametrize("bad", [None, float("nan"), float("inf"), float("-inf")])
+def test_finite_check_sees_every_place(n, bad):
+    for place in {0, n // 2, n - 1}:
+        x = torch.zeros((1, n), device=DEV)
+        if bad is not None:
+            x[0, place] = bad
+        ops.check_finite(x)
+        if bad is None:
+            ops.raise_on_status(torch.device(DEV))
+        else:
+            with pytest.raises(NonFiniteLogits):
+                ops.raise_on_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("K,N,T", [(64, 40, 128), (61, 33, 127), (128, 32, 200), (3, 1, 129), (136, 5, 3), (130, 5, 3)])
+def test_few_outputs(K, N, T):
+    torch.manual_seed(K)
+    x, w = torch.randn((T, K), device=DEV).bfloat16(), torch.randn((N, K), device=DEV).bfloat16()
+    close(ops.small_linear_f32(x, w), x.double() @ w.double().T)
