@@ -45,10 +45,6 @@ constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2, STAGE_BYTES = 
 constexpr int TMEM_COLS = 256;
 constexpr int STAGING_BYTES = BM * 128 * 2;          // the epilogue's 128 rows x 128 columns of bfloat16
 constexpr int GEMM_THREADS = 192;
-// What sharing a tile among two or four pairs costs, in slabs of 0.3 us.  Measured (us, a pair per tile / shared): N x K = 2304 x 9216,
-// 256 rows 46.7 / 22.0, 640 rows 47.0 / 30.3; 2304 x 2048, 256 rows 15.1 / 10.8, 640 rows 15.6 / 12.8; 768 x 2304, 2048 rows 16.8 / 13.3;
-// 256 x 2304, 2048 rows 15.7 / 10.2; 2304 x 1152 (18 slabs), 256 rows 11.2 / 9.8.
-constexpr int SPLIT_COST_2 = 8, SPLIT_COST_4 = 10;
 
 
 // `bar` is a shared::cluster address: the leader's barrier, whichever CTA of the pair loads
@@ -64,10 +60,9 @@ __device__ __forceinline__ void umma_bf16(unsigned tmem_d, uint64_t adesc, uint6
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 // arrives, once everything issued so far is done, on the barrier at this offset in both CTAs of the pair
-// (`ctas`: their bits among the cluster's)
-__device__ __forceinline__ void umma_commit_pair(unsigned bar, unsigned ctas = 3) {
+__device__ __forceinline__ void umma_commit_pair(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"((unsigned short)ctas) : "memory");
+                 ::"r"(bar), "h"((unsigned short)3) : "memory");
 }
 
 
@@ -308,232 +303,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
 }
 
-// ---- few tiles: several pairs per tile ---------------------------------------------------------------------------------
-// A product of few rows and few columns has fewer 256 x 256 tiles than the device has pairs, and its time is one tile's walk over
-// K (144 slabs of 0.3 us for 9216).  Here a cluster of S pairs shares a tile: pair s takes a share of the slabs, and when it is
-// done hands every other pair the columns that pair finishes (256 / S of them), as float32: each epilogue warp lays them into its
-// idle ring and one thread sends them by bulk shared-to-shared copies, counted in bytes on the receiver's mbarrier.  The shares are
-// summed in their order, so a result does not depend on which pair comes last.  The place for what comes in stands beside the
-// ring (a pair may finish while another still walks), which therefore has fewer stages.  One tile per cluster, all clusters at once.
-template <int S>
-struct SplitPlan {
-    static constexpr int CW = BN / S;                                  // columns that a pair finishes
-    static constexpr int STAGES = S == 2 ? 5 : 4;
-    static constexpr int PIECE = 32 * CW * 4;                          // bytes of a warp's rows from one other pair
-    static constexpr int IN = STAGES * STAGE_BYTES;                    // [other pairs][4 warps] pieces that come in
-    static constexpr int OUT = (S - 1) * 4 * PIECE;                    // where the finished rows are staged, behind what goes out
-    static constexpr int BARS = IN + (S - 1) * 4 * PIECE, BYTES = BARS + 256 + 1024;
-    static_assert(OUT + BM * CW * 2 <= IN, "the ring holds what goes out and the finished rows");
-};
-struct __align__(8) SplitBarriers {
-    uint64_t full[5], empty[5];      // as above, per pair
-    uint64_t acc_ready;              // in each CTA
-    uint64_t come[4];                // in each CTA, per epilogue warp: the other pairs' shares of its rows are here (bytes)
-    uint32_t tmem_base;
-    uint32_t failed;
-};
-static_assert(sizeof(SplitBarriers) <= 256, "");
 
-template <int S>
-__global__ void __launch_bounds__(GEMM_THREADS)
-gemm_tcgen05_2cta_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                               bf16* __restrict__ C, int M, int N, int K, int act, ActConsts actk, int* __restrict__ status) {
-    using P = SplitPlan<S>;
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    SplitBarriers* bars = reinterpret_cast<SplitBarriers*>(smem + P::BARS);
-    volatile uint32_t* failed = &bars->failed;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned crank = cluster_rank(), rank = crank & 1, leader = crank & ~1u;
-    const int share = (int)(crank >> 1);
-    const int tile = blockIdx.x / (2 * S), m_tiles = (M + 2 * BM - 1) / (2 * BM);
-    const int m0 = (tile % m_tiles) * (2 * BM) + (int)rank * BM, n0 = (tile / m_tiles) * BN;
-    const int nk = (K + BK - 1) / BK, kb0 = nk * share / S, kb1 = nk * (share + 1) / S;
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < P::STAGES; ++s) {
-            mbar_init(smem_u32(&bars->full[s]), 1);
-            mbar_init(smem_u32(&bars->empty[s]), 1);
-        }
-        mbar_init(smem_u32(&bars->acc_ready), 1);
-        for (int w = 0; w < 4; ++w) mbar_init(smem_u32(&bars->come[w]), 1);
-        bars->failed = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        for (int w = 0; w < 4; ++w) mbar_expect_tx(smem_u32(&bars->come[w]), (S - 1) * P::PIECE);
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&bars->tmem_base)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    cluster_barrier();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const unsigned tmem = bars->tmem_base;
-    pdl_wait();
-
-    if (warp == 0) {
-        if (lane == 0) {
-            const int brow = n0 + (int)rank * (BN / 2);
-            for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-                const int s = it % P::STAGES;
-                if (it >= P::STAGES && !mbar_wait(smem_u32(&bars->empty[s]), ((it / P::STAGES) - 1) & 1)) {
-                    atomicOr(status, 1);
-                    *failed = 1;
-                    break;
-                }
-                const unsigned full_local = smem_u32(&bars->full[s]), full_leader = map_to_rank(full_local, leader);
-                const unsigned a_dst = smem_u32(smem + s * STAGE_BYTES), b_dst = a_dst + A_BYTES;
-                if (rank == 0) mbar_expect_tx(full_local, 2 * STAGE_BYTES);
-                tma_load_2d_pair(a_dst, &map_a, full_leader, kb * BK, m0);
-                tma_load_2d_pair(b_dst, &map_b, full_leader, kb * BK, brow);
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
-            const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)((2 * BM) >> 4) << 24);
-            for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-                const int s = it % P::STAGES;
-                if (!mbar_wait(smem_u32(&bars->full[s]), (it / P::STAGES) & 1)) {
-                    atomicOr(status, 2);
-                    *failed = 1;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const unsigned a_addr = smem_u32(smem + s * STAGE_BYTES), b_addr = a_addr + A_BYTES;
-#pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k)
-                    umma_bf16(tmem, umma_desc(a_addr + k * UMMA_K * 2), umma_desc(b_addr + k * UMMA_K * 2), idesc, (it > 0 || k > 0) ? 1u : 0u);
-                umma_commit_pair(smem_u32(&bars->empty[s]), 3u << leader);
-            }
-            umma_commit_pair(smem_u32(&bars->acc_ready), 3u << leader);
-        }
-    } else {
-        const int quarter = warp & 3;
-        bool ok = mbar_wait_warp(smem_u32(&bars->acc_ready), 0);
-        if (!ok) atomicOr(status, 4);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned lane_addr = tmem + ((unsigned)(quarter * 32) << 16);
-        // a piece: a warp's 32 rows as [columns / 4][lane] times 16 bytes, so that stores and loads are whole 512-byte lines
-        if (ok) {
-#pragma unroll 1
-            for (int d = 1; d < S; ++d) {                               // every pair begins with another
-                const int other = (share + d) % S, place = share < other ? share : share - 1;
-                unsigned char* out = smem + ((d - 1) * 4 + quarter) * P::PIECE;
-#pragma unroll 1
-                for (int c = 0; c < P::CW; c += 32) {
-                    uint32_t v[32];
-                    tmem_ld32(lane_addr + other * P::CW + c, v);
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4)
-                        *reinterpret_cast<uint4*>(out + (c + j) * 128 + lane * 16) = make_uint4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the copy below reads what was stored
-                __syncwarp();
-                if (lane == 0)
-                    bulk_copy_to_rank(smem_u32(smem + P::IN + (place * 4 + quarter) * P::PIECE), smem_u32(out), P::PIECE,
-                                      smem_u32(&bars->come[quarter]), 2 * other + rank);
-            }
-            ok = mbar_wait_warp(smem_u32(&bars->come[quarter]), 0);
-            if (!ok) atomicOr(status, 4);
-        }
-        if (ok && *failed == 0) {
-            constexpr int CHUNKS = P::CW / 8, ROW = P::CW * 2;
-            unsigned char* mine = smem + P::OUT + quarter * (32 * ROW);
-            const unsigned char* from = smem + P::IN + quarter * P::PIECE + lane * 16;
-#pragma unroll 1
-            for (int c = 0; c < P::CW; c += 32) {
-                uint32_t v[32];
-                tmem_ld32(lane_addr + share * P::CW + c, v);
-                float f[32];
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) {
-                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                    for (int i = 0; i < S; ++i) {                       // the shares in their order
-                        float4 x;
-                        if (i == share) x = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]), __uint_as_float(v[j + 2]), __uint_as_float(v[j + 3]));
-                        else x = *reinterpret_cast<const float4*>(from + (i < share ? i : i - 1) * (4 * P::PIECE) + (c + j) * 128);
-                        sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
-                    }
-                    f[j] = sum.x; f[j + 1] = sum.y; f[j + 2] = sum.z; f[j + 3] = sum.w;
-                }
-                if (act >= QNN_ACT_ALONE) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) f[j] = activate_fast(f[j], act - QNN_ACT_ALONE, actk);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int ch = c / 8 + j;
-                    uint4 pk;
-                    pk.x = pack_bf16(f[j * 8 + 0], f[j * 8 + 1]);
-                    pk.y = pack_bf16(f[j * 8 + 2], f[j * 8 + 3]);
-                    pk.z = pack_bf16(f[j * 8 + 4], f[j * 8 + 5]);
-                    pk.w = pack_bf16(f[j * 8 + 6], f[j * 8 + 7]);
-                    *reinterpret_cast<uint4*>(mine + lane * ROW + ((ch ^ (lane & (CHUNKS - 1))) << 4)) = pk;
-                }
-            }
-            __syncwarp();
-            constexpr int AT_ONCE = 32 / CHUNKS;                        // rows per store instruction
-#pragma unroll 4
-            for (int rr = 0; rr < 32; rr += AT_ONCE) {
-                const int r = rr + lane / CHUNKS, pos = lane % CHUNKS;
-                const int row = m0 + quarter * 32 + r, col = n0 + share * P::CW + ((pos ^ (r & (CHUNKS - 1))) << 3);
-                const uint4 pk = *reinterpret_cast<const uint4*>(mine + r * ROW + (pos << 4));
-                if (row < M && col < N) *reinterpret_cast<uint4*>(C + (size_t)row * N + col) = pk;
-            }
-        }
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    cluster_barrier();           // nobody leaves while another still copies to or from it, or its pair's tensor memory is in use
-    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
-}
-
-template <int S>
-cudaLaunchConfig_t split_config(int tiles, cudaLaunchAttribute* attr, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * S * tiles);
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = SplitPlan<S>::BYTES;
-    cfg.stream = st;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2 * S;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cfg;
-}
-
-// clusters of 2 S CTAs that the device holds at once (0: none), asked once per process
-template <int S>
-int split_clusters() {
-    static const int n = [] {
-        int c = 0;
-        cudaLaunchAttribute attr[2];
-        const cudaLaunchConfig_t cfg = split_config<S>(1, attr, nullptr);
-        if (cudaFuncSetAttribute(gemm_tcgen05_2cta_split_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitPlan<S>::BYTES) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&c, gemm_tcgen05_2cta_split_kernel<S>, &cfg) != cudaSuccess) {
-            (void)cudaGetLastError();
-            return 0;
-        }
-        return c;
-    }();
-    return n;
-}
-
-template <int S>
-int launch_split(const CUtensorMap& map_a, const CUtensorMap& map_b, bf16* C, int M, int N, int K, int act, ActConsts actk,
-                 int* status, int tiles, cudaStream_t st) {
-    cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg = split_config<S>(tiles, attr, st);
-    cfg.numAttrs = qnn::pdl_enabled() ? 2 : 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_tcgen05_2cta_split_kernel<S>, map_a, map_b, C, M, N, K, act, actk, status);
-    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
-}
 
 }  // namespace
 
@@ -597,18 +367,6 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
         }
     }
     if (max_pairs < 0) return QNN_ERR_UNSUPPORTED;
-    // Several pairs per tile where one each leaves SMs idle: the walk gets S times shorter, and sharing costs some slabs' time.  Only
-    // where all clusters run at once.
-    if (epi == EPI_NONE && N % 8 == 0) {
-        const int nk = (K + BK - 1) / BK;
-        const long long alone = (ntiles + max_pairs - 1) / max_pairs * nk;
-        int best = 1;
-        long long slabs = alone;
-        if (nk >= 8 && ntiles <= split_clusters<2>() && nk / 2 + SPLIT_COST_2 < slabs) { best = 2; slabs = nk / 2 + SPLIT_COST_2; }
-        if (nk >= 16 && ntiles <= split_clusters<4>() && nk / 4 + SPLIT_COST_4 < slabs) best = 4;
-        if (best == 4) return launch_split<4>(map_a, map_b, (bf16*)C, M, N, K, act, ActConsts{act_a, act_b}, status, (int)ntiles, st);
-        if (best == 2) return launch_split<2>(map_a, map_b, (bf16*)C, M, N, K, act, ActConsts{act_a, act_b}, status, (int)ntiles, st);
-    }
     const int pairs = ntiles < max_pairs ? (int)ntiles : max_pairs;
     cfg.gridDim = dim3(2 * pairs);
     cfg.numAttrs = (qnn::pdl_enabled() && 2ll * pairs <= qnn::pdl_max_grid()) ? 2 : 1;
