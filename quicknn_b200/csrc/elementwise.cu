@@ -58,15 +58,13 @@ __global__ void embed_rmsnorm_kernel(const int* __restrict__ tokens, const W* __
     }
 }
 
-// Both for rows of eights: without a norm `normed` is null.
+// The rows alone, eight elements per thread.  (With the norm, and rmsnorm_kernel: a row's sum keeps the order it has always had, so
+// that a model's results stay the same bit for bit.)
 template <typename W>
 __global__ void __launch_bounds__(qnn::ROW8_THREADS)
 embed_vec_kernel(const int* __restrict__ tokens, const W* __restrict__ table, int table_dt, float scale,
-                 float* __restrict__ out, int H, int V, const void* __restrict__ w, int w_dt, float eps,
-                 float offset, void* __restrict__ normed, int normed_dt) {
-    __shared__ float red[32];
-    float g[8], v[8];
-    if (normed != nullptr) qnn::row8_load(w, w_dt, 0, H, g);        // no kernel of a step writes weights
+                 float* __restrict__ out, int H, int V) {
+    float v[8];
     pdl_wait();
     const int tok = tokens[blockIdx.x];
     const size_t base = (size_t)blockIdx.x * H;
@@ -75,11 +73,6 @@ embed_vec_kernel(const int* __restrict__ tokens, const W* __restrict__ table, in
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= scale;
     qnn::row8_store(out, QNN_DT_F32, base, H, v);
-    if (normed == nullptr) return;
-    const float inv = rsqrtf(qnn::block_sum(qnn::squares8(v), red) / (float)H + eps);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * (g[e] + offset);
-    qnn::row8_store(normed, normed_dt, base, H, v);
 }
 
 QNN_API int qnn_embed_rmsnorm(const int* tokens, const void* table, int table_dtype, float scale, float* out,
@@ -87,15 +80,6 @@ QNN_API int qnn_embed_rmsnorm(const int* tokens, const void* table, int table_dt
                               int T, int H, int V, cudaStream_t st) {
     if (T <= 0) return 0;
     const float off = unit_offset ? 1.f : 0.f;
-    if (qnn::row8_fits(H, {table, out, w, normed})) {
-        if (table_dtype == QNN_DT_BF16)
-            qnn::launch_pdl(embed_vec_kernel<bf16>, dim3(T), dim3(qnn::row8_threads(H)), 0, st, tokens, (const bf16*)table, table_dtype,
-                            scale, out, H, V, w, w_dt, eps, off, normed, normed_dt);
-        else
-            qnn::launch_pdl(embed_vec_kernel<float>, dim3(T), dim3(qnn::row8_threads(H)), 0, st, tokens, (const float*)table, table_dtype,
-                            scale, out, H, V, w, w_dt, eps, off, normed, normed_dt);
-        QNN_LAUNCH_CHECK();
-    }
     const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
     if (table_dtype == QNN_DT_BF16)
         qnn::launch_pdl(embed_rmsnorm_kernel<bf16>, dim3(T), dim3(threads), 0, st, tokens, (const bf16*)table, scale, out, H,
@@ -112,10 +96,10 @@ QNN_API int qnn_embed(const int* tokens, const void* table, int table_dtype, flo
     if (qnn::row8_fits(H, {table, out})) {
         if (table_dtype == QNN_DT_BF16)
             qnn::launch_pdl(embed_vec_kernel<bf16>, dim3(T), dim3(qnn::row8_threads(H)), 0, st, tokens, (const bf16*)table, table_dtype,
-                            scale, out, H, V, (const void*)nullptr, 0, 0.f, 0.f, (void*)nullptr, 0);
+                            scale, out, H, V);
         else
             qnn::launch_pdl(embed_vec_kernel<float>, dim3(T), dim3(qnn::row8_threads(H)), 0, st, tokens, (const float*)table, table_dtype,
-                            scale, out, H, V, (const void*)nullptr, 0, 0.f, 0.f, (void*)nullptr, 0);
+                            scale, out, H, V);
         QNN_LAUNCH_CHECK();
     }
     const int threads = H >= 1024 ? 256 : 128;
@@ -148,30 +132,11 @@ __global__ void rmsnorm_kernel(const void* __restrict__ x, int x_dt, const void*
     }
 }
 
-__global__ void __launch_bounds__(qnn::ROW8_THREADS)
-rmsnorm_vec_kernel(const void* __restrict__ x, int x_dt, const void* __restrict__ w, int w_dt, float eps,
-                   float offset, void* __restrict__ out, int out_dt, int H) {
-    __shared__ float red[32];
-    const size_t base = (size_t)blockIdx.x * H;
-    float g[8], v[8];
-    qnn::row8_load(w, w_dt, 0, H, g);
-    pdl_wait();
-    qnn::row8_load(x, x_dt, base, H, v);
-    const float inv = rsqrtf(qnn::block_sum(qnn::squares8(v), red) / (float)H + eps);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * (g[e] + offset);
-    qnn::row8_store(out, out_dt, base, H, v);
-}
-
 static inline int norm_threads(int H) { return H >= 2048 ? 512 : (H >= 512 ? 256 : 128); }
 
 QNN_API int qnn_rmsnorm(const void* x, int x_dt, const void* w, int w_dt, float eps, int unit_offset,
                         void* out, int out_dt, int T, int H, cudaStream_t st) {
     if (T <= 0) return 0;
-    if (qnn::row8_fits(H, {x, w, out})) {
-        qnn::launch_pdl(rmsnorm_vec_kernel, dim3(T), dim3(qnn::row8_threads(H)), 0, st, x, x_dt, w, w_dt, eps, unit_offset ? 1.f : 0.f, out, out_dt, H);
-        QNN_LAUNCH_CHECK();
-    }
     qnn::launch_pdl(rmsnorm_kernel, dim3(T), dim3(norm_threads(H)), 0, st, x, x_dt, w, w_dt, eps, unit_offset ? 1.f : 0.f, out, out_dt, H);
     QNN_LAUNCH_CHECK();
 }

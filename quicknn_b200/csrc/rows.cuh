@@ -5,7 +5,7 @@
 // of the step writes is asked for before the wait for the kernel in front) and by bytes where it has many.  Measured against the
 // walk (us, one launch after another): add and RMS norm, 2048 rows of 2304, 18.6 -> 9.3 (6.1 TB/s), 8 rows 4.8 -> 2.7; add and layer
 // norm, 2813 rows of 1536, 21.1 -> 12.7; the same of the mean of two branches 37.4 -> 22.8; norm of a 768-wide piece of 2048 rows
-// 5.3 -> 3.8; embedding and norm, 8 rows of 2304, 5.8 -> 2.9.
+// 5.3 -> 3.8.
 #pragma once
 #include <initializer_list>
 
