@@ -22,6 +22,15 @@
 // For the gated epilogue rank 0 loads the 128 gate rows and rank 1 the 128 matching up rows, so every
 // accumulator row holds gate | up side by side, as in the single-CTA kernel.
 //
+// The plain product also comes with tiles of 128 or 64 columns: a product of few rows and few columns has fewer 256 x 256 tiles than
+// the device has pairs, and its time is one tile's walk over K.  A slab of a narrow tile takes hardly less time than one of 256
+// columns (about 0.27 instead of 0.30 us: an MMA occupies its issuer for about 100 cycles whatever its width), but more pairs share
+// the fetching and a tile is written sooner.  Measured (us, 256 columns / as chosen): 256 rows of 2304 x 9216 46.7 / 42.8, of 2304 x
+// 2048 15.1 / 13.3, 640 rows 15.6 / 14.6, 2048 rows of 256 x 2304 15.7 / 14.0, 256 rows of 1152 x 768 8.9 / 7.1.  An element's
+// sum runs over K in the same order whatever the tile, so the results are the same bit for bit.  (Sharing a tile's K among
+// clusters of two or four pairs, summed through distributed shared memory, took 22 and 30 us for 256 and 640 rows of 2304 x 9216, but
+// rounds differently, which shows in the ids that a model samples.)
+//
 // Every wait on an mbarrier is bounded (see gemm_tcgen05.cu); the two cluster barriers are reached by
 // every thread of both CTAs on every path, in bounded time.
 #include "common.cuh"
@@ -40,11 +49,17 @@ inline int make_map(CUtensorMap* map, const void* base, long long rows, long lon
     return make_map_bf16(map, base, rows, width, box_rows, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 6, UMMA_K = 16;       // BM: rows per CTA; the pair does 256
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = (BN / 2) * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;   // per CTA
-constexpr int TMEM_COLS = 256;
+constexpr int BM = 128, BK = 64, UMMA_K = 16;        // BM: rows per CTA; the pair does 256
+constexpr int A_BYTES = BM * BK * 2;                 // per CTA
+constexpr int MAX_STAGES = 8;
+template <int BN>                                    // columns of a pair's tile
+struct Tile {
+    static constexpr int B_BYTES = (BN / 2) * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;                // per CTA
+    static constexpr int STAGES = BN == 256 ? 6 : MAX_STAGES, TMEM_COLS = BN;                         // TMEM_COLS: per accumulator
+};
 constexpr int STAGING_BYTES = BM * 128 * 2;          // the epilogue's 128 rows x 128 columns of bfloat16
 constexpr int GEMM_THREADS = 192;
+constexpr int SLAB_256 = 30, SLAB_128 = 28, SLAB_64 = 27;      // time of a slab by the tile's columns, in 10 ns
 
 
 // `bar` is a shared::cluster address: the leader's barrier, whichever CTA of the pair loads
@@ -67,8 +82,8 @@ __device__ __forceinline__ void umma_commit_pair(unsigned bar) {
 
 
 struct __align__(8) Barriers {
-    uint64_t full[STAGES];      // leader only: the slabs of both CTAs have landed (TMA bytes)
-    uint64_t empty[STAGES];     // in each CTA: the MMAs that read the stage are done
+    uint64_t full[MAX_STAGES];      // leader only: the slabs of both CTAs have landed (TMA bytes)
+    uint64_t empty[MAX_STAGES];     // in each CTA: the MMAs that read the stage are done
     uint64_t acc_ready[2];      // in each CTA: an accumulator is complete
     uint64_t acc_free[2];       // leader only: the epilogues of both CTAs have read an accumulator
     uint32_t tmem_base;
@@ -79,10 +94,12 @@ __device__ __forceinline__ bool has_failed(Barriers* b) { return *reinterpret_ca
 
 // Persistent: a pair of CTAs per TPC walks over 256-row tiles t = pair, pair + pairs, ... (row tiles
 // fastest, so the pairs that run together share their B slabs in L2).
-template <int EPI>
+template <int EPI, int BN>
 __global__ void __launch_bounds__(GEMM_THREADS)
 gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          bf16* __restrict__ C, int M, int N, int K, int act, ActConsts actk, int* __restrict__ status) {
+    static_assert(EPI == EPI_NONE || BN == 256, "a gated tile holds 128 gate and 128 up columns");
+    constexpr int STAGES = Tile<BN>::STAGES, STAGE_BYTES = Tile<BN>::STAGE_BYTES, TMEM_COLS = Tile<BN>::TMEM_COLS;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* staging = smem + STAGES * STAGE_BYTES;
@@ -210,8 +227,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 unsigned char* mine = staging + quarter * (32 * 256);
 #pragma unroll 1
                 for (int h0 = 0; h0 < OUT_COLS; h0 += 128) {
+                    constexpr int PART = OUT_COLS < 128 ? OUT_COLS : 128;
 #pragma unroll 1
-                    for (int c0 = h0; c0 < h0 + 128; c0 += 32) {
+                    for (int c0 = h0; c0 < h0 + PART; c0 += 32) {
                         uint32_t v[32];
                         tmem_ld32(lane_addr + c0, v);
                         float f[32];
@@ -252,7 +270,8 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         const int row = m0 + quarter * 32 + r;
                         const int col = n0 + h0 + ((pos ^ (r & 15)) << 3);
                         const uint4 pk = *reinterpret_cast<const uint4*>(mine + r * 256 + (pos << 4));
-                        if (row < M && col < Nout) *reinterpret_cast<uint4*>(C + (size_t)row * Nout + col) = pk;
+                        const bool staged = PART == 128 || (pos ^ (r & 15)) < PART / 8;
+                        if (staged && row < M && col < Nout) *reinterpret_cast<uint4*>(C + (size_t)row * Nout + col) = pk;
                     }
                     __syncwarp();
                 }
@@ -316,13 +335,7 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
     if (K <= 0 || (K & 7) || ((((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) != 0)) return QNN_ERR_UNSUPPORTED;
     if (epi != EPI_NONE && epi != EPI_GATED) return QNN_ERR_ARGUMENT;
     if (epi == EPI_GATED && (N & 1)) return QNN_ERR_ARGUMENT;
-    CUtensorMap map_a, map_b;
-    int rc = make_map(&map_a, A, M, K, BM);
-    if (rc) return rc;
-    rc = make_map(&map_b, B, N, K, BN / 2);
-    if (rc) return rc;
     const int Nout = epi == EPI_GATED ? N / 2 : N;
-    const int cols = epi == EPI_GATED ? BN / 2 : BN;
     static int sm_count = 0;
     if (sm_count == 0) {
         int dev = 0;
@@ -330,14 +343,33 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
             cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
             sm_count = 148;
     }
-    const long long ntiles = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((Nout + cols - 1) / cols);
+    // The tile's columns: what takes the fewest rounds of tiles times the time of a slab (64 inner elements)
+    const long long m_tiles = (M + 2 * BM - 1) / (2 * BM);
+    const int pairs_about = sm_count / 2 > 0 ? sm_count / 2 : 1;
+    int cols = epi == EPI_GATED ? 128 : 256;
+    if (epi == EPI_NONE) {
+        auto time = [&](int c, int slab) { return (m_tiles * ((N + c - 1) / c) + pairs_about - 1) / pairs_about * slab; };
+        long long best = time(256, SLAB_256);
+        if (time(128, SLAB_128) < best) { cols = 128; best = time(128, SLAB_128); }
+        if (time(64, SLAB_64) < best) cols = 64;
+    }
+    const long long ntiles = m_tiles * ((Nout + cols - 1) / cols);
     if (ntiles > 0x3fffffffLL) return QNN_ERR_UNSUPPORTED;
-    const size_t smem = (size_t)STAGES * STAGE_BYTES + STAGING_BYTES + sizeof(Barriers) + 1024;
-    void (*kern)(CUtensorMap, CUtensorMap, bf16*, int, int, int, int, ActConsts, int*) =
-        epi == EPI_GATED ? gemm_tcgen05_2cta_kernel<EPI_GATED> : gemm_tcgen05_2cta_kernel<EPI_NONE>;
-    static bool configured[2] = {false, false};
+    CUtensorMap map_a, map_b;
+    int rc = make_map(&map_a, A, M, K, BM);
+    if (rc) return rc;
+    rc = make_map(&map_b, B, N, K, epi == EPI_GATED ? 128 : cols / 2);
+    if (rc) return rc;
+    const int which = epi == EPI_GATED ? 3 : (cols == 256 ? 0 : (cols == 128 ? 1 : 2));
+    void (*const kerns[4])(CUtensorMap, CUtensorMap, bf16*, int, int, int, int, ActConsts, int*) = {
+        gemm_tcgen05_2cta_kernel<EPI_NONE, 256>, gemm_tcgen05_2cta_kernel<EPI_NONE, 128>, gemm_tcgen05_2cta_kernel<EPI_NONE, 64>,
+        gemm_tcgen05_2cta_kernel<EPI_GATED, 256>};
+    const int rings[4] = {Tile<256>::STAGES * Tile<256>::STAGE_BYTES, Tile<128>::STAGES * Tile<128>::STAGE_BYTES,
+                          Tile<64>::STAGES * Tile<64>::STAGE_BYTES, Tile<256>::STAGES * Tile<256>::STAGE_BYTES};
+    const auto kern = kerns[which];
+    const size_t smem = (size_t)rings[which] + STAGING_BYTES + sizeof(Barriers) + 1024;
+    static bool configured[4] = {false, false, false, false};
     static int max_pairs = 0;
-    const int which = epi == EPI_GATED ? 1 : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = smem;
