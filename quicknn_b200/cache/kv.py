@@ -52,6 +52,11 @@ class LineView:
     has_readers: bool = False       # another scheduled layer reads this line after its writer (set by the model)
 
 
+# Page tables and lengths up to this size go to the device together, however few rows changed: a copy of 32 KB takes the stream
+# about 1 us longer than one of a row, and every copy takes the host 4 us and the stream 2.
+TABLES_IN_ONE_COPY = 32 << 10
+
+
 class CacheGroup:
     def __init__(self, need: CacheNeed, lines: List[int], n_pages: int, max_slots: int, max_seq: int,
                  dtype: torch.dtype, device):
@@ -67,8 +72,8 @@ class CacheGroup:
         shape = (len(lines), n_pages, need.n_kv_heads, PAGE, need.head_dim)
         self.k = torch.zeros(shape, dtype=dtype, device=device)
         self.v = torch.zeros(shape, dtype=dtype, device=device) if need.values else self.k
-        self.table_host = np.zeros((max_slots, self.pages_per_seq), dtype=np.int32)
-        self.table_dev = torch.zeros((max_slots, self.pages_per_seq), dtype=torch.int32, device=device)
+        self.table_host: np.ndarray = None      # [slots, pages per sequence], views that the cache gives
+        self.table_dev: torch.Tensor = None
         self.held: List[List[int]] = [[] for _ in range(max_slots)]
         self.dirty: set = set()
 
@@ -109,9 +114,21 @@ class KVCache:
                 self._line_group[line] = (len(self.groups), i)
             self.groups.append(g)
         self.uploader = PinnedUploader(device, entries=32)
-        self.lengths_host = np.zeros(max_slots, dtype=np.int32)
+        # the page tables of all groups and the lengths, one array here and one on the device: a step that changes some of them
+        # sends them in one copy
+        at, places = 0, []
+        for g in self.groups:
+            places.append(at)
+            at += _round_up(max_slots * g.pages_per_seq, 4)
+        self._tables_host = np.zeros(at + max_slots, dtype=np.int32)
+        self._tables_dev = torch.zeros(at + max_slots, dtype=torch.int32, device=device)
+        for g, p in zip(self.groups, places):
+            shape = (max_slots, g.pages_per_seq)
+            n = max_slots * g.pages_per_seq
+            g.table_host, g.table_dev = self._tables_host[p:p + n].reshape(shape), self._tables_dev[p:p + n].view(shape)
+        self.lengths_host = self._tables_host[at:]
         self.longest_host = np.zeros(max_slots, dtype=np.int32)    # the longest that a slot's sequence has been: what its rings have overwritten
-        self.lengths_dev = torch.zeros(max_slots, dtype=torch.int32, device=device)
+        self.lengths_dev = self._tables_dev[at:]
         self._lengths_dirty = False
         def regions(needed) -> Dict[int, torch.Tensor]:
             out: Dict[int, torch.Tensor] = {}
@@ -224,6 +241,11 @@ class KVCache:
 
     def sync(self) -> None:
         """Bring the device copies of the page tables and lengths up to date."""
+        if self._tables_host.nbytes <= TABLES_IN_ONE_COPY and any(g.dirty for g in self.groups):
+            self.uploader.send(self._tables_dev, self._tables_host)
+            for g in self.groups:
+                g.dirty.clear()
+            self._lengths_dirty = False
         for g in self.groups:
             if g.dirty:
                 rows = sorted(g.dirty)

@@ -4,11 +4,14 @@ A copy from ordinary host memory makes the caller wait until the stream has drai
 from pinned memory does not, but reads the pinned bytes when the stream gets to it, by which
 time the host may have written the next step's values.  So every array is first copied into
 the next buffer of a ring of pinned buffers and sent from there; a buffer is reused only after
-the copy that read it has run (an event per buffer says so).
+the copy that read it has run (an event per buffer says so).  The ring is native code
+(``csrc/upload.cu``): a step sends two or three such arrays before its first kernel.
 """
 from __future__ import annotations
 
-from typing import List, Optional
+import ctypes
+import weakref
+from typing import Optional
 
 import numpy as np
 import torch
@@ -20,10 +23,17 @@ class PinnedUploader:
         self.on_gpu = self.device.type == "cuda"
         self.entries = entries
         self._nbytes = nbytes
-        self._bufs: List[Optional[torch.Tensor]] = [None] * entries
-        self._events: List[Optional[torch.cuda.Event]] = [None] * entries
-        self._next = 0
+        self._ring: Optional[int] = None
+        self._lib = None
         self.bytes_sent = 0
+
+    def _open(self) -> None:
+        from ..kernels import lib
+        self._lib = lib
+        ring = ctypes.c_void_p()
+        lib.check(lib.load().qnn_upload_ring(self.entries, self._nbytes, ctypes.byref(ring)), "upload_ring", 0)
+        self._ring = ring.value
+        weakref.finalize(self, lib.load().qnn_upload_ring_free, ring.value)
 
     def send(self, dst: torch.Tensor, src: np.ndarray) -> None:
         """dst (contiguous, on the device) = src, ordered on the current stream."""
@@ -37,16 +47,10 @@ class PinnedUploader:
         if not self.on_gpu:
             dst.view(torch.uint8).reshape(-1).copy_(torch.from_numpy(src.view(np.uint8).reshape(-1)))
             return
-        k = self._next
-        self._next = (k + 1) % self.entries
-        if self._events[k] is not None:
-            self._events[k].synchronize()
-        buf = self._bufs[k]
-        if buf is None or buf.numel() < n:
-            buf = torch.empty(max(n, self._nbytes), dtype=torch.uint8, pin_memory=True)
-            self._bufs[k] = buf
-        buf.numpy()[:n] = src.view(np.uint8).reshape(-1)
-        dst.view(torch.uint8).reshape(-1).copy_(buf[:n], non_blocking=True)
-        if self._events[k] is None:
-            self._events[k] = torch.cuda.Event()
-        self._events[k].record()
+        if not dst.is_cuda:
+            raise ValueError("upload into a tensor that is not on the device")
+        if self._ring is None:
+            self._open()
+        stream = torch._C._cuda_getCurrentRawStream(dst.device.index)
+        self._lib.check(self._lib.load().qnn_upload(self._ring, dst.data_ptr(), src.__array_interface__["data"][0], n, stream),
+                        "upload", 0)

@@ -38,7 +38,7 @@ def dt_code(t: torch.Tensor) -> int:
 
 
 def _p(t: Optional[torch.Tensor]):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -50,11 +50,13 @@ def _stream():
     two plain C calls where this torch has them (``torch.cuda.current_stream()`` walks a dozen Python frames, a
     third of the host time of a short step)."""
     if _raw_stream is not None and _raw_device is not None:
-        return ctypes.c_void_p(_raw_stream(_raw_device()))
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _raw_stream(_raw_device())
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _req(t: torch.Tensor, name: str, dtype=None, dim=None) -> None:
+    if t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype is dtype) and (dim is None or t.dim() == dim):
+        return
     if not t.is_cuda:
         raise _lib.KernelError(f"{name} must be a CUDA tensor: quicknn_b200 has no CPU path")
     if not t.is_contiguous():
@@ -316,7 +318,9 @@ def status_words(device) -> torch.Tensor:
 
 
 def _status_word(device) -> torch.Tensor:
-    return status_words(device)[0:1]
+    """The first of them (the launchers take its address)."""
+    t = _status.get(device)
+    return status_words(device)[0:1] if t is None else t
 
 
 def finite_flag(device) -> torch.Tensor:
@@ -922,7 +926,7 @@ def add_scaled_rmsnorm(resid: torch.Tensor, y: torch.Tensor, scale: float, w_nex
 
 
 def _col_ptr(t: torch.Tensor, col: int):
-    return ctypes.c_void_p(t.data_ptr() + col * t.element_size())
+    return t.data_ptr() + col * t.element_size()
 
 
 def rmsnorm_cols(x: torch.Tensor, col0: int, n: int, weight: torch.Tensor, eps: float, out: torch.Tensor,
@@ -1065,7 +1069,7 @@ def _memory_chunks(qk: torch.Tensor, q_col: int, k_col: int, values: torch.Tenso
     n_local, n_norm, n_decay = units * dim * vdim, units * dim if normaliser else 0, 2 * units * (dim if per_channel else 1)
     scratch = torch.empty(n_local + n_norm + n_decay, dtype=torch.float32, device=qk.device)
     ldw = 0 if key_weight is None else key_weight.shape[1]
-    at = lambda n: ctypes.c_void_p(scratch.data_ptr() + 4 * n)  # noqa: E731
+    at = lambda n: scratch.data_ptr() + 4 * n  # noqa: E731
     for r in range(rounds):
         _lib.check(_lib.load().qnn_memory_chunks(
             _col_ptr(qk, q_col), _col_ptr(qk, k_col), qk.shape[1], dt_code(qk), _col_ptr(values, v_col), values.shape[1],
