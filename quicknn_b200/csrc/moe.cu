@@ -391,6 +391,77 @@ __device__ __forceinline__ void mma_tile_product(const bf16* const* w, int col0,
     }
 }
 
+// The same for tiles of up to 16 rows (decode steps: one or two rows per expert), where a block's time is the latency of its weights:
+// one block of inner elements ahead in registers leaves 2 KB per warp in flight.  Here a lane copies its pieces of the weights
+// asynchronously into places of its own in shared memory, AHEAD blocks before their use and across the pieces of the rows, and
+// reads back what it copied itself, so that no barrier stands in that stream; the rows' pieces of 256 are double-buffered, one
+// barrier each.  The order of the sums is the same.  Measured: a decode step of eight sequences with four routed layers (16 experts of
+// 2304 x 2304, two per row, 48 us of weights a layer) 990 -> 881 us.  (A warp per 8 columns with the rows straight from the caches,
+// three or four blocks ahead in registers: 1097.)
+template <int NM> struct FewRing {
+    static constexpr int AHEAD = 8 / NM;                                     // blocks of 32 inner elements in flight
+    static constexpr int WARP = AHEAD * NM * MMA_NW * 32 * 16, XS = 16 * MMA_PITCH * 2;      // bytes: a warp's ring; one buffer of rows
+    static constexpr int BYTES = MMA_WARPS * WARP + 2 * XS;
+};
+template <int NM, typename Fill>
+__device__ __forceinline__ void few_tile_product(const bf16* const* w, int col0, int n_cols, int K, unsigned char* smem,
+                                                 float (&acc)[NM][1][MMA_NW][4], Fill fill) {
+    using R = FewRing<NM>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3, blocks = K / 32;
+    unsigned char* ring = smem + warp * R::WARP + lane * 16;
+    bf16* xs = reinterpret_cast<bf16*>(smem + MMA_WARPS * R::WARP);
+    const bf16* wrow[NM][MMA_NW];
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+        for (int t = 0; t < MMA_NW; ++t) {
+            const int c = min((warp * MMA_NW + t) * 8 + g, n_cols - 1);
+            wrow[m][t] = w[m] + (size_t)(col0 + c) * K + 8 * tg;
+        }
+    auto ask = [&](int i) {                                                  // a group per block, empty beyond the last
+        if (i < blocks) {
+            unsigned char* at = ring + (i % R::AHEAD) * (NM * MMA_NW * 512);
+#pragma unroll
+            for (int m = 0; m < NM; ++m)
+#pragma unroll
+                for (int t = 0; t < MMA_NW; ++t)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(at + (m * MMA_NW + t) * 512)),
+                                 "l"(wrow[m][t] + i * 32) : "memory");
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+#pragma unroll
+    for (int i = 0; i < R::AHEAD; ++i) ask(i);
+    fill(0, min(MMA_KC, K), xs);
+    __syncthreads();
+    for (int k0 = 0, buf = 0; k0 < K; k0 += MMA_KC, buf ^= 1) {
+        const int kn = min(MMA_KC, K - k0);
+        const bf16* x = xs + buf * (R::XS / 2);
+        if (k0 + MMA_KC < K) fill(k0 + MMA_KC, min(MMA_KC, K - k0 - MMA_KC), xs + (buf ^ 1) * (R::XS / 2));
+        for (int kb = 0; kb < kn; kb += 32) {
+            const int i = (k0 + kb) / 32;
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(R::AHEAD - 1) : "memory");
+            const unsigned char* at = ring + (i % R::AHEAD) * (NM * MMA_NW * 512);
+            uint4 b[NM][MMA_NW];
+#pragma unroll
+            for (int m = 0; m < NM; ++m)
+#pragma unroll
+                for (int t = 0; t < MMA_NW; ++t) b[m][t] = *reinterpret_cast<const uint4*>(at + (m * MMA_NW + t) * 512);
+            const uint4 lo = *reinterpret_cast<const uint4*>(x + (size_t)g * MMA_PITCH + kb + 8 * tg);
+            const uint4 hi = *reinterpret_cast<const uint4*>(x + (size_t)(g + 8) * MMA_PITCH + kb + 8 * tg);
+#pragma unroll
+            for (int m = 0; m < NM; ++m)
+#pragma unroll
+                for (int t = 0; t < MMA_NW; ++t) {
+                    mma_bf16(acc[m][0][t], lo.x, hi.x, lo.y, hi.y, b[m][t].x, b[m][t].y);
+                    mma_bf16(acc[m][0][t], lo.z, hi.z, lo.w, hi.w, b[m][t].z, b[m][t].w);
+                }
+            ask(i + R::AHEAD);                                               // the place is read: its numbers are in registers
+        }
+        __syncthreads();                                                     // this piece is read, the next one written
+    }
+}
+
 template <int MT, int NM>
 __global__ void __launch_bounds__(MMA_WARPS * 32)
 moe_gate_up_mma_kernel(const bf16* __restrict__ x, int W, const bf16* __restrict__ w_gu, int ff,
@@ -416,7 +487,7 @@ moe_gate_up_mma_kernel(const bf16* __restrict__ x, int W, const bf16* __restrict
 #pragma unroll
     for (int m = 0; m < NM; ++m) w2[m] = wg + (size_t)m * ff * W;
     float acc[NM][MT][MMA_NW][4] = {};
-    mma_tile_product<MT, NM>(w2, col0, n_cols, W, xs, acc, [&](int k0, int kn) {
+    auto fill = [&](int k0, int kn, bf16* xs) {
         for (int idx = threadIdx.x; idx < MT * 16 * (MMA_KC / 8); idx += blockDim.x) {
             const int r = idx / (MMA_KC / 8), kk = (idx - r * (MMA_KC / 8)) * 8;
             const int row = src_row[r];
@@ -431,7 +502,13 @@ moe_gate_up_mma_kernel(const bf16* __restrict__ x, int W, const bf16* __restrict
             }
             Vec16<bf16>::store(xs + (size_t)r * MMA_PITCH + kk, v);
         }
-    });
+    };
+    if constexpr (MT == 1) {
+        __syncthreads();                                        // src_row, src_w
+        few_tile_product<NM>(w2, col0, n_cols, W, smem_raw, acc, fill);
+    } else {
+        mma_tile_product<MT, NM>(w2, col0, n_cols, W, xs, acc, [&](int k0, int kn) { fill(k0, kn, xs); });
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -462,14 +539,16 @@ moe_down_mma_kernel(const bf16* __restrict__ hidden, int ff, const bf16* __restr
     const int col0 = blockIdx.y * MMA_COLS, n_cols = min(MMA_COLS, W - col0);
     const bf16* const w1[1] = {w_down + (size_t)e * W * ff};
     float acc[1][MT][MMA_NW][4] = {};
-    mma_tile_product<MT, 1>(w1, col0, n_cols, ff, xs, acc, [&](int k0, int kn) {
+    auto fill = [&](int k0, int kn, bf16* xs) {
         for (int idx = threadIdx.x; idx < MT * 16 * (MMA_KC / 8); idx += blockDim.x) {
             const int r = idx / (MMA_KC / 8), kk = (idx - r * (MMA_KC / 8)) * 8;
             uint4 v = make_uint4(0u, 0u, 0u, 0u);
             if (r < rows && kk < kn) v = *reinterpret_cast<const uint4*>(hidden + (size_t)(p0 + r) * ff + k0 + kk);
             *reinterpret_cast<uint4*>(xs + (size_t)r * MMA_PITCH + kk) = v;
         }
-    });
+    };
+    if constexpr (MT == 1) few_tile_product<1>(w1, col0, n_cols, ff, smem_raw, acc, fill);
+    else mma_tile_product<MT, 1>(w1, col0, n_cols, ff, xs, acc, [&](int k0, int kn) { fill(k0, kn, xs); });
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -628,9 +707,9 @@ QNN_API int qnn_moe_gate_up(const void* x, int dtype, int W, const void* w_gu, i
     if (mma_takes(dtype, W, x, w_gu)) {
         const dim3 mgrid(max_tiles, (ff + MMA_COLS - 1) / MMA_COLS);
         if (mgrid.y > 65535) return QNN_ERR_UNSUPPORTED;
-        const size_t smem = (size_t)tile_rows * MMA_PITCH * sizeof(bf16);
 #define QNN_GU_MMA(MT, NM)                                                                                             \
         {                                                                                                              \
+            const size_t smem = MT == 1 ? FewRing<NM>::BYTES : (size_t)tile_rows * MMA_PITCH * sizeof(bf16);           \
             static bool set = false;                                                                                   \
             if (smem > 48 * 1024 && !set) {                                                                            \
                 cudaFuncSetAttribute(moe_gate_up_mma_kernel<MT, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
@@ -683,7 +762,12 @@ QNN_API int qnn_moe_down(const void* hidden, int dtype, int ff, const void* w_do
             launch_pdl(moe_down_mma_kernel<4>, mgrid, dim3(MMA_WARPS * 32), smem, st, (const bf16*)hidden, ff,
                        (const bf16*)w_down, W, offsets, perm, sel_w, tiles, n_tiles, scale_output, ys);
         } else {
-            launch_pdl(moe_down_mma_kernel<1>, mgrid, dim3(MMA_WARPS * 32), smem, st, (const bf16*)hidden, ff,
+            static bool set = false;
+            if (!set) {
+                cudaFuncSetAttribute(moe_down_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FewRing<1>::BYTES);
+                set = true;
+            }
+            launch_pdl(moe_down_mma_kernel<1>, mgrid, dim3(MMA_WARPS * 32), FewRing<1>::BYTES, st, (const bf16*)hidden, ff,
                        (const bf16*)w_down, W, offsets, perm, sel_w, tiles, n_tiles, scale_output, ys);
         }
         QNN_LAUNCH_CHECK();
