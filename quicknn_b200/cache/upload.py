@@ -17,6 +17,11 @@ import numpy as np
 import torch
 
 
+def _close(native, ring: int, slab: torch.Tensor) -> None:
+    """Waits for the copies that still read the pinned memory, which goes back to torch's allocator with its last reference."""
+    native.qnn_upload_ring_free(ring)
+
+
 class PinnedUploader:
     def __init__(self, device, entries: int = 8, nbytes: int = 1 << 16):
         self.device = torch.device(device)
@@ -30,10 +35,11 @@ class PinnedUploader:
     def _open(self) -> None:
         from ..kernels import lib
         self._lib = lib
-        ring = ctypes.c_void_p()
-        lib.check(lib.load().qnn_upload_ring(self.entries, self._nbytes, ctypes.byref(ring)), "upload_ring", 0)
+        ring, native = ctypes.c_void_p(), lib.load()
+        slab = torch.empty(self.entries * self._nbytes, dtype=torch.uint8, pin_memory=True)
+        lib.check(native.qnn_upload_ring(self.entries, self._nbytes, slab.data_ptr(), ctypes.byref(ring)), "upload_ring", 0)
         self._ring = ring.value
-        weakref.finalize(self, lib.load().qnn_upload_ring_free, ring.value)
+        weakref.finalize(self, _close, native, ring.value, slab)
 
     def send(self, dst: torch.Tensor, src: np.ndarray) -> None:
         """dst (contiguous, on the device) = src, ordered on the current stream."""

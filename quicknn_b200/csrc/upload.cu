@@ -15,14 +15,14 @@ struct Buffer {
     void* bytes;
     size_t size;
     cudaEvent_t sent;
+    bool own;                    // allocated here: an array that was larger than the caller's pieces
 };
 struct Ring {
     int n, next;
-    size_t least;
     Buffer* buffers;
 };
 
-int fill(Buffer& b, size_t n, size_t least) {
+int fill(Buffer& b, size_t n) {
     if (b.sent != nullptr) {
         const cudaError_t e = cudaEventSynchronize(b.sent);
         if (e != cudaSuccess) return (int)e;
@@ -34,26 +34,32 @@ int fill(Buffer& b, size_t n, size_t least) {
         }
     }
     if (b.size < n) {
-        const size_t size = n > least ? n : least;
         void* p = nullptr;
-        const cudaError_t e = cudaHostAlloc(&p, size, cudaHostAllocDefault);
+        const cudaError_t e = cudaHostAlloc(&p, n, cudaHostAllocDefault);
         if (e != cudaSuccess) return (int)e;
-        if (b.bytes != nullptr) (void)cudaFreeHost(b.bytes);
+        if (b.own) (void)cudaFreeHost(b.bytes);
         b.bytes = p;
-        b.size = size;
+        b.size = n;
+        b.own = true;
     }
     return 0;
 }
 
 }  // namespace
 
-// A ring of `entries` buffers of at least `least` bytes each (made as they are first used, on the device that is current then).
-QNN_API int qnn_upload_ring(int entries, long long least, void** ring) {
-    if (entries < 1 || least < 1 || ring == nullptr) return QNN_ERR_ARGUMENT;
-    Ring* r = new (std::nothrow) Ring{entries, 0, (size_t)least, new (std::nothrow) Buffer[entries]()};
+// A ring of `entries` buffers of `each` bytes, pieces of the pinned memory at `slab` (the caller's, kept until the ring is free: an
+// allocation of pinned memory takes about 1 ms, so the pieces come from one that a caching allocator may have at hand); a larger array
+// gets a buffer of its own.  Events are made as buffers are first used, on the device that is current then.
+QNN_API int qnn_upload_ring(int entries, long long each, void* slab, void** ring) {
+    if (entries < 1 || each < 1 || slab == nullptr || ring == nullptr) return QNN_ERR_ARGUMENT;
+    Ring* r = new (std::nothrow) Ring{entries, 0, new (std::nothrow) Buffer[entries]()};
     if (r == nullptr || r->buffers == nullptr) {
         delete r;
         return (int)cudaErrorMemoryAllocation;
+    }
+    for (int i = 0; i < entries; ++i) {
+        r->buffers[i].bytes = (char*)slab + (size_t)i * (size_t)each;
+        r->buffers[i].size = (size_t)each;
     }
     *ring = r;
     return 0;
@@ -65,7 +71,7 @@ QNN_API int qnn_upload(void* ring, void* dst, const void* src, long long n, cuda
     if (n == 0) return 0;
     Ring* r = (Ring*)ring;
     Buffer& b = r->buffers[r->next];
-    const int rc = fill(b, (size_t)n, r->least);
+    const int rc = fill(b, (size_t)n);
     if (rc != 0) return rc;
     r->next = (r->next + 1) % r->n;
     memcpy(b.bytes, src, (size_t)n);
@@ -84,7 +90,7 @@ QNN_API int qnn_upload_ring_free(void* ring) {
             (void)cudaEventSynchronize(b.sent);
             (void)cudaEventDestroy(b.sent);
         }
-        if (b.bytes != nullptr) (void)cudaFreeHost(b.bytes);
+        if (b.own) (void)cudaFreeHost(b.bytes);
     }
     delete[] r->buffers;
     delete r;
