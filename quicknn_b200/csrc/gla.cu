@@ -352,6 +352,80 @@ __global__ void mlstm_gates_kernel(const float* __restrict__ pre, long long ldp,
     if (slot >= 0 && lane == 0) mstate[(size_t)slot * state_stride + h] = m;
 }
 
+// The same for sequences of many rows.  With a warp per (sequence, head) the walk took 75 cycles a row: its chain of two operations
+// stood behind the shuffles that bring a row's numbers to every lane, and between walks the warp formed the next 32 rows' gates.
+// Here a block takes four heads of a sequence, 64 rows at a time: four lanes of one warp walk a chunk, a head each, from shared
+// memory, while the other warps form the log gates of the chunk after it and the exponentials of the one before.  The walk's order,
+// and so every bit of m, is the same.  Measured: three sequences of 2813 rows, the longest 1777, 12 heads: 68 -> MLSTM_US us.
+constexpr int GATE_ROWS = 64, GATE_HEADS = 4, GATE_THREADS = 256;
+struct GateChunk {
+    float f[GATE_ROWS][GATE_HEADS], i[GATE_ROWS][GATE_HEADS], before[GATE_ROWS][GATE_HEADS], after[GATE_ROWS][GATE_HEADS];
+};
+__global__ void __launch_bounds__(GATE_THREADS)
+mlstm_gates_rows_kernel(const float* __restrict__ pre, long long ldp, const void* __restrict__ bias, int b_dt, float cap,
+                        const int* __restrict__ seq_row0, const int* __restrict__ seq_len, const int* __restrict__ slots,
+                        float* __restrict__ mstate, long long state_stride, float* __restrict__ gates, int H) {
+    __shared__ GateChunk chunk[3];
+    pdl_wait();
+    const int h0 = blockIdx.x * GATE_HEADS, b = blockIdx.y, slot = slots[b], row0 = seq_row0[b], n = seq_len[b];
+    const int heads = min(GATE_HEADS, H - h0), chunks = (n + GATE_ROWS - 1) / GATE_ROWS;
+    const bool live = slot >= 0;
+    const size_t ldg = (size_t)3 * H;
+    constexpr int CELLS = GATE_ROWS * GATE_HEADS, HELPERS = GATE_THREADS - 32;
+    auto form = [&](int c, int thread, int threads) {                  // the log gates of chunk c
+        GateChunk& k = chunk[c % 3];
+        for (int x = thread; x < CELLS; x += threads) {
+            const int r = x / GATE_HEADS, j = x % GATE_HEADS, t = c * GATE_ROWS + r, h = h0 + j;
+            float gi = -INFINITY, gf = 0.f;                            // rows beyond the sequence change nothing: m -> max(m, -inf)
+            if (t < n && j < heads) {
+                const float zi = pre[(size_t)(row0 + t) * ldp + h] + load_as_f(bias, b_dt, h);
+                const float zf = pre[(size_t)(row0 + t) * ldp + H + h] + load_as_f(bias, b_dt, H + h);
+                gi = cap * tanhf(zi / cap);
+                const float u = cap * tanhf(zf / cap);
+                gf = fminf(u, 0.f) - log1pf(expf(-fabsf(u)));
+            }
+            k.i[r][j] = gi;
+            k.f[r][j] = gf;
+        }
+    };
+    auto finish = [&](int c, int thread, int threads) {                // the gates of chunk c, walked
+        const GateChunk& k = chunk[c % 3];
+        for (int x = thread; x < CELLS; x += threads) {
+            const int r = x / GATE_HEADS, j = x % GATE_HEADS, t = c * GATE_ROWS + r;
+            if (t >= n || j >= heads) continue;
+            float* gr = gates + (size_t)(row0 + t) * ldg + h0 + j;
+            gr[0] = live ? expf(k.f[r][j] + k.before[r][j] - k.after[r][j]) : 0.f;
+            gr[H] = live ? expf(k.i[r][j] - k.after[r][j]) : 0.f;
+            gr[2 * H] = live ? expf(-k.after[r][j]) : 1.f;
+        }
+    };
+    const bool walker = threadIdx.x < 32;
+    const int lane = threadIdx.x & 31;
+    float m = walker && live && lane < heads ? mstate[(size_t)slot * state_stride + h0 + lane] : 0.f;
+    form(0, threadIdx.x, GATE_THREADS);
+    for (int c = 0; c < chunks; ++c) {
+        __syncthreads();
+        if (walker) {
+            if (lane < GATE_HEADS) {
+                GateChunk& k = chunk[c % 3];
+#pragma unroll 16
+                for (int r = 0; r < GATE_ROWS; ++r) {
+                    const float next = fmaxf(m + k.f[r][lane], k.i[r][lane]);
+                    k.before[r][lane] = m;
+                    k.after[r][lane] = next;
+                    m = next;
+                }
+            }
+        } else {
+            if (c + 1 < chunks) form(c + 1, threadIdx.x - 32, HELPERS);
+            if (c > 0) finish(c - 1, threadIdx.x - 32, HELPERS);
+        }
+    }
+    __syncthreads();
+    if (chunks > 0) finish(chunks - 1, threadIdx.x, GATE_THREADS);
+    if (walker && live && lane < heads) mstate[(size_t)slot * state_stride + h0 + lane] = m;
+}
+
 // Gates of a matrix memory whose forget gate also decides what is written.  rows: [T, ld] of T with the query columns
 // (nq of them, from column q_col) and the forget gate's pre-activations (nf, from column f_col).  The queries get
 // silu in place; f = l + (1 - l) sigmoid(z + bias), float32, goes to `f_out` [T, nf] (l: a lower bound per channel).
@@ -522,6 +596,11 @@ QNN_API int qnn_mlstm_gates(const float* pre, long long ldp, const void* bias, i
                             int H, int B, cudaStream_t st) {
     if (B <= 0) return 0;
     if (H <= 0 || !(cap > 0.f) || (seq_row0 == nullptr) != (seq_len == nullptr)) return QNN_ERR_ARGUMENT;
+    if (seq_len != nullptr && B <= 65535) {              // prompts and portions; a warp per (sequence, head) serves single rows
+        launch_pdl(mlstm_gates_rows_kernel, dim3((H + GATE_HEADS - 1) / GATE_HEADS, B), dim3(GATE_THREADS), 0, st, pre, ldp, bias, b_dt,
+                   cap, seq_row0, seq_len, slots, mstate, state_stride, gates, H);
+        QNN_LAUNCH_CHECK();
+    }
     const int warps = 4;
     launch_pdl(mlstm_gates_kernel, dim3(((size_t)B * H + warps - 1) / warps), dim3(warps * 32), 0, st, pre, ldp, bias, b_dt,
                cap, seq_row0, seq_len, slots, mstate, state_stride, gates, H, B);
