@@ -24,6 +24,8 @@
 // 20 cycles per product and scheduler, six products per pair of float32 tiles).  Measured at 2048 rows, 9 heads of 128 x 256, a
 // decay per channel: 46 + 10 + 33 us; the walk in segments of 256 rows took 330.  Three prompts of 2813 rows, 12 heads of
 // 64 x 128, a gate per head: 38 + 8 + 26 us against 550.
+// A number that is Inf or NaN reaches what depends on it and nothing else, as in the walk: rows before it, other columns of a value's
+// head and other heads keep their results (what does depend on it is Inf or NaN; the parts of an Inf are Inf and NaN).
 // Steps whose states would not stay in L2 run in rounds of rows (the caller's scratch limits them), each from the slots'
 // states and back into them.
 #include <atomic>
@@ -86,6 +88,8 @@ __device__ __forceinline__ void store_split1(char* at, int part_bytes, float x) 
     *reinterpret_cast<uint16_t*>(at + part_bytes) = (uint16_t)(__float_as_uint(r) >> 16);
     *reinterpret_cast<uint16_t*>(at + 2 * part_bytes) = (uint16_t)(__float_as_uint(r - upper(r)) >> 16);
 }
+// two bfloat16 numbers: not 0 where one of them is Inf or NaN (an exponent of ones carries into the sign's place)
+__device__ __forceinline__ uint32_t exponent_carry(uint32_t w) { return ((w & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
 __device__ __forceinline__ float bf_at(const char* at) { return __uint_as_float((uint32_t)*reinterpret_cast<const uint16_t*>(at) << 16); }
 
 // A chunk's decay as the sum of two floats: where every chunk has the same decay, close to 1, its rounding would not average out
@@ -240,13 +244,15 @@ __global__ void __launch_bounds__(LOCAL_THREADS) memory_chunk_local_kernel(const
         stage_rows<TQ, DIM, LOCAL_THREADS>(q, a.ldq, n, sm + L::Q);
         stage_rows<TQ, DIM, LOCAL_THREADS>(k, a.ldq, n, sm + L::K);
     }
+    uint32_t carries = 0u;
     for (int i = tid; i < CH * (vdim / 8); i += LOCAL_THREADS) {
         const int t = i / (vdim / 8), x = i - t * (vdim / 8);
         uint4 w = make_uint4(0u, 0u, 0u, 0u);
         if (t < n) w = *reinterpret_cast<const uint4*>(a.v + (size_t)(row0 + t) * a.ldv + h * vdim + x * 8);
         *reinterpret_cast<uint4*>(sm + L::V + t * VP + x * 16) = w;
+        carries |= exponent_carry(w.x) | exponent_carry(w.y) | exponent_carry(w.z) | exponent_carry(w.w);
     }
-    __syncthreads();
+    const bool endless = __syncthreads_or(carries != 0u);        // a value that is Inf or NaN
 
     // ---- A [t][s], s <= t, 16 x 16 blocks (i, j): a warp per block ---------------------------------------------------------
     Tile prod[2];                                                // columns s = 16 j + 8 nt + 2 (lane & 3) + {0, 1}
@@ -455,6 +461,20 @@ __global__ void __launch_bounds__(LOCAL_THREADS) memory_chunk_local_kernel(const
         for (int col0 = (warp & 3) * 32; col0 < vdim; col0 += 128) {
             Tile o[4];
             for (int j = 0; j <= i; ++j) {
+                if (endless && j == i) {                         // the zeros above A's diagonal must not meet an Inf or NaN
+                    for (int s = 0; s < SB; ++s)
+#pragma unroll
+                        for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const int t = g + (e >> 1) * 8, col = min(col0 + nt * 8 + l2 + (e & 1), vdim - 1);
+                                if (s > t) continue;
+                                const char* at = sm + L::A + (i * SB + t) * Z::AP + (i * SB + s) * 2;
+                                const float w = bf_at(at) + (bf_at(at + Z::AMAT) + bf_at(at + 2 * Z::AMAT));
+                                o[nt].hi[e] += w * bf_at(sm + L::V + (i * SB + s) * VP + col * 2);
+                            }
+                    continue;
+                }
                 uint32_t x[3][4], y[2][4];
 #pragma unroll
                 for (int p = 0; p < 3; ++p) ldsm4(x[p], a_row(base + L::A + p * Z::AMAT + i * SB * Z::AP + j * 32, Z::AP, lane));

@@ -103,6 +103,56 @@ def test_chunks_against_64_bits(lens, slots, D, V, kind, monkeypatch):
     assert results[0][1] <= results[1][1] + 2 ** -24 and results[0][3] <= results[1][3] + 2 ** -24, results
 
 
+@pytest.mark.parametrize("place", ["value", "key", "query", "decay", "state"])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("kind", ["channels", "gates", "float_keys"])
+def test_numbers_that_are_not_finite_stay_where_they_belong(kind, bad, place, monkeypatch):
+    """Inf or NaN in one number: the results that are not finite are those of the walk, and all others are what they are without it."""
+    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FROM", 1)
+    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FROM_WIDE", 1)
+    H, D, V, lens, slots = 2, 64, 40, [150, 70], [1, 0]
+    T, ones = sum(lens), kind == "gates"
+    proj, row0, d_row0, d_lens, q, k, v = inputs(lens, H, D, V, 11)
+    rows = torch.cat([torch.randn((T, 2 * H * D), device=DEV), proj[:, 2 * H * D:2 * H * D + H * V].float()], 1) if kind == "float_keys" else proj
+    if kind == "float_keys":
+        q, k = (x.double().reshape(T, H, D) for x in rows[:, :2 * H * D].split(H * D, 1))
+    gates = 0.5 + 0.5 * torch.rand((T, H * D if kind == "channels" else 2 * H), device=DEV)
+    start = torch.randn((2, H, D, V + ones), device=DEV)
+    d_slots = torch.tensor(slots, dtype=torch.int32, device=DEV)
+    dec = gates.double().reshape(T, H, D) if kind == "channels" else gates[:, :H, None].double()
+    w = gates[:, H:].double() if ones else torch.ones((T, H), device=DEV).double()
+    clean, _ = recurrence(q, k, v, dec, w, D ** -0.5, start, row0, lens, slots, ones)
+    for at in (0, 5, 15, 37, 63, 64, 149, 150, 215):             # rows of the first and of the second sequence
+        p, r, g, st = proj.clone(), rows.clone(), gates.clone(), start.clone()
+        if place == "value":
+            p[at, 2 * H * D + V + 3] = bad                       # head 1, column 3
+            r[at, 2 * H * D + V + 3] = bad
+        elif place in ("key", "query"):
+            c = (H * D if place == "key" else 0) + D + 7         # head 1, channel 7
+            p[at, c] = bad
+            r[at, c] = bad
+        elif place == "decay":
+            g[at, D + 7 if kind == "channels" else 1] = bad
+        else:
+            st[at % 2, 1, 7, 3] = bad
+        got = []
+        for longest in (max(lens), 0):
+            s = st.clone() if kind == "channels" else st.reshape(2, -1).clone()
+            if kind == "channels":
+                out = ops.gla_scan(p, 0, H * D, 2 * H * D, g, D ** -0.5, d_row0, d_lens, d_slots, s, 2, H, D, V, longest=longest)
+            else:
+                own = kind == "float_keys" and longest > 0
+                src = r if kind == "float_keys" else p
+                out = ops.memory_scan(src, 0, H * D, 2 * H * D, g, 2 * H, g if ones else None, H, D ** -0.5, ones, d_row0, d_lens, d_slots, s, 2,
+                                      H, D, V, longest=longest, values=p if own else None)
+            got.append((out.reshape(clean.shape), s.reshape(start.shape)))
+        (out, s), (walked, s_walked) = got
+        fine = walked.isfinite()
+        assert torch.equal(out.isfinite(), fine) and torch.equal(s.isfinite(), s_walked.isfinite()), at
+        assert not fine.all() and fine.any()
+        assert ((out.double() - clean)[fine].abs().max() / clean.abs().max()).item() < TOL, at
+
+
 def test_what_is_refused_or_walks():
     """Other sizes, float32 values and short steps keep the row-by-row scan; a step that walks takes no values of its own."""
     bf = torch.bfloat16
