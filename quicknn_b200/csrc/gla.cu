@@ -57,7 +57,7 @@ gla_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
                 const int* __restrict__ seq_len, const int* __restrict__ slots, float* __restrict__ state,
                 float* __restrict__ out, long long ldo, int H, int dim, int vdim, int seg_len, int nseg,
                 int decay_per_head, const float* __restrict__ kw, long long ldw, int ones_col, long long state_stride,
-                int key_from_decay) {
+                int key_from_decay, int max_rows) {
     using C = GlaChunk<RPT, CPT>;
     constexpr int DIMP = RPT * GLA_SHARE;                    // key channels with padding
     constexpr bool AHEAD = RPT <= 16;                        // the next chunk's loads in registers while this one is walked
@@ -77,6 +77,7 @@ gla_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __res
         slot = slots[blockIdx.z];
         row0 = seq_row0 ? seq_row0[blockIdx.z] : blockIdx.z;
         n = seq_len ? seq_len[blockIdx.z] : 1;
+        if (max_rows > 0 && n >= max_rows) return;           // longer sequences of the step are taken elsewhere
     }
     const int part = threadIdx.x & (GLA_SHARE - 1), grp = threadIdx.x / GLA_SHARE;
     const int col = c0 + grp * CPT;                          // the first of this lane's columns
@@ -456,6 +457,7 @@ struct ScanExtra {
     int ones_col = -1;
     long long state_stride = 0;         // 0: H * dim * vdim
     int key_from_decay = 0;             // the keys are 1 - decay (per key channel), k is not read
+    int max_rows = 0;                   // > 0: only sequences of fewer rows (not in segments)
 };
 
 template <typename T>
@@ -477,7 +479,7 @@ int scan_launch(const void* q, const void* k, const void* v, long long ld, const
         }                                                                                                            \
         launch_pdl(gla_scan_kernel<T, RPTV, CPTV>, grid, dim3(GLA_THREADS), smem, st, (const T*)q, (const T*)k,     \
                    (const T*)v, ld, decay, ldd, q_scale, seq_row0, seq_len, slots, state, out, ldo, H, dim, vdim,    \
-                   seg_len, nseg, x.decay_per_head, x.kw, x.ldw, x.ones_col, stride, x.key_from_decay);             \
+                   seg_len, nseg, x.decay_per_head, x.kw, x.ldw, x.ones_col, stride, x.key_from_decay, x.max_rows); \
     }
     if (rpt <= 4) QNN_GLA(4, 4)
     else if (rpt <= 8) QNN_GLA(8, 4)
@@ -518,15 +520,17 @@ int scan_segments(const void* q, const void* k, const void* v, long long ld, con
 // of each sequence, negative for a row of no sequence (its output is zero, no state is touched); state:
 // [slots, H, dim, vdim] float32; out: [rows, H*vdim] float32.  dim up to 256.
 // key_from_decay != 0: the keys are 1 - decay, formed in float32 as the rows are staged; k is not read (may be null).
+// max_rows > 0: sequences of that many rows and more are left alone, output and state (qnn_memory_chunks takes them).
 QNN_API int qnn_gla_scan(const void* q, const void* k, const void* v, long long ld, int dtype, const float* decay,
                          long long ldd, float q_scale, const int* seq_row0, const int* seq_len, const int* slots,
                          float* state, float* out, long long ldo, int B, int H, int dim, int vdim, int key_from_decay,
-                         cudaStream_t st) {
+                         int max_rows, cudaStream_t st) {
     if (B <= 0) return 0;
     if (H <= 0 || dim <= 0 || vdim <= 0 || H > 65535 || B > 65535) return QNN_ERR_ARGUMENT;
     if ((seq_row0 == nullptr) != (seq_len == nullptr)) return QNN_ERR_ARGUMENT;
     ScanExtra x;
     x.key_from_decay = key_from_decay ? 1 : 0;
+    x.max_rows = max_rows;
     if (dtype == QNN_DT_BF16)
         return scan_launch<bf16>(q, k, v, ld, decay, ldd, q_scale, seq_row0, seq_len, slots, state, out, ldo, B, H, dim,
                                  vdim, 0, 1, st, x);
@@ -558,14 +562,14 @@ QNN_API int qnn_gla_scan_segments(const void* q, const void* k, const void* v, l
 // kw[row * ldw + h], or null for 1.  normaliser != 0: the state has one column more than the rows have value columns,
 // which is fed 1 in every row (n_t = d_t n_{t-1} + w_t k_t); out then has vdim + 1 columns per head, the last n_t . q_t.
 // state: the slot's [H, dim, vdim (+1)] floats start at state + slot * state_stride.  seg_len > 0: in segments, with
-// scratch [B * nseg, H, dim, vdim (+1)] zeroed by the caller and seg_decay [B * nseg, H].
+// scratch [B * nseg, H, dim, vdim (+1)] zeroed by the caller and seg_decay [B * nseg, H].  max_rows as above (without segments).
 QNN_API int qnn_memory_scan(const void* q, const void* k, const void* v, long long ld, int dtype, const float* decay,
                             long long ldd, const float* kw, long long ldw, float q_scale, int normaliser,
                             const int* seq_row0, const int* seq_len, const int* slots, float* state, long long state_stride,
                             float* out, long long ldo, int B, int H, int dim, int vdim, int seg_len, int nseg,
-                            float* scratch, float* seg_decay, cudaStream_t st) {
+                            float* scratch, float* seg_decay, int max_rows, cudaStream_t st) {
     if (B <= 0) return 0;
-    if (H <= 0 || dim <= 0 || vdim <= 0 || H > 65535 || B > 65535) return QNN_ERR_ARGUMENT;
+    if (H <= 0 || dim <= 0 || vdim <= 0 || H > 65535 || B > 65535 || (seg_len > 0 && max_rows > 0)) return QNN_ERR_ARGUMENT;
     if ((seq_row0 == nullptr) != (seq_len == nullptr)) return QNN_ERR_ARGUMENT;
     const int vs = vdim + (normaliser ? 1 : 0);
     if (state_stride < (long long)H * dim * vs) return QNN_ERR_ARGUMENT;
@@ -575,6 +579,7 @@ QNN_API int qnn_memory_scan(const void* q, const void* k, const void* v, long lo
     x.ldw = ldw;
     x.ones_col = normaliser ? vdim : -1;
     x.state_stride = state_stride;
+    x.max_rows = max_rows;
     if (seg_len > 0) {
         if (nseg < 1 || (long long)B * nseg > 65535 || seq_row0 == nullptr || scratch == nullptr || seg_decay == nullptr)
             return QNN_ERR_ARGUMENT;

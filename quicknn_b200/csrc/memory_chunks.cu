@@ -26,7 +26,8 @@
 // 64 x 128, a gate per head: 38 + 8 + 26 us against 550.
 // A number that is Inf or NaN reaches what depends on it and nothing else, as in the walk: rows before it, other columns of a value's
 // head and other heads keep their results (what does depend on it is Inf or NaN; the parts of an Inf are Inf and NaN).
-// Steps whose states would not stay in L2 run in rounds of rows (the caller's scratch limits them), each from the slots'
+// A block takes a chunk that there is: the chunks of all sequences are counted through, so unequal sequences cost what their rows do.
+// Steps whose states would not stay in L2 run in rounds of chunks (the caller's scratch limits them), each from the slots'
 // states and back into them.
 #include <atomic>
 
@@ -49,22 +50,50 @@ struct ChunkArgs {
     const float* kw;                              // w: kw[row * ldw + h], null: 1
     long long ldw;
     float q_scale;
-    const int *seq_row0, *seq_len, *slots;
+    const int *seq_row0, *seq_len, *slots;        // [B]
+    int B, least;                                 // sequences of fewer than `least` rows are not this path's
     float* out;                                   // [rows, ldo], vs columns per head
     long long ldo;
     float* state;                                 // slot s: [H, DIM, vs] at state + s * state_stride
     long long state_stride;
-    float* local;                                 // [B * nch, H, DIM, vdim]
-    float* local_n;                               // [B * nch, H, DIM]: the normaliser's column (vs = vdim + 1)
-    float* chunk_decay;                           // [B * nch, H (, DIM)] pairs
-    int first, nch, H, vdim, vs, key_from_decay;  // this round: rows first .. first + 64 nch of every sequence
+    float* local;                                 // [units, H, DIM, vdim]
+    float* local_n;                               // [units, H, DIM]: the normaliser's column (vs = vdim + 1)
+    float* chunk_decay;                           // [units, H (, DIM)] pairs
+    int unit0, units;                             // this round's chunks, counted through all sequences in order
+    int H, vdim, vs, key_from_decay;
 };
 
-// the chunk of a block: its first row and how many rows it has (none: beyond the sequence)
-__device__ __forceinline__ int chunk_rows(const ChunkArgs& a, int b, int c, int& row0) {
-    const int at = a.first + c * CH;
-    row0 = a.seq_row0[b] + at;
-    return min(CH, a.seq_len[b] - at);
+__device__ __forceinline__ int chunks_of(int rows, int least) { return rows >= least ? (rows + CH - 1) / CH : 0; }
+__device__ __forceinline__ int inclusive_sum(int x, int lane, int n) {       // of the first n lanes
+    for (int o = 1; o < 32 && o < n; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    return x;
+}
+// The chunk of a block, unit `u` of the step: its first row, the slot of its sequence, and how many rows it has (0: there are not so
+// many chunks).  Every warp finds it by itself, 32 sequences at a time.
+__device__ __forceinline__ int find_chunk(const ChunkArgs& a, int u, int lane, int& row0, int& slot) {
+    for (int b0 = 0; b0 < a.B; b0 += 32) {
+        const int b = b0 + lane;
+        const bool has = b < a.B;
+        const int len = has ? a.seq_len[b] : 0, first = has ? a.seq_row0[b] : 0, s = has ? a.slots[b] : -1;
+        const int mine = chunks_of(len, a.least), upto = inclusive_sum(mine, lane, a.B), at = (u - (upto - mine)) * CH;
+        const bool here = has && at >= 0 && u < upto;            // in one lane at most; sums over the warp are uniform registers
+        if (__any_sync(0xffffffffu, here)) {
+            row0 = __reduce_add_sync(0xffffffffu, here ? first + at : 0);
+            slot = __reduce_add_sync(0xffffffffu, here ? s : 0);
+            return __reduce_add_sync(0xffffffffu, here ? min(CH, len - at) : 0);
+        }
+        u -= __shfl_sync(0xffffffffu, upto, 31);           // (more sequences to come: all 32 lanes have one)
+    }
+    return 0;
+}
+// chunks of the sequences before sequence b
+__device__ __forceinline__ int chunks_before(const ChunkArgs& a, int b, int lane) {
+    int n = 0;
+    for (int i = lane; i < b; i += 32) n += chunks_of(a.seq_len[i], a.least);
+    return b == 0 ? 0 : __reduce_add_sync(0xffffffffu, n);
 }
 
 template <typename TQ, int DIM>
@@ -202,16 +231,16 @@ __global__ void __launch_bounds__(LOCAL_THREADS) memory_chunk_local_kernel(const
     using Z = Sizes<TQ, DIM>;
     using L = LocalPlan<TQ, DIM, CHANNELS>;
     extern __shared__ __align__(16) char sm[];
-    const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     pdl_wait();
-    int row0;
-    const int n = chunk_rows(a, b, c, row0), vdim = a.vdim;
+    int row0 = 0, slot = -1;
+    const int n = find_chunk(a, a.unit0 + blockIdx.y, lane, row0, slot), vdim = a.vdim;
     if (n <= 0) return;
-    if (a.slots[b] < 0) {                                        // rows of no sequence: nothing but zeros
+    if (slot < 0) {                                        // rows of no sequence: nothing but zeros
         for (int i = tid; i < n * a.vs; i += LOCAL_THREADS) a.out[(size_t)(row0 + i / a.vs) * a.ldo + h * a.vs + i % a.vs] = 0.f;
         return;
     }
-    const size_t unit = ((size_t)b * a.nch + c) * a.H + h;
+    const size_t unit = (size_t)blockIdx.y * a.H + h;
     const int VP = vdim * 2 + 16;
     const unsigned base = (unsigned)__cvta_generic_to_shared(sm);
     float* Dd = reinterpret_cast<float*>(sm + L::D);             // [s][t mod 16]
@@ -245,12 +274,19 @@ __global__ void __launch_bounds__(LOCAL_THREADS) memory_chunk_local_kernel(const
         stage_rows<TQ, DIM, LOCAL_THREADS>(k, a.ldq, n, sm + L::K);
     }
     uint32_t carries = 0u;
-    for (int i = tid; i < CH * (vdim / 8); i += LOCAL_THREADS) {
-        const int t = i / (vdim / 8), x = i - t * (vdim / 8);
-        uint4 w = make_uint4(0u, 0u, 0u, 0u);
-        if (t < n) w = *reinterpret_cast<const uint4*>(a.v + (size_t)(row0 + t) * a.ldv + h * vdim + x * 8);
-        *reinterpret_cast<uint4*>(sm + L::V + t * VP + x * 16) = w;
-        carries |= exponent_carry(w.x) | exponent_carry(w.y) | exponent_carry(w.z) | exponent_carry(w.w);
+    constexpr int NV = CH * MAX_VDIM / 8 / LOCAL_THREADS;
+    uint4 w[NV];
+    const int pieces = vdim / 8;
+#pragma unroll
+    for (int e = 0; e < NV; ++e) {
+        const int i = tid + e * LOCAL_THREADS, t = i / pieces, x = i - t * pieces;
+        w[e] = t < n ? *reinterpret_cast<const uint4*>(a.v + (size_t)(row0 + t) * a.ldv + h * vdim + x * 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int e = 0; e < NV; ++e) {
+        const int i = tid + e * LOCAL_THREADS, t = i / pieces, x = i - t * pieces;
+        if (t < CH) *reinterpret_cast<uint4*>(sm + L::V + t * VP + x * 16) = w[e];
+        carries |= exponent_carry(w[e].x) | exponent_carry(w[e].y) | exponent_carry(w[e].z) | exponent_carry(w[e].w);
     }
     const bool endless = __syncthreads_or(carries != 0u);        // a value that is Inf or NaN
 
@@ -573,17 +609,20 @@ __global__ void __launch_bounds__(LOCAL_THREADS) memory_chunk_local_kernel(const
 // The state before every chunk, in place of the states that the chunks build from nothing: a thread per four columns of a
 // state row (or one number of the normaliser), eight chunks' loads in flight.
 template <int DIM, bool CHANNELS>
-__global__ void __launch_bounds__(256) memory_chunk_prefix_kernel(const ChunkArgs a) {
+__global__ void __launch_bounds__(256, CHANNELS ? 2 : 3) memory_chunk_prefix_kernel(const ChunkArgs a) {
     const int h = blockIdx.y, b = blockIdx.z, q4 = a.vdim / 4;
     const int e = blockIdx.x * 256 + threadIdx.x, n4 = DIM * q4;
     pdl_wait();
-    const int slot = a.slots[b], rows = a.seq_len[b] - a.first;
-    if (slot < 0 || rows <= 0 || e >= n4 + (a.vs > a.vdim ? DIM : 0)) return;
-    const int nb = min(a.nch, (rows + CH - 1) / CH);
+    const int slot = a.slots[b], chunks = chunks_of(a.seq_len[b], a.least);
+    if (slot < 0 || chunks == 0) return;
+    // the sequence's chunks that this round holds
+    const int start = chunks_before(a, b, threadIdx.x & 31) - a.unit0;
+    const int from = max(start, 0), nb = min(start + chunks, a.units) - from;
+    if (nb <= 0 || e >= n4 + (a.vs > a.vdim ? DIM : 0)) return;
     const bool column = e >= n4;                                 // the normaliser's
     const int ch = column ? e - n4 : e / q4, col = column ? a.vdim : (e - ch * q4) * 4;
     float* st = a.state + (size_t)slot * a.state_stride + ((size_t)h * DIM + ch) * a.vs + col;
-    const size_t u0 = (size_t)b * a.nch * a.H + h;
+    const size_t u0 = (size_t)from * a.H + h;
     const float2* dec = reinterpret_cast<const float2*>(a.chunk_decay) + (CHANNELS ? u0 * DIM + ch : u0);
     const size_t dstep = CHANNELS ? (size_t)a.H * DIM : (size_t)a.H;
     if (column) {
@@ -600,24 +639,31 @@ __global__ void __launch_bounds__(256) memory_chunk_prefix_kernel(const ChunkArg
     const size_t step = (size_t)a.H * DIM * a.vdim;
     float* at = a.local + (u0 * DIM + ch) * a.vdim + col;
     float4 carry = make_float4(st[0], st[1], st[2], st[3]);
+    // (offsets from the first chunk with a decay per channel, pointers that move with one per head: the compiler's registers then let two
+    // and three blocks onto an SM.  9 heads of 128 x 256: 2048 rows 9.3 us, with pointers 11.8; a gate per head, 8 x 300 rows 18.6, with offsets 23.2)
     for (int i0 = 0; i0 < nb; i0 += 8) {
+        const int left = nb - i0, first = CHANNELS ? i0 : 0;
         float4 x[8];
         float2 d[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            if (i0 + i < nb) {
-                x[i] = *reinterpret_cast<const float4*>(at + (i0 + i) * step);
-                d[i] = dec[(i0 + i) * dstep];
+            if (i < left) {
+                x[i] = *reinterpret_cast<const float4*>(at + (first + i) * step);
+                d[i] = dec[(first + i) * dstep];
             }
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            if (i0 + i < nb) {
-                *reinterpret_cast<float4*>(at + (i0 + i) * step) = carry;
+            if (i < left) {
+                *reinterpret_cast<float4*>(at + (first + i) * step) = carry;
                 carry.x = decayed(d[i], carry.x, x[i].x);
                 carry.y = decayed(d[i], carry.y, x[i].y);
                 carry.z = decayed(d[i], carry.z, x[i].z);
                 carry.w = decayed(d[i], carry.w, x[i].w);
             }
+        if constexpr (!CHANNELS) {
+            at += 8 * step;
+            dec += 8 * dstep;
+        }
     }
     st[0] = carry.x; st[1] = carry.y; st[2] = carry.z; st[3] = carry.w;
 }
@@ -637,12 +683,10 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) memory_chunk_out_kernel(const 
     using Z = Sizes<TQ, DIM>;
     using L = OutPlan<TQ, DIM, CHANNELS>;
     extern __shared__ __align__(16) char sm[];
-    const int h = blockIdx.x, c = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int vdim = a.vdim;
     pdl_wait();
-    int row0;
-    const int n = chunk_rows(a, b, c, row0), vdim = a.vdim;
-    if (n <= 0 || a.slots[b] < 0) return;
-    const size_t unit = ((size_t)b * a.nch + c) * a.H + h;
+    const size_t unit = (size_t)blockIdx.y * a.H + h;
     const unsigned base = (unsigned)__cvta_generic_to_shared(sm);
     const float* S = a.local + unit * DIM * vdim;
     constexpr int NL = DIM * L::COLS / 4 / OUT_THREADS;          // float4 of a slice per thread
@@ -654,7 +698,10 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) memory_chunk_out_kernel(const 
             nx[e] = col0 + x * 4 < vdim ? *reinterpret_cast<const float4*>(S + (size_t)r * vdim + col0 + x * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     };
-    fetch(0);
+    fetch(0);                                                    // (of scratch that nobody wrote, where there is no chunk)
+    int row0 = 0, slot = -1;
+    const int n = find_chunk(a, a.unit0 + blockIdx.y, lane, row0, slot);
+    if (n <= 0 || slot < 0) return;
     float* P = reinterpret_cast<float*>(sm + L::P);
     if constexpr (CHANNELS) {
         double* Fs = reinterpret_cast<double*>(sm + L::P);
@@ -792,7 +839,7 @@ __global__ void __launch_bounds__(OUT_THREADS, 2) memory_chunk_out_kernel(const 
 }
 
 template <typename TQ, int DIM, bool CHANNELS>
-int launch(const ChunkArgs& a, int B, cudaStream_t st) {
+int launch(const ChunkArgs& a, cudaStream_t st) {
     using L = LocalPlan<TQ, DIM, CHANNELS>;
     using O = OutPlan<TQ, DIM, CHANNELS>;
     static std::atomic<uint64_t> asked{0};                       // devices on which the kernels may have their shared memory
@@ -804,10 +851,10 @@ int launch(const ChunkArgs& a, int B, cudaStream_t st) {
         if (rc != 0) return rc;
         asked.fetch_or(1ull << (dev & 63), std::memory_order_relaxed);
     }
-    const dim3 grid(a.H, a.nch, B);
+    const dim3 grid(a.H, a.units);
     const int elements = DIM * (a.vdim / 4) + (a.vs > a.vdim ? DIM : 0);
     launch_pdl(memory_chunk_local_kernel<TQ, DIM, CHANNELS>, grid, dim3(LOCAL_THREADS), L::bytes(a.vdim), st, a);
-    launch_pdl(memory_chunk_prefix_kernel<DIM, CHANNELS>, dim3((elements + 255) / 256, a.H, B), dim3(256), 0, st, a);
+    launch_pdl(memory_chunk_prefix_kernel<DIM, CHANNELS>, dim3((elements + 255) / 256, a.H, a.B), dim3(256), 0, st, a);
     launch_pdl(memory_chunk_out_kernel<TQ, DIM, CHANNELS>, grid, dim3(OUT_THREADS), O::BYTES, st, a);
     return (int)cudaGetLastError();
 }
@@ -817,16 +864,18 @@ int launch(const ChunkArgs& a, int B, cudaStream_t st) {
 // q, k: [rows, H * dim] of `qk_dtype` (float32 only with one decay per head), row pitch ldq; v: [rows, H * vdim] bfloat16, row
 // pitch ldv; per_channel: decay[row * ldd + h * dim + channel], otherwise decay[row * ldd + h] (ldd = 0: the same in every row)
 // and kw[row * ldw + h] (null: 1).  normaliser: vs = vdim + 1 state and output columns per head, the last one's value being 1
-// (one decay per head only).  key_from_decay: the keys are 1 - decay, k is not read (per channel only).  `first`, `nch`: this
-// round's rows first .. first + 64 nch of every sequence; local [B * nch, H, dim, vdim], local_n [B * nch, H, dim] (normaliser) and
-// chunk_decay [B * nch, H (, dim), 2] (on 8 bytes) are scratch.  dim 64 or 128, vdim a multiple of 8 up to 256; rows on 16 bytes.
+// (one decay per head only).  key_from_decay: the keys are 1 - decay, k is not read (per channel only).  Sequences of fewer than
+// `least` rows are left alone.  The chunks of the others count through all sequences in order: this round takes unit0 .. unit0 +
+// units - 1 (there may be fewer), and a step's rounds come in order.  local [units, H, dim, vdim], local_n [units, H, dim]
+// (normaliser) and chunk_decay [units, H (, dim), 2] (on 8 bytes) are scratch.  dim 64 or 128, vdim a multiple of 8 up to 256;
+// rows on 16 bytes.
 QNN_API int qnn_memory_chunks(const void* q, const void* k, long long ldq, int qk_dtype, const void* v, long long ldv,
                               const float* decay, long long ldd, int per_channel, const float* kw, long long ldw, float q_scale,
                               int normaliser, int key_from_decay, const int* seq_row0, const int* seq_len, const int* slots,
                               float* state, long long state_stride, float* out, long long ldo, int B, int H, int dim, int vdim,
-                              int first, int nch, float* local, float* local_n, float* chunk_decay, cudaStream_t st) {
-    if (B <= 0 || nch <= 0) return 0;
-    if (H <= 0 || B > 65535 || nch > 65535 || H > 65535 || first < 0 || first % CH != 0) return QNN_ERR_ARGUMENT;
+                              int least, int unit0, int units, float* local, float* local_n, float* chunk_decay, cudaStream_t st) {
+    if (B <= 0 || units <= 0) return 0;
+    if (H <= 0 || B > 65535 || units > 65535 || H > 65535 || unit0 < 0 || least < 1) return QNN_ERR_ARGUMENT;
     if (!seq_row0 || !seq_len || !slots || !state || !out || !local || !chunk_decay || (normaliser && !local_n)) return QNN_ERR_ARGUMENT;
     if ((dim != 64 && dim != 128) || vdim < 8 || vdim > MAX_VDIM || vdim % 8 != 0) return QNN_ERR_UNSUPPORTED;
     const int elt = qk_dtype == QNN_DT_BF16 ? 2 : 4;
@@ -834,10 +883,10 @@ QNN_API int qnn_memory_chunks(const void* q, const void* k, long long ldq, int q
     if (odd(q) || (!key_from_decay && odd(k)) || odd(v) || ldq * elt % 16 != 0 || ldv % 8 != 0 || odd(local) || ((uintptr_t)chunk_decay & 7) != 0) return QNN_ERR_UNSUPPORTED;
     if (per_channel && (qk_dtype != QNN_DT_BF16 || normaliser || kw != nullptr || odd(decay) || ldd % 4 != 0)) return QNN_ERR_UNSUPPORTED;
     if (!per_channel && key_from_decay) return QNN_ERR_UNSUPPORTED;
-    ChunkArgs a{q, k, ldq, (const bf16*)v, ldv, decay, ldd, kw, ldw, q_scale, seq_row0, seq_len, slots, out, ldo, state,
-                state_stride, local, local_n, chunk_decay, first, nch, H, vdim, vdim + (normaliser ? 1 : 0), key_from_decay};
+    ChunkArgs a{q, k, ldq, (const bf16*)v, ldv, decay, ldd, kw, ldw, q_scale, seq_row0, seq_len, slots, B, least, out, ldo, state,
+                state_stride, local, local_n, chunk_decay, unit0, units, H, vdim, vdim + (normaliser ? 1 : 0), key_from_decay};
     if (((uintptr_t)out & 7) != 0) return QNN_ERR_UNSUPPORTED;
-    if (per_channel) return dim == 128 ? launch<bf16, 128, true>(a, B, st) : launch<bf16, 64, true>(a, B, st);
-    if (qk_dtype == QNN_DT_BF16) return dim == 128 ? launch<bf16, 128, false>(a, B, st) : launch<bf16, 64, false>(a, B, st);
-    return dim == 128 ? launch<float, 128, false>(a, B, st) : launch<float, 64, false>(a, B, st);
+    if (per_channel) return dim == 128 ? launch<bf16, 128, true>(a, st) : launch<bf16, 64, true>(a, st);
+    if (qk_dtype == QNN_DT_BF16) return dim == 128 ? launch<bf16, 128, false>(a, st) : launch<bf16, 64, false>(a, st);
+    return dim == 128 ? launch<float, 128, false>(a, st) : launch<float, 64, false>(a, st);
 }

@@ -69,6 +69,7 @@ class StepBatch:
     want_rows: torch.Tensor         # [R] int32: rows whose logits are returned
     act_dtype: torch.dtype
     max_q_len: int = 1              # longest run of tokens that one sequence brings
+    min_q_len: int = 0              # the shortest (0: unknown)
     seq_row0: Optional[torch.Tensor] = None   # [B] int32: first row of each sequence in the packed batch
     seq_len: Optional[torch.Tensor] = None    # [B] int32: tokens that each sequence brings
     max_seq: int = 0

@@ -173,7 +173,7 @@ class Engine:
             whole = WholeSequences(views[4], views[8], views[6], views[7], views[9], views[10], views[11],
                                    total=int(extra[2].sum()), longest=int(extra[2].max()), most_new=int(arrays[7].max()))
         step = StepBatch(mode, T, B, views[0], views[1], views[2], views[3], views[4], views[5],
-                         self.model.dtype, max_q_len=int(arrays[7].max()), seq_row0=views[6], seq_len=views[7],
+                         self.model.dtype, max_q_len=int(arrays[7].max()), min_q_len=int(arrays[7].min()), seq_row0=views[6], seq_len=views[7],
                          max_seq=self.max_seq, tuning=self.tuning, longest=longest, spread=spread, whole=whole)
         self._give_scratch(step)
         logits = self.model.forward(step, self.cache)

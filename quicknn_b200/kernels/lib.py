@@ -86,7 +86,7 @@ _SIGNATURES: Dict[str, list] = {
                         c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_vp, c_int, c_int, c_vp],
     "qnn_small_linear_f32": [c_vp, c_int, c_vp, c_int, c_vp, c_int, c_int, c_int, c_vp, c_int, c_float, c_vp],
     "qnn_gla_scan": [c_vp, c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_float, c_vp, c_vp, c_vp, c_vp,
-                     c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_vp],
+                     c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp],
     "qnn_gla_scan_segments": [c_vp, c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_float, c_vp, c_vp, c_vp, c_vp,
                               c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_int, c_vp],
     "qnn_bounded_gates": [c_vp, c_int, c_ll, c_int, c_int, c_int, c_int, c_int, c_vp, c_int, c_vp, c_int, c_vp, c_vp],
@@ -115,12 +115,12 @@ _SIGNATURES: Dict[str, list] = {
                       c_vp, c_int, c_vp, c_vp, c_int, c_float, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int,
                       c_vp, c_int, c_int, c_vp],
     "qnn_memory_scan": [c_vp, c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_ll, c_float, c_int, c_vp, c_vp, c_vp, c_vp,
-                        c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp],
+                        c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_int, c_vp],
     "qnn_upload_ring": [c_int, c_ll, c_vp, c_vp],
     "qnn_upload": [c_vp, c_vp, c_vp, c_ll, c_vp],
     "qnn_upload_ring_free": [c_vp],
     "qnn_memory_chunks": [c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_ll, c_int, c_vp, c_ll, c_float, c_int, c_int, c_vp, c_vp,
-                          c_vp, c_vp, c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp],
+                          c_vp, c_vp, c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp],
     "qnn_mlstm_gates": [c_vp, c_ll, c_vp, c_int, c_float, c_vp, c_vp, c_vp, c_vp, c_ll, c_vp, c_int, c_int, c_vp],
     "qnn_group_rmsnorm": [c_vp, c_int, c_vp, c_int, c_float, c_int, c_vp, c_int, c_int, c_int, c_vp],
     "qnn_add2_group_rmsnorm": [c_vp, c_vp, c_int, c_vp, c_int, c_vp, c_int, c_float, c_int, c_vp, c_int, c_int, c_int, c_vp],

@@ -1045,6 +1045,13 @@ MEMORY_CHUNK = 64            # rows of a chunk of qnn_memory_chunks
 # One prompt of 2048 rows, 9 heads of 128 x 256: 89 against 330 us (the walk in segments); 2813 rows in three prompts, 12 heads
 # of 64 x 128, a gate per head: 72 against 550 us.
 MEMORY_CHUNKS_FROM, MEMORY_CHUNKS_FROM_WIDE = 96, 160
+# A chunk costs a state written and read three times however few rows it has.  Where the sequences have more heads than two thirds of
+# the SMs (FREE), those of fewer than BESIDE rows walk beside the chunks of the others, and the longest has to be longer by what the
+# walk takes: the others' mean, or the device full of their rows.  Measured (us, everything walks / everything in chunks / so; 9
+# heads of 128 x 256 and 12 of 64 x 128, a decay per channel): 63 single rows and 300: 158 / 330 / 133 and 103 / 136 / 50; 63 single rows and
+# 2048: 4690 (in segments) / 428 / 201 and 1688 / 192 / 95; 20 x 5 and 2 x 200: 95 / 120 / 93 and 68 / 66 / 39; 63 x 40 and 300: 300 / 404 / (317) 300
+# and 148 / 157 / 109; 31 x 60 and 500: 301 / 202 / 192 and 186 / 93 / 92; 7 x 30 and 300, not so many heads: 118 / 69 / (85) 69 and 91 / 31 / (48) 31.
+MEMORY_CHUNKS_BESIDE, MEMORY_CHUNKS_FREE, MEMORY_CHUNKS_WALK_ROWS = 48, 98, 20
 MEMORY_CHUNKS_SCRATCH = 80 << 20      # bytes of chunk states per round, which then stay in L2 between the three kernels
 
 
@@ -1052,20 +1059,37 @@ def memory_chunks_fit(values_dtype: torch.dtype, dim: int, vdim: int, longest: i
     """Whether prompts run in chunks of 64 rows on the tensor cores: bfloat16 values, heads of 64 or 128 key channels and up to
     256 value columns, rows and first columns (``columns``) on 16 bytes, and a sequence that is long enough.  Everything
     else (single tokens, short steps, float32 models, other sizes) walks the rows one by one."""
-    least = MEMORY_CHUNKS_FROM_WIDE if per_channel and dim > 64 else MEMORY_CHUNKS_FROM
-    return (values_dtype == torch.bfloat16 and longest >= least and dim in (64, 128) and vdim % 8 == 0
+    return (values_dtype == torch.bfloat16 and longest >= _memory_chunks_from(dim, per_channel) and dim in (64, 128) and vdim % 8 == 0
             and 8 <= vdim <= 256 and all(c % 8 == 0 for c in columns))
+
+
+def _memory_chunks_from(dim: int, per_channel: bool) -> int:
+    return MEMORY_CHUNKS_FROM_WIDE if per_channel and dim > 64 else MEMORY_CHUNKS_FROM
+
+
+def memory_chunks_least(dim: int, n_heads: int, n_seqs: int, rows: int, longest: int, shortest: int = 0, per_channel: bool = False) -> int:
+    """The rows from which a sequence of the step (``rows`` in all) runs in chunks, if its sizes fit: 0 none does, 1 all do,
+    otherwise the shorter ones walk their rows beside them.  ``shortest``: the fewest rows of a sequence (0: unknown)."""
+    start = _memory_chunks_from(dim, per_channel)
+    if longest < start:
+        return 0
+    if n_seqs * n_heads <= MEMORY_CHUNKS_FREE or n_seqs == 1 or shortest >= MEMORY_CHUNKS_BESIDE:
+        return 1
+    others = rows - longest
+    walk = min(MEMORY_CHUNKS_BESIDE, -(-others // (n_seqs - 1))) + others // MEMORY_CHUNKS_WALK_ROWS
+    return MEMORY_CHUNKS_BESIDE if longest >= start + walk else 0
 
 
 def _memory_chunks(qk: torch.Tensor, q_col: int, k_col: int, values: torch.Tensor, v_col: int, decay: torch.Tensor, decay_ld: int,
                    per_channel: bool, key_weight: Optional[torch.Tensor], kw_col: int, q_scale: float, normaliser: bool,
                    key_from_decay: bool, seq_row0: torch.Tensor, seq_len: torch.Tensor, slots: torch.Tensor, state: torch.Tensor,
-                   state_stride: int, out: torch.Tensor, n_seqs: int, n_heads: int, dim: int, vdim: int, longest: int) -> None:
-    chunks = -(-longest // MEMORY_CHUNK)
-    at_once = max(1, min(chunks, MEMORY_CHUNKS_SCRATCH // (4 * n_seqs * n_heads * dim * vdim)))
+                   state_stride: int, out: torch.Tensor, n_seqs: int, n_heads: int, dim: int, vdim: int, least: int) -> None:
+    T = qk.shape[0]
+    chunks = (T + 63 * min(n_seqs, T // least)) // MEMORY_CHUNK      # no step of T rows has more: a sequence's last one may be short
+    at_once = max(1, min(chunks, MEMORY_CHUNKS_SCRATCH // (4 * n_heads * dim * vdim), 65535))
     rounds = -(-chunks // at_once)
     at_once = -(-chunks // rounds)
-    units = n_seqs * at_once * n_heads
+    units = at_once * n_heads
     n_local, n_norm, n_decay = units * dim * vdim, units * dim if normaliser else 0, 2 * units * (dim if per_channel else 1)
     scratch = torch.empty(n_local + n_norm + n_decay, dtype=torch.float32, device=qk.device)
     ldw = 0 if key_weight is None else key_weight.shape[1]
@@ -1075,22 +1099,23 @@ def _memory_chunks(qk: torch.Tensor, q_col: int, k_col: int, values: torch.Tenso
             _col_ptr(qk, q_col), _col_ptr(qk, k_col), qk.shape[1], dt_code(qk), _col_ptr(values, v_col), values.shape[1],
             _p(decay), int(decay_ld), int(per_channel), _col_ptr(key_weight, kw_col) if key_weight is not None else None, ldw,
             float(q_scale), int(normaliser), int(key_from_decay), _p(seq_row0), _p(seq_len), _p(slots), _p(state),
-            int(state_stride), _p(out), out.shape[1], n_seqs, n_heads, dim, vdim, r * at_once * MEMORY_CHUNK, at_once,
+            int(state_stride), _p(out), out.shape[1], n_seqs, n_heads, dim, vdim, least, r * at_once, at_once,
             at(0), at(n_local), at(n_local + n_norm), _stream()), "memory_chunks", 3)
 
 
 def gla_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torch.Tensor, q_scale: float,
              seq_row0: Optional[torch.Tensor], seq_len: Optional[torch.Tensor], slots: torch.Tensor,
              state: torch.Tensor, n_seqs: int, n_heads: int, dim: int, vdim: int, longest: int = 0,
-             key_from_decay: bool = False) -> torch.Tensor:
+             key_from_decay: bool = False, shortest: int = 0) -> torch.Tensor:
     """The recurrence S = diag(a) S + k v^T, o = S^T (q q_scale) over the rows of every sequence in order, from the
     state of the sequence's slot and back into it.  ``proj`` holds q and k ([*, heads*dim]) and v ([*, heads*vdim])
     from the given columns on; ``decay`` the decays a, float32 [rows, heads*dim]; returns o, float32 [rows, heads*vdim].
 
-    ``longest``: the most rows that one sequence brings (0: unknown).  Where ``memory_chunks_fit`` the rows run in chunks
-    on the tensor cores.  Otherwise, from 512 rows on, the sequences are cut into segments of 256 rows that run side by side (the recurrence is linear in the state: each segment's own state and
-    decay product first, a short pass over the segments in order, then the outputs); results differ from the walk
-    in one piece by rounding only.  ``key_from_decay``: the keys are 1 - a, formed in float32 inside the scan (what the
+    ``longest``, ``shortest``: the most and the fewest rows that one sequence brings (0: unknown).  Where ``memory_chunks_fit`` the
+    rows run in chunks on the tensor cores (of all sequences, or beside short ones that walk: ``memory_chunks_least``).
+    Otherwise, from 512 rows on, the sequences are cut into segments of 256 rows that run side by side (the recurrence is linear
+    in the state: each segment's own state and decay product first, a short pass over the segments in order, then the outputs);
+    results differ from the walk in one piece by rounding only.  ``key_from_decay``: the keys are 1 - a, formed in float32 inside the scan (what the
     forget gate lets go is what is written); ``k_col`` is then not read."""
     _req(proj, "proj", None, 2)
     _req(decay, "decay", torch.float32, 2)
@@ -1106,13 +1131,17 @@ def gla_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torc
     if seq_row0 is None and T < n_seqs:
         raise ValueError("gla_scan: fewer rows than sequences")
     out = torch.empty((T, n_heads * vdim), dtype=torch.float32, device=proj.device)
+    least = 0
     if (seq_row0 is not None and memory_chunks_fit(proj.dtype, dim, vdim, longest, proj.shape[1], q_col, k_col, v_col,
                                                          per_channel=True)
             and (proj.data_ptr() | decay.data_ptr()) % 16 == 0):
+        least = memory_chunks_least(dim, n_heads, n_seqs, T, longest, shortest, True)
+    if least > 0:
         _memory_chunks(proj, q_col, k_col, proj, v_col, decay, decay.shape[1], True, None, 0, q_scale, False, key_from_decay,
-                       seq_row0, seq_len, slots, state, n_heads * dim * vdim, out, n_seqs, n_heads, dim, vdim, longest)
-        return out
-    if seq_row0 is not None and longest >= GLA_SEGMENTS_FROM and n_seqs * -(-longest // GLA_SEGMENT) <= 65535:
+                       seq_row0, seq_len, slots, state, n_heads * dim * vdim, out, n_seqs, n_heads, dim, vdim, least)
+        if least == 1:
+            return out
+    if least == 0 and seq_row0 is not None and longest >= GLA_SEGMENTS_FROM and n_seqs * -(-longest // GLA_SEGMENT) <= 65535:
         nseg = -(-longest // GLA_SEGMENT)
         scratch = torch.zeros((n_seqs * nseg, n_heads, dim, vdim), dtype=torch.float32, device=proj.device)
         seg_decay = torch.empty((n_seqs * nseg, n_heads * dim), dtype=torch.float32, device=proj.device)
@@ -1125,7 +1154,7 @@ def gla_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: torc
     _lib.check(_lib.load().qnn_gla_scan(
         _col_ptr(proj, q_col), _col_ptr(proj, k_col), _col_ptr(proj, v_col), proj.shape[1], dt_code(proj), _p(decay),
         decay.shape[1], float(q_scale), _p(seq_row0), _p(seq_len), _p(slots), _p(state),
-        _p(out), out.shape[1], n_seqs, n_heads, dim, vdim, int(key_from_decay), _stream()), "gla_scan")
+        _p(out), out.shape[1], n_seqs, n_heads, dim, vdim, int(key_from_decay), least, _stream()), "gla_scan")
     return out
 
 
@@ -1502,7 +1531,7 @@ def memory_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: t
                 key_weight: Optional[torch.Tensor], kw_col: int, q_scale: float, normaliser: bool,
                 seq_row0: Optional[torch.Tensor],
                 seq_len: Optional[torch.Tensor], slots: torch.Tensor, state: torch.Tensor, n_seqs: int, n_heads: int,
-                dim: int, vdim: int, longest: int = 0, values: Optional[torch.Tensor] = None) -> torch.Tensor:
+                dim: int, vdim: int, longest: int = 0, values: Optional[torch.Tensor] = None, shortest: int = 0) -> torch.Tensor:
     """S_t = d_t S_{t-1} + w_t k_t v_t^T, o_t = S_t^T (q_t q_scale) over the rows of every sequence in order, from
     the state of the sequence's slot and back into it; d and w are one float32 number per (row, head).
 
@@ -1512,7 +1541,7 @@ def memory_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: t
     being n_t . q_t.  ``state``: float32 [slots, floats per slot], a slot's [heads, dim, vdim (+1)] first.  Returns
     float32 [rows, heads * (vdim (+1))].  Long sequences run in chunks, or in segments side by side, like ``gla_scan``.
     ``values``: the rows that hold v (from ``v_col`` on) where they are not ``proj``'s: bfloat16 beside float32 queries and
-    keys, for steps that ``memory_chunks_fit``."""
+    keys, for steps that ``memory_chunks_fit``; where some sequences walk (``memory_chunks_least``), ``proj`` holds v too."""
     _req(proj, "proj", None, 2)
     _req(decay, "decay", torch.float32)
     _req(slots, "slots", torch.int32, 1)
@@ -1529,20 +1558,25 @@ def memory_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: t
             raise ValueError("memory_scan: a key weight per (row, head)")
     ldw = 0 if key_weight is None else key_weight.shape[1]
     out = torch.empty((T, n_heads * vs), dtype=torch.float32, device=proj.device)
-    rows = proj if values is None else values
+    rows, least = proj if values is None else values, 0
     if (seq_row0 is not None and memory_chunks_fit(rows.dtype, dim, vdim, longest, rows.shape[1], v_col, proj.shape[1], q_col, k_col)
             and (proj.data_ptr() | rows.data_ptr()) % 16 == 0):
+        least = memory_chunks_least(dim, n_heads, n_seqs, T, longest, shortest)
+    if least > 0:
         _req(rows, "values", None, 2)
         if rows.shape[0] != T:
             raise ValueError("memory_scan: a row of values per row")
+        if least > 1 and v_col + n_heads * vdim > proj.shape[1]:
+            raise ValueError("memory_scan: sequences that walk need their values beside the queries and keys")
         _memory_chunks(proj, q_col, k_col, rows, v_col, decay, decay_ld, False, key_weight, kw_col, q_scale, normaliser, False,
-                       seq_row0, seq_len, slots, state, state.shape[1], out, n_seqs, n_heads, dim, vdim, longest)
-        return out
-    if values is not None:
+                       seq_row0, seq_len, slots, state, state.shape[1], out, n_seqs, n_heads, dim, vdim, least)
+        if least == 1:
+            return out
+    elif values is not None:
         raise ValueError("memory_scan: values of their own need a step that runs in chunks")
     seg_len = nseg = 0
     scratch = seg_decay = None
-    if seq_row0 is not None and longest >= GLA_SEGMENTS_FROM and n_seqs * -(-longest // GLA_SEGMENT) <= 65535:
+    if least == 0 and seq_row0 is not None and longest >= GLA_SEGMENTS_FROM and n_seqs * -(-longest // GLA_SEGMENT) <= 65535:
         seg_len = _segment_rows(longest, n_seqs * n_heads * -(-vs // (64 if dim <= 128 else 32)), proj.device)
         if n_seqs * -(-longest // seg_len) > 65535:
             seg_len = GLA_SEGMENT
@@ -1553,7 +1587,7 @@ def memory_scan(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, decay: t
         _col_ptr(proj, q_col), _col_ptr(proj, k_col), _col_ptr(proj, v_col), proj.shape[1], dt_code(proj), _p(decay),
         int(decay_ld), _col_ptr(key_weight, kw_col) if key_weight is not None else None, ldw, float(q_scale), int(normaliser), _p(seq_row0), _p(seq_len), _p(slots), _p(state),
         state.shape[1], _p(out), out.shape[1], n_seqs, n_heads, dim, vdim, seg_len, nseg, _p(scratch), _p(seg_decay),
-        _stream()), "memory_scan", 4 if seg_len else 1)
+        least, _stream()), "memory_scan", 4 if seg_len else 1)
     return out
 
 

@@ -82,7 +82,7 @@ class GatedLinearAttention(Mixer):
                          None if step.mode == "decode" else step.seq_row0,
                          None if step.mode == "decode" else step.seq_len,
                          step.slots, line.state, step.n_seqs, H, d, vd,
-                         longest=0 if step.mode == "decode" else step.max_q_len)
+                         longest=0 if step.mode == "decode" else step.max_q_len, shortest=step.min_q_len)
         g = ops.gla_norm_gate(o, self.norm, self.eps, p, 2 * H * d + H * vd, H, vd)
         return project(g, self.w_o)
 
@@ -148,6 +148,6 @@ class HGRN2(Mixer):
         decode = step.mode == "decode"
         o = ops.gla_scan(p, 0, 0, 2 * H * d, f, 1.0, None if decode else step.seq_row0,
                          None if decode else step.seq_len, step.slots, line.state, step.n_seqs, H, d, vd,
-                         longest=0 if decode else step.max_q_len, key_from_decay=True)
+                         longest=0 if decode else step.max_q_len, key_from_decay=True, shortest=step.min_q_len)
         n = ops.head_norm_gate(o, vd, H, vd, self.eps, None, 0, "none", weight=self.norm, out_dtype=p.dtype)
         return project(n, self.w_o)

@@ -62,10 +62,10 @@ class _MatrixMemory(Mixer):
         return None
 
     def _rows(self, step):
-        """(first rows, row counts, longest) of the step's sequences; a decode step is a row each."""
+        """(first rows, row counts, longest, shortest) of the step's sequences; a decode step is a row each."""
         if step.mode == "decode":
-            return None, None, 0
-        return step.seq_row0, step.seq_len, step.max_q_len
+            return None, None, 0, 0
+        return step.seq_row0, step.seq_len, step.max_q_len, step.min_q_len
 
 
 @MIXERS.register("retention")
@@ -104,15 +104,17 @@ class Retention(_MatrixMemory):
     def forward(self, x: torch.Tensor, step, line) -> torch.Tensor:
         H, d, vd = self.n_heads, self.dim, self.vdim
         p = project(x, self.w_in)                                         # q | k | v | gate
-        row0, lens, longest = self._rows(step)
-        # rotated q and k as float32 rows for the scan; v stays where it is if the scan runs in chunks, and beside them if not
-        chunks = row0 is not None and ops.memory_chunks_fit(p.dtype, d, vd, longest, p.shape[1], 2 * H * d)
-        beside = 0 if chunks else H * vd
+        row0, lens, longest, shortest = self._rows(step)
+        # rotated q and k as float32 rows for the scan; v stays where it is for sequences in chunks, and lies beside them for others
+        least = 0
+        if row0 is not None and ops.memory_chunks_fit(p.dtype, d, vd, longest, p.shape[1], 2 * H * d):
+            least = ops.memory_chunks_least(d, H, step.n_seqs, p.shape[0], longest, shortest)
+        beside = 0 if least == 1 else H * vd
         rows = torch.empty((p.shape[0], H * 2 * d + beside), dtype=torch.float32, device=p.device)
         ops.head_prep(p, 0, H, H, beside, d, dst=rows, rot_dim=self.rot_dim, inv_freq=self.position.inv_freq,
                       interleaved=getattr(self.position, "layout", "half") == "interleaved", tok_pos=step.tok_pos)
         o = ops.memory_scan(rows, 0, H * d, 2 * H * d, self.decay_dev, 0, None, 0, float(d) ** -0.5, False, row0, lens,
-                            step.slots, line.state, step.n_seqs, H, d, vd, longest=longest, values=p if chunks else None)
+                            step.slots, line.state, step.n_seqs, H, d, vd, longest=longest, values=p if least > 0 else None, shortest=shortest)
         g = ops.head_norm_gate(o, vd, H, vd, self.eps, p, 2 * H * d + H * vd, "silu")
         return project(g, self.w_o)
 
@@ -154,9 +156,9 @@ class LightningAttention(_MatrixMemory):
         H, d, vd = self.n_heads, self.dim, self.vdim
         p = project(x, self.w_in, epilogue=ops.EPI_ACT, activation="silu")          # silu(q | k | v)
         g = project(x, self.w_gate)
-        row0, lens, longest = self._rows(step)
+        row0, lens, longest, shortest = self._rows(step)
         o = ops.memory_scan(p, 0, H * d, 2 * H * d, self.decay_dev, 0, None, 0, 1.0, False, row0, lens, step.slots,
-                            line.state, step.n_seqs, H, d, vd, longest=longest)
+                            line.state, step.n_seqs, H, d, vd, longest=longest, shortest=shortest)
         # one norm over all heads together: a single "head" as wide as the row, a weight per column
         n = ops.head_norm_gate(o, H * vd, 1, H * vd, self.eps, g, 0, "sigmoid", weight=self.norm)
         return project(n, self.w_o)
@@ -203,12 +205,12 @@ class MatrixLSTM(_MatrixMemory):
     def forward(self, x: torch.Tensor, step, line) -> torch.Tensor:
         H, d, vd = self.n_heads, self.dim, self.vdim
         p = project(x, self.w_in)                                         # q | k | v | gate
-        row0, lens, longest = self._rows(step)
+        row0, lens, longest, shortest = self._rows(step)
         pre = ops.small_linear_f32(x, self.w_gates)                       # the gates' pre-activations, float32
         gates = ops.mlstm_gates(pre, self.b_gates, self.cap, row0, lens, step.slots, line.state, self._m_offset,
                                 step.n_seqs, H)                           # decay | key weight | e^-m
         o = ops.memory_scan(p, 0, H * d, 2 * H * d, gates, 3 * H, gates, H, float(d) ** -0.5, True, row0, lens,
-                            step.slots, line.state, step.n_seqs, H, d, vd, longest=longest)
+                            step.slots, line.state, step.n_seqs, H, d, vd, longest=longest, shortest=shortest)
         g = ops.head_norm_gate(o, vd + 1, H, vd, self.eps, p, 2 * H * d + H * vd, "sigmoid", weight=self.norm,
                                den=gates, den_col=2 * H)
         return project(g, self.w_o)

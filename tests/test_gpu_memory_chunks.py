@@ -46,6 +46,12 @@ def off(got, want):
     return (d.abs().max() / want.abs().max()).item(), (d.norm() / want.norm()).item()
 
 
+def everything_in_chunks(monkeypatch):
+    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FREE", 1 << 30)
+    for name in ("MEMORY_CHUNKS_FROM", "MEMORY_CHUNKS_FROM_WIDE"):
+        monkeypatch.setattr(ops, name, 1)
+
+
 # lengths about the edges of a chunk (64) and a sub-chunk (16), the longest first, last and among others; slot -1: no sequence
 LENGTHS = [([64], [0]), ([1, 65, 16], [2, 0, 3]), ([79, 128, 17], [1, -1, 0]), ([321], [3]), ([15, 200, 63, 64], [0, 1, 2, 3])]
 
@@ -53,12 +59,12 @@ LENGTHS = [([64], [0]), ([1, 65, 16], [2, 0, 3]), ([79, 128, 17], [1, -1, 0]), (
 @pytest.mark.parametrize("lens,slots", LENGTHS)
 @pytest.mark.parametrize("D,V", [(64, 8), (64, 128), (128, 24), (128, 256)])
 @pytest.mark.parametrize("kind", ["channels", "complement", "constant", "gates", "float_keys"])
-def test_chunks_against_64_bits(lens, slots, D, V, kind, monkeypatch):
+@pytest.mark.parametrize("at_once", [1, 2, 3, 1000])             # chunks of a round, of one sequence or several; the last round may have fewer
+def test_chunks_against_64_bits(lens, slots, D, V, kind, at_once, monkeypatch):
     H, T = 3, sum(lens)
     proj, row0, d_row0, d_lens, q, k, v = inputs(lens, H, D, V, 5 + D + V + T)
-    monkeypatch.setattr(ops, "MEMORY_CHUNKS_SCRATCH", 1 if T % 2 else 80 << 20)       # a chunk per round, or all at once
-    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FROM", 1)
-    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FROM_WIDE", 1)
+    monkeypatch.setattr(ops, "MEMORY_CHUNKS_SCRATCH", 4 * H * D * V * at_once)
+    everything_in_chunks(monkeypatch)
     ones = kind == "gates"
     state = torch.randn((4, H, D, V + ones), device=DEV)
     d_slots = torch.tensor(slots, dtype=torch.int32, device=DEV)
@@ -108,8 +114,7 @@ def test_chunks_against_64_bits(lens, slots, D, V, kind, monkeypatch):
 @pytest.mark.parametrize("kind", ["channels", "gates", "float_keys"])
 def test_numbers_that_are_not_finite_stay_where_they_belong(kind, bad, place, monkeypatch):
     """Inf or NaN in one number: the results that are not finite are those of the walk, and all others are what they are without it."""
-    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FROM", 1)
-    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FROM_WIDE", 1)
+    everything_in_chunks(monkeypatch)
     H, D, V, lens, slots = 2, 64, 40, [150, 70], [1, 0]
     T, ones = sum(lens), kind == "gates"
     proj, row0, d_row0, d_lens, q, k, v = inputs(lens, H, D, V, 11)
@@ -151,6 +156,59 @@ def test_numbers_that_are_not_finite_stay_where_they_belong(kind, bad, place, mo
         assert torch.equal(out.isfinite(), fine) and torch.equal(s.isfinite(), s_walked.isfinite()), at
         assert not fine.all() and fine.any()
         assert ((out.double() - clean)[fine].abs().max() / clean.abs().max()).item() < TOL, at
+
+
+@pytest.mark.parametrize("lens,slots", [([1, 300, 47, 48, 1], [0, 1, 2, 3, 4]), ([1] * 40 + [241] + [2] * 9 + [64, 130], [-1] + list(range(1, 52)))])
+@pytest.mark.parametrize("D,V", [(64, 24), (128, 64)])
+@pytest.mark.parametrize("kind", ["channels", "gates", "float_keys"])
+def test_short_sequences_beside_a_prompt_walk(lens, slots, D, V, kind, monkeypatch):
+    """A step of unequal sequences: the long ones run in chunks, one among many others included; those of a few rows walk, and give the
+    walk's results bit for bit."""
+    monkeypatch.setattr(ops, "MEMORY_CHUNKS_FREE", 0)            # as if the heads were many
+    H, T, ones = 2, sum(lens), kind == "gates"
+    proj, row0, d_row0, d_lens, q, k, v = inputs(lens, H, D, V, 3)
+    rows = proj
+    if kind == "float_keys":
+        rows = torch.cat([torch.randn((T, 2 * H * D), device=DEV), proj[:, 2 * H * D:2 * H * D + H * V].float()], 1)
+        q, k = (x.double().reshape(T, H, D) for x in rows[:, :2 * H * D].split(H * D, 1))
+    gates = 0.5 + 0.5 * torch.rand((T, H * D if kind == "channels" else 2 * H), device=DEV)
+    start = torch.randn((len(lens), H, D, V + ones), device=DEV)
+    d_slots = torch.tensor(slots, dtype=torch.int32, device=DEV)
+    dec = gates.double().reshape(T, H, D) if kind == "channels" else gates[:, :H, None].double()
+    w = gates[:, H:].double() if ones else torch.ones((T, H), device=DEV).double()
+    want, end = recurrence(q, k, v, dec, w, D ** -0.5, start, row0, lens, slots, ones)
+    got = []
+    for longest, shortest in ((max(lens), min(lens)), (max(lens), 0), (0, 0)):
+        s = start.clone() if kind == "channels" else start.reshape(len(lens), -1).clone()
+        if kind == "channels":
+            out = ops.gla_scan(proj, 0, H * D, 2 * H * D, gates, D ** -0.5, d_row0, d_lens, d_slots, s, len(lens), H, D, V, longest=longest,
+                               shortest=shortest)
+        else:
+            out = ops.memory_scan(rows, 0, H * D, 2 * H * D, gates, 2 * H, gates if ones else None, H, D ** -0.5, ones, d_row0, d_lens,
+                                  d_slots, s, len(lens), H, D, V, longest=longest, shortest=shortest,
+                                  values=proj if kind == "float_keys" and longest > 0 else None)
+        got.append((out.reshape(want.shape), s.reshape(start.shape)))
+        assert max(off(got[-1][0], want) + off(got[-1][1], end)) < TOL
+    for out, s in got[:2]:
+        for r0, n, slot in zip(row0, lens, slots):
+            same = torch.equal(out[r0:r0 + n], got[2][0][r0:r0 + n])
+            assert same if n < ops.MEMORY_CHUNKS_BESIDE or slot < 0 else not same, (n, slot)
+            if n < ops.MEMORY_CHUNKS_BESIDE and slot >= 0:
+                assert torch.equal(s[slot], got[2][1][slot])
+
+
+def test_scratch_has_a_limit():
+    """A prompt beside many sequences: the scratch is bounded whatever their number."""
+    lens, H, D, V = [1] * 71 + [200], 9, 128, 256
+    proj, row0, d_row0, d_lens, *_ = inputs(lens, H, D, V, 2)
+    gates, state = torch.rand((sum(lens), 2 * H), device=DEV), torch.zeros((72, H * D * V), device=DEV)
+    d_slots = torch.arange(72, dtype=torch.int32, device=DEV)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    out = ops.memory_scan(proj, 0, H * D, 2 * H * D, gates, 2 * H, None, 0, 1.0, False, d_row0, d_lens, d_slots, state, 72, H, D, V, longest=200)
+    # 271 rows are at most nine chunks, if five sequences of 48 rows and more have a short last one; a chunk per sequence were 72
+    assert torch.cuda.max_memory_allocated() - before <= 4 * out.numel() + 9 * 4 * H * D * V + (1 << 20)
 
 
 def test_what_is_refused_or_walks():
