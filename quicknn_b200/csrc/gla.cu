@@ -16,7 +16,8 @@
 // n_t . q_t.  `state_stride` is the distance between two slots' states in floats (a slot may keep more than S).
 //
 //   qnn_mlstm_gates     from the pre-activations of an input and a forget gate per (row, head): the soft-capped log
-//                       gates, the running maximum m_t = max(f_t + m_{t-1}, i_t) from the slot's m and back into it,
+//                       gates, the running maximum m_t = max(f_t + m_{t-1}, i_t) from the slot's m and back into it
+//                       (a thread per single row and head; a block per sequence of several rows and four heads),
 //                       and per row the decay exp(f_t + m_{t-1} - m_t), the key weight exp(i_t - m_t) and exp(-m_t)
 //   qnn_head_norm_gate  qnn_gla_norm_gate with its options: a denominator max(|n.q|, e) + 1e-6 first, the norm's weight
 //                       per column of a head, per column of the row, or none, and silu or sigmoid of the gate
@@ -304,60 +305,44 @@ head_norm_gate_wide_kernel(const float* __restrict__ o, long long ldo, int hs, c
 // ---- gates of a matrix memory with a running maximum ---------------------------------------------------------------
 // pre: float32 [rows, ldp] with the input gate's pre-activation of head h at column h and the forget gate's at H + h;
 // bias: [2H] (input gates, then forget gates).  i = cap tanh((pre_i + b_i) / cap); f = log sigmoid(cap tanh((pre_f +
-// b_f) / cap)).  A warp takes 32 rows at a time: every lane forms one row's log gates (the hyperbolic tangents, the
-// logarithm), then all lanes walk m_t = max(f_t + m_{t-1}, i_t) through the 32 rows in order.  gates: float32 [rows, 3H]: the decay exp(f_t + m_{t-1} - m_t), the key weight exp(i_t - m_t),
-// exp(-m_t).  A warp per (sequence, head); m of the slot's head at mstate[slot * state_stride + h].
-__global__ void mlstm_gates_kernel(const float* __restrict__ pre, long long ldp, const void* __restrict__ bias, int b_dt,
-                                   float cap, const int* __restrict__ seq_row0, const int* __restrict__ seq_len,
-                                   const int* __restrict__ slots, float* __restrict__ mstate, long long state_stride,
-                                   float* __restrict__ gates, int H, int B) {
-    pdl_wait();
-    const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (unit >= B * H) return;
-    const int b = unit / H, h = unit - b * H;
-    const int slot = slots[b];
-    const int row0 = seq_row0 ? seq_row0[b] : b, n = seq_len ? seq_len[b] : 1;
-    const float bi = load_as_f(bias, b_dt, h), bf = load_as_f(bias, b_dt, H + h);
-    float m = slot >= 0 ? mstate[(size_t)slot * state_stride + h] : 0.f;
-    const size_t ldg = (size_t)3 * H;
-    for (int t0 = 0; t0 < n; t0 += 32) {
-        const int t = t0 + lane;
-        float gi = -INFINITY, gf = 0.f;                        // rows beyond the sequence change nothing: m -> max(m, -inf)
-        if (t < n) {
-            const float zi = pre[(size_t)(row0 + t) * ldp + h] + bi, zf = pre[(size_t)(row0 + t) * ldp + H + h] + bf;
-            gi = cap * tanhf(zi / cap);
-            const float c = cap * tanhf(zf / cap);
-            gf = fminf(c, 0.f) - log1pf(expf(-fabsf(c)));
-        }
-        // the rows of the chunk in order; every lane walks them all, so m is the same bit for bit whether a row came
-        // in a prompt, in a portion or alone
-        float before = m, mt = m;
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j) {
-            const float fj = __shfl_sync(0xffffffffu, gf, j), ij = __shfl_sync(0xffffffffu, gi, j);
-            const float next = fmaxf(m + fj, ij);
-            if (lane == j) {
-                before = m;
-                mt = next;
-            }
-            m = next;
-        }
-        if (t < n) {
-            float* gr = gates + (size_t)(row0 + t) * ldg;
-            const bool live = slot >= 0;
-            gr[h] = live ? expf(gf + before - mt) : 0.f;
-            gr[H + h] = live ? expf(gi - mt) : 0.f;
-            gr[2 * H + h] = live ? expf(-mt) : 1.f;
-        }
-    }
-    if (slot >= 0 && lane == 0) mstate[(size_t)slot * state_stride + h] = m;
+// b_f) / cap)).  m_t = max(f_t + m_{t-1}, i_t) through a sequence's rows in order; gates: float32 [rows, 3H]: the decay
+// exp(f_t + m_{t-1} - m_t), the key weight exp(i_t - m_t), exp(-m_t).  m of the slot's head at mstate[slot * state_stride + h].  m is
+// the same bit for bit whether a row came in a prompt, in a portion or alone.
+__device__ __forceinline__ float log_input_gate(float z, float cap) { return cap * tanhf(z / cap); }
+__device__ __forceinline__ float log_forget_gate(float z, float cap) {
+    const float c = cap * tanhf(z / cap);
+    return fminf(c, 0.f) - log1pf(expf(-fabsf(c)));
+}
+// rows of no sequence (live false): nothing is kept or written
+__device__ __forceinline__ void store_gates(float* at, int H, bool live, float gi, float gf, float before, float after) {
+    at[0] = live ? expf(gf + before - after) : 0.f;
+    at[H] = live ? expf(gi - after) : 0.f;
+    at[2 * H] = live ? expf(-after) : 1.f;
 }
 
-// The same for sequences of many rows.  With a warp per (sequence, head) the walk took 75 cycles a row: its chain of two operations
-// stood behind the shuffles that bring a row's numbers to every lane, and between walks the warp formed the next 32 rows' gates.
+// one row per sequence (row b): a thread per (row, head)
+__global__ void mlstm_gates_kernel(const float* __restrict__ pre, long long ldp, const void* __restrict__ bias, int b_dt,
+                                   float cap, const int* __restrict__ slots, float* __restrict__ mstate, long long state_stride,
+                                   float* __restrict__ gates, int H, int B) {
+    pdl_wait();
+    const int unit = blockIdx.x * blockDim.x + threadIdx.x;
+    if (unit >= B * H) return;
+    const int b = unit / H, h = unit - b * H, slot = slots[b];
+    const bool live = slot >= 0;
+    const float zi = pre[(size_t)b * ldp + h] + load_as_f(bias, b_dt, h);
+    const float zf = pre[(size_t)b * ldp + H + h] + load_as_f(bias, b_dt, H + h);
+    const float gi = log_input_gate(zi, cap), gf = log_forget_gate(zf, cap);
+    float* const kept = mstate + (size_t)(live ? slot : 0) * state_stride + h;
+    const float m = live ? *kept : 0.f, next = fmaxf(m + gf, gi);
+    store_gates(gates + (size_t)b * 3 * H + h, H, live, gi, gf, m, next);
+    if (live) *kept = fmaxf(next, -INFINITY);              // gates that are not numbers leave no maximum behind
+}
+
+// Sequences of several rows.  The walk is the chain: with a warp per (sequence, head) it took 75 cycles a row, its two operations
+// behind the shuffles that brought a row's numbers to every lane, and between walks the warp formed the next 32 rows' gates.
 // Here a block takes four heads of a sequence, 64 rows at a time: four lanes of one warp walk a chunk, a head each, from shared
-// memory, while the other warps form the log gates of the chunk after it and the exponentials of the one before.  The walk's order,
-// and so every bit of m, is the same.  Measured: three sequences of 2813 rows, the longest 1777, 12 heads: 68 -> MLSTM_US us.
+// memory, while the other warps form the log gates of the chunk after it and the exponentials of the one before.  Measured, 12 heads:
+// one sequence of 2048 rows 68 -> 44 us, three of 1777, 731 and 301 60 -> 38, eight of 16 2.25 -> 2.15, 64 of one 2.47 -> 2.35.
 constexpr int GATE_ROWS = 64, GATE_HEADS = 4, GATE_THREADS = 256;
 struct GateChunk {
     float f[GATE_ROWS][GATE_HEADS], i[GATE_ROWS][GATE_HEADS], before[GATE_ROWS][GATE_HEADS], after[GATE_ROWS][GATE_HEADS];
@@ -381,9 +366,8 @@ mlstm_gates_rows_kernel(const float* __restrict__ pre, long long ldp, const void
             if (t < n && j < heads) {
                 const float zi = pre[(size_t)(row0 + t) * ldp + h] + load_as_f(bias, b_dt, h);
                 const float zf = pre[(size_t)(row0 + t) * ldp + H + h] + load_as_f(bias, b_dt, H + h);
-                gi = cap * tanhf(zi / cap);
-                const float u = cap * tanhf(zf / cap);
-                gf = fminf(u, 0.f) - log1pf(expf(-fabsf(u)));
+                gi = log_input_gate(zi, cap);
+                gf = log_forget_gate(zf, cap);
             }
             k.i[r][j] = gi;
             k.f[r][j] = gf;
@@ -394,10 +378,7 @@ mlstm_gates_rows_kernel(const float* __restrict__ pre, long long ldp, const void
         for (int x = thread; x < CELLS; x += threads) {
             const int r = x / GATE_HEADS, j = x % GATE_HEADS, t = c * GATE_ROWS + r;
             if (t >= n || j >= heads) continue;
-            float* gr = gates + (size_t)(row0 + t) * ldg + h0 + j;
-            gr[0] = live ? expf(k.f[r][j] + k.before[r][j] - k.after[r][j]) : 0.f;
-            gr[H] = live ? expf(k.i[r][j] - k.after[r][j]) : 0.f;
-            gr[2 * H] = live ? expf(-k.after[r][j]) : 1.f;
+            store_gates(gates + (size_t)(row0 + t) * ldg + h0 + j, H, live, k.i[r][j], k.f[r][j], k.before[r][j], k.after[r][j]);
         }
     };
     const bool walker = threadIdx.x < 32;
@@ -409,13 +390,15 @@ mlstm_gates_rows_kernel(const float* __restrict__ pre, long long ldp, const void
         if (walker) {
             if (lane < GATE_HEADS) {
                 GateChunk& k = chunk[c % 3];
-#pragma unroll 16
-                for (int r = 0; r < GATE_ROWS; ++r) {
-                    const float next = fmaxf(m + k.f[r][lane], k.i[r][lane]);
-                    k.before[r][lane] = m;
-                    k.after[r][lane] = next;
-                    m = next;
-                }
+                const int rows = min(GATE_ROWS, n - c * GATE_ROWS);
+                for (int r0 = 0; r0 < rows; r0 += 16)                  // a short sequence does not walk a whole chunk
+#pragma unroll
+                    for (int r = r0; r < r0 + 16; ++r) {
+                        const float next = fmaxf(m + k.f[r][lane], k.i[r][lane]);
+                        k.before[r][lane] = m;
+                        k.after[r][lane] = next;
+                        m = next;
+                    }
             }
         } else {
             if (c + 1 < chunks) form(c + 1, threadIdx.x - 32, HELPERS);
@@ -424,7 +407,7 @@ mlstm_gates_rows_kernel(const float* __restrict__ pre, long long ldp, const void
     }
     __syncthreads();
     if (chunks > 0) finish(chunks - 1, threadIdx.x, GATE_THREADS);
-    if (walker && live && lane < heads) mstate[(size_t)slot * state_stride + h0 + lane] = m;
+    if (walker && live && lane < heads) mstate[(size_t)slot * state_stride + h0 + lane] = fmaxf(m, -INFINITY);
 }
 
 // Gates of a matrix memory whose forget gate also decides what is written.  rows: [T, ld] of T with the query columns
@@ -601,14 +584,14 @@ QNN_API int qnn_mlstm_gates(const float* pre, long long ldp, const void* bias, i
                             int H, int B, cudaStream_t st) {
     if (B <= 0) return 0;
     if (H <= 0 || !(cap > 0.f) || (seq_row0 == nullptr) != (seq_len == nullptr)) return QNN_ERR_ARGUMENT;
-    if (seq_len != nullptr && B <= 65535) {              // prompts and portions; a warp per (sequence, head) serves single rows
-        launch_pdl(mlstm_gates_rows_kernel, dim3((H + GATE_HEADS - 1) / GATE_HEADS, B), dim3(GATE_THREADS), 0, st, pre, ldp, bias, b_dt,
-                   cap, seq_row0, seq_len, slots, mstate, state_stride, gates, H);
+    if (seq_len == nullptr) {
+        launch_pdl(mlstm_gates_kernel, dim3((unsigned)(((size_t)B * H + 127) / 128)), dim3(128), 0, st, pre, ldp, bias, b_dt, cap, slots,
+                   mstate, state_stride, gates, H, B);
         QNN_LAUNCH_CHECK();
     }
-    const int warps = 4;
-    launch_pdl(mlstm_gates_kernel, dim3(((size_t)B * H + warps - 1) / warps), dim3(warps * 32), 0, st, pre, ldp, bias, b_dt,
-               cap, seq_row0, seq_len, slots, mstate, state_stride, gates, H, B);
+    for (int b0 = 0; b0 < B; b0 += 65535)                // rows of the grid
+        launch_pdl(mlstm_gates_rows_kernel, dim3((H + GATE_HEADS - 1) / GATE_HEADS, B - b0 < 65535 ? B - b0 : 65535), dim3(GATE_THREADS), 0, st,
+                   pre, ldp, bias, b_dt, cap, seq_row0 + b0, seq_len + b0, slots + b0, mstate, state_stride, gates, H);
     QNN_LAUNCH_CHECK();
 }
 
