@@ -160,9 +160,11 @@ __global__ void small_linear_warp_kernel(const TX* __restrict__ x, const TW* __r
 // memory (the weight rows of neighbouring outputs lie K elements apart: read directly, every load of a warp
 // would touch 32 lines).
 // With many rows a block owns 32 of them and a thread four: a weight's element then serves four sums and a row's elements come four
-// at a time (one row per thread reads shared memory twice for every product: 2048 rows, 1152 outputs of 64, 57 -> 35 us).  The order
-// of a sum is the same.
-constexpr int SL_ROWS = 8, SL_OUTS = 32, SL_MAXK = 128;
+// at a time (one row per thread reads shared memory twice for every product).  The order of a sum is the same.  A block then takes about
+// three times as long, so that it pays from where the blocks of 8 rows are more than four per SM (measured, 8 / 32 rows a block, us:
+// 576 of them, 128 rows, 1152 outputs of 64, 5.5 / 6.1; 612, 136 rows, 8.5 / 6.9; 512, 2048 rows, 64 outputs of 128, 9.6 / 10.9; 640, 640
+// rows, 256 outputs of 64, 8.7 / 6.9; 9216, 2048 rows, 1152 outputs of 64, 52 / 30; few outputs of 64, 1024 rows, 3.0 / 4.9).
+constexpr int SL_ROWS = 8, SL_OUTS = 32, SL_MAXK = 128, SL_MANY_BLOCKS = 4 * 148;
 template <typename TX, typename TW>
 __global__ void __launch_bounds__(SL_ROWS * SL_OUTS)
 small_linear_rows_kernel(const TX* __restrict__ x, const TW* __restrict__ w, float* __restrict__ out, int T, int N, int K,
@@ -334,11 +336,12 @@ QNN_API int qnn_small_linear_f32(const void* x, int x_dt, const void* w, int w_d
     if (K <= 0 || (bias != nullptr && !(tau > 0.f))) return QNN_ERR_ARGUMENT;
     const float inv_tau = bias != nullptr ? 1.f / tau : 0.f;
     const size_t total = (size_t)T * N;
+    const bool many = (long long)((T + SL_ROWS - 1) / SL_ROWS) * ((N + SL_OUTS - 1) / SL_OUTS) > SL_MANY_BLOCKS;
 #define QNN_SL(TX, TW)                                                                                               \
     if (K > SL_MAXK)                                                                                                 \
         launch_pdl(small_linear_warp_kernel<TX, TW>, dim3((unsigned)((total + 7) / 8)), dim3(256), 0, st,            \
                    (const TX*)x, (const TW*)w, out, N, K, total, bias, bias_dt, inv_tau);                            \
-    else if (T >= 128)                                                                                               \
+    else if (many)                                                                                                   \
         launch_pdl(small_linear_rows_kernel<TX, TW>, dim3((N + SL_OUTS - 1) / SL_OUTS, (T + 4 * SL_ROWS - 1) / (4 * SL_ROWS)), \
                    dim3(SL_ROWS * SL_OUTS), 0, st, (const TX*)x, (const TW*)w, out, T, N, K, bias, bias_dt, inv_tau); \
     else                                                                                                             \

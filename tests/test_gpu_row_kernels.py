@@ -74,7 +74,8 @@ def test_finite_check_sees_every_place(n, bad):
                 ops.raise_on_status(torch.device(DEV))
 
 
-@pytest.mark.parametrize("K,N,T", [(64, 40, 128), (61, 33, 127), (128, 32, 200), (3, 1, 129), (136, 5, 3), (130, 5, 3)])
+@pytest.mark.parametrize("K,N,T", [(64, 40, 128), (61, 33, 127), (128, 32, 200), (3, 1, 129), (136, 5, 3), (130, 5, 3),
+                                   (64, 256, 592), (64, 256, 593), (61, 257, 640), (3, 1152, 140), (128, 1152, 129)])    # to 592 blocks of 8 rows, and beyond
 def test_few_outputs(K, N, T):
     torch.manual_seed(K)
     x, w = torch.randn((T, K), device=DEV).bfloat16(), torch.randn((N, K), device=DEV).bfloat16()
