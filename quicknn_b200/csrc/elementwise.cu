@@ -58,8 +58,11 @@ __global__ void embed_rmsnorm_kernel(const int* __restrict__ tokens, const W* __
     }
 }
 
-// The rows alone, eight elements per thread.  (With the norm, and rmsnorm_kernel: a row's sum keeps the order it has always had, so
+// The rows alone, eight elements per thread, for steps of up to 384 rows: there the loads' latency counts (64 rows of 2304 2.8 -> 1.6 us,
+// 384 rows 3.0 -> 2.8).  With more rows the walk's stores, neighbours in neighbouring lanes, are the faster (512 rows of 2304 3.1 against
+// 3.2, 1024 rows of 6144 7.0 against 8.7).  (With the norm, and rmsnorm_kernel: a row's sum keeps the order it has always had, so
 // that a model's results stay the same bit for bit.)
+constexpr int EMBED_VEC_ROWS = 384;
 template <typename W>
 __global__ void __launch_bounds__(qnn::ROW8_THREADS)
 embed_vec_kernel(const int* __restrict__ tokens, const W* __restrict__ table, int table_dt, float scale,
@@ -93,7 +96,7 @@ QNN_API int qnn_embed_rmsnorm(const int* tokens, const void* table, int table_dt
 QNN_API int qnn_embed(const int* tokens, const void* table, int table_dtype, float scale, float* out,
                       int T, int H, int V, cudaStream_t st) {
     if (T <= 0) return 0;
-    if (qnn::row8_fits(H, {table, out})) {
+    if (T <= EMBED_VEC_ROWS && qnn::row8_fits(H, {table, out})) {
         if (table_dtype == QNN_DT_BF16)
             qnn::launch_pdl(embed_vec_kernel<bf16>, dim3(T), dim3(qnn::row8_threads(H)), 0, st, tokens, (const bf16*)table, table_dtype,
                             scale, out, H, V);

@@ -59,6 +59,16 @@ def test_norms_and_adds(W, dtype, T):
     close(ops.embed(ids, table, 3.0), 3.0 * D(table)[ids.long()])
 
 
+@pytest.mark.parametrize("T", [383, 384, 385])
+@pytest.mark.parametrize("W", [8, 2304, 2305])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_embedding_of_many_rows(T, W, dtype):
+    torch.manual_seed(T)
+    table = torch.randn((50, W), device=DEV).to(dtype)
+    ids = torch.randint(0, 50, (T,), dtype=torch.int32, device=DEV)
+    assert torch.equal(ops.embed(ids, table, 3.0), 3.0 * table.float()[ids.long()])
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 4095, 4096, 4097, 1 << 20])
 @pytest.mark.parametrize("bad", [None, float("nan"), float("inf"), float("-inf")])
 def test_finite_check_sees_every_place(n, bad):
