@@ -46,9 +46,10 @@ layernorm_vec_kernel(const void* __restrict__ x, int x_dt, const void* __restric
     __shared__ float red[32];
     const size_t base = (size_t)blockIdx.x * H;
     float g[8], v[8];
-    row8_load(w, w_dt, 0, H, g);
+    row8_ask(w, w_dt, H);
     pdl_wait();
     row8_load(x, x_dt, base, H, v);
+    row8_load(w, w_dt, 0, H, g);
     const float mean = block_sum(sum8(v), red) / (float)H;
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = (int)threadIdx.x * 8 < H ? v[e] - mean : 0.f;
@@ -58,7 +59,7 @@ layernorm_vec_kernel(const void* __restrict__ x, int x_dt, const void* __restric
     row8_store(out, out_dt, base, H, v);
 }
 
-// resid += layernorm(v) * g of a row in registers (g and the stream's row r were asked for before)
+// resid += layernorm(v) * g of a row in registers (g and the stream's row r were loaded before)
 __device__ __forceinline__ void add_layernorm_of_row8(float (&v)[8], const float (&r)[8], const float (&g)[8], float* red,
                                                       float* __restrict__ resid, float eps, void* __restrict__ copy, int copy_dt, int H) {
     const size_t base = (size_t)blockIdx.x * H;
@@ -79,12 +80,14 @@ add_layernorm_vec_kernel(float* __restrict__ resid, const void* __restrict__ y, 
     __shared__ float red[32];
     const size_t base = (size_t)blockIdx.x * H;
     float g[8], b[8], v[8], r[8];
-    row8_load(w, w_dt, 0, H, g);
-    if (bias != nullptr) row8_load(bias, b_dt, 0, H, b);
-    else zero8(b);
+    row8_ask(w, w_dt, H);
+    if (bias != nullptr) row8_ask(bias, b_dt, H);
     pdl_wait();
     row8_load(y, y_dt, base, H, v);
     row8_load(resid, QNN_DT_F32, base, H, r);
+    if (bias != nullptr) row8_load(bias, b_dt, 0, H, b);
+    else zero8(b);
+    row8_load(w, w_dt, 0, H, g);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] += b[e];
     add_layernorm_of_row8(v, r, g, red, resid, eps, copy, copy_dt, H);
@@ -180,12 +183,13 @@ add_mean_layernorm_vec_kernel(float* __restrict__ resid, Branches br, int y_dt, 
     __shared__ float red[32];
     const size_t base = (size_t)blockIdx.x * H;
     float g[8], r[8], y[MAX_BRANCHES][8], mean[8];
-    row8_load(w, w_dt, 0, H, g);
+    row8_ask(w, w_dt, H);
     pdl_wait();
 #pragma unroll
     for (int b = 0; b < MAX_BRANCHES; ++b)
         if (b < br.n) row8_load(br.y[b], y_dt, base, H, y[b]);
     row8_load(resid, QNN_DT_F32, base, H, r);
+    row8_load(w, w_dt, 0, H, g);
     zero8(mean);
 #pragma unroll
     for (int b = 0; b < MAX_BRANCHES; ++b)

@@ -42,10 +42,11 @@ add_scaled_rmsnorm_vec_kernel(float* __restrict__ resid, const void* __restrict_
     __shared__ float red[32];
     const size_t base = (size_t)blockIdx.x * H;
     float g[8], v[8], r[8];
-    if (out != nullptr) row8_load(w, w_dt, 0, H, g);         // no kernel of a step writes weights
+    if (out != nullptr) row8_ask(w, w_dt, H);
     pdl_wait();
     row8_load(y, y_dt, base, H, v);
     row8_load(resid, QNN_DT_F32, base, H, r);
+    if (out != nullptr) row8_load(w, w_dt, 0, H, g);
 #pragma unroll
     for (int e = 0; e < 8; ++e) r[e] = r[e] + scale * v[e];
     row8_store(resid, QNN_DT_F32, base, H, r);
@@ -62,9 +63,10 @@ rmsnorm_strided_vec_kernel(const void* __restrict__ x, int x_dt, long long ldx, 
                            void* __restrict__ out2, long long ldo2, int N) {
     __shared__ float red[32];
     float g[8], v[8];
-    row8_load(w, w_dt, 0, N, g);
+    row8_ask(w, w_dt, N);
     pdl_wait();
     row8_load(x, x_dt, (size_t)blockIdx.x * ldx, N, v);
+    row8_load(w, w_dt, 0, N, g);
     const float inv = rsqrtf(block_sum(squares8(v), red) / (float)N + eps);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = v[e] * inv * g[e];

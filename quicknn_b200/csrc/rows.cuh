@@ -1,8 +1,9 @@
 // A row per block in registers, eight neighbouring elements per thread: what the row kernels (norms, adds, copies) share.
 //
 // Rows of a multiple of 8 elements up to 8192 whose starts lie on 16 bytes go this way; others keep the kernels that walk a row
-// element by element.  Bound by latency where a step has few rows (the loads of a row are all in flight at once, and what no kernel
-// of the step writes is asked for before the wait for the kernel in front) and by bytes where it has many.  Measured against the
+// element by element.  Bound by latency where a step has few rows (the loads of a row are all in flight at once, and weights are
+// asked into L2 before the wait for the kernel in front, which may be the one that writes them: they are read behind it) and by
+// bytes where it has many.  Measured against the
 // walk (us, one launch after another): add and RMS norm, 2048 rows of 2304, 18.6 -> 9.3 (6.1 TB/s), 8 rows 4.8 -> 2.7; add and layer
 // norm, 2813 rows of 1536, 21.1 -> 12.7; the same of the mean of two branches 37.4 -> 22.8; norm of a 768-wide piece of 2048 rows
 // 5.3 -> 3.8.
@@ -36,6 +37,11 @@ __device__ __forceinline__ void row8_load(const void* p, int dt, size_t base, in
     const int j = threadIdx.x * 8;
     if (j < n) load8_as_f(p, dt, base + j, v);
     else zero8(v);
+}
+// asks the lines of a row of weights into L2, where whoever writes them writes them too; nothing is read
+__device__ __forceinline__ void row8_ask(const void* p, int dt, int n) {
+    const int j = threadIdx.x * 8, size = dt == QNN_DT_BF16 ? 2 : 4;
+    if (j < n && j * size % 128 < 8 * size) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)p + (size_t)j * size));
 }
 __device__ __forceinline__ void row8_store(void* p, int dt, size_t base, int n, const float (&v)[8]) {
     const int j = threadIdx.x * 8;

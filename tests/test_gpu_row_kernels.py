@@ -69,6 +69,39 @@ def test_embedding_of_many_rows(T, W, dtype):
     assert torch.equal(ops.embed(ids, table, 3.0), 3.0 * table.float()[ids.long()])
 
 
+def test_weights_that_the_kernel_in_front_writes():
+    """A norm may follow the kernel that writes its weights, and reads what that kernel wrote."""
+    torch.manual_seed(1)
+    W, n, f32 = 2304, 4 << 20, torch.float32
+    x, y, r0 = (torch.randn((4, W), device=DEV) for _ in range(3))
+    out = torch.empty((4, W), device=DEV)
+    for i in range(40):
+        src = torch.randn(n, device=DEV).bfloat16()
+        want = src[-2 * W:].float()
+        torch.cuda.synchronize()
+        w = ops.cast(src, f32)[-2 * W:-W]                        # its last blocks write what the norm reads
+        got = [ops.layernorm(x, w, 1e-5, f32)]
+        w, b = ops.cast(src, f32)[-2 * W:].split(W)
+        got.append(r0.clone())                                   # (queued before the cast below)
+        w, b = ops.cast(src, f32)[-2 * W:].split(W)
+        ops.add_layernorm(got[1], y, w, 1e-5, bias=b)
+        got.append(r0.clone())
+        w = ops.cast(src, f32)[-W:]
+        ops.add_mean_layernorm(got[2], [x, y], [x[0], y[0]], 1e-6, w, 1e-5)
+        r = r0.clone()
+        w = ops.cast(src, f32)[-W:]
+        got.append(ops.add_scaled_rmsnorm(r, y, 0.5, w, 1e-6, False, f32))
+        w = ops.cast(src, f32)[-W:]
+        got.append(ops.rmsnorm_cols(x, 0, W, w, 1e-6, out).clone())
+        D, v, b = (lambda t: t.double()), want[:W].double(), want[W:].double()
+        close(got[0], layernorm(D(x), 1e-5) * v)
+        close(got[1], D(r0) + layernorm(D(y) + b, 1e-5) * v)
+        mean = (rms(D(x), 1e-6) * D(x[0]) + rms(D(y), 1e-6) * D(y[0])) / 2
+        close(got[2], D(r0) + layernorm(mean, 1e-5) * b)
+        close(got[3], rms(D(r0) + 0.5 * D(y), 1e-6) * b)
+        close(got[4], rms(D(x), 1e-6) * b)
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 4095, 4096, 4097, 1 << 20])
 @pytest.mark.parametrize("bad", [None, float("nan"), float("inf"), float("-inf")])
 def test_finite_check_sees_every_place(n, bad):
