@@ -12,6 +12,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "per_device.h"
+
 #define QNN_ERR_UNSUPPORTED 10001
 #define QNN_ERR_ARGUMENT 10002
 
@@ -217,6 +219,15 @@ inline long long pdl_max_grid() {
         v = e ? atoll(e) : 1184;
     }
     return v;
+}
+
+// lets `kernel` have up to `bytes` of dynamic shared memory on the current device; `asked`: a static of the kernel's launcher
+template <typename... KArgs>
+inline int allow_shared(OncePerDevice& asked, void (*kernel)(KArgs...), size_t bytes) {
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return (int)e;
+    return asked.run(device, [&] { return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); });
 }
 
 template <typename... KArgs, typename... Args>

@@ -29,8 +29,6 @@
 // A block takes a chunk that there is: the chunks of all sequences are counted through, so unequal sequences cost what their rows do.
 // Steps whose states would not stay in L2 run in rounds of chunks (the caller's scratch limits them), each from the slots'
 // states and back into them.
-#include <atomic>
-
 #include "mma_split.cuh"
 
 using namespace qnn;
@@ -842,15 +840,9 @@ template <typename TQ, int DIM, bool CHANNELS>
 int launch(const ChunkArgs& a, cudaStream_t st) {
     using L = LocalPlan<TQ, DIM, CHANNELS>;
     using O = OutPlan<TQ, DIM, CHANNELS>;
-    static std::atomic<uint64_t> asked{0};                       // devices on which the kernels may have their shared memory
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (!(asked.load(std::memory_order_relaxed) >> (dev & 63) & 1) || dev > 63) {
-        int rc = (int)cudaFuncSetAttribute(memory_chunk_local_kernel<TQ, DIM, CHANNELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::bytes(MAX_VDIM));
-        if (rc == 0) rc = (int)cudaFuncSetAttribute(memory_chunk_out_kernel<TQ, DIM, CHANNELS>, cudaFuncAttributeMaxDynamicSharedMemorySize, O::BYTES);
-        if (rc != 0) return rc;
-        asked.fetch_or(1ull << (dev & 63), std::memory_order_relaxed);
-    }
+    static OncePerDevice local_asked, out_asked;
+    if (int rc = allow_shared(local_asked, memory_chunk_local_kernel<TQ, DIM, CHANNELS>, L::bytes(MAX_VDIM))) return rc;
+    if (int rc = allow_shared(out_asked, memory_chunk_out_kernel<TQ, DIM, CHANNELS>, O::BYTES)) return rc;
     const dim3 grid(a.H, a.units);
     const int elements = DIM * (a.vdim / 4) + (a.vs > a.vdim ? DIM : 0);
     launch_pdl(memory_chunk_local_kernel<TQ, DIM, CHANNELS>, grid, dim3(LOCAL_THREADS), L::bytes(a.vdim), st, a);

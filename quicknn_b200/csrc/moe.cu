@@ -710,12 +710,9 @@ QNN_API int qnn_moe_gate_up(const void* x, int dtype, int W, const void* w_gu, i
 #define QNN_GU_MMA(MT, NM)                                                                                             \
         {                                                                                                              \
             const size_t smem = MT == 1 ? FewRing<NM>::BYTES : (size_t)tile_rows * MMA_PITCH * sizeof(bf16);           \
-            static bool set = false;                                                                                   \
-            if (smem > 48 * 1024 && !set) {                                                                            \
-                cudaFuncSetAttribute(moe_gate_up_mma_kernel<MT, NM>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                     (int)smem);                                                                       \
-                set = true;                                                                                            \
-            }                                                                                                          \
+            static OncePerDevice asked;                                                                                \
+            if (smem > 48 * 1024)                                                                                      \
+                if (int rc = allow_shared(asked, moe_gate_up_mma_kernel<MT, NM>, smem)) return rc;                     \
             launch_pdl(moe_gate_up_mma_kernel<MT, NM>, mgrid, dim3(MMA_WARPS * 32), smem, st, (const bf16*)x, W,      \
                        (const bf16*)w_gu, ff, offsets, perm, sel_w, tiles, n_tiles, top, scale_input, act, limit,      \
                        alpha, (bf16*)hidden);                                                                          \
@@ -754,19 +751,13 @@ QNN_API int qnn_moe_down(const void* hidden, int dtype, int ff, const void* w_do
         if (mgrid.y > 65535) return QNN_ERR_UNSUPPORTED;
         const size_t smem = (size_t)tile_rows * MMA_PITCH * sizeof(bf16);
         if (tile_rows == 64) {
-            static bool set = false;
-            if (!set) {
-                cudaFuncSetAttribute(moe_down_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                set = true;
-            }
+            static OncePerDevice asked;
+            if (int rc = allow_shared(asked, moe_down_mma_kernel<4>, smem)) return rc;
             launch_pdl(moe_down_mma_kernel<4>, mgrid, dim3(MMA_WARPS * 32), smem, st, (const bf16*)hidden, ff,
                        (const bf16*)w_down, W, offsets, perm, sel_w, tiles, n_tiles, scale_output, ys);
         } else {
-            static bool set = false;
-            if (!set) {
-                cudaFuncSetAttribute(moe_down_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, FewRing<1>::BYTES);
-                set = true;
-            }
+            static OncePerDevice asked;
+            if (int rc = allow_shared(asked, moe_down_mma_kernel<1>, FewRing<1>::BYTES)) return rc;
             launch_pdl(moe_down_mma_kernel<1>, mgrid, dim3(MMA_WARPS * 32), FewRing<1>::BYTES, st, (const bf16*)hidden, ff,
                        (const bf16*)w_down, W, offsets, perm, sel_w, tiles, n_tiles, scale_output, ys);
         }
