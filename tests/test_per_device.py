@@ -7,7 +7,7 @@ import pytest
 from quicknn_b200.kernels.build import CSRC
 
 PROGRAM = r"""
-#include <cstdio>
+#include <initializer_list>
 #include "per_device.h"
 int main() {
     static qnn::OncePerDevice once;
