@@ -10,6 +10,7 @@ the copy that read it has run (an event per buffer says so).  The ring is native
 from __future__ import annotations
 
 import ctypes
+import threading
 import weakref
 from typing import Optional
 
@@ -30,19 +31,23 @@ class PinnedUploader:
         self._nbytes = nbytes
         self._ring: Optional[int] = None
         self._lib = None
+        self._opening = threading.Lock()
         self.bytes_sent = 0
 
     def _open(self) -> None:
         from ..kernels import lib
-        self._lib = lib
-        ring, native = ctypes.c_void_p(), lib.load()
-        slab = torch.empty(self.entries * self._nbytes, dtype=torch.uint8, pin_memory=True)
-        lib.check(native.qnn_upload_ring(self.entries, self._nbytes, slab.data_ptr(), ctypes.byref(ring)), "upload_ring", 0)
-        self._ring = ring.value
-        weakref.finalize(self, _close, native, ring.value, slab)
+        with self._opening:
+            if self._ring is not None:
+                return
+            ring, native = ctypes.c_void_p(), lib.load()
+            slab = torch.empty(self.entries * self._nbytes, dtype=torch.uint8, pin_memory=True)
+            lib.check(native.qnn_upload_ring(self.entries, self._nbytes, slab.data_ptr(), ctypes.byref(ring)), "upload_ring", 0)
+            self._lib = lib
+            self._ring = ring.value
+            weakref.finalize(self, _close, native, ring.value, slab)
 
     def send(self, dst: torch.Tensor, src: np.ndarray) -> None:
-        """dst (contiguous, on the device) = src, ordered on the current stream."""
+        """dst (contiguous) = src, ordered on the current stream of dst's device; a dst in host memory gets the bytes at once."""
         src = np.ascontiguousarray(src)
         n = src.nbytes
         if dst.numel() * dst.element_size() != n or not dst.is_contiguous():
@@ -50,13 +55,11 @@ class PinnedUploader:
         self.bytes_sent += n
         if n == 0:
             return
-        if not self.on_gpu:
+        if not self.on_gpu or not dst.is_cuda:
             dst.view(torch.uint8).reshape(-1).copy_(torch.from_numpy(src.view(np.uint8).reshape(-1)))
             return
-        if not dst.is_cuda:
-            raise ValueError("upload into a tensor that is not on the device")
         if self._ring is None:
             self._open()
         stream = torch._C._cuda_getCurrentRawStream(dst.device.index)
-        self._lib.check(self._lib.load().qnn_upload(self._ring, dst.data_ptr(), src.__array_interface__["data"][0], n, stream),
+        self._lib.check(self._lib.load().qnn_upload(self._ring, dst.data_ptr(), src.__array_interface__["data"][0], n, dst.device.index, stream),
                         "upload", 0)

@@ -4,6 +4,10 @@
 // reads the pinned bytes when the stream gets to it, by which time the host may have written the next step's values.  So every
 // array goes into the next buffer of the ring and is sent from there; a buffer is written again only after the copy that read
 // it has run.  The same over torch tensors and events took about 18 us of host time a copy, this 4.
+//
+// Several threads may send through one ring (a call from Python gives the interpreter away): a lock holds the choice of a buffer, the
+// bytes and the copy together.  An event belongs to the device it was made on; a buffer that goes to another one next gets another.
+#include <mutex>
 #include <new>
 #include <string.h>
 
@@ -15,23 +19,45 @@ struct Buffer {
     void* bytes;
     size_t size;
     cudaEvent_t sent;
+    int device;                  // of the event
     bool own;                    // allocated here: an array that was larger than the caller's pieces
 };
 struct Ring {
     int n, next;
     Buffer* buffers;
+    std::mutex lock;
 };
 
-int fill(Buffer& b, size_t n) {
+// the device that is current while this lives
+struct OnDevice {
+    int before = -1;
+    cudaError_t rc;
+    explicit OnDevice(int device) {
+        rc = cudaGetDevice(&before);
+        if (rc == cudaSuccess && before != device) rc = cudaSetDevice(device);
+        else before = -1;
+    }
+    ~OnDevice() {
+        if (before >= 0) (void)cudaSetDevice(before);
+    }
+};
+
+int fill(Buffer& b, size_t n, int device) {
     if (b.sent != nullptr) {
         const cudaError_t e = cudaEventSynchronize(b.sent);
         if (e != cudaSuccess) return (int)e;
-    } else {
+        if (b.device != device) {
+            (void)cudaEventDestroy(b.sent);
+            b.sent = nullptr;
+        }
+    }
+    if (b.sent == nullptr) {
         const cudaError_t e = cudaEventCreateWithFlags(&b.sent, cudaEventDisableTiming);
         if (e != cudaSuccess) {
             b.sent = nullptr;
             return (int)e;
         }
+        b.device = device;
     }
     if (b.size < n) {
         void* p = nullptr;
@@ -49,11 +75,14 @@ int fill(Buffer& b, size_t n) {
 
 // A ring of `entries` buffers of `each` bytes, pieces of the pinned memory at `slab` (the caller's, kept until the ring is free: an
 // allocation of pinned memory takes about 1 ms, so the pieces come from one that a caching allocator may have at hand); a larger array
-// gets a buffer of its own.  Events are made as buffers are first used, on the device that is current then.
+// gets a buffer of its own.  Events are made as buffers are first used.
 QNN_API int qnn_upload_ring(int entries, long long each, void* slab, void** ring) {
     if (entries < 1 || each < 1 || slab == nullptr || ring == nullptr) return QNN_ERR_ARGUMENT;
-    Ring* r = new (std::nothrow) Ring{entries, 0, new (std::nothrow) Buffer[entries]()};
-    if (r == nullptr || r->buffers == nullptr) {
+    Ring* r = new (std::nothrow) Ring();
+    if (r == nullptr) return (int)cudaErrorMemoryAllocation;
+    r->n = entries;
+    r->buffers = new (std::nothrow) Buffer[entries]();
+    if (r->buffers == nullptr) {
         delete r;
         return (int)cudaErrorMemoryAllocation;
     }
@@ -65,13 +94,16 @@ QNN_API int qnn_upload_ring(int entries, long long each, void* slab, void** ring
     return 0;
 }
 
-// dst (device) = the n bytes at src, ordered on the stream; src may change as soon as this returns.
-QNN_API int qnn_upload(void* ring, void* dst, const void* src, long long n, cudaStream_t st) {
-    if (ring == nullptr || n < 0 || (n > 0 && (dst == nullptr || src == nullptr))) return QNN_ERR_ARGUMENT;
+// dst (on `device`) = the n bytes at src, ordered on the stream, one of that device's; src may change as soon as this returns.
+QNN_API int qnn_upload(void* ring, void* dst, const void* src, long long n, int device, cudaStream_t st) {
+    if (ring == nullptr || n < 0 || device < 0 || (n > 0 && (dst == nullptr || src == nullptr))) return QNN_ERR_ARGUMENT;
     if (n == 0) return 0;
     Ring* r = (Ring*)ring;
+    const OnDevice there(device);
+    if (there.rc != cudaSuccess) return (int)there.rc;
+    const std::lock_guard<std::mutex> held(r->lock);
     Buffer& b = r->buffers[r->next];
-    const int rc = fill(b, (size_t)n);
+    const int rc = fill(b, (size_t)n, device);
     if (rc != 0) return rc;
     r->next = (r->next + 1) % r->n;
     memcpy(b.bytes, src, (size_t)n);

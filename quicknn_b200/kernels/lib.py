@@ -117,7 +117,7 @@ _SIGNATURES: Dict[str, list] = {
     "qnn_memory_scan": [c_vp, c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_ll, c_float, c_int, c_vp, c_vp, c_vp, c_vp,
                         c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_int, c_vp],
     "qnn_upload_ring": [c_int, c_ll, c_vp, c_vp],
-    "qnn_upload": [c_vp, c_vp, c_vp, c_ll, c_vp],
+    "qnn_upload": [c_vp, c_vp, c_vp, c_ll, c_int, c_vp],
     "qnn_upload_ring_free": [c_vp],
     "qnn_memory_chunks": [c_vp, c_vp, c_ll, c_int, c_vp, c_ll, c_vp, c_ll, c_int, c_vp, c_ll, c_float, c_int, c_int, c_vp, c_vp,
                           c_vp, c_vp, c_ll, c_vp, c_ll, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp],
