@@ -28,8 +28,9 @@
 // the fetching and a tile is written sooner.  Measured (us, 256 columns / as chosen): 256 rows of 2304 x 9216 46.7 / 42.8, of 2304 x
 // 2048 15.1 / 13.3, 640 rows 15.6 / 14.6, 2048 rows of 256 x 2304 15.7 / 14.0, 256 rows of 1152 x 768 8.9 / 7.1.  An element's
 // sum runs over K in the same order whatever the tile, so the results are the same bit for bit.  (Sharing a tile's K among
-// clusters of two or four pairs, summed through distributed shared memory, took 22 and 30 us for 256 and 640 rows of 2304 x 9216, but
-// rounds differently, which shows in the ids that a model samples.)
+// clusters of two or four pairs, summed through distributed shared memory in a fixed order, took 22 and 30 us for 256 and 640 rows of
+// 2304 x 9216.  It is not in: it moves results by rounding, and with them ids that a model samples, where these are to stay the same.
+// No precision speaks against it; the products of up to 128 rows share their K.)
 //
 // Every wait on an mbarrier is bounded (see gemm_tcgen05.cu); the two cluster barriers are reached by
 // every thread of both CTAs on every path, in bounded time.
@@ -328,12 +329,13 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 // The product of qnn_gemm_tcgen05 (same arguments, same meaning of `status`) computed by pairs of CTAs.
 // Returns QNN_ERR_UNSUPPORTED when the device cannot hold a pair (the caller then uses the single-CTA
-// kernel).
+// kernel).  tile_cols: columns of a plain product's tile (64, 128 or 256), 0 to have them chosen.
 QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, int N, int K, int epi, int act,
-                                  float act_a, float act_b, int* status, cudaStream_t st) {
+                                  float act_a, float act_b, int tile_cols, int* status, cudaStream_t st) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0 || (K & 7) || ((((uintptr_t)A | (uintptr_t)B | (uintptr_t)C) & 15) != 0)) return QNN_ERR_UNSUPPORTED;
     if (epi != EPI_NONE && epi != EPI_GATED) return QNN_ERR_ARGUMENT;
+    if (tile_cols != 0 && (epi != EPI_NONE || (tile_cols != 64 && tile_cols != 128 && tile_cols != 256))) return QNN_ERR_ARGUMENT;
     if (epi == EPI_GATED && (N & 1)) return QNN_ERR_ARGUMENT;
     const int Nout = epi == EPI_GATED ? N / 2 : N;
     static int sm_count = 0;
@@ -347,7 +349,9 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
     const long long m_tiles = (M + 2 * BM - 1) / (2 * BM);
     const int pairs_about = sm_count / 2 > 0 ? sm_count / 2 : 1;
     int cols = epi == EPI_GATED ? 128 : 256;
-    if (epi == EPI_NONE) {
+    if (tile_cols != 0) {
+        cols = tile_cols;
+    } else if (epi == EPI_NONE) {
         auto time = [&](int c, int slab) { return (m_tiles * ((N + c - 1) / c) + pairs_about - 1) / pairs_about * slab; };
         long long best = time(256, SLAB_256);
         if (time(128, SLAB_128) < best) { cols = 128; best = time(128, SLAB_128); }

@@ -354,12 +354,12 @@ GEMM_2CTA = os.environ.get("QNN_GEMM_2CTA", "1") != "0"
 
 
 def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_NONE, activation: str = "gelu_tanh",
-                 pair: Optional[bool] = None, out: Optional[torch.Tensor] = None, act_consts=(0.0, 0.0)):
+                 pair: Optional[bool] = None, out: Optional[torch.Tensor] = None, act_consts=(0.0, 0.0), tile_cols: int = 0):
     """x w^T for whole prompts on the 5th-generation tensor cores (bfloat16, any M; K a multiple of 8).
     Epilogues: none, gated (w = [gate; up] stacked), or an activation alone (``"xielu"`` with its two
     constants in ``act_consts``).  With more than 128 rows pairs of CTAs
-    compute 256 x 256 tiles (``pair``; QNN_GEMM_2CTA=0 keeps one CTA per tile).  Returns None when
-    the sizes are refused."""
+    compute tiles of 256 rows and 256, 128 or 64 columns (``pair``; QNN_GEMM_2CTA=0 keeps one CTA per tile), ``tile_cols`` of
+    them if given.  Returns None when the sizes are refused."""
     _req(x, "x", torch.bfloat16, 2)
     _req(w, "w", torch.bfloat16, 2)
     M, K = x.shape
@@ -383,7 +383,7 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_NONE, 
     if pair is None:
         pair = GEMM_2CTA and M > 128
     if pair:
-        code = L.qnn_gemm_tcgen05_2cta(_p(x), _p(w), _p(out), M, N, K, epilogue, act_code, ka, kb,
+        code = L.qnn_gemm_tcgen05_2cta(_p(x), _p(w), _p(out), M, N, K, epilogue, act_code, ka, kb, tile_cols,
                                        _p(_status_word(x.device)), _stream())
         if code != _lib.ERR_UNSUPPORTED:
             _lib.check(code, "gemm_tcgen05_2cta")

@@ -1,26 +1,35 @@
 """Whole-prompt products with tiles of 256, 128 and 64 columns: an element's sum runs over the inner size in one order whatever the
-tile, so a product of few rows (narrow tiles) gives bit for bit what the same rows give among many (tiles of 256 columns)."""
+tile, so every width gives the same bits, and so do the same rows among many."""
 import pytest
 import torch
 
 from quicknn_b200.kernels import ops
+from quicknn_b200.kernels.lib import KernelError
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
-MANY = 20000             # rows from which every product here takes tiles of 256 columns
+MANY = 20000             # rows for more tiles than there are pairs of SMs, whatever their width
 
 
 @pytest.mark.parametrize("M", [129, 256, 257, 640, 1025, 2048])
 @pytest.mark.parametrize("N,K", [(8, 1024), (64, 64), (72, 2304), (256, 1160), (264, 136), (768, 2304), (2304, 2048), (2304, 9216), (4100, 520)])
-def test_narrow_tiles(M, N, K):
+def test_tile_widths(M, N, K):
     torch.manual_seed(M + N + K)
     x, w = torch.randn((MANY, K), device=DEV).bfloat16(), (torch.randn((N, K), device=DEV) * 0.05).bfloat16()
-    many = ops.gemm_tcgen05(x, w)
-    out = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)          # nothing is written behind the last row
-    got = ops.gemm_tcgen05(x[:M], w, out=out[:M])
-    assert (out[M] == 7.0).all() and torch.equal(got, many[:M])
+    many = ops.gemm_tcgen05(x, w, tile_cols=256)
+    act = ops.gemm_tcgen05(x, w, epilogue=ops.EPI_ACT, activation="silu", tile_cols=256)
     want = x[:M].double() @ w.double().T
-    assert ((got.double() - want).norm() / want.norm()).item() < 2e-3            # bfloat16's own rounding
-    assert torch.equal(ops.gemm_tcgen05(x[:M], w, epilogue=ops.EPI_ACT, activation="silu"),
-                       ops.gemm_tcgen05(x, w, epilogue=ops.EPI_ACT, activation="silu")[:M])
+    assert ((many[:M].double() - want).norm() / want.norm()).item() < 2e-3       # bfloat16's own rounding
+    for cols in (0, 64, 128, 256):
+        out = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device=DEV)      # nothing is written behind the last row
+        got = ops.gemm_tcgen05(x[:M], w, out=out[:M], tile_cols=cols)
+        assert (out[M] == 7.0).all() and torch.equal(got, many[:M]), cols
+        assert torch.equal(ops.gemm_tcgen05(x[:M], w, epilogue=ops.EPI_ACT, activation="silu", tile_cols=cols), act[:M]), cols
     ops.raise_on_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("cols,epilogue", [(32, ops.EPI_NONE), (192, ops.EPI_NONE), (-64, ops.EPI_NONE), (128, ops.EPI_GATED)])
+def test_other_widths_are_refused(cols, epilogue):
+    x = torch.zeros((256, 64), dtype=torch.bfloat16, device=DEV)
+    with pytest.raises(KernelError):
+        ops.gemm_tcgen05(x, x, epilogue=epilogue, tile_cols=cols)
