@@ -14,10 +14,16 @@
 //
 // Queries, keys and values are bfloat16 numbers as they come (retention's rotated queries and keys are float32); every other
 // matrix is float32 and meets them in three bfloat16 parts (mma_split.cuh), so products keep float32's 24 bits; sums are float32.
-// Decays between two rows are products of the rows' decays (in 64 bits, rounded once), all at most 1 where decays are; nothing is
-// divided and no logarithm is taken, so no decay is too strong.  Within 16 rows (a sub-chunk) the per-channel decays stand between query and
-// key and those products run on the FMA pipes; between sub-chunks j < i they part into (suffix of j) (whole sub-chunks between)
-// (prefix of i), and the products are matrix products again.
+// Decays between two rows are products of the rows' decays, all at most 1 where decays are; nothing is
+// divided and no logarithm is taken, so no decay is too strong.  One per head: in 64 bits, rounded once.  Within 16 rows (a sub-chunk)
+// the per-channel decays stand between query and key, and those products, decays included, run in float32 on the FMA pipes; between
+// sub-chunks j < i they part into (suffix of j) (whole sub-chunks between) (prefix of i), each in 64 bits and rounded once, and the
+// products are matrix products again.
+//
+// Against the recurrence in 64 bits, on what eight layers of Fuposun and Tumudra at two widths hand over (2-norm, the row-by-row walk in
+// brackets): a decay per channel around 0.92: outputs 0.9e-7 to 1.1e-7 (1.0e-7 to 1.1e-7), states 5.8e-8 (6.1e-8 to 6.7e-8); constant decays from 0.97 on:
+// 1.0e-7 to 1.4e-7 (2.1e-7 to 5.4e-7), 5e-8 to 8e-8 (2.4e-7 to 8.4e-7); an mLSTM's gates around 0.5: 0.7e-7 to 1.0e-7 (0.8e-7 to 1.1e-7), states
+// 3.6e-8 to 6.7e-8 (2.8e-8 to 5.1e-8: two roundings for the last row where here there are five).
 //
 // Bound by: the chunk states' way through L2 (written once, read and written by the prefix, read once: 16 bytes per state
 // element and chunk, 1.2 MB of state per chunk at 9 heads of 128 x 256), and in the outputs' kernel by the rate of mma.sync (about

@@ -8,7 +8,8 @@
 //   qnn_add_bias           y[t, :] += bias
 //   qnn_activation         out = act(x) elementwise (gelu_tanh, silu, squared relu)
 //
-// All sums are float32; a block per row; the order of a row's sums depends on the width only.
+// All sums are float32; a block per row; the order of a row's sums depends on the width and on whether the rows lie on 16 bytes
+// (rows.cuh), not on the other rows.
 #include "rows.cuh"
 
 using namespace qnn;

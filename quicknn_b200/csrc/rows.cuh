@@ -6,7 +6,9 @@
 // bytes where it has many.  Measured against the
 // walk (us, one launch after another): add and RMS norm, 2048 rows of 2304, 18.6 -> 9.3 (6.1 TB/s), 8 rows 4.8 -> 2.7; add and layer
 // norm, 2813 rows of 1536, 21.1 -> 12.7; the same of the mean of two branches 37.4 -> 22.8; norm of a 768-wide piece of 2048 rows
-// 5.3 -> 3.8.
+// 5.3 -> 3.8.  Wide rows, add and RMS norm / layer norm / add and layer norm / norm of a piece: 8192 wide, 8 rows, add and layer norm
+// 9.9 -> 3.6; 2048 rows 59 -> 36 / 34 -> 20 / 83 -> 62 / 30 -> 15; 6144 wide, 2048 rows 41 -> 28 / 27 -> 16 / 57 -> 47 / 23 -> 12.  (Add and layer norm of 512
+// or 1024 rows of 6144 lose 4 %, 11.2 -> 11.7: a block of 768 threads has an SM to itself.)
 #pragma once
 #include <initializer_list>
 

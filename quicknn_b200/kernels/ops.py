@@ -1012,7 +1012,8 @@ def small_linear_f32(x: torch.Tensor, w: torch.Tensor, decay_bias: Optional[torc
                      tau: Optional[float] = None) -> torch.Tensor:
     """x w^T with float32 sums and a float32 result, whatever the element types: for the few outputs that feed
     float32 math (a gate per head, decay logits).  With ``decay_bias`` and ``tau`` the result is the decay
-    sigmoid(x w^T + bias)^(1/tau) itself.  A plain kernel; the order of a sum depends on the inner size only."""
+    sigmoid(x w^T + bias)^(1/tau) itself.  A plain kernel; the order of a sum depends on the inner size and, beyond 128,
+    on whether the rows lie on 16 bytes."""
     _req(x, "x", None, 2)
     _req(w, "w", None, 2)
     T, K = x.shape

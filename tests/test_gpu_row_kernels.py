@@ -69,6 +69,83 @@ def test_embedding_of_many_rows(T, W, dtype):
     assert torch.equal(ops.embed(ids, table, 3.0), 3.0 * table.float()[ids.long()])
 
 
+# (columns of the rows, first column, of the result's rows, first columns): eights on 16 bytes; then a pitch or a first column that is not
+PIECES = [(2048, 256, 1024, 64, 576), (264, 8, 520, 0, 264), (1032, 8, 1032, 8, 520), (2049, 8, 1024, 64, 576), (2048, 3, 1024, 64, 576),
+          (2048, 256, 1028, 64, 576), (2048, 256, 1024, 60, 576), (2048, 256, 1024, 64, 577), (1028, 4, 1028, 4, 516)]
+
+
+@pytest.mark.parametrize("ldx,col,ldo,out1,out2", PIECES)
+@pytest.mark.parametrize("dtype,out_dtype", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32), (torch.float32, torch.bfloat16)])
+@pytest.mark.parametrize("T", [1, 9])
+@pytest.mark.parametrize("twice", [False, True])
+def test_pieces_of_rows(ldx, col, ldo, out1, out2, dtype, out_dtype, T, twice):
+    n = 256
+    torch.manual_seed(ldx + col)
+    x, w = torch.randn((T, ldx), device=DEV).to(dtype), torch.randn(n, device=DEV).to(dtype)
+    out = torch.full((T, ldo), 7.0, device=DEV).to(out_dtype)
+    ops.rmsnorm_cols(x, col, n, w, 1e-6, out, out1, out2 if twice else None)
+    want = rms(x[:, col:col + n].double(), 1e-6) * w.double()
+    rest = torch.ones(ldo, dtype=torch.bool, device=DEV)
+    for at in [out1] + ([out2] if twice else []):
+        close(out[:, at:at + n], want, out_dtype)
+        rest[at:at + n] = False
+    assert (out[:, rest] == 7.0).all()                               # and nothing beside the pieces
+    if dtype == out_dtype:
+        got = torch.full((T, ldo), 7.0, device=DEV).to(dtype)
+        ops.copy_col_range(x, col, n, got, out1)
+        keep = torch.full((T, ldo), 7.0, device=DEV).to(dtype)
+        keep[:, out1:out1 + n] = x[:, col:col + n]
+        assert torch.equal(got, keep)
+        piece = x[:, col:col + n].contiguous()
+        got.fill_(7.0)
+        ops.copy_cols(piece, got, out1)
+        assert torch.equal(got, keep)
+
+
+@pytest.mark.parametrize("W", [8, 264, 4096, 4104, 100])
+@pytest.mark.parametrize("branches", [1, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_one_and_four_branches(W, branches, dtype):
+    torch.manual_seed(W)
+    ys, ws = [torch.randn((5, W), device=DEV).to(dtype) for _ in range(branches)], [torch.randn(W, device=DEV).to(dtype) for _ in range(branches)]
+    w, stream = torch.randn(W, device=DEV).to(dtype), torch.randn((5, W), device=DEV)
+    r = stream.clone()
+    ops.add_mean_layernorm(r, ys, ws, 1e-6, w, 1e-5)
+    mean = sum(rms(y.double(), 1e-6) * v.double() for y, v in zip(ys, ws)) / branches
+    close(r, stream.double() + layernorm(mean, 1e-5) * w.double())
+
+
+@pytest.mark.parametrize("offset", [0, 1, 8])
+@pytest.mark.parametrize("W", [8, 2304])
+def test_rows_that_do_not_start_on_16_bytes(W, offset):
+    """Widths of eights: only where the memory starts decides the way."""
+    torch.manual_seed(W)
+    take = lambda t: torch.cat([t.new_zeros(offset), t.reshape(-1)])[offset:].view(t.shape)  # noqa: E731
+    for dtype in (torch.float32, torch.bfloat16):
+        x, w = take(torch.randn((3, W), device=DEV).to(dtype)), take(torch.randn(W, device=DEV).to(dtype))
+        r0 = take(torch.randn((3, W), device=DEV))
+        close(ops.layernorm(x, w, 1e-5, dtype), layernorm(x.double(), 1e-5) * w.double(), dtype)
+        r = take(r0)
+        ops.add_layernorm(r, x, w, 1e-5)
+        close(r, r0.double() + layernorm(x.double(), 1e-5) * w.double())
+        r = take(r0)
+        want = r0.double() + 0.5 * x.double()
+        close(ops.add_scaled_rmsnorm(r, x, 0.5, w, 1e-6, False, torch.float32), rms(want, 1e-6) * w.double())
+        close(r, want)
+
+
+@pytest.mark.parametrize("inner", [8, 264, 2304, 33])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_clamped_gate(inner, dtype, offset):
+    torch.manual_seed(inner)
+    gu = (4 * torch.randn(7 * 2 * inner + offset, device=DEV)).to(dtype)[offset:].view(7, 2 * inner)
+    g, u = gu.double().split(inner, 1)
+    g, u = g.clamp(max=7.0), u.clamp(-7.0, 7.0)
+    want = g * torch.sigmoid(1.7 * g) * (u + 1)
+    close(ops.gated_act_clamped(gu, 7.0, 1.7), want, dtype)
+
+
 def test_weights_that_the_kernel_in_front_writes():
     """A norm may follow the kernel that writes its weights, and reads what that kernel wrote."""
     torch.manual_seed(1)
