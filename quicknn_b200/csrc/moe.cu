@@ -17,7 +17,7 @@
 // else (float32, other inner sizes) on plain FMA kernels, 16 rows x 128 columns per block, 32 inner elements at a
 // time through shared memory.  Sums run over the inner size in a fixed order, so a row's result does not depend on
 // which other rows share its tile.
-#include "common.cuh"
+#include "mma_split.cuh"
 
 using namespace qnn;
 
@@ -335,6 +335,7 @@ moe_down_kernel(const T* __restrict__ hidden, int ff, const T* __restrict__ w_do
 
 constexpr int MMA_WARPS = 4, MMA_NW = 2, MMA_COLS = MMA_WARPS * MMA_NW * 8, MMA_KC = 256, MMA_PITCH = MMA_KC + 32;
 
+// (volatile, unlike mma_split.cuh's: few_tile_product's copies into a place must not be asked for before the product that read it)
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -425,8 +426,7 @@ __device__ __forceinline__ void few_tile_product(const bf16* const* w, int col0,
             for (int m = 0; m < NM; ++m)
 #pragma unroll
                 for (int t = 0; t < MMA_NW; ++t)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(at + (m * MMA_NW + t) * 512)),
-                                 "l"(wrow[m][t] + i * 32) : "memory");
+                    cp16((unsigned)__cvta_generic_to_shared(at + (m * MMA_NW + t) * 512), wrow[m][t] + i * 32);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };

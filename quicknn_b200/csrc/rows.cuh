@@ -40,10 +40,11 @@ __device__ __forceinline__ void row8_load(const void* p, int dt, size_t base, in
     if (j < n) load8_as_f(p, dt, base + j, v);
     else zero8(v);
 }
-// asks the lines of a row of weights into L2, where whoever writes them writes them too; nothing is read
+// asks the lines of a row of weights into L2, where whoever writes them writes them too; nothing is read.  The first block does it for
+// all (every block: add and layer norm of 2048 rows of 2304 11.7 -> 12.3 us)
 __device__ __forceinline__ void row8_ask(const void* p, int dt, int n) {
     const int j = threadIdx.x * 8, size = dt == QNN_DT_BF16 ? 2 : 4;
-    if (j < n && j * size % 128 < 8 * size) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)p + (size_t)j * size));
+    if (blockIdx.x == 0 && j < n && j * size % 128 < 8 * size) asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)p + (size_t)j * size));
 }
 __device__ __forceinline__ void row8_store(void* p, int dt, size_t base, int n, const float (&v)[8]) {
     const int j = threadIdx.x * 8;
