@@ -25,11 +25,12 @@
 // 1.0e-7 to 1.4e-7 (2.1e-7 to 5.4e-7), 5e-8 to 8e-8 (2.4e-7 to 8.4e-7); an mLSTM's gates around 0.5: 0.7e-7 to 1.0e-7 (0.8e-7 to 1.1e-7), states
 // 3.6e-8 to 6.7e-8 (2.8e-8 to 5.1e-8: two roundings for the last row where here there are five).
 //
-// Bound by: the chunk states' way through L2 (written once, read and written by the prefix, read once: 16 bytes per state
-// element and chunk, 1.2 MB of state per chunk at 9 heads of 128 x 256), and in the outputs' kernel by the rate of mma.sync (about
-// 20 cycles per product and scheduler, six products per pair of float32 tiles).  Measured at 2048 rows, 9 heads of 128 x 256, a
-// decay per channel: 46 + 10 + 33 us; the walk in segments of 256 rows took 330.  Three prompts of 2813 rows, 12 heads of
-// 64 x 128, a gate per head: 38 + 8 + 26 us against 550.
+// Bound by latency, not by a unit (one prompt of 4096 rows, 9 heads of 128 x 256, a decay per channel): a block of 512 threads per SM, or
+// two of 256 in the outputs' kernel, fill a quarter of the warps; the tensor pipe is busy 20 and 33 % of the time, L2 18 and 15 %, and warps
+// wait in turn at the barriers between a block's stages, for shared memory and for the pipe (about 20 cycles per product and
+// scheduler, six products per pair of float32 tiles).  The prefix is bound by the chunk states' way: 16 bytes per state element and
+// chunk, written once, read and written by the prefix, read once, 1.2 MB of state per chunk.  Measured at 2048 rows: 47 + 9 + 35 us; the
+// walk in segments of 256 rows took 320.  Prompts of 1777, 731 and 301 rows, 12 heads of 64 x 128, a gate per head: 36 + 9 + 25 us against 820.
 // A number that is Inf or NaN reaches what depends on it and nothing else, as in the walk: rows before it, other columns of a value's
 // head and other heads keep their results (what does depend on it is Inf or NaN; the parts of an Inf are Inf and NaN).
 // A block takes a chunk that there is: the chunks of all sequences are counted through, so unequal sequences cost what their rows do.
