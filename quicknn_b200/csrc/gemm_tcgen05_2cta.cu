@@ -23,10 +23,9 @@
 // accumulator row holds gate | up side by side, as in the single-CTA kernel.
 //
 // The plain product also comes with tiles of 128 or 64 columns: a product of few rows and few columns has fewer 256 x 256 tiles than
-// the device has pairs, and its time is one tile's walk over K.  A slab of a narrow tile takes hardly less time than one of 256
-// columns (about 0.27 instead of 0.30 us: an MMA occupies its issuer for about 100 cycles whatever its width), but more pairs share
-// the fetching and a tile is written sooner.  Measured (us, 256 columns / as chosen): 256 rows of 2304 x 9216 46.7 / 42.8, of 2304 x
-// 2048 15.1 / 13.3, 640 rows 15.6 / 14.6, 2048 rows of 256 x 2304 15.7 / 14.0, 256 rows of 1152 x 768 8.9 / 7.1.  An element's
+// the device has pairs, and its time is one tile's walk over K.  A slab takes about 0.16, 0.18 and 0.30 us at 64, 128 and 256
+// columns.  Measured (us, 256 columns / as chosen): 256 rows of 2304 x 9216 46.5 / 26.5, 640 rows 46.6 / 28.7, 1024 rows 46.9 / 32.1;
+// 256 rows of 2304 x 2048 15.1 / 9.1, 640 rows 15.3 / 10.3; 256 rows of 4096 x 2304 16.4 / 10.6.  An element's
 // sum runs over K in the same order whatever the tile, so the results are the same bit for bit.  (Sharing a tile's K among
 // clusters of two or four pairs, summed through distributed shared memory in a fixed order, took 22 and 30 us for 256 and 640 rows of
 // 2304 x 9216.  It is not in: it moves results by rounding, and with them ids that a model samples, where these are to stay the same.
@@ -60,7 +59,7 @@ struct Tile {
 };
 constexpr int STAGING_BYTES = BM * 128 * 2;          // the epilogue's 128 rows x 128 columns of bfloat16
 constexpr int GEMM_THREADS = 192;
-constexpr int SLAB_256 = 30, SLAB_128 = 28, SLAB_64 = 27;      // time of a slab by the tile's columns, in 10 ns
+constexpr int SLAB_256 = 30, SLAB_128 = 18, SLAB_64 = 16;      // time of a slab by the tile's columns, in 10 ns
 
 
 // `bar` is a shared::cluster address: the leader's barrier, whichever CTA of the pair loads
@@ -141,7 +140,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     pdl_wait();
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- producer (both CTAs) ---------------------------------------------------------
             int it = 0;                                    // slabs issued so far, over all tiles
             for (int tile = pair; tile < ntiles && !has_failed(bars); tile += pairs) {
@@ -166,7 +165,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             // ---- tensor-core issue (leader) ----------------------------------------------------
             // instruction descriptor: D float32, A and B bfloat16, both K-major, N >> 3, M >> 4 (M = 256 over the pair)
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)((2 * BM) >> 4) << 24);

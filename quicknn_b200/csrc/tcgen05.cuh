@@ -18,6 +18,17 @@ constexpr unsigned WAIT_HINT_NS = 1000u;                // longest suspension in
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
+// True in one lane of a warp whose lanes all come here.  TMA and tcgen05 instructions stand behind this and not behind
+// `lane == 0`: the compiler then knows that one thread issues them and keeps their addresses and descriptors in uniform
+// registers.  Behind `lane == 0` a tcgen05.mma held its issuer for about 100 cycles whatever its size, so tiles narrower
+// than 256 columns were bound by issue (0.27 us for 64 of the inner size; now 0.16 at 64 columns, 0.18 at 128; 640 rows
+// of 2304 x 9216 43.4 -> 28.7 us).
+__device__ __forceinline__ bool elect_one() {
+    unsigned one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one)::"memory");
+    return one != 0;
+}
+
 // ---- mbarriers ---------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
