@@ -117,7 +117,7 @@ gemm_skinny_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
     // producer asks for the weight tiles of the first ring of stages, and only then waits for that kernel,
     // whose output the activation loads read; every other thread waits before it touches global memory.
     const int n_it = kb1 - kb0;
-    const int ahead = (warp == 0 && lane == 0) ? min(stages, n_it) : 0;
+    const int ahead = min(stages, n_it);
     auto load_weights = [&](int it) {
         const int s = it % stages, kb = kb0 + it;
         const unsigned full = smem_u32(&bars->full[s]);
@@ -130,12 +130,13 @@ gemm_skinny_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
             tma_load_2d(w_dst, &map_w, full, kb * BK, n0);
         }
     };
-    for (int it = 0; it < ahead; ++it) load_weights(it);
+    if (warp == 0 && elect_one())
+        for (int it = 0; it < ahead; ++it) load_weights(it);
     pdl_wait();
     bool have_acc = false;     // epilogue warps: the accumulator is complete (else this CTA contributes zeros)
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             for (int it = 0; it < n_it; ++it) {
                 const int s = it % stages;
                 if (it >= ahead) {
@@ -151,7 +152,7 @@ gemm_skinny_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // D float32, A (weights) and B (activations) bfloat16, both K-major, N = NM, M = 128
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(NM >> 3) << 17) | ((unsigned)(BW >> 4) << 24);
             for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
@@ -221,7 +222,7 @@ gemm_skinny_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gr
             }
             if (KS > 1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // visible to the copy engine
             asm volatile("bar.sync 1, 128;" ::: "memory");                   // the four epilogue warps
-            if (KS > 1 && warp == 2 && lane == 0) {
+            if (KS > 1 && warp == 2 && elect_one()) {
                 const unsigned part_addr = smem_u32(part), recv_addr = smem_u32(recv);
                 for (int q = 0; q < KS; ++q) {
                     // rank q finishes rows [q * RPB, (q + 1) * RPB) of a plain tile; of a gated tile RPB / 2 gate rows

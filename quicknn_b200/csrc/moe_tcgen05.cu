@@ -96,7 +96,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const int ntiles = m_tiles * n_tiles;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- producer -------------------------------------------------------------------
             int it = 0;                                    // slabs issued so far, over all tiles
             for (int tile = blockIdx.x; tile < ntiles && !has_failed(bars); tile += gridDim.x) {
@@ -124,7 +124,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- tensor-core issue ------------------------------------------------------------
             // instruction descriptor: D float32, A and B bfloat16, both K-major, N >> 3, M >> 4
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
