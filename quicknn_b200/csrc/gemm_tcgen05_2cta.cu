@@ -22,10 +22,11 @@
 // For the gated epilogue rank 0 loads the 128 gate rows and rank 1 the 128 matching up rows, so every
 // accumulator row holds gate | up side by side, as in the single-CTA kernel.
 //
-// The plain product also comes with tiles of 128 or 64 columns: a product of few rows and few columns has fewer 256 x 256 tiles than
-// the device has pairs, and its time is one tile's walk over K.  A slab takes about 0.16, 0.18 and 0.30 us at 64, 128 and 256
-// columns.  Measured (us, 256 columns / as chosen): 256 rows of 2304 x 9216 46.5 / 26.5, 640 rows 46.6 / 28.7, 1024 rows 46.9 / 32.1;
-// 256 rows of 2304 x 2048 15.1 / 9.1, 640 rows 15.3 / 10.3; 256 rows of 4096 x 2304 16.4 / 10.6.  An element's
+// The plain product comes with tiles of 64, 96, .. 256 columns: its time is the rounds of tiles that the pairs take times one
+// tile's walk over K, and a slab takes 0.16 us at 64 columns, 0.18 at 128, 0.24 at 192 and 0.30 at 256 (at 256 the tensor cores' time,
+// below that of fetching: the 16 KB of A stay).  Measured (us, 256 columns / 128 / as chosen): of 2304 x 9216 256 rows 46.4 / 28.5 / 26.3 (64), 640
+// rows 46.5 / 29.5 / 28.6 (96), 1280 rows 50.7 / 51.4 / 41.4 (192), 2809 rows 93.0 / 87.4 / 83.5 (192); of 4096 x 2304 640 rows 17.8 /
+// 17.1 / 15.3 (192), 1280 rows 27.8 / 23.2 / 21.2 (160); of 1536 x 6144 2048 rows 36.4 / 35.1 / 28.9 (192).  An element's
 // sum runs over K in the same order whatever the tile, so the results are the same bit for bit.  (Sharing a tile's K among
 // clusters of two or four pairs, summed through distributed shared memory in a fixed order, took 22 and 30 us for 256 and 640 rows of
 // 2304 x 9216.  It is not in: it moves results by rounding, and with them ids that a model samples, where these are to stay the same.
@@ -55,11 +56,14 @@ constexpr int MAX_STAGES = 8;
 template <int BN>                                    // columns of a pair's tile
 struct Tile {
     static constexpr int B_BYTES = (BN / 2) * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;                // per CTA
-    static constexpr int STAGES = BN == 256 ? 6 : MAX_STAGES, TMEM_COLS = BN;                         // TMEM_COLS: per accumulator
+    static constexpr int STAGES = BN >= 192 ? 6 : (BN >= 160 ? 7 : MAX_STAGES), RING_BYTES = STAGES * STAGE_BYTES;
+    static constexpr int TMEM_COLS = BN <= 64 ? 64 : (BN <= 128 ? 128 : 256);                         // per accumulator: a power of two
+    static_assert(BN % 32 == 0 && STAGE_BYTES % 1024 == 0, "the instruction's columns; the swizzle's 8 rows of 128 bytes");
+    static_assert(RING_BYTES + BM * 128 * 2 + 1024 + 256 <= 232448, "a CTA's shared memory");
 };
 constexpr int STAGING_BYTES = BM * 128 * 2;          // the epilogue's 128 rows x 128 columns of bfloat16
 constexpr int GEMM_THREADS = 192;
-constexpr int SLAB_256 = 30, SLAB_128 = 18, SLAB_64 = 16;      // time of a slab by the tile's columns, in 10 ns
+constexpr int SLAB_NS[7] = {160, 167, 175, 205, 235, 268, 300};      // time of a slab in tiles of 64, 96, .. 256 columns
 
 
 // `bar` is a shared::cluster address: the leader's barrier, whichever CTA of the pair loads
@@ -227,9 +231,9 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                 unsigned char* mine = staging + quarter * (32 * 256);
 #pragma unroll 1
                 for (int h0 = 0; h0 < OUT_COLS; h0 += 128) {
-                    constexpr int PART = OUT_COLS < 128 ? OUT_COLS : 128;
+                    const int part = min(OUT_COLS - h0, 128);
 #pragma unroll 1
-                    for (int c0 = h0; c0 < h0 + PART; c0 += 32) {
+                    for (int c0 = h0; c0 < h0 + part; c0 += 32) {
                         uint32_t v[32];
                         tmem_ld32(lane_addr + c0, v);
                         float f[32];
@@ -270,7 +274,7 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
                         const int row = m0 + quarter * 32 + r;
                         const int col = n0 + h0 + ((pos ^ (r & 15)) << 3);
                         const uint4 pk = *reinterpret_cast<const uint4*>(mine + r * 256 + (pos << 4));
-                        const bool staged = PART == 128 || (pos ^ (r & 15)) < PART / 8;
+                        const bool staged = OUT_COLS % 128 == 0 || (pos ^ (r & 15)) < part / 8;
                         if (staged && row < M && col < Nout) *reinterpret_cast<uint4*>(C + (size_t)row * Nout + col) = pk;
                     }
                     __syncwarp();
@@ -323,8 +327,24 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 }
 
 
+typedef void (*Kernel)(CUtensorMap, CUtensorMap, bf16*, int, int, int, int, ActConsts, int*);
+
+// Columns of a plain product's tile: what takes the fewest rounds of tiles times the time of a slab.
+int plain_tile_cols(long long M, long long N, int sm_count) {
+    const long long m_tiles = (M + 2 * BM - 1) / (2 * BM), pairs = sm_count / 2 > 0 ? sm_count / 2 : 1;
+    long long best = 0;
+    int cols = 256;
+    for (int c = 256; c >= 64; c -= 32) {
+        const long long t = (m_tiles * ((N + c - 1) / c) + pairs - 1) / pairs * SLAB_NS[c / 32 - 2];
+        if (c == 256 || t < best) best = t, cols = c;
+    }
+    return cols;
+}
 
 }  // namespace
+
+// The columns that qnn_gemm_tcgen05_2cta chooses for a plain product of this size on a device of so many SMs.
+QNN_API int qnn_gemm_tcgen05_2cta_cols(int M, int N, int sm_count) { return plain_tile_cols(M, N, sm_count); }
 
 // The product of qnn_gemm_tcgen05 (same arguments, same meaning of `status`) computed by pairs of CTAs.
 // Returns QNN_ERR_UNSUPPORTED when the device cannot hold a pair (the caller then uses the single-CTA
@@ -344,18 +364,8 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
             cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
             sm_count = 148;
     }
-    // The tile's columns: what takes the fewest rounds of tiles times the time of a slab (64 inner elements)
     const long long m_tiles = (M + 2 * BM - 1) / (2 * BM);
-    const int pairs_about = sm_count / 2 > 0 ? sm_count / 2 : 1;
-    int cols = epi == EPI_GATED ? 128 : 256;
-    if (tile_cols != 0) {
-        cols = tile_cols;
-    } else if (epi == EPI_NONE) {
-        auto time = [&](int c, int slab) { return (m_tiles * ((N + c - 1) / c) + pairs_about - 1) / pairs_about * slab; };
-        long long best = time(256, SLAB_256);
-        if (time(128, SLAB_128) < best) { cols = 128; best = time(128, SLAB_128); }
-        if (time(64, SLAB_64) < best) cols = 64;
-    }
+    const int cols = epi == EPI_GATED ? 128 : (tile_cols != 0 ? tile_cols : plain_tile_cols(M, N, sm_count));
     const long long ntiles = m_tiles * ((Nout + cols - 1) / cols);
     if (ntiles > 0x3fffffffLL) return QNN_ERR_UNSUPPORTED;
     CUtensorMap map_a, map_b;
@@ -363,15 +373,16 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
     if (rc) return rc;
     rc = make_map(&map_b, B, N, K, epi == EPI_GATED ? 128 : cols / 2);
     if (rc) return rc;
-    const int which = epi == EPI_GATED ? 3 : (cols == 256 ? 0 : (cols == 128 ? 1 : 2));
-    void (*const kerns[4])(CUtensorMap, CUtensorMap, bf16*, int, int, int, int, ActConsts, int*) = {
-        gemm_tcgen05_2cta_kernel<EPI_NONE, 256>, gemm_tcgen05_2cta_kernel<EPI_NONE, 128>, gemm_tcgen05_2cta_kernel<EPI_NONE, 64>,
-        gemm_tcgen05_2cta_kernel<EPI_GATED, 256>};
-    const int rings[4] = {Tile<256>::STAGES * Tile<256>::STAGE_BYTES, Tile<128>::STAGES * Tile<128>::STAGE_BYTES,
-                          Tile<64>::STAGES * Tile<64>::STAGE_BYTES, Tile<256>::STAGES * Tile<256>::STAGE_BYTES};
-    const auto kern = kerns[which];
-    const size_t smem = (size_t)rings[which] + STAGING_BYTES + sizeof(Barriers) + 1024;
-    static bool configured[4] = {false, false, false, false};
+    struct Form { Kernel kernel; int ring_bytes; };
+    static const Form forms[8] = {        // gated, then plain by columns: 64, 96, .. 256
+        {gemm_tcgen05_2cta_kernel<EPI_GATED, 256>, Tile<256>::RING_BYTES}, {gemm_tcgen05_2cta_kernel<EPI_NONE, 64>, Tile<64>::RING_BYTES},
+        {gemm_tcgen05_2cta_kernel<EPI_NONE, 96>, Tile<96>::RING_BYTES},    {gemm_tcgen05_2cta_kernel<EPI_NONE, 128>, Tile<128>::RING_BYTES},
+        {gemm_tcgen05_2cta_kernel<EPI_NONE, 160>, Tile<160>::RING_BYTES},  {gemm_tcgen05_2cta_kernel<EPI_NONE, 192>, Tile<192>::RING_BYTES},
+        {gemm_tcgen05_2cta_kernel<EPI_NONE, 224>, Tile<224>::RING_BYTES},  {gemm_tcgen05_2cta_kernel<EPI_NONE, 256>, Tile<256>::RING_BYTES}};
+    const int which = epi == EPI_GATED ? 0 : cols / 32 - 1;
+    const Kernel kern = forms[which].kernel;
+    const size_t smem = (size_t)forms[which].ring_bytes + STAGING_BYTES + sizeof(Barriers) + 1024;
+    static bool configured[8] = {};
     static int max_pairs = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GEMM_THREADS);

@@ -358,8 +358,8 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, *, epilogue: int = EPI_NONE, 
     """x w^T for whole prompts on the 5th-generation tensor cores (bfloat16, any M; K a multiple of 8).
     Epilogues: none, gated (w = [gate; up] stacked), or an activation alone (``"xielu"`` with its two
     constants in ``act_consts``).  With more than 128 rows pairs of CTAs
-    compute tiles of 256 rows and 256, 128 or 64 columns (``pair``; QNN_GEMM_2CTA=0 keeps one CTA per tile), ``tile_cols`` of
-    them if given.  Returns None when the sizes are refused."""
+    compute tiles of 256 rows and 64, 96, .. 256 columns (``pair``; QNN_GEMM_2CTA=0 keeps one CTA per tile); ``tile_cols``: 64, 128
+    or 256 of them instead of a choice by size.  Returns None when the sizes are refused."""
     _req(x, "x", torch.bfloat16, 2)
     _req(w, "w", torch.bfloat16, 2)
     M, K = x.shape

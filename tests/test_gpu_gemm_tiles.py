@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from quicknn_b200.kernels import ops
-from quicknn_b200.kernels.lib import KernelError
+from quicknn_b200.kernels.lib import KernelError, load
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -33,3 +33,19 @@ def test_other_widths_are_refused(cols, epilogue):
     x = torch.zeros((256, 64), dtype=torch.bfloat16, device=DEV)
     with pytest.raises(KernelError):
         ops.gemm_tcgen05(x, x, epilogue=epilogue, tile_cols=cols)
+
+
+@pytest.mark.parametrize("cols", range(64, 257, 32))
+def test_chosen_widths(cols):
+    """Every width that is chosen by itself, at products that it is chosen for: the bits of 256 columns."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    chosen = load().qnn_gemm_tcgen05_2cta_cols
+    sizes = [(M, N) for M in range(200, 3000, 200) for N in range(8, 4400, 8) if chosen(M, N, sms) == cols]
+    K = 328
+    for M, N in (sizes[0], sizes[len(sizes) // 2], sizes[-1]):
+        torch.manual_seed(M + N)
+        x, w = torch.randn((M - 3, K), device=DEV).bfloat16(), (torch.randn((N, K), device=DEV) * 0.05).bfloat16()
+        out = torch.full((M - 2, N), 7.0, dtype=torch.bfloat16, device=DEV)
+        got = ops.gemm_tcgen05(x, w, out=out[:M - 3])
+        assert torch.equal(got, ops.gemm_tcgen05(x, w, tile_cols=256)) and (out[M - 3] == 7.0).all(), (M, N)
+    ops.raise_on_status(torch.device(DEV))
