@@ -674,7 +674,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 template <int HD, bool FIXED>
 int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, long long out_stride, const int* seq_row0,
-                const int* seq_len, const int* seq_q0, int B, int max_len, int nq, int nkv, float scale, float cap,
+                const int* seq_len, const int* seq_q0, int q_tiles, int B, int max_len, int nq, int nkv, float scale, float cap,
                 int window, int* status, const float* slopes, const float* sinks, cudaStream_t st) {
     const long long width = ld;                    // the rows may be wider than what is read of them
     CUtensorMap map_q, map_kv;
@@ -690,7 +690,8 @@ int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, 
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    const int ntq = (max_len + BM - 1) / BM;
+    // query tiles of a sequence, of which only the last q_tiles (0: all) hold wanted rows
+    const int all_tiles = (max_len + BM - 1) / BM, ntq = q_tiles > 0 && q_tiles < all_tiles ? q_tiles : all_tiles;
     static int sm_count = 0;
     if (sm_count == 0) {
         int dev = 0;
@@ -713,8 +714,11 @@ int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, 
     // tiles on 148 SMs) pairs for every tile need a second round of CTAs (41.0 us), pairs for the two heaviest levels
     // only, so that everything still starts together, took 41.7 us, single CTAs 37.7 us: the cluster launch and the
     // hand-over cost more than the shorter key walk saves, so such a grid runs single CTAs.
+    // Of sequences that go on from cached tokens the tiles of wanted rows count: three of them, 203 rows behind 1100 to 2900 tokens,
+    // 8 heads, are 72 tiles and run as pairs (a step of Gemma 2 2B 5557 -> 5174 us, with the grid of 600 CTAs, most of
+    // them without work, gone).
     int levels = 0;
-    if (ntq >= 2 && !no_split && 2 * singles <= sm_count && key_tiles >= 12) levels = ntq;
+    if (all_tiles >= 2 && !no_split && 2 * singles <= sm_count && key_tiles >= 12) levels = ntq;
     const bool want_split = levels > 0;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(THREADS);
@@ -757,13 +761,14 @@ int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, 
 // qkv: this step's projections, [T rows, (nq + 2 nkv) * hd] bfloat16, rotated, rows ld elements apart; sequence b occupies rows
 // seq_row0[b] .. + seq_len[b] - 1.  seq_q0 (may be null): row seq_q0[b] of sequence b is the first whose output is
 // wanted; the rows before it bring keys and values only (qnn_attn_extend_gather lays cached tokens out that way) and
-// their output rows hold nothing of use.  Head sizes 64, 128 and 256; QNN_ERR_UNSUPPORTED for others.  `status` as in
+// their output rows hold nothing of use; most_wanted: no sequence has more wanted rows than that (0: unknown).  Head sizes
+// 64, 128 and 256; QNN_ERR_UNSUPPORTED for others.  `status` as in
 // qnn_gemm_tcgen05 (bits: 2 K/V wait, 4 S wait, 8 P wait, 16 ring wait, 32 Q wait, 64 product wait, 128 wait for
 // the other half of a pair).  seq_row0 and seq_len are read before the kernel waits for the kernel launched
 // in front of it on the stream: that kernel must not be the one that writes them (copies from the host and
 // kernels further back are complete by then).
 QNN_API int qnn_attn_prefill_tcgen05(const void* qkv, long long ld, long long total_rows, void* out, long long out_stride,
-                                     const int* seq_row0, const int* seq_len, const int* seq_q0, int B, int max_len,
+                                     const int* seq_row0, const int* seq_len, const int* seq_q0, int most_wanted, int B, int max_len,
                                      int nq, int nkv, int hd, float scale, float cap, int window, int* status,
                                      const float* slopes, const float* sinks, cudaStream_t st) {
     if (B <= 0 || max_len <= 0) return 0;
@@ -772,7 +777,9 @@ QNN_API int qnn_attn_prefill_tcgen05(const void* qkv, long long ld, long long to
     if (B > 65535 || nq > 32767 || (max_len + BM - 1) / BM > 65535) return QNN_ERR_UNSUPPORTED;
     if (ld < (long long)(nq + 2 * nkv) * hd) return QNN_ERR_ARGUMENT;
     if ((ld & 7) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || (out_stride * 2) % 16) return QNN_ERR_UNSUPPORTED;
-#define QNN_ATTN_ARGS qkv, ld, total_rows, out, out_stride, seq_row0, seq_len, seq_q0, B, max_len, nq, nkv, scale, cap, window, status, slopes, sinks, st
+    // the last most_wanted rows of a sequence may begin anywhere in a tile
+    const int q_tiles = seq_q0 != nullptr && most_wanted > 0 ? (int)(((long long)most_wanted + 2 * BM - 2) / BM) : 0;
+#define QNN_ATTN_ARGS qkv, ld, total_rows, out, out_stride, seq_row0, seq_len, seq_q0, q_tiles, B, max_len, nq, nkv, scale, cap, window, status, slopes, sinks, st
     // With a softcap up to 70 the exponent cap * log2(e) stays below 101, so that neither exp(score) nor a row's
     // sum over a million keys leaves float32: the fixed-reference softmax with both groups of warps.  QNN_ATTN_FIXED=0
     // keeps the running maximum (for comparisons).

@@ -652,7 +652,7 @@ def attn_prefill(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, tok_
         _req(seq_len, "seq_len", torch.int32, 1)
         if ATTN_TCGEN05:
             code = L.qnn_attn_prefill_tcgen05(
-                _p(qkv), ld, T, _p(out), out.shape[1], _p(seq_row0), _p(seq_len), None, seq_row0.numel(), int(max_len),
+                _p(qkv), ld, T, _p(out), out.shape[1], _p(seq_row0), _p(seq_len), None, 0, seq_row0.numel(), int(max_len),
                 n_heads, n_kv, head_dim, float(scale), float(cap or 0.0), int(window or 0),
                 _p(_status_word(qkv.device)), _p(slopes), _p(sinks), _stream())
             if code != _lib.ERR_UNSUPPORTED:
@@ -720,8 +720,9 @@ def attn_shared_tensor_core(q: torch.Tensor, n_heads: int, n_kv: int, head_dim: 
         _p(new_row0), _p(new_len), _p(row0), _p(rows), B, most, n_heads, n_kv, head_dim, 1, _stream()), "attn_extend_gather")
     out_rows = torch.empty((total, n_heads * head_dim), dtype=q.dtype, device=q.device)
     code = L.qnn_attn_prefill_tcgen05(
-        _p(rows), width, total, _p(out_rows), out_rows.shape[1], _p(row0), _p(length), _p(start), B, most, n_heads, n_kv,
-        head_dim, float(scale), float(cap or 0.0), int(window or 0), _p(_status_word(q.device)), _p(slopes), _p(sinks), _stream())
+        _p(rows), width, total, _p(out_rows), out_rows.shape[1], _p(row0), _p(length), _p(start),
+        0 if whole is None else whole.most_new, B, most, n_heads, n_kv, head_dim, float(scale), float(cap or 0.0), int(window or 0),
+        _p(_status_word(q.device)), _p(slopes), _p(sinks), _stream())
     if code == _lib.ERR_UNSUPPORTED:
         return None
     _lib.check(code, "attn_prefill_tcgen05")
@@ -760,8 +761,8 @@ def attn_extend(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, k_poo
             n_heads, n_kv, head_dim, 0, _stream()), "attn_extend_gather")
         out_rows = torch.empty((whole.total, n_heads * head_dim), dtype=qkv.dtype, device=qkv.device)
         code = L.qnn_attn_prefill_tcgen05(
-            _p(rows), rows.shape[1], whole.total, _p(out_rows), out_rows.shape[1], _p(whole.row0), _p(whole.length), _p(whole.start), B,
-            whole.longest, n_heads, n_kv, head_dim, float(scale), float(cap or 0.0), int(window or 0),
+            _p(rows), rows.shape[1], whole.total, _p(out_rows), out_rows.shape[1], _p(whole.row0), _p(whole.length), _p(whole.start),
+            whole.most_new, B, whole.longest, n_heads, n_kv, head_dim, float(scale), float(cap or 0.0), int(window or 0),
             _p(_status_word(qkv.device)), _p(slopes), _p(sinks), _stream())
         if code != _lib.ERR_UNSUPPORTED:
             _lib.check(code, "attn_prefill_tcgen05")
