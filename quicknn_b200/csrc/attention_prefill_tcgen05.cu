@@ -19,12 +19,17 @@
 //                       product reads.  Without a softcap: a running maximum, and O is rescaled in tensor memory only
 //                       when a row maximum has grown by more than 8 since the value the row's exponentials are taken
 //                       against (the stale maximum cancels in the final division; P stays below e^8).
-//   warps 6..9          a second softmax group, with a softcap only (FIXED).  A capped score lies in [-cap, cap], so
-//                       exp(score) can neither overflow nor vanish in float32 and needs no running maximum:
+//   warps 6..9          a second softmax group: warps 2..5 take the lower tile of each pair, warps 6..9 the upper one, so
+//                       two tiles are in the softmax at any time.  With a running maximum the groups tell each other
+//                       their maxima of a pair through shared memory (an mbarrier per 32 rows) and take their
+//                       exponentials against one reference; group 0 rescales O.  With a softcap (FIXED) a capped score
+//                       lies in [-cap, cap], so exp(score) can neither overflow nor vanish in float32:
 //                       p = exp(cap tanh(s / cap)) against the fixed reference 0, the same softmax (it is invariant
-//                       under the shift) with nothing carried from tile to tile but a row's sum.  The tiles are then
-//                       independent: warps 2..5 take the lower tile of each pair, warps 6..9 the upper one, two tiles
-//                       are in the softmax at any time, no maximum is tracked and O is never rescaled.
+//                       under the shift) with nothing carried from tile to tile but a row's sum.
+// Both groups' arithmetic runs on pairs of scores (f32x2 instructions: the same rounding, half the issue slots), which
+// the softmax is bound by.  us before / after both groups and pairs, no softcap: 8 heads of 256, one prompt of 2048 43.2 /
+// 37.4, four of 1024 34.1 / 30.6; 8 heads of 128, 1777 + 731 + 301 tokens 37.1 / 29.7; with a softcap (pairs alone, the same
+// bits): 35.6 / 34.9, 31.7 / 29.2, 29.2 / 27.5; 1500 tokens under a window of 300 18.2 / 15.5.
 // What set the pace, in the order in which it was found (clock64 around the waits of each role): the softmax chain of
 // one warp per scheduler (2350 cycles per tile); the issue of 16 + 4 products per tile by one thread (1850); shared
 // memory bandwidth (Q, K, V, P and the TMA writes: 224 KB per tile, 160 with Q in tensor memory).  One prompt of 8192
@@ -89,16 +94,53 @@ __device__ __forceinline__ float exp2_fast(float x) {
 // 0, 2, 4, 6, 8 of every 8 columns done this way, 8 heads of 256, one prompt: 2048 tokens 36.8 / 36.1 / 35.1 / 35.2 /
 // 38.4 us, 8192 tokens 243 / 241 / 238 / 239 / 253 us; 32 heads of 128 at 8192: 831 / 815 / 796 / 800 / 869 us.
 constexpr int POLY = 4;            // of every 8 columns of a row
-__device__ __forceinline__ float exp2_poly(float x) {
-    const float magic = 12582912.f;
-    const float xf = x + magic;
-    const float f = x - (xf - magic);
-    float p = fmaf(f, 0.055171407759189606f, 0.24261075258255005f);
-    p = fmaf(p, f, 0.6932609677314758f);
-    p = fmaf(p, f, 0.9999281167984009f);
-    return __int_as_float(__float_as_int(p) + (__float_as_int(xf) << 23));
-}
 
+// Two floats in a register pair: one instruction does both, each rounded like the single operation.
+__device__ __forceinline__ uint64_t two(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void one_by_one(uint64_t v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// (a, b) <- exp(cap tanh(score / cap)) of two scores; `poly`: 2^x by the polynomial described at POLY
+__device__ __forceinline__ uint64_t capped_exp2(float& a, float& b, uint64_t k1, uint64_t k2, bool poly) {
+    float x, y;
+    one_by_one(mul2(two(a, b), k1), x, y);
+    const uint64_t t = two(tanh_fast(x), tanh_fast(y));
+    if (poly) {
+        const uint64_t magic = two(12582912.f, 12582912.f), minus = two(-1.f, -1.f);
+        const uint64_t xf = fma2(t, k2, magic);
+        const uint64_t f = fma2(t, k2, fma2(xf, minus, magic));
+        uint64_t q = fma2(f, two(0.055171407759189606f, 0.055171407759189606f), two(0.24261075258255005f, 0.24261075258255005f));
+        q = fma2(q, f, two(0.6932609677314758f, 0.6932609677314758f));
+        q = fma2(q, f, two(0.9999281167984009f, 0.9999281167984009f));
+        float qa, qb, na, nb;
+        one_by_one(q, qa, qb);
+        one_by_one(xf, na, nb);
+        a = __int_as_float(__float_as_int(qa) + (__float_as_int(na) << 23));
+        b = __int_as_float(__float_as_int(qb) + (__float_as_int(nb) << 23));
+    } else {
+        one_by_one(mul2(t, k2), x, y);
+        a = exp2_fast(x);
+        b = exp2_fast(y);
+    }
+    return two(a, b);
+}
 
 struct __align__(8) Barriers {
     uint64_t q_full;
@@ -111,16 +153,17 @@ struct __align__(8) Barriers {
     uint64_t s_free;          // the softmax warps have read it (8 arrivals: 4 warps for each tile of the pair)
     uint64_t p_ready[2];      // P_j is in shared memory and O has been corrected
     uint64_t pv_done[2];      // O += P_j V_j has completed
+    uint64_t max_ready[4];    // both groups' row maxima of a pair of key tiles are there (one for each 32 rows)
     uint64_t merge_full;      // rank 0 of a pair: rank 1's partial result has arrived (bytes)
     uint32_t tmem_base;
     uint32_t failed;
+    float row_max[2][2][BM];  // what the groups tell each other: by pair parity and group
 };
 
 __device__ __forceinline__ bool has_failed(Barriers* b) { return *reinterpret_cast<volatile uint32_t*>(&b->failed) != 0; }
 
 // HD: head size, 64, 128 or 256 (the operands are walked in blocks of 64 head elements = 128 bytes)
-// FIXED: softcap with a fixed reference, both softmax groups at work (see the head of this file); else the running
-// maximum, warps 2..5 only.
+// FIXED: softcap with a fixed reference (see the head of this file); else the running maximum.
 template <int HD, bool FIXED>
 __global__ void __launch_bounds__(THREADS)
 attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
@@ -148,6 +191,14 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     unsigned char* sQ = sK + KP_BYTES;                              // Q on its way to tensor memory: K stage 1, before its first use
     unsigned char* sOut = sV;                                       // the output rows, once every product is done
     Barriers* bars = reinterpret_cast<Barriers*>(sP + 2 * P_BYTES);
+    // At head size 256 there is no room for a whole KB of alignment.  A block's memory starts on one anyway; if it ever did not, this
+    // says so instead of running past the end.
+    unsigned dynamic_bytes;
+    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynamic_bytes));
+    if ((unsigned)(reinterpret_cast<unsigned char*>(bars + 1) - smem_raw) > dynamic_bytes) {
+        if (threadIdx.x == 0) atomicOr(status, 256);
+        return;
+    }
 
     // grid (heads [x 2 ranks], sequences, query tiles): the query tile is the slowest index, so that CTAs are
     // handed out from the heaviest tiles of all heads down to the lightest
@@ -197,6 +248,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mbar_init(smem_u32(&bars->p_ready[i]), 4);               // one arrival per softmax warp
             mbar_init(smem_u32(&bars->pv_done[i]), 1);
         }
+        for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&bars->max_ready[i]), 2);
         mbar_init(smem_u32(&bars->merge_full), 1);
         if (split && rank == 0) mbar_expect_tx(smem_u32(&bars->merge_full), MERGE_O_BYTES + MERGE_ML_BYTES);
         bars->failed = 0;
@@ -369,9 +421,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         const int key_hi = min(row, len - 1);
         const int key_lo = (window > 0 && row - window + 1 > 0) ? row - window + 1 : 0;
         const unsigned key_span = key_hi >= key_lo ? (unsigned)(key_hi - key_lo) : 0u;
-        // FIXED: this group's tiles are group, group + 2, ...; else group 0 takes them all and group 1 none
-        for (int j = FIXED ? group : (group == 0 ? 0 : nt); j < nt && alive; j += FIXED ? 2 : 1) {
-            const int bsel = j & 1;                      // half of the pair = S columns = P buffer
+        const uint64_t k1_2 = two(k1, k1), k2_2 = two(k2, k2);
+        bool started = false;                            // running maximum: the row has seen a key
+        // this group's tiles: group, group + 2, ... (nt is even)
+        for (int j = group; j < nt && alive; j += 2) {
+            const int bsel = group;                      // half of the pair = S columns = P buffer
             if (!mbar_wait_warp(smem_u32(&bars->s_ready), (j >> 1) & 1)) {
                 atomicOr(status, 4);
                 bars->failed = 1;
@@ -405,68 +459,87 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             bool rescale = false;
             if (FIXED) {
                 // exp(capped score) against the reference 0: k2 = cap log2(e), the exponent stays within +-k2
-                float rs4[4] = {0.f, 0.f, 0.f, 0.f};
+                uint64_t rs01 = two(0.f, 0.f), rs23 = two(0.f, 0.f);      // sums of the columns c % 4
                 if (interior) {
 #pragma unroll
-                    for (int c = 0; c < BN; ++c) {
-                        const float e = tanh_fast(s[c] * k1) * k2;
-                        const float pv = (c & 7) < POLY ? exp2_poly(e) : exp2_fast(e);
-                        s[c] = pv;
-                        rs4[c & 3] += pv;
+                    for (int c = 0; c < BN; c += 4) {
+                        rs01 = add2(rs01, capped_exp2(s[c], s[c + 1], k1_2, k2_2, (c & 7) < POLY));
+                        rs23 = add2(rs23, capped_exp2(s[c + 2], s[c + 3], k1_2, k2_2, (c & 7) < POLY));
                     }
                 } else {
 #pragma unroll
-                    for (int c = 0; c < BN; ++c) {
-                        const bool seen = (unsigned)(col0 + c - key_lo) <= key_span;      // key_lo <= column <= key_hi
-                        const float e = tanh_fast(s[c] * k1) * k2;
-                        const float pv = seen ? ((c & 7) < POLY ? exp2_poly(e) : exp2_fast(e)) : 0.f;
-                        s[c] = pv;
-                        rs4[c & 3] += pv;
+                    for (int c = 0; c < BN; c += 4) {
+#pragma unroll
+                        for (int i = 0; i < 4; i += 2) (void)capped_exp2(s[c + i], s[c + i + 1], k1_2, k2_2, (c & 7) < POLY);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            s[c + i] = (unsigned)(col0 + c + i - key_lo) <= key_span ? s[c + i] : 0.f;      // key_lo <= column <= key_hi
+                        rs01 = add2(rs01, two(s[c], s[c + 1]));
+                        rs23 = add2(rs23, two(s[c + 2], s[c + 3]));
                     }
                 }
-                l_sum += (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
+                float r0s, r1s, r2s, r3s;
+                one_by_one(rs01, r0s, r1s);
+                one_by_one(rs23, r2s, r3s);
+                l_sum += (r0s + r1s) + (r2s + r3s);
             } else {
             float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
             // the distance bias of the tile's first column; a column adds slope_u times its place in the tile, so the
             // bias costs one multiply-add per score and no conversion
             const float bias0 = slope_u * (float)(col0 - row);
-            if (interior) {
-#pragma unroll
-                for (int c = 0; c < BN; ++c) {
-                    const float bias = fmaf(slope_u, (float)c, bias0);     // (float)c is a constant of the unrolled loop
-                    const float x = cap > 0.f ? tanh_fast(s[c] * k1) + bias : fmaf(s[c], k1, bias);
-                    s[c] = x;
-                    mx4[c & 3] = fmaxf(mx4[c & 3], x);
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < BN; ++c) {
-                    const float bias = fmaf(slope_u, (float)c, bias0);
-                    float x = cap > 0.f ? tanh_fast(s[c] * k1) + bias : fmaf(s[c], k1, bias);
-                    const bool seen = (unsigned)(col0 + c - key_lo) <= key_span;      // key_lo <= column <= key_hi
-                    x = seen ? x : -CUDART_INF_F;
-                    s[c] = x;
-                    mx4[c & 3] = fmaxf(mx4[c & 3], x);
-                }
-            }
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            m_run = fmaxf(m_run, mx);
-            if (m_run != -CUDART_INF_F && (j == 0 || m_run > m_used + step || l_sum == 0.f)) {
-                // take the exponentials against the new maximum from here on
-                corr = (l_sum == 0.f) ? 0.f : exp2_fast((m_used - m_run) * k2);
-                rescale = (j > 0);
-                m_used = m_run;
-            }
-            const float moff = m_used * k2;
-            float rs4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int c = 0; c < BN; ++c) {
-                const float p = exp2_fast(fmaf(s[c], k2, -moff));         // exp(-inf) = 0 for masked keys
-                s[c] = p;
-                rs4[c & 3] += p;
+                const float bias = fmaf(slope_u, (float)c, bias0);         // (float)c is a constant of the unrolled loop
+                s[c] = cap > 0.f ? tanh_fast(s[c] * k1) + bias : fmaf(s[c], k1, bias);
             }
-            const float rs = (rs4[0] + rs4[1]) + (rs4[2] + rs4[3]);
-            l_sum = l_sum * corr + rs;
+            if (!interior) {
+#pragma unroll
+                for (int c = 0; c < BN; ++c)
+                    if ((unsigned)(col0 + c - key_lo) > key_span) s[c] = -CUDART_INF_F;     // outside key_lo .. key_hi
+            }
+#pragma unroll
+            for (int c = 0; c < BN; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], s[c]);
+            // The groups take their exponentials against one reference, so each learns the other's maximum of the row.  A group
+            // writes the place of pair J + 2 only when the other has arrived for J + 1, that is, has read J.
+            const int J = j >> 1;
+            float(*const told)[BM] = bars->row_max[J & 1];
+            const float mine = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            told[group][rloc] = mine;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bars->max_ready[quarter]));
+            if (!mbar_wait_warp(smem_u32(&bars->max_ready[quarter]), J & 1)) {
+                atomicOr(status, 4);
+                bars->failed = 1;
+                alive = false;
+                break;
+            }
+            m_run = fmaxf(m_run, fmaxf(mine, told[group ^ 1][rloc]));
+            if (m_run != -CUDART_INF_F && (!started || m_run > m_used + step)) {
+                // take the exponentials against the new maximum from here on (a row without keys so far has only zeros in O)
+                corr = started ? exp2_fast((m_used - m_run) * k2) : 0.f;
+                rescale = started;
+                m_used = m_run;
+                started = true;
+            }
+            const float moff = m_used * k2;
+            const uint64_t less = two(-moff, -moff);
+            uint64_t rs01 = two(0.f, 0.f), rs23 = two(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < BN; c += 4) {
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                    float x, y;
+                    one_by_one(fma2(two(s[c + i], s[c + i + 1]), k2_2, less), x, y);
+                    s[c + i] = exp2_fast(x);                               // exp(-inf) = 0 for masked keys
+                    s[c + i + 1] = exp2_fast(y);
+                }
+                rs01 = add2(rs01, two(s[c], s[c + 1]));
+                rs23 = add2(rs23, two(s[c + 2], s[c + 3]));
+            }
+            float r0s, r1s, r2s, r3s;
+            one_by_one(rs01, r0s, r1s);
+            one_by_one(rs23, r2s, r3s);
+            l_sum = l_sum * corr + ((r0s + r1s) + (r2s + r3s));
             }
             // P_j overwrites the buffer that P_{j-2} V_{j-2} read: that product (issued by another thread than S, so
             // s_ready says nothing about it) has to be done.  Whoever writes P_j has seen every earlier phase of this
@@ -489,7 +562,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     *reinterpret_cast<uint4*>(prow + ((ch ^ (rloc & 7)) << 4)) = pk;
                 }
             }
-            if (!FIXED && __any_sync(0xffffffffu, rescale)) {
+            // group 0 rescales: P V of the second group's tile comes after its own
+            if (!FIXED && group == 0 && __any_sync(0xffffffffu, rescale)) {
                 if (j >= 1 && !mbar_wait_warp(smem_u32(&bars->pv_done[(j - 1) & 1]), ((j - 1) >> 1) & 1)) {
                     atomicOr(status, 64);
                     bars->failed = 1;
@@ -521,7 +595,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // done in order, so after that the one before the very last is over too, and the very last may be asked for.
         if (alive && nt > 0) {
             const int jl = nt - 1;
-            const int jmine = (FIXED && (jl & 1) != group) ? jl - 1 : jl;
+            const int jmine = (jl & 1) != group ? jl - 1 : jl;
             if (jmine >= 0 && jmine != jl && !mbar_wait_warp(smem_u32(&bars->pv_done[jmine & 1]), (jmine >> 1) & 1)) {
                 atomicOr(status, 64);
                 bars->failed = 1;
@@ -533,8 +607,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 alive = false;
             }
         }
-        if (FIXED) {
-            // a row's sum is the sum of its two groups' sums (both against the reference 0); the second group
+        {
+            // a row's sum is the sum of its two groups' sums (both against the same reference); the second group
             // leaves its own at the end of the P buffers, which no product reads any more
             float* l_second = reinterpret_cast<float*>(sP + 2 * P_BYTES - BM * 4);
             if (group == 1) l_second[rloc] = alive ? l_sum : 0.f;
@@ -682,7 +756,9 @@ int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, 
     if (rc) return rc;
     rc = make_map(&map_kv, qkv, total_rows, width, BN);
     if (rc) return rc;
-    const size_t smem = (size_t)k_stages(HD) * 2 * BN * HD * 2 + (size_t)v_stages(HD) * BN * HD * 2 + 2 * P_BYTES + sizeof(Barriers) + 1024;
+    constexpr size_t layout = (size_t)k_stages(HD) * 2 * BN * HD * 2 + (size_t)v_stages(HD) * BN * HD * 2 + 2 * P_BYTES + sizeof(Barriers);
+    static_assert(layout <= 227 * 1024, "a block's shared memory");
+    const size_t smem = layout + 1024 < 227 * 1024 ? layout + 1024 : 227 * 1024;           // with room to align it, where there is
     auto kern = attn_prefill_tcgen05_kernel<HD, FIXED>;
     static bool configured = false;
     if (!configured) {
@@ -764,7 +840,7 @@ int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, 
 // their output rows hold nothing of use; most_wanted: no sequence has more wanted rows than that (0: unknown).  Head sizes
 // 64, 128 and 256; QNN_ERR_UNSUPPORTED for others.  `status` as in
 // qnn_gemm_tcgen05 (bits: 2 K/V wait, 4 S wait, 8 P wait, 16 ring wait, 32 Q wait, 64 product wait, 128 wait for
-// the other half of a pair).  seq_row0 and seq_len are read before the kernel waits for the kernel launched
+// the other half of a pair, 256 shared memory that does not start on a KB).  seq_row0 and seq_len are read before the kernel waits for the kernel launched
 // in front of it on the stream: that kernel must not be the one that writes them (copies from the host and
 // kernels further back are complete by then).
 QNN_API int qnn_attn_prefill_tcgen05(const void* qkv, long long ld, long long total_rows, void* out, long long out_stride,
