@@ -364,23 +364,35 @@ attn_decode_mma_kernel(const bf16* __restrict__ q, size_t q_stride, const bf16* 
 // plain grid followed by the combine kernel; clusters of 2 and 4 measured equal or slightly faster.
 constexpr int CLUSTER_MAX = 4;
 
-template <int HD, bool CLUSTER>
-constexpr int stages() { return 3; }   // of the cp.async pipeline
-
-template <int HD, int MMA_WARPS, bool CLUSTER>
+// Stages ST of the cp.async pipeline: 3.  A grid of more CTAs than the device holds at once takes 2 at head size 256: a third of the
+// shared memory less, so three CTAs share an SM instead of two and one's start (slot, length, page row, first tile) and merge hide
+// behind the others' keys.  Decode steps of Gemma 2 2B, us, 3 / 2 stages: 64 sequences of 512 to 2048 tokens 3512 / 3233, 32 of
+// them 2561 / 2465, 64 of 1200 3286 / 3285; where all CTAs fit at once the deeper ring is the better one (8 of 6900 tokens 2013 / 2202).
+// A tile's sums do not depend on it.
+template <int HD, int MMA_WARPS, int MMA_STAGES>
 size_t smem_bytes(int max_pages) {
-    constexpr int MMA_STAGES = stages<HD, CLUSTER>();
     size_t smem = (size_t)MMA_WARPS * MMA_STAGES * 2 * TILE * HD * 2;
     const size_t merge = (size_t)(MMA_WARPS + 1) * 8 * (HD + 2) * sizeof(float);
     if (smem < merge) smem = merge;
     return smem + ((size_t)max_pages + 2) * sizeof(int);
 }
 
+template <int HD, int MMA_WARPS, int ST>
+int allow_memory() {                                 // before the device is asked what it holds, too
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, MMA_WARPS, ST>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    return 0;
+}
+
 // How many clusters of `size` CTAs of this kernel the device holds at once (asked once per size; 0: none, or
 // clusters are switched off).  Clusters are placed inside a GPC, so fewer CTAs may fit than as a plain grid.
-template <int HD, int MMA_WARPS>
+template <int HD, int MMA_WARPS, int ST>
 int clusters_at_once(size_t smem, int size) {
-    constexpr int ST = stages<HD, true>();
     static int known[CLUSTER_MAX + 1] = {-1, -1, -1, -1, -1};
     if (size < 1 || size > CLUSTER_MAX) return 0;
     if (known[size] < 0) {
@@ -409,9 +421,8 @@ int clusters_at_once(size_t smem, int size) {
 }
 
 // CTAs of this kernel that the device holds at once as a plain grid (asked once).
-template <int HD, int MMA_WARPS>
+template <int HD, int MMA_WARPS, int ST>
 int ctas_at_once(size_t smem) {
-    constexpr int ST = stages<HD, false>();
     static int known = -1;
     if (known < 0) {
         int per_sm = 0, dev = 0, sms = 0;
@@ -432,42 +443,31 @@ int ctas_at_once(size_t smem) {
 // it holds plain ones (a grid of several rounds loses little then).  Measured at head size 256, 24
 // sequences x 4 kv heads x 3 ranges at context 8192: 96 clusters of 3 do not fit at once where 288 plain
 // CTAs do, and a step of 6 layers took 1.58 ms against 1.08 ms with the combine kernel.
-template <int HD, int MMA_WARPS>
-bool merge_in_clusters(size_t smem_plain, size_t smem_cluster, int size, long long clusters) {
-    const int at_once = clusters_at_once<HD, MMA_WARPS>(smem_cluster, size);
+template <int HD, int MMA_WARPS, int ST>
+bool merge_in_clusters(size_t smem, int size, long long clusters) {
+    const int at_once = clusters_at_once<HD, MMA_WARPS, ST>(smem, size);
     if (at_once <= 0) return false;
     if (clusters <= at_once) return true;
-    return (long long)at_once * size * 100 >= (long long)ctas_at_once<HD, MMA_WARPS>(smem_plain) * 95;
+    return (long long)at_once * size * 100 >= (long long)ctas_at_once<HD, MMA_WARPS, ST>(smem) * 95;
 }
 
-template <int HD, int MMA_WARPS>
-int launch(const void* q, long long q_stride, const void* k_pool, const void* v_pool, const int* page_table,
+template <int HD, int MMA_WARPS, int ST>
+int launch_staged(const void* q, long long q_stride, const void* k_pool, const void* v_pool, const int* page_table,
            int max_pages, int page_size, int ring, const int* slots, const int* slot_len, int B, int nq, int nkv,
            float scale, float cap, int window, float* part_o, float* part_ml, int n_splits, void* out,
            long long out_stride, int* combined, const float* slopes, const float* sinks, cudaStream_t st) {
-    const size_t smem = smem_bytes<HD, MMA_WARPS, false>(max_pages);
-    const size_t smem_c = smem_bytes<HD, MMA_WARPS, true>(max_pages);
-    if (smem > 220 * 1024 || smem_c > 220 * 1024) return QNN_ERR_UNSUPPORTED;
-    constexpr int ST = stages<HD, false>(), STC = stages<HD, true>();
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, MMA_WARPS, ST>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, MMA_WARPS, STC>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    const size_t smem = smem_bytes<HD, MMA_WARPS, ST>(max_pages);
+    if (smem > 220 * 1024) return QNN_ERR_UNSUPPORTED;
+    if (const int rc = allow_memory<HD, MMA_WARPS, ST>()) return rc;
     const int G = nq / nkv;
     dim3 grid(n_splits, nkv * ((G + 7) / 8), B);
     *combined = 0;
     if (out != nullptr && n_splits <= CLUSTER_MAX &&
-        merge_in_clusters<HD, MMA_WARPS>(smem, smem_c, n_splits, (long long)grid.y * grid.z)) {
+        merge_in_clusters<HD, MMA_WARPS, ST>(smem, n_splits, (long long)grid.y * grid.z)) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;
         cfg.blockDim = dim3(MMA_WARPS * 32);
-        cfg.dynamicSmemBytes = smem_c;
+        cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -478,7 +478,7 @@ int launch(const void* q, long long q_stride, const void* k_pool, const void* v_
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = (qnn::pdl_enabled() && (long long)grid.x * grid.y * grid.z <= qnn::pdl_max_grid()) ? 2 : 1;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HD, MMA_WARPS, STC>, (const bf16*)q,
+        cudaError_t e = cudaLaunchKernelEx(&cfg, attn_decode_mma_kernel<HD, MMA_WARPS, ST>, (const bf16*)q,
                                            (size_t)q_stride, (const bf16*)k_pool, (const bf16*)v_pool, page_table,
                                            max_pages, page_size, ring, slots, slot_len, nq, nkv, scale, cap, window,
                                            part_o, part_ml, n_splits, (bf16*)out, (size_t)out_stride, slopes, sinks);
@@ -490,6 +490,24 @@ int launch(const void* q, long long q_stride, const void* k_pool, const void* v_
                                              page_table, max_pages, page_size, ring, slots, slot_len, nq, nkv, scale,
                                              cap, window, part_o, part_ml, n_splits, (bf16*)nullptr, (size_t)0, slopes, sinks);
     return (int)cudaGetLastError();
+}
+
+template <int HD, int MMA_WARPS>
+int launch(const void* q, long long q_stride, const void* k_pool, const void* v_pool, const int* page_table,
+           int max_pages, int page_size, int ring, const int* slots, const int* slot_len, int B, int nq, int nkv,
+           float scale, float cap, int window, float* part_o, float* part_ml, int n_splits, void* out,
+           long long out_stride, int* combined, const float* slopes, const float* sinks, cudaStream_t st) {
+#define QNN_STAGED(ST) launch_staged<HD, MMA_WARPS, ST>(q, q_stride, k_pool, v_pool, page_table, max_pages, page_size, ring, slots,     \
+                                                        slot_len, B, nq, nkv, scale, cap, window, part_o, part_ml, n_splits, out, \
+                                                        out_stride, combined, slopes, sinks, st)
+    if constexpr (HD == 256 && MMA_WARPS == 2) {
+        const size_t smem = smem_bytes<HD, MMA_WARPS, 3>(max_pages);
+        if (const int rc = allow_memory<HD, MMA_WARPS, 3>()) return rc;
+        const long long ctas = (long long)n_splits * nkv * ((nq / nkv + 7) / 8) * B;
+        if (smem <= 220 * 1024 && ctas > ctas_at_once<HD, MMA_WARPS, 3>(smem)) return QNN_STAGED(2);
+    }
+    return QNN_STAGED(3);
+#undef QNN_STAGED
 }
 
 }  // namespace
