@@ -156,32 +156,67 @@ __global__ void head_prep_kernel(const T* src, long long lds, void* dst, int dst
     }
 }
 
-// The same with 16-byte accesses: a lane holds eight consecutive columns of a head (heads of up to 256 columns, a
-// multiple of 8).  The pair of an interleaved rotation lies inside a lane; the partner of a half-split pair lies
-// rot/16 lanes away and comes by shuffle.  Element types are read at run time (rows and pools of bfloat16 or float32).
+// The same with 16-byte accesses: a lane holds eight consecutive columns of a head (heads of up to 256 columns, a multiple of 8), so
+// `lph` lanes (a power of two: 8, 16 or 32) hold a head and a warp 32 / lph of them.  The pair of an interleaved rotation lies inside a
+// lane; the partner of a half-split pair lies rot/16 lanes away and comes by shuffle.  Element types are read at run time (rows and
+// pools of bfloat16 or float32).  Bound by instructions and by the chain load -> sum -> store of a head where a step has many rows, so
+// what is the same for every head of a token (a lane's angles, the norms' weights) is held in registers, and the first heads' rows are
+// asked for before the angles are formed.  us, a warp per head / now: 8 + 4 heads of 128, 8 rows 7.7 / 3.9, 2809 rows 25.8 / 18.7;
+// 12 + 12 heads of 64, 2048 rows 39.0 / 13.5; 8 + 4 heads of 256, 2048 rows 27.8 / 20.6.
+// WHOLE_W: the norms' weights are read in pieces of eight (16-byte aligned, norm_dim a multiple of 8); else one by one.
+__device__ __forceinline__ float group_sum(float v, int lph) {
+    for (int o = lph >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+template <bool WHOLE_W>
 __global__ void head_prep_vec_kernel(const void* src, int s_dt, long long lds, void* dst, int d_dt, long long ldd, int nq,
                                      int nk, int nv, int hd, int norm_dim, int rot, int interleaved,
                                      const void* __restrict__ bias, int b_dt, const void* __restrict__ wq,
                                      const void* __restrict__ wk, int w_dt, float eps, const float* __restrict__ inv_freq,
                                      const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, void* k_pool,
                                      void* v_pool, const int* __restrict__ page_table, int max_pages, int page_size,
-                                     int ring, const int* __restrict__ slot_len, int write_cache, int flags) {
+                                     int ring, const int* __restrict__ slot_len, int write_cache, int flags, int lph) {
     const int norm_whole = flags & QNN_PREP_WHOLE;
     const bool norm_last = flags & QNN_PREP_NORM_LAST, plain = flags & QNN_PREP_PLAIN_NORM;
     const bool v_is_k = flags & QNN_PREP_VALUES_ARE_KEYS;
     extern __shared__ float sm[];                   // [rot/2] (cos, sin) pairs, then [nq + nk] sums
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
+    const int hpw = 32 / lph, sub = lane / lph, at = lane & (lph - 1), heads = nq + nk;
+    const int col = at * 8, rh = rot / 2;
+    const bool active = col < hd;
     pdl_wait();
     const int t = blockIdx.x;
+    const size_t in_row = (size_t)t * lds, out_row = (size_t)t * ldd;
+    auto load_head = [&](int h, float (&v)[8]) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        if (active && h < heads) {
+            load8_as_f(src, s_dt, in_row + (size_t)h * hd + col, v);
+            if (bias != nullptr) {
+                float b[8];
+                load8_as_f(bias, b_dt, (size_t)h * hd + col, b);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] += b[e];
+            }
+        }
+    };
+    float v[8];
+    load_head(warp * hpw + sub, v);
     const int pos = tok_pos != nullptr ? tok_pos[t] : 0;
     const int slot = tok_slot != nullptr ? tok_slot[t] : -1;
-    const int rh = rot / 2;
+    float wqv[8], wkv[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) wqv[e] = wkv[e] = 1.f;
+    if (WHOLE_W && !norm_whole && col < norm_dim) {
+        if (wq != nullptr) load8_as_f(wq, w_dt, col, wqv);
+        if (wk != nullptr) load8_as_f(wk, w_dt, col, wkv);
+    }
     float2* angles = reinterpret_cast<float2*>(sm);
     for (int j = threadIdx.x; j < rh; j += blockDim.x) {
         float sn, cs;
         sincosf((float)pos * inv_freq[j], &sn, &cs);
         angles[j] = make_float2(cs, sn);
     }
-    __syncthreads();
     size_t cache_base = 0;
     bool wr = write_cache && slot >= 0;
     if (wr && ring > 0 && pos + ring < slot_len[slot]) wr = false;
@@ -191,118 +226,118 @@ __global__ void head_prep_vec_kernel(const void* src, int s_dt, long long lds, v
         cache_base = ((size_t)page * nk * page_size + (r % page_size)) * hd;
     }
     const size_t head_stride = (size_t)page_size * hd;
-    const size_t in_row = (size_t)t * lds, out_row = (size_t)t * ldd;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-    const int col = lane * 8, shift = rh / 8;
-    const bool active = col < hd;
     float inv_q = 0.f, inv_k = 0.f;
     if (norm_whole) {
         float* sums = sm + 2 * rh;
-        for (int h = warp; h < nq + nk; h += nwarp) {
-            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (active) {
-                load8_as_f(src, s_dt, in_row + (size_t)h * hd + col, v);
-                if (bias != nullptr) {
-                    float b[8];
-                    load8_as_f(bias, b_dt, (size_t)h * hd + col, b);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] += b[e];
-                }
-            }
-            float ss = 0.f;
+        for (int h0 = warp * hpw; h0 < heads; h0 += nwarp * hpw) {
+            float x[8], ss = 0.f;
+            load_head(h0 + sub, x);
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-                if (col + e < norm_dim) ss += v[e] * v[e];
-            ss = warp_sum(ss);
-            if (lane == 0) sums[h] = ss;
+                if (col + e < norm_dim) ss += x[e] * x[e];
+            ss = group_sum(ss, lph);
+            if (at == 0 && h0 + sub < heads) sums[h0 + sub] = ss;
         }
         __syncthreads();
         float sq = 0.f, sk = 0.f;
         for (int h = 0; h < nq; ++h) sq += sums[h];
-        for (int h = nq; h < nq + nk; ++h) sk += sums[h];
+        for (int h = nq; h < heads; ++h) sk += sums[h];
         inv_q = rsqrtf(sq / (float)(nq > 0 ? nq * norm_dim : 1) + eps);
         inv_k = rsqrtf(sk / (float)(nk > 0 ? nk * norm_dim : 1) + eps);
+    } else {
+        __syncthreads();
     }
-    for (int h = warp; h < nq + nk; h += nwarp) {
-        const bool is_k = h >= nq;
-        const size_t c0 = (size_t)h * hd;
-        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (active) {
-            load8_as_f(src, s_dt, in_row + c0 + col, v);
-            if (bias != nullptr) {
-                float b[8];
-                load8_as_f(bias, b_dt, c0 + col, b);
+    // this lane's angles: of pair (col + e) / 2, or of column c and its partner (the lower one's sine with a minus)
+    const bool low = col < rh, turns = col < rot;
+    const int partner = interleaved || !turns ? lane : (low ? lane + rh / 8 : lane - rh / 8);
+    float cs[8], sn[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] += b[e];
-            }
+    for (int e = 0; e < 8; ++e) {
+        cs[e] = 1.f;
+        sn[e] = 0.f;
+        const int c = interleaved ? (col + e) >> 1 : (low ? col + e : col + e - rh);
+        if (col + e < rot) {
+            const float2 a = angles[c];
+            cs[e] = a.x;
+            sn[e] = interleaved || !low ? a.y : -a.y;
         }
+    }
+    const bool any_norm = wq != nullptr || wk != nullptr || (plain && norm_dim > 0);
+    for (int h0 = warp * hpw; h0 < heads; h0 += nwarp * hpw) {
+        const int h = h0 + sub;
+        if (h0 != warp * hpw) load_head(h, v);
+        const bool is_k = h >= nq, store = active && h < heads;
+        const size_t c0 = (size_t)h * hd;
         const void* w = is_k ? wk : wq;
         const bool normed = w != nullptr || (plain && norm_dim > 0);
-        if (is_k && v_is_k && active) {
+        if (is_k && v_is_k && store) {
             store8_from_f(dst, d_dt, out_row + (size_t)(h + nk) * hd + col, v);
             if (wr && v_pool != nullptr)
                 store8_from_f(v_pool, d_dt, cache_base + (size_t)(h - nq) * head_stride + col, v);
         }
-        auto norm = [&]() {
+        auto norm = [&]() {                        // (the lanes of a warp may hold heads with and without a norm: all sum)
             float ss = 0.f;
 #pragma unroll
             for (int e = 0; e < 8; ++e)
                 if (col + e < norm_dim) ss += v[e] * v[e];
-            ss = warp_sum(ss);
+            ss = group_sum(ss, lph);
+            if (!normed) return;
             const float inv = norm_whole ? (is_k ? inv_k : inv_q) : rsqrtf(ss / (float)norm_dim + eps);
-            const size_t w0 = norm_whole ? (size_t)(is_k ? h - nq : h) * norm_dim : 0;
+            if (WHOLE_W) {
+                float wv[8];
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (col + e < norm_dim) v[e] = v[e] * inv * (w != nullptr ? load_as_f(w, w_dt, w0 + col + e) : 1.f);
+                for (int e = 0; e < 8; ++e) wv[e] = is_k ? wkv[e] : wqv[e];
+                if (norm_whole && h < heads && col < norm_dim)
+                    load8_as_f(w, w_dt, (size_t)(is_k ? h - nq : h) * norm_dim + col, wv);
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (col + e < norm_dim) v[e] = v[e] * inv * wv[e];
+            } else if (h < heads) {
+                const size_t w0 = norm_whole ? (size_t)(is_k ? h - nq : h) * norm_dim : 0;
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (col + e < norm_dim) v[e] = v[e] * inv * (w != nullptr ? load_as_f(w, w_dt, w0 + col + e) : 1.f);
+            }
         };
-        if (normed && !norm_last) norm();
+        if (any_norm && !norm_last) norm();
         if (rot > 0) {
             if (interleaved) {
 #pragma unroll
                 for (int e = 0; e < 8; e += 2) {
+                    const float a = v[e], b = v[e + 1];
                     if (col + e < rot) {
-                        const float2 cs = angles[(col + e) >> 1];
-                        const float a = v[e], b = v[e + 1];
-                        v[e] = a * cs.x - b * cs.y;
-                        v[e + 1] = b * cs.x + a * cs.y;
+                        v[e] = a * cs[e] - b * sn[e];
+                        v[e + 1] = b * cs[e] + a * sn[e];
                     }
                 }
             } else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
-                    const float above = __shfl_down_sync(0xffffffffu, v[e], shift);     // column c + rot/2
-                    const float below = __shfl_up_sync(0xffffffffu, v[e], shift);       // column c - rot/2
-                    const int c = col + e;
-                    if (c < rh) {
-                        const float2 cs = angles[c];
-                        v[e] = v[e] * cs.x - above * cs.y;
-                    } else if (c < rot) {
-                        const float2 cs = angles[c - rh];
-                        v[e] = v[e] * cs.x + below * cs.y;
-                    }
+                    const float other = __shfl_sync(0xffffffffu, v[e], partner);
+                    if (turns) v[e] = v[e] * cs[e] + other * sn[e];
                 }
             }
         }
-        if (normed && norm_last) norm();
-        if (active) {
+        if (any_norm && norm_last) norm();
+        if (store) {
             store8_from_f(dst, d_dt, out_row + c0 + col, v);
             if (is_k && wr) store8_from_f(k_pool, d_dt, cache_base + (size_t)(h - nq) * head_stride + col, v);
         }
     }
-    const size_t v0 = (size_t)(nq + nk) * hd;
+    const size_t v0 = (size_t)heads * hd;
     const bool v_cache = wr && v_pool != nullptr;
     if (nv > 0 && !v_is_k && (bias != nullptr || v_cache || src != (const void*)dst)) {
         for (int c = threadIdx.x * 8; c < nv; c += blockDim.x * 8) {
-            float v[8];
-            load8_as_f(src, s_dt, in_row + v0 + c, v);
+            float x[8];
+            load8_as_f(src, s_dt, in_row + v0 + c, x);
             if (bias != nullptr) {
                 float b[8];
                 load8_as_f(bias, b_dt, v0 + c, b);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) v[e] += b[e];
+                for (int e = 0; e < 8; ++e) x[e] += b[e];
             }
-            store8_from_f(dst, d_dt, out_row + v0 + c, v);
-            if (v_cache) store8_from_f(v_pool, d_dt, cache_base + (size_t)(c / hd) * head_stride + (c % hd), v);
+            store8_from_f(dst, d_dt, out_row + v0 + c, x);
+            if (v_cache) store8_from_f(v_pool, d_dt, cache_base + (size_t)(c / hd) * head_stride + (c % hd), x);
         }
     }
 }
@@ -345,10 +380,15 @@ QNN_API int qnn_head_prep(const void* src, int dtype, long long lds, void* dst, 
                          (ldd * ed) % 16 == 0 && ((uintptr_t)bias % 16 == 0) && ((uintptr_t)k_pool % 16 == 0) &&
                          ((uintptr_t)v_pool % 16 == 0);
     if (aligned && hd % 8 == 0 && hd <= 256 && nv % 8 == 0 && (interleaved ? rot % 2 == 0 : rot % 16 == 0)) {
-        launch_pdl(head_prep_vec_kernel, dim3(T), dim3(warps * 32), ((size_t)rot + heads) * sizeof(float), st, src, dtype, lds,
-                   dst, dst_dt, ldd, nq, nk, nv, hd, norm_dim, rot, interleaved, bias, b_dt, wq, wk, w_dt, eps, inv_freq,
-                   tok_pos, tok_slot, k_pool, v_pool, page_table, max_pages, page_size, ring, slot_len, write_cache,
-                   flags);
+        int lph = 8;
+        while (lph * 8 < hd) lph *= 2;
+        const int full = (heads * lph + 31) / 32;       // warps that hold every head at once
+        if (full < warps) warps = full < 1 ? 1 : full;
+        const bool whole_w = norm_dim % 8 == 0 && (((uintptr_t)wq | (uintptr_t)wk) & 15) == 0;
+        launch_pdl(whole_w ? head_prep_vec_kernel<true> : head_prep_vec_kernel<false>, dim3(T), dim3(warps * 32),
+                   ((size_t)rot + heads) * sizeof(float), st, src, dtype, lds, dst, dst_dt, ldd, nq, nk, nv, hd, norm_dim, rot,
+                   interleaved, bias, b_dt, wq, wk, w_dt, eps, inv_freq, tok_pos, tok_slot, k_pool, v_pool, page_table, max_pages,
+                   page_size, ring, slot_len, write_cache, flags, lph);
         QNN_LAUNCH_CHECK();
     }
     const size_t smem = ((size_t)rot + (size_t)warps * hd + heads) * sizeof(float);
