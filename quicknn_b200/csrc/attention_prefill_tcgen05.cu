@@ -8,9 +8,8 @@
 //                       tiles is one operand of 128 rows (hd/64 boxes of 128 x 64), free again once S is formed.
 //   warp 10 (one lane)  TMA producer of V, tiles of 64 keys, free only after O += P V.  128-byte swizzle throughout.
 //   warp 1  (one lane)  issues S[128 x 128] = Q K^T for a pair of tiles: hd/16 tcgen05.mma of N = 128 whose A operand,
-//                       Q, is read from tensor memory.  Issuing one tcgen05.mma occupies its thread for about 100
-//                       cycles whatever its size (N = 32, 64, 128 alike; 138 at N = 256 with A from tensor memory,
-//                       171 with A from shared memory), so products of N = 64 cost their issue, not their work.
+//                       Q, is read from tensor memory.  (Pairs of tiles date from when an MMA held its issuer for about
+//                       100 cycles; with an elected lane, see elect_one, four prompts of 1024 take 28.5 instead of 29.5 us.)
 //   warp 11 (one lane)  issues O[128 x hd] += P_j V_j (4 tcgen05.mma of N = hd, V as MN-major operand) for every tile.
 //   warps 2..5          softmax, one thread per query row (tensor-memory lane = row, so row maxima and sums need no
 //                       shuffles): first they copy Q from shared to tensor memory; then per tile tcgen05.ld of S
@@ -287,7 +286,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     const int kx = (nq + kh) * HD, vx = (nq + nkv + kh) * HD;     // columns of K and V in the qkv rows
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- producer of Q and K --------------------------------------------------------------------
             // K of a pair of tiles is one operand of 128 rows; its stage is free again as soon as S of the pair has
             // been formed.  (The boxes of 128 rows x 64 columns are those of Q: the same tensor map.)
@@ -315,7 +314,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
         }
     } else if (warp == 10) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- producer of V: a stage is free only after O += P_j V_j ------------------------------------
             for (int j = 0; j < nt; ++j) {
                 const int s = j % VS;
@@ -333,11 +332,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- tensor-core issue of S ----------------------------------------------------------------
-            // Issuing one tcgen05.mma occupies its thread for about 100 cycles whatever its size (measured: N = 32,
-            // 64 and 128 alike, 138 at N = 256), so S is formed for two key tiles at once, 16 products of N = 128 with
-            // Q from tensor memory (M 128, B = K of the pair, K-major), and P V is issued by a thread of its own.
+            // S is formed for two key tiles at once, 16 products of N = 128 with Q from tensor memory (M 128, B = K of the
+            // pair, K-major), and P V is issued by a thread of its own.
             // Operand descriptors differ only in their address field (bits 0..13, the address in 16-byte units; every
             // operand lies below 256 KB, so adding an offset never carries out of the field): one descriptor is
             // formed once and each product adds its offset.
@@ -364,7 +362,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             }
         }
     } else if (warp == 11) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- tensor-core issue of O += P_j V_j: M 128, N hd, A (P) K-major, B (V) MN-major -----------------
             const unsigned idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(HD >> 3) << 17) | ((unsigned)(BM >> 4) << 24);
             const uint64_t v_desc0 = umma_desc(smem_u32(sV), BN * 128, 1024);
