@@ -161,15 +161,16 @@ __global__ void head_prep_kernel(const T* src, long long lds, void* dst, int dst
 // lane; the partner of a half-split pair lies rot/16 lanes away and comes by shuffle.  Element types are read at run time (rows and
 // pools of bfloat16 or float32).  Bound by instructions and by the chain load -> sum -> store of a head where a step has many rows, so
 // what is the same for every head of a token (a lane's angles, the norms' weights) is held in registers, and the first heads' rows are
-// asked for before the angles are formed.  us, a warp per head / now: 8 + 4 heads of 128, 8 rows 7.7 / 3.9, 2809 rows 25.8 / 18.7;
-// 12 + 12 heads of 64, 2048 rows 39.0 / 13.5; 8 + 4 heads of 256, 2048 rows 27.8 / 20.6.
+// asked for before the angles are formed.  us, a warp per head / now: 8 + 4 heads of 128, 8 rows 7.7 / 4.0, 2809 rows 25.8 / 17.5;
+// 12 + 12 heads of 64, 2048 rows 39.0 / 11.8; 8 + 4 heads of 256, 2048 rows 27.8 / 19.5.  (64 registers; with the 91 that the compiler takes
+// by itself 18.6, 13.8 and 20.6.)
 // WHOLE_W: the norms' weights are read in pieces of eight (16-byte aligned, norm_dim a multiple of 8); else one by one.
 __device__ __forceinline__ float group_sum(float v, int lph) {
     for (int o = lph >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 template <bool WHOLE_W>
-__global__ void head_prep_vec_kernel(const void* src, int s_dt, long long lds, void* dst, int d_dt, long long ldd, int nq,
+__global__ void __launch_bounds__(256, 4) head_prep_vec_kernel(const void* src, int s_dt, long long lds, void* dst, int d_dt, long long ldd, int nq,
                                      int nk, int nv, int hd, int norm_dim, int rot, int interleaved,
                                      const void* __restrict__ bias, int b_dt, const void* __restrict__ wq,
                                      const void* __restrict__ wk, int w_dt, float eps, const float* __restrict__ inv_freq,
