@@ -159,14 +159,26 @@ struct __align__(8) Barriers {
     float row_max[2][2][BM];  // what the groups tell each other: by pair parity and group
 };
 
+// Where the keys and values of a PAGED launch lie: pages of BN positions, [page][kv head][position][hd]
+struct Pages {
+    bf16* v_pool;
+    const int* table;         // [slot][max_pages]
+    const int* slots;         // of the step's sequences
+    int max_pages;
+};
+
 __device__ __forceinline__ bool has_failed(Barriers* b) { return *reinterpret_cast<volatile uint32_t*>(&b->failed) != 0; }
 
 // HD: head size, 64, 128 or 256 (the operands are walked in blocks of 64 head elements = 128 bytes)
 // FIXED: softcap with a fixed reference (see the head of this file); else the running maximum.
-template <int HD, bool FIXED>
+// PAGED: sequences that go on from cached tokens, all of whose keys and values are in the cache.  A page is a key tile, so the producers
+// load pages where they would load packed rows (map_k and map_v are the pools'); the packed rows (map_q) hold the new tokens only,
+// position seq_q0[b] of sequence b at row seq_row0[b], and so does `out`.  (3 x 203 rows behind 1100 to 2900 tokens, 8 heads of 256: 40 us; the
+// copy out of the pages, 17 us of a layer, and the two small copies around it, 10, are not needed.)
+template <int HD, bool FIXED, bool PAGED>
 __global__ void __launch_bounds__(THREADS)
-attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kv,
-                            bf16* __restrict__ out, size_t out_stride, const int* __restrict__ seq_row0,
+attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                            const __grid_constant__ CUtensorMap map_v, const Pages pages, bf16* __restrict__ out, size_t out_stride, const int* __restrict__ seq_row0,
                             const int* __restrict__ seq_len, const int* __restrict__ seq_q0, int nq, int nkv,
                             float scale, float cap, int window, int* __restrict__ status, int split_levels,
                             const float* __restrict__ slopes, const float* __restrict__ sinks) {
@@ -216,7 +228,8 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // seq_q0: the first rows of a sequence may be there for their keys and values only (a sequence that goes on from
     // cached tokens); query tiles that end before row seq_q0[b] are left out (both CTAs of a pair agree on this)
     if (seq_q0 != nullptr && (qt + 1) * BM <= seq_q0[b]) return;
-    const int r0 = qt * BM, row0 = seq_row0[b];
+    const int q0 = PAGED ? seq_q0[b] : 0;                            // the first position that has a row
+    const int r0 = qt * BM, row0 = seq_row0[b] - q0;                 // row of position 0 (PAGED: may be negative; loads give zeros there)
     const int kh = h / (nq / nkv);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int last_row = min(r0 + BM, len) - 1;
@@ -285,6 +298,10 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     bool alive = true;
     const int kx = (nq + kh) * HD, vx = (nq + nkv + kh) * HD;     // columns of K and V in the qkv rows
 
+    // PAGED: the pools' row of a key tile (beyond the sequence: of its last page, whose keys no row sees)
+    const int* const my_pages = PAGED ? pages.table + (size_t)pages.slots[b] * pages.max_pages : nullptr;
+    auto page_row = [&](int tile) { return (my_pages[min(tile, (len - 1) / BN)] * nkv + kh) * BN; };
+
     if (warp == 0) {
         if (elect_one()) {
             // ---- producer of Q and K --------------------------------------------------------------------
@@ -294,6 +311,15 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             mbar_expect_tx(qf, Q_BYTES);
             for (int d = 0; d < HD / 64; ++d)
                 tma_load_2d(smem_u32(sQ + d * (BM * 128)), &map_q, qf, h * HD + d * 64, row0 + r0);
+            int lower = 0, upper = 0;                                // PAGED: the pools' rows of the pair's two pages, read a pair ahead
+            auto ask = [&](int J) {
+                if (PAGED && J < np) {
+                    const int tile = (jp0 + J * stride) * 2;
+                    lower = page_row(tile);
+                    upper = page_row(tile + 1);
+                }
+            };
+            ask(0);
             for (int J = 0; J < np; ++J) {
                 const int s = J % KS;
                 if (J >= KS && !mbar_wait(smem_u32(&bars->k_empty[s]), ((J / KS) - 1) & 1)) {
@@ -309,13 +335,30 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const unsigned kfull = smem_u32(&bars->k_full[s]);
                 unsigned char* kdst = sK + s * KP_BYTES;
                 mbar_expect_tx(kfull, KP_BYTES);
-                for (int d = 0; d < HD / 64; ++d)
-                    tma_load_2d(smem_u32(kdst + d * (2 * BN * 128)), &map_q, kfull, kx + d * 64, row0 + (jp0 + J * stride) * 2 * BN);
+                if constexpr (PAGED) {
+                    for (int d = 0; d < HD / 64; ++d) {
+                        tma_load_2d(smem_u32(kdst + d * (2 * BN * 128)), &map_k, kfull, d * 64, lower);
+                        tma_load_2d(smem_u32(kdst + d * (2 * BN * 128) + BN * 128), &map_k, kfull, d * 64, upper);
+                    }
+                    ask(J + 1);
+                } else {
+                    for (int d = 0; d < HD / 64; ++d)
+                        tma_load_2d(smem_u32(kdst + d * (2 * BN * 128)), &map_q, kfull, kx + d * 64, row0 + (jp0 + J * stride) * 2 * BN);
+                }
             }
         }
     } else if (warp == 10) {
+        if (PAGED && last_row == len - 1 && len % BN != 0) {
+            // The cells behind the sequence in its last page hold what an earlier sequence left.  Their weights are zero, but zero
+            // times Inf or NaN is not: they are cleared first (by every CTA that loads the page).
+            uint4* cells = reinterpret_cast<uint4*>(pages.v_pool + ((size_t)page_row(len / BN) + len % BN) * HD);
+            for (int i = lane; i < (BN - len % BN) * (HD / 8); i += 32) cells[i] = make_uint4(0u, 0u, 0u, 0u);
+            asm volatile("fence.proxy.async;" ::: "memory");
+            __syncwarp();
+        }
         if (elect_one()) {
             // ---- producer of V: a stage is free only after O += P_j V_j ------------------------------------
+            int v_row = PAGED && nt > 0 ? page_row(jp0 * 2) : 0;     // read a tile ahead
             for (int j = 0; j < nt; ++j) {
                 const int s = j % VS;
                 if (j >= VS && !mbar_wait(smem_u32(&bars->v_empty[s]), ((j / VS) - 1) & 1)) {
@@ -326,9 +369,11 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 const unsigned vfull = smem_u32(&bars->v_full[s]);
                 unsigned char* vdst = sV + s * V_BYTES;
                 mbar_expect_tx(vfull, V_BYTES);
-                const int y = row0 + ((jp0 + (j >> 1) * stride) * 2 + (j & 1)) * BN;
+                const int tile = (jp0 + (j >> 1) * stride) * 2 + (j & 1);
+                const int y = PAGED ? v_row : row0 + tile * BN;
                 for (int d = 0; d < HD / 64; ++d)
-                    tma_load_2d(smem_u32(vdst + d * (BN * 128)), &map_kv, vfull, vx + d * 64, y);
+                    tma_load_2d(smem_u32(vdst + d * (BN * 128)), &map_v, vfull, (PAGED ? 0 : vx) + d * 64, y);
+                if (PAGED && j + 1 < nt) v_row = page_row((jp0 + ((j + 1) >> 1) * stride) * 2 + ((j + 1) & 1));
             }
         }
     } else if (warp == 1) {
@@ -728,7 +773,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
             constexpr int RPI = 32 / CPR;                        // rows that one warp-wide store covers
             for (int rr = 0; rr < 32; rr += RPI) {
                 const int rl = quarter * 32 + rr + lane / CPR, pos = lane % CPR;
-                if (r0 + rl >= len) continue;
+                if (r0 + rl >= len || (PAGED && r0 + rl < q0)) continue;
                 const uint4 pk = *reinterpret_cast<const uint4*>(sOut + rl * (HD * 2) + (pos << 4));
                 bf16* dst = out + (size_t)(row0 + r0 + rl) * out_stride + (size_t)h * HD + ((pos ^ (rl & (CPR - 1))) << 3);
                 *reinterpret_cast<uint4*>(dst) = pk;
@@ -744,20 +789,26 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 
 
-template <int HD, bool FIXED>
-int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, long long out_stride, const int* seq_row0,
+struct Cache { const void *k_pool, *v_pool; long long rows; const int *table, *slots; int max_pages; };   // k_pool null: packed rows
+
+template <int HD, bool FIXED, bool PAGED>
+int launch_attn(const Cache& cache, const void* qkv, long long ld, long long total_rows, void* out, long long out_stride, const int* seq_row0,
                 const int* seq_len, const int* seq_q0, int q_tiles, int B, int max_len, int nq, int nkv, float scale, float cap,
                 int window, int* status, const float* slopes, const float* sinks, cudaStream_t st) {
     const long long width = ld;                    // the rows may be wider than what is read of them
-    CUtensorMap map_q, map_kv;
+    CUtensorMap map_q, map_k, map_v;
     int rc = make_map(&map_q, qkv, total_rows, width, BM);
     if (rc) return rc;
-    rc = make_map(&map_kv, qkv, total_rows, width, BN);
+    rc = PAGED ? make_map(&map_k, cache.k_pool, cache.rows, HD, BN) : 0;
     if (rc) return rc;
+    rc = PAGED ? make_map(&map_v, cache.v_pool, cache.rows, HD, BN) : make_map(&map_v, qkv, total_rows, width, BN);
+    if (rc) return rc;
+    if (!PAGED) map_k = map_v;
+    const Pages pages = {(bf16*)cache.v_pool, cache.table, cache.slots, cache.max_pages};
     constexpr size_t layout = (size_t)k_stages(HD) * 2 * BN * HD * 2 + (size_t)v_stages(HD) * BN * HD * 2 + 2 * P_BYTES + sizeof(Barriers);
     static_assert(layout <= 227 * 1024, "a block's shared memory");
     const size_t smem = layout + 1024 < 227 * 1024 ? layout + 1024 : 227 * 1024;           // with room to align it, where there is
-    auto kern = attn_prefill_tcgen05_kernel<HD, FIXED>;
+    auto kern = attn_prefill_tcgen05_kernel<HD, FIXED, PAGED>;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -825,9 +876,39 @@ int launch_attn(const void* qkv, long long ld, long long total_rows, void* out, 
     } else {
         cfg.numAttrs = pdl ? 1 : 0;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map_q, map_kv, (bf16*)out, (size_t)out_stride, seq_row0, seq_len, seq_q0, nq,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map_q, map_k, map_v, pages, (bf16*)out, (size_t)out_stride, seq_row0, seq_len, seq_q0, nq,
                                        nkv, scale, cap, window, status, split, slopes, sinks);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+template <bool PAGED>
+int prefill_tcgen05(const Cache& cache, const void* qkv, long long ld, long long total_rows, void* out, long long out_stride,
+                    const int* seq_row0, const int* seq_len, const int* seq_q0, int most_wanted, int B, int max_len, int nq, int nkv, int hd,
+                    float scale, float cap, int window, int* status, const float* slopes, const float* sinks, cudaStream_t st) {
+    if (B <= 0 || max_len <= 0) return 0;
+    if (hd != 64 && hd != 128 && hd != 256) return QNN_ERR_UNSUPPORTED;
+    if (nkv <= 0 || nq % nkv) return QNN_ERR_ARGUMENT;
+    if (B > 65535 || nq > 32767 || (max_len + BM - 1) / BM > 65535) return QNN_ERR_UNSUPPORTED;
+    if (ld < (long long)(nq + 2 * nkv) * hd) return QNN_ERR_ARGUMENT;
+    if ((ld & 7) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || (out_stride * 2) % 16) return QNN_ERR_UNSUPPORTED;
+    // the last most_wanted rows of a sequence may begin anywhere in a tile
+    const int q_tiles = seq_q0 != nullptr && most_wanted > 0 ? (int)(((long long)most_wanted + 2 * BM - 2) / BM) : 0;
+#define QNN_ATTN_ARGS cache, qkv, ld, total_rows, out, out_stride, seq_row0, seq_len, seq_q0, q_tiles, B, max_len, nq, nkv, scale, cap, window, status, slopes, sinks, st
+    // With a softcap up to 70 the exponent cap * log2(e) stays below 101, so that neither exp(score) nor a row's
+    // sum over a million keys leaves float32: the fixed-reference softmax with both groups of warps.  QNN_ATTN_FIXED=0
+    // keeps the running maximum (for comparisons).
+    static int fixed_ok = -1;
+    if (fixed_ok < 0) {
+        const char* e = getenv("QNN_ATTN_FIXED");
+        fixed_ok = (e && e[0] == '0') ? 0 : 1;
+    }
+    const bool fixed = fixed_ok && cap > 0.f && cap <= 70.f && slopes == nullptr;
+    switch (hd) {
+        case 64: return fixed ? launch_attn<64, true, PAGED>(QNN_ATTN_ARGS) : launch_attn<64, false, PAGED>(QNN_ATTN_ARGS);
+        case 128: return fixed ? launch_attn<128, true, PAGED>(QNN_ATTN_ARGS) : launch_attn<128, false, PAGED>(QNN_ATTN_ARGS);
+        default: return fixed ? launch_attn<256, true, PAGED>(QNN_ATTN_ARGS) : launch_attn<256, false, PAGED>(QNN_ATTN_ARGS);
+    }
+#undef QNN_ATTN_ARGS
 }
 
 }  // namespace
@@ -845,28 +926,24 @@ QNN_API int qnn_attn_prefill_tcgen05(const void* qkv, long long ld, long long to
                                      const int* seq_row0, const int* seq_len, const int* seq_q0, int most_wanted, int B, int max_len,
                                      int nq, int nkv, int hd, float scale, float cap, int window, int* status,
                                      const float* slopes, const float* sinks, cudaStream_t st) {
-    if (B <= 0 || max_len <= 0) return 0;
-    if (hd != 64 && hd != 128 && hd != 256) return QNN_ERR_UNSUPPORTED;
-    if (nkv <= 0 || nq % nkv) return QNN_ERR_ARGUMENT;
-    if (B > 65535 || nq > 32767 || (max_len + BM - 1) / BM > 65535) return QNN_ERR_UNSUPPORTED;
-    if (ld < (long long)(nq + 2 * nkv) * hd) return QNN_ERR_ARGUMENT;
-    if ((ld & 7) || ((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || (out_stride * 2) % 16) return QNN_ERR_UNSUPPORTED;
-    // the last most_wanted rows of a sequence may begin anywhere in a tile
-    const int q_tiles = seq_q0 != nullptr && most_wanted > 0 ? (int)(((long long)most_wanted + 2 * BM - 2) / BM) : 0;
-#define QNN_ATTN_ARGS qkv, ld, total_rows, out, out_stride, seq_row0, seq_len, seq_q0, q_tiles, B, max_len, nq, nkv, scale, cap, window, status, slopes, sinks, st
-    // With a softcap up to 70 the exponent cap * log2(e) stays below 101, so that neither exp(score) nor a row's
-    // sum over a million keys leaves float32: the fixed-reference softmax with both groups of warps.  QNN_ATTN_FIXED=0
-    // keeps the running maximum (for comparisons).
-    static int fixed_ok = -1;
-    if (fixed_ok < 0) {
-        const char* e = getenv("QNN_ATTN_FIXED");
-        fixed_ok = (e && e[0] == '0') ? 0 : 1;
-    }
-    const bool fixed = fixed_ok && cap > 0.f && cap <= 70.f && slopes == nullptr;
-    switch (hd) {
-        case 64: return fixed ? launch_attn<64, true>(QNN_ATTN_ARGS) : launch_attn<64, false>(QNN_ATTN_ARGS);
-        case 128: return fixed ? launch_attn<128, true>(QNN_ATTN_ARGS) : launch_attn<128, false>(QNN_ATTN_ARGS);
-        default: return fixed ? launch_attn<256, true>(QNN_ATTN_ARGS) : launch_attn<256, false>(QNN_ATTN_ARGS);
-    }
-#undef QNN_ATTN_ARGS
+    return prefill_tcgen05<false>(Cache{}, qkv, ld, total_rows, out, out_stride, seq_row0, seq_len, seq_q0, most_wanted, B, max_len, nq, nkv, hd, scale, cap, window, status, slopes, sinks, st);
+}
+
+// Attention of a step that continues sequences, over the paged cache, which holds every key and value by now, this step's included
+// (no ring that has wrapped): sequence b's new rows are rows seq_row0[b] .. of qkv and of out, at positions start[b] .. length[b] - 1; no
+// sequence brings more than most_new of them, none is longer than `longest`.  Pools: [pool_pages, nkv, 64, hd]; page_table: [slots, max_pages].
+// The value cells behind a sequence in its last page are cleared.  What it saves is the copy of whole sequences out of the pages into
+// packed rows and of the wanted rows out of the result.
+QNN_API int qnn_attn_extend_tcgen05(const void* qkv, long long ld, long long total_rows, void* out, long long out_stride, const int* seq_row0,
+                                    const int* length, const int* start, int most_new, int B, int longest, int nq, int nkv, int hd,
+                                    float scale, float cap, int window, int* status, const float* slopes, const float* sinks,
+                                    const void* k_pool, const void* v_pool, long long pool_pages, const int* page_table, int max_pages,
+                                    const int* slots, cudaStream_t st) {
+    if (start == nullptr || k_pool == nullptr || v_pool == nullptr || page_table == nullptr || slots == nullptr || most_new <= 0)
+        return QNN_ERR_ARGUMENT;
+    const long long rows = pool_pages * nkv * BN;
+    if (rows <= 0 || rows > 0x7fffffffLL || (((uintptr_t)k_pool | (uintptr_t)v_pool) & 15) != 0) return QNN_ERR_UNSUPPORTED;
+    const Cache cache = {k_pool, v_pool, rows, page_table, slots, max_pages};
+    return prefill_tcgen05<true>(cache, qkv, ld, total_rows, out, out_stride, seq_row0, length, start, most_new, B, longest, nq, nkv, hd, scale,
+                                 cap, window, status, slopes, sinks, st);
 }

@@ -595,6 +595,7 @@ ATTN_TCGEN05 = os.environ.get("QNN_ATTN", "tcgen05") != "mma"
 # generic kernel (a warp per row and kv head that walks the keys one after the other), 512 rows on 7000: 152 us against
 # 8477; so always, where the sizes allow.
 EXTEND_TENSOR_CORE_FROM = int(os.environ.get("QNN_EXTEND_TC_FROM", "1"))
+EXTEND_PAGED = os.environ.get("QNN_EXTEND_PAGED", "1") != "0"       # 0: such steps go through packed copies of the sequences
 
 
 def attention_refusal(dtype: torch.dtype, n_heads: int, n_kv: int, head_dim: int) -> Optional[str]:
@@ -778,6 +779,34 @@ def attn_extend(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, k_poo
         _p(k_pool), _p(v_pool), _p(page_table), page_table.shape[1], page_size, ring, _p(out), out.shape[1],
         _p(tok_pos), _p(tok_row0), _p(tok_slot), T, n_heads, n_kv, head_dim, float(scale), float(cap or 0.0),
         int(window or 0), _p(slopes), _p(sinks), _stream()), "attn_extend")
+    return out
+
+
+def extends_in_pages(qkv: torch.Tensor, head_dim: int, line, whole) -> bool:
+    """Whether attn_extend_paged takes a step that continues sequences: many bfloat16 rows, and a cache line that holds every position
+    (no ring, or none that has wrapped) in pages of 64."""
+    return (whole is not None and ATTN_TCGEN05 and EXTEND_PAGED and qkv.dtype == torch.bfloat16 and head_dim in (64, 128, 256)
+            and whole.most_new >= EXTEND_TENSOR_CORE_FROM and line.writes and line.has_values and line.k.dtype == torch.bfloat16
+            and line.page_size == 64 and (not line.ring or whole.longest <= line.ring))
+
+
+def attn_extend_paged(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, line, scale: float, cap: Optional[float],
+                      window: Optional[int], whole, slopes: Optional[torch.Tensor] = None, sinks: Optional[torch.Tensor] = None):
+    """``attn_extend`` where this step's keys and values are in the cache line already (and ``extends_in_pages`` holds): the
+    tensor-core prompt kernel reads the pages themselves."""
+    ld = _rows(qkv, "qkv", torch.bfloat16)
+    _check_per_head(slopes, sinks, n_heads)
+    for n, t in (("k_pool", line.k), ("v_pool", line.v)):
+        _req(t, n, torch.bfloat16, 4)
+        if tuple(t.shape[1:]) != (n_kv, 64, head_dim):
+            raise ValueError(f"{n} has shape {tuple(t.shape)}, expected [pages, {n_kv}, 64, {head_dim}]")
+    _req(line.page_table, "page_table", torch.int32, 2)
+    out = torch.empty((qkv.shape[0], n_heads * head_dim), dtype=qkv.dtype, device=qkv.device)
+    _lib.check(_lib.load().qnn_attn_extend_tcgen05(
+        _p(qkv), ld, qkv.shape[0], _p(out), out.shape[1], _p(whole.new_row0), _p(whole.length), _p(whole.start), whole.most_new,
+        whole.row0.numel(), whole.longest, n_heads, n_kv, head_dim, float(scale), float(cap or 0.0), int(window or 0),
+        _p(_status_word(qkv.device)), _p(slopes), _p(sinks), _p(line.k), _p(line.v), line.k.shape[0], _p(line.page_table),
+        line.page_table.shape[1], _p(whole.slots), _stream()), "attn_extend_tcgen05")
     return out
 
 

@@ -284,10 +284,15 @@ class AttentionMixer(Mixer):
                 qkv, gate_col = project(x, self.w_qkvg), self.w_qkv.shape[0]
             else:
                 qkv = project(x, self.w_qkv)
+            paged = extend and self._reads_pages(qkv, step, line)
             if self.prep is None:
-                self.position.place(qkv, h, step, line, append=not extend)
+                self.position.place(qkv, h, step, line, append=not extend or paged)
             else:
-                self.position.place(qkv, h, step, line, append=not extend, prep=self.prep)
+                self.position.place(qkv, h, step, line, append=not extend or paged, prep=self.prep)
+            if paged:
+                a = ops.attn_extend_paged(qkv, h.n_heads, h.n_kv_heads, h.head_dim, line, self.scale, self.softcap, self.window,
+                                          step.whole, slopes=self.slopes, sinks=self.sinks)
+                return ops.sigmoid_gate_(a, project(x, self.w_out_gate)) if self.out_gate else a
         if line.has_readers and line.writes and not self.shared_kv and step.mode != "decode":
             step.shared_rows[line.index] = (qkv, h)          # for the layers that read this line later in the step
         a = self.attend(qkv, step, line)
@@ -315,6 +320,11 @@ class AttentionMixer(Mixer):
                                    self.window, whole=getattr(step, "whole", None), slopes=self.slopes, sinks=self.sinks)
         return ops.attn_prefill(packed, self.n_heads, nkv, D, step.tok_pos, step.tok_row0, self.scale, self.softcap,
                                 self.window, step.seq_row0, step.seq_len, step.max_q_len, slopes=self.slopes, sinks=self.sinks)
+
+    def _reads_pages(self, qkv: torch.Tensor, step, line) -> bool:
+        """Whether a step that continues sequences appends its keys and values first and then attends over the pages: not in a ring
+        that the new rows would overwrite, nor where other layers still have to read the line as earlier steps left it."""
+        return not self.shared_kv and not line.has_readers and ops.extends_in_pages(qkv, self.head_dim, line, getattr(step, "whole", None))
 
     def attend(self, qkv: torch.Tensor, step, line) -> torch.Tensor:
         """Attention of the packed q|k|v rows of a step, by the step's mode.  In prefill and decode the keys and
