@@ -1,0 +1,64 @@
+"""Gates per head and router logits of a prompt's many rows (tensor cores, 8 rows a block) beside those of few rows: both as far from
+64 bits as float32 sums are, whatever the width, the outputs and the rows left over."""
+import pytest
+import torch
+
+from quicknn_b200.kernels import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+MANY = 256
+
+
+def off(a, want):
+    return ((a.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("T", [MANY, MANY + 1, MANY + 7, 700])
+@pytest.mark.parametrize("W,E,extra", [(8, 2, 0), (40, 16, 1), (264, 17, 0), (1536, 31, 1), (2304, 16, 0), (2304, 32, 0)])
+@pytest.mark.parametrize("score", ["sigmoid", "softmax"])
+def test_route(T, W, E, extra, score):
+    torch.manual_seed(T + W + E)
+    x, w = torch.randn((T, W), device=DEV).bfloat16(), (torch.randn((E + extra, W), device=DEV) * 2 * W ** -0.5).bfloat16()
+    z = x.double() @ w.double().T
+    s = torch.sigmoid(z[:, :E]) if score == "sigmoid" else z[:, :E].softmax(-1)
+    top = min(2, E)
+    res = ops.moe_route(x, w, top, score, False, **({"extra": extra} if extra else {}))
+    sel_e, sel_w = res[0].view(T, top).long(), res[1].view(T, top)
+    assert (sel_e >= 0).all() and (sel_e < E).all() and (sel_e.sort(-1).values.diff(dim=-1) > 0).all()
+    want = s.gather(1, sel_e)
+    best = s.topk(top, -1).values
+    assert off(sel_w, want) < 1e-6 and ((best - want).abs() <= 1e-6 * best.abs() + 1e-7).all()         # the best, ties by rounding aside
+    if extra:
+        assert off(res[2], z[:, E:]) < 1e-6
+    few = [ops.moe_route(x[lo:lo + 100].contiguous(), w, top, score, False, **({"extra": extra} if extra else {})) for lo in range(0, T, 100)]
+    same = torch.cat([f[0] for f in few]).view(T, top).long() == sel_e
+    assert same.float().mean().item() > 0.999
+
+
+@pytest.mark.parametrize("T", [MANY, MANY + 1, 700])
+@pytest.mark.parametrize("W,H,D", [(8, 1, 8), (264, 9, 256), (1536, 12, 64), (2304, 16, 8), (2304, 17, 128), (2304, 32, 16)])
+@pytest.mark.parametrize("dt", ["bfloat16", "float32"])
+def test_gate_heads(T, W, H, D, dt):
+    torch.manual_seed(T + W + H)
+    x, w = torch.randn((T, W), device=DEV).bfloat16(), (torch.randn((H, W), device=DEV) * W ** -0.5).bfloat16()
+    o = torch.randn((T, H * D), device=DEV).to(getattr(torch, dt))
+    want = (o.double().view(T, H, D) * torch.sigmoid(x.double() @ w.double().T)[:, :, None]).view(T, -1)
+    few = torch.cat([ops.gate_heads(o[lo:lo + 100].clone(), x[lo:lo + 100].contiguous(), w, H) for lo in range(0, T, 100)])
+    got = ops.gate_heads(o.clone(), x, w, H)
+    if dt == "float32":
+        assert off(got, want) < 2e-7 and off(got, want) < 1.1 * off(few, want) + 1e-8
+    else:
+        assert off(got, want) < 2.0 ** -8
+
+
+def test_values_that_are_not_finite_stay_in_their_row():
+    T, W, H, D = 300, 264, 9, 16
+    torch.manual_seed(1)
+    x, w = torch.randn((T, W), device=DEV).bfloat16(), torch.randn((H, W), device=DEV).bfloat16()
+    o = torch.randn((T, H * D), device=DEV)
+    clean = ops.gate_heads(o.clone(), x, w, H)
+    x[17, 3], x[42, 100] = float("nan"), float("inf")
+    got = ops.gate_heads(o.clone(), x, w, H)
+    others = torch.tensor([t not in (17, 42) for t in range(T)], device=DEV)
+    assert torch.equal(got[others], clean[others]) and got[17].isnan().all()
