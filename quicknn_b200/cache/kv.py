@@ -140,6 +140,8 @@ class KVCache:
 
         self.state = regions(states)
         self.block_state = regions(block_states)
+        # a slot's part of every state, made when the slot is first used: one call clears a new sequence's
+        self._slot_states: List[Optional[List[torch.Tensor]]] = [None] * max_slots
 
     def _all_states(self) -> List[torch.Tensor]:
         return list(self.state.values()) + list(self.block_state.values())
@@ -150,8 +152,11 @@ class KVCache:
         self.lengths_host[slot] = 0
         self.longest_host[slot] = 0
         self._lengths_dirty = True
-        for t in self._all_states():
-            t[slot].zero_()
+        if self.state or self.block_state:
+            parts = self._slot_states[slot]
+            if parts is None:
+                parts = self._slot_states[slot] = [t[slot] for t in self._all_states()]
+            torch._foreach_zero_(parts)
         return slot
 
     def free(self, slot: int) -> None:

@@ -38,7 +38,9 @@ class PagePool:
     def take(self, n: int) -> List[int]:
         if n > len(self._free):
             raise CacheFull(f"{n} pages wanted, {len(self._free)} free of {self.n_pages - 1}")
-        out = [self._free.pop() for _ in range(n)]
+        keep = len(self._free) - n
+        out = self._free[keep:][::-1]
+        del self._free[keep:]
         for p in out:
             self._held[p] = True
         return out
