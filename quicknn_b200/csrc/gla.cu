@@ -244,8 +244,9 @@ __global__ void gla_segment_prefix_kernel(float* __restrict__ scratch, const flo
 // a warp per (row, head).  o: float32 rows of H heads, `hs` columns apart, of which the first vdim are normed; with `den`
 // (float32 [rows, ldden], one per head) a head is first divided by max(|o[vdim]|, den) + 1e-6, o[vdim] being the
 // normaliser's product with the query.  w_mode: 0 no weight, 1 a weight per column of a head (shared by the heads),
-// 2 a weight per column of the row.  gate_act: 0 silu, 1 sigmoid.
-template <typename T>
+// 2 a weight per column of the row.  gate_act: 0 silu, 1 sigmoid.  N: a lane's columns at most; all of a head's loads are in flight at once
+// (read where they are needed, the gate and the head's second reading came behind the sum).
+template <typename T, int N>
 __global__ void head_norm_gate_kernel(const float* __restrict__ o, long long ldo, int hs, const float* __restrict__ den,
                                       long long ldden, const void* __restrict__ w, int w_dt, int w_mode, float eps,
                                       const T* __restrict__ g, long long ldg, int gate_act, T* __restrict__ out,
@@ -255,20 +256,30 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, long long ldo
     if (unit >= rows * H) return;
     const int t = unit / H, h = unit - t * H;
     const float* orow = o + (size_t)t * ldo + (size_t)h * hs;
+    float v[N], gv[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int j = lane + 32 * i;
+        v[i] = j < vdim ? orow[j] : 0.f;
+        gv[i] = j < vdim && gate_act != 2 ? to_f(g[(size_t)t * ldg + h * vdim + j]) : 0.f;
+    }
     float scale = 1.f;
     if (den != nullptr) scale = 1.f / (fmaxf(fabsf(orow[vdim]), den[(size_t)t * ldden + h]) + 1e-6f);
     float ss = 0.f;
-    for (int j = lane; j < vdim; j += 32) {
-        const float v = orow[j] * scale;
-        ss += v * v;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        v[i] *= scale;
+        ss += v[i] * v[i];
     }
     ss = warp_sum(ss);
     const float inv = rsqrtf(ss / (float)vdim + eps);
-    for (int j = lane; j < vdim; j += 32) {
-        const float gv = gate_act == 2 ? 0.f : to_f(g[(size_t)t * ldg + h * vdim + j]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const int j = lane + 32 * i;
+        if (j >= vdim) break;
         const float wv = w_mode == 0 ? 1.f : load_as_f(w, w_dt, w_mode == 2 ? (size_t)h * vdim + j : (size_t)j);
-        const float ga = gate_act == 2 ? 1.f : (gate_act == 1 ? 1.f / (1.f + expf(-gv)) : silu(gv));
-        out[(size_t)t * ld_out + h * vdim + j] = from_f<T>(orow[j] * scale * inv * wv * ga);
+        const float ga = gate_act == 2 ? 1.f : (gate_act == 1 ? 1.f / (1.f + expf(-gv[i])) : silu(gv[i]));
+        out[(size_t)t * ld_out + h * vdim + j] = from_f<T>(v[i] * inv * wv * ga);
     }
 }
 
@@ -614,12 +625,18 @@ QNN_API int qnn_head_norm_gate(const float* o, long long ldo, int hs, const floa
     }
     const int warps = 4;
     const dim3 grid(((size_t)rows * H + warps - 1) / warps);
-    if (dtype == QNN_DT_BF16)
-        launch_pdl(head_norm_gate_kernel<bf16>, grid, dim3(warps * 32), 0, st, o, ldo, hs, den, ldden, w, w_dt, w_mode, eps,
-                   (const bf16*)g, ldg, gate_act, (bf16*)out, ld_out, rows, H, vdim);
-    else
-        launch_pdl(head_norm_gate_kernel<float>, grid, dim3(warps * 32), 0, st, o, ldo, hs, den, ldden, w, w_dt, w_mode, eps,
-                   (const float*)g, ldg, gate_act, (float*)out, ld_out, rows, H, vdim);
+#define QNN_HNG(T, N)                                                                                                             \
+    launch_pdl(head_norm_gate_kernel<T, N>, grid, dim3(warps * 32), 0, st, o, ldo, hs, den, ldden, w, w_dt, w_mode, eps, (const T*)g, ldg, \
+               gate_act, (T*)out, ld_out, rows, H, vdim)
+#define QNN_HNG_T(T)                                                                                                              \
+    if (vdim <= 128) QNN_HNG(T, 4);                                                                                               \
+    else if (vdim <= 256) QNN_HNG(T, 8);                                                                                          \
+    else QNN_HNG(T, 16)
+    if (vdim > 512) return QNN_ERR_UNSUPPORTED;
+    if (dtype == QNN_DT_BF16) { QNN_HNG_T(bf16); }
+    else { QNN_HNG_T(float); }
+#undef QNN_HNG_T
+#undef QNN_HNG
     QNN_LAUNCH_CHECK();
 }
 

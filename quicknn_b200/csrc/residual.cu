@@ -228,6 +228,61 @@ small_linear_thread_kernel(const TX* __restrict__ x, const TW* __restrict__ w, f
     out[(size_t)(t0 + r) * N + n0 + c] = finish(d, bias, bias_dt, inv_tau, n0 + c);
 }
 
+// Both on the tensor cores, for bfloat16 rows and weights and many rows (sums as in row_dots).  Long rows and up to 32 outputs: 8 rows a
+// block.  Short rows: a block does 64 rows of 64 outputs, a warp 16 outputs of 32 rows.  us, the forms above / now: 2809 rows of 1536, 24
+// outputs 22.3 / 6.2, 640 rows 6.8 / 5.3, 256 rows 4.5 / 5.2; 2048 rows of 64, 1152 outputs with a decay 33.4 / 12.3, 640 rows 14.8 / 6.7.
+constexpr int SL_DOTS_FROM = 512, SL_TILE = 64;
+template <int MT>
+__global__ void __launch_bounds__(256)
+small_linear_dots_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, float* __restrict__ out, int T, int N, int K,
+                         const void* __restrict__ bias, int bias_dt, float inv_tau) {
+    __shared__ __align__(16) double part[8 * MT * 16 * DOT_ROWS];
+    __shared__ float dots[DOT_ROWS][MT * 16];
+    pdl_wait();
+    const int t0 = blockIdx.x * DOT_ROWS, rows = min(DOT_ROWS, T - t0);
+    row_dots<MT>(x + (size_t)t0 * K, K, rows, w, N, K, 8, part, &dots[0][0], MT * 16);
+    for (int i = threadIdx.x; i < rows * N; i += blockDim.x) {
+        const int r = i / N, n = i - r * N;
+        out[(size_t)t0 * N + i] = finish(dots[r][n], bias, bias_dt, inv_tau, n);
+    }
+}
+__global__ void __launch_bounds__(256)
+small_linear_short_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, float* __restrict__ out, int T, int N, int K,
+                          const void* __restrict__ bias, int bias_dt, float inv_tau) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int n0 = blockIdx.x * SL_TILE + (warp & 3) * 16 + g, t0 = blockIdx.y * SL_TILE + (warp >> 2) * 32;
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    double acc[4][4];
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][e] = 0.0;
+    pdl_wait();
+    for (int k = q * 8; k - q * 8 < K; k += 32) {
+        const bool in = k < K;
+        const uint4 lo = in && n0 < N ? *reinterpret_cast<const uint4*>(w + (size_t)n0 * K + k) : none;
+        const uint4 hi = in && n0 + 8 < N ? *reinterpret_cast<const uint4*>(w + (size_t)(n0 + 8) * K + k) : none;
+        const uint32_t first[4] = {lo.x, hi.x, lo.y, hi.y}, second[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int t = t0 + m * 8 + g;
+            const uint4 b = in && t < T ? *reinterpret_cast<const uint4*>(x + (size_t)t * K + k) : none;
+            float f[4], s[4];
+            mma_first(f, first, b.x, b.y);
+            mma_first(s, second, b.z, b.w);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[m][e] += (double)f[e] + (double)s[e];
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int t = t0 + m * 8 + 2 * q + (e & 1), n = n0 + (e >> 1) * 8;
+            if (t < T && n < N) out[(size_t)t * N + n] = finish((float)acc[m][e], bias, bias_dt, inv_tau, n);
+        }
+}
+
 // out[t, h, :] = o[t, h, :] * scale * sigmoid(x[t, :] . w[h, :]) (out may be o; without w: sigmoid(x[t, h])): the gate per head formed (float32) and
 // applied in one kernel; a block per row, the warps share the heads.  A lane's terms and the order of their sum depend on
 // the width only.
@@ -280,8 +335,8 @@ __global__ void gate_heads_kernel(const TX* __restrict__ x, long long ldx, const
 }
 
 // The same for the many rows of a prompt, 8 per block, the logits on the tensor cores (see row_dots).  us, a block per row / now: 2048 rows of
-// 2304, 9 heads of 128 12.7 / 6.5, 512 rows 6.0 / 5.9, 4096 rows 21.5 / 9.6.
-constexpr int GATE_FROM = 256, GATE_WARPS = 8;
+// 2304, 9 heads of 128 12.8 / 7.2, 1024 rows 7.6 / 6.1, 512 rows 6.0 / 6.4.
+constexpr int GATE_FROM = 1024, GATE_WARPS = 8;
 template <int MT>
 __global__ void __launch_bounds__(GATE_WARPS * 32)
 gate_heads_rows_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w, int W, const void* o, int o_dt, void* out,
@@ -367,6 +422,18 @@ QNN_API int qnn_small_linear_f32(const void* x, int x_dt, const void* w, int w_d
     const float inv_tau = bias != nullptr ? 1.f / tau : 0.f;
     const size_t total = (size_t)T * N;
     const bool many = (long long)((T + SL_ROWS - 1) / SL_ROWS) * ((N + SL_OUTS - 1) / SL_OUTS) > SL_MANY_BLOCKS;
+    if (x_dt == QNN_DT_BF16 && w_dt == QNN_DT_BF16 && K % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
+        if (T >= SL_DOTS_FROM && K > SL_MAXK && N <= 32) {
+            launch_pdl(N <= 16 ? small_linear_dots_kernel<1> : small_linear_dots_kernel<2>, dim3((T + DOT_ROWS - 1) / DOT_ROWS), dim3(256), 0, st,
+                       (const bf16*)x, (const bf16*)w, out, T, N, K, bias, bias_dt, inv_tau);
+            QNN_LAUNCH_CHECK();
+        }
+        if (T >= 256 && K <= SL_MAXK && many && (T + SL_TILE - 1) / SL_TILE <= 65535) {
+            launch_pdl(small_linear_short_kernel, dim3((N + SL_TILE - 1) / SL_TILE, (T + SL_TILE - 1) / SL_TILE), dim3(256), 0, st,
+                       (const bf16*)x, (const bf16*)w, out, T, N, K, bias, bias_dt, inv_tau);
+            QNN_LAUNCH_CHECK();
+        }
+    }
 #define QNN_SL(TX, TW)                                                                                               \
     if (K > SL_MAXK)                                                                                                 \
         launch_pdl(small_linear_warp_kernel<TX, TW>, dim3((unsigned)((total + 7) / 8)), dim3(256), 0, st,            \

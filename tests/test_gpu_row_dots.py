@@ -36,7 +36,7 @@ def test_route(T, W, E, extra, score):
     assert same.float().mean().item() > 0.999
 
 
-@pytest.mark.parametrize("T", [MANY, MANY + 1, 700])
+@pytest.mark.parametrize("T", [1024, 1025, 1500])
 @pytest.mark.parametrize("W,H,D", [(8, 1, 8), (264, 9, 256), (1536, 12, 64), (2304, 16, 8), (2304, 17, 128), (2304, 32, 16)])
 @pytest.mark.parametrize("dt", ["bfloat16", "float32"])
 def test_gate_heads(T, W, H, D, dt):
@@ -53,7 +53,7 @@ def test_gate_heads(T, W, H, D, dt):
 
 
 def test_values_that_are_not_finite_stay_in_their_row():
-    T, W, H, D = 300, 264, 9, 16
+    T, W, H, D = 1030, 264, 9, 16
     torch.manual_seed(1)
     x, w = torch.randn((T, W), device=DEV).bfloat16(), torch.randn((H, W), device=DEV).bfloat16()
     o = torch.randn((T, H * D), device=DEV)
@@ -62,3 +62,19 @@ def test_values_that_are_not_finite_stay_in_their_row():
     got = ops.gate_heads(o.clone(), x, w, H)
     others = torch.tensor([t not in (17, 42) for t in range(T)], device=DEV)
     assert torch.equal(got[others], clean[others]) and got[17].isnan().all()
+
+
+@pytest.mark.parametrize("T", [MANY, MANY + 1, 700])
+@pytest.mark.parametrize("K,N", [(136, 1), (1536, 24), (2304, 32), (264, 17), (8, 700), (64, 1152), (72, 577), (128, 640)])
+@pytest.mark.parametrize("decay", [False, True])
+def test_small_linear(T, K, N, decay):
+    """Long rows with few outputs, short rows with many."""
+    torch.manual_seed(T + K + N)
+    x, w = torch.randn((T, K), device=DEV).bfloat16(), (torch.randn((N, K), device=DEV) * K ** -0.5).bfloat16()
+    bias = torch.randn(N, device=DEV)
+    kw = dict(decay_bias=bias, tau=8.0) if decay else {}
+    z = x.double() @ w.double().T
+    want = torch.sigmoid(z + bias.double()) ** 0.125 if decay else z
+    got = ops.small_linear_f32(x, w, **kw)
+    few = torch.cat([ops.small_linear_f32(x[lo:lo + 100].contiguous(), w, **kw) for lo in range(0, T, 100)])
+    assert off(got, want) < 2e-7 and off(got, want) < 1.1 * off(few, want) + 1e-8
