@@ -50,56 +50,6 @@ __device__ __forceinline__ void split_tiles(const float (&x)[4], const float (&y
     split(y[0], y[1], s.h[2], s.m[2], s.l[2]);
     split(y[2], y[3], s.h[3], s.m[3], s.l[3]);
 }
-// Products of 8 bfloat16 rows with up to MT * 16 rows of weights, for the few outputs per row that feed float32 math (gates, router
-// logits): dots[row][output], from all warps of the block (`warps` of them share the width in pieces of 32; `part` is scratch for
-// warps * MT * 128 doubles).  x: `rows` (1 to 8) of them, ldx apart; w: n rows of `width`; both on 16 bytes, width a multiple of 8.  A dot
-// product per warp, row and output on the FMA pipe costs a load and an unpacking of both factors per product of eight, most of its
-// time; here a warp's instruction does 16 outputs of 8 rows.  Every piece's sums of 16 start from zero and are added in float64 (a few
-// additions per output), so that neither the tensor cores' cutting of an accumulator's last bits nor the additions' rounding adds
-// up: no further from 64 bits than float32 sums (measured).  The order of sums depends on the width and the warps only.
-constexpr int DOT_ROWS = 8;
-template <int MT>
-__device__ __forceinline__ void row_dots(const bf16* x, long long ldx, int rows, const bf16* w, int n, int width, int warps, double* part,
-                                         float* dots, int ldd) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    double acc[MT][4];
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[m][e] = 0.0;
-    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll 3
-    for (int k0 = warp * 32; k0 < width; k0 += warps * 32) {
-        const int k = k0 + t * 8;
-        const bool in = k < width;
-        const uint4 b = in && g < rows ? *reinterpret_cast<const uint4*>(x + (size_t)g * ldx + k) : none;
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            const int r = m * 16 + g;
-            const uint4 lo = in && r < n ? __ldg(reinterpret_cast<const uint4*>(w + (size_t)r * width + k)) : none;
-            const uint4 hi = in && r + 8 < n ? __ldg(reinterpret_cast<const uint4*>(w + (size_t)(r + 8) * width + k)) : none;
-            const uint32_t first[4] = {lo.x, hi.x, lo.y, hi.y}, second[4] = {lo.z, hi.z, lo.w, hi.w};
-            float f[4], s[4];
-            mma_first(f, first, b.x, b.y);
-            mma_first(s, second, b.z, b.w);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[m][e] += (double)f[e] + (double)s[e];
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < MT; ++m) {                               // [warp][output][row]
-        double* at = part + ((size_t)warp * MT * 16 + m * 16 + g) * DOT_ROWS + 2 * t;
-        *reinterpret_cast<double2*>(at) = make_double2(acc[m][0], acc[m][1]);
-        *reinterpret_cast<double2*>(at + 8 * DOT_ROWS) = make_double2(acc[m][2], acc[m][3]);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < MT * 16 * DOT_ROWS; i += blockDim.x) {
-        double d = 0.0;
-        for (int u = 0; u < warps; ++u) d += part[u * MT * 16 * DOT_ROWS + i];
-        if (i / DOT_ROWS < n) dots[(i % DOT_ROWS) * ldd + i / DOT_ROWS] = (float)d;
-    }
-    __syncthreads();
-}
 __device__ __forceinline__ void cp16(unsigned dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }

@@ -18,6 +18,7 @@
 // time through shared memory.  Sums run over the inner size in a fixed order, so a row's result does not depend on
 // which other rows share its tile.
 #include "mma_split.cuh"
+#include "row_dots.cuh"
 
 using namespace qnn;
 
@@ -177,20 +178,19 @@ __global__ void moe_route_kernel(const TX* __restrict__ x, const TW* __restrict_
     choose_experts(t, s, E, top, score_fn, renorm, correction, out_scale, sel_e, sel_w, n_groups, keep_groups);
 }
 
-// The same for the many rows of a prompt: 8 rows per block, their logits on the tensor cores (see row_dots), then a warp per row.
-// us, a block per row / now: 2048 rows of 2304, 16 experts 18.2 / 6.1, 256 rows 6.4 / 5.0, 4096 rows 29.9 / 10.8.
+// The same, bit for bit, for the many rows of a prompt: 8 rows per block (see row_dots), then a warp per row.  us, a block per row / now:
+// 16 experts of rows of 2304, 256 rows 6.4 / 6.3, 512 rows 7.5 / 6.4, 2048 rows 18.1 / 9.2, 4096 rows 29.9 / 17.1; 32 experts of 1536, 256 rows
+// 7.9 / 7.7, 2048 rows 22.2 / 11.3; below 256 rows a block per row is as fast.  Bound by the issue of loads, unpacking and products.
 constexpr int ROUTE_FROM = 256;
-template <int MT>
 __global__ void __launch_bounds__(DOT_ROWS * 32)
 moe_route_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wr, int T, int W, int E, int top, int score_fn, int renorm,
                       const float* __restrict__ correction, float out_scale, int* __restrict__ sel_e, float* __restrict__ sel_w,
                       int extra, float* __restrict__ extra_out, int n_groups, int keep_groups) {
-    __shared__ __align__(16) double part[DOT_ROWS * MT * 16 * DOT_ROWS];
     extern __shared__ float sc[];                       // per row: [E + extra] logits, [E] ranking values, [groups]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, per_row = 2 * E + extra + n_groups;
     pdl_wait();
     const int t0 = blockIdx.x * DOT_ROWS, rows = min(DOT_ROWS, T - t0), t = t0 + warp;
-    row_dots<MT>(x + (size_t)t0 * W, W, rows, wr, E + extra, W, DOT_ROWS, part, sc, per_row);
+    row_dots(x + (size_t)t0 * W, W, rows, wr, E + extra, W, sc, per_row);
     if (warp >= rows) return;
     float* s = sc + (size_t)warp * per_row;
     for (int j = lane; j < extra; j += 32) extra_out[(size_t)t * extra + j] = s[E + j];
@@ -696,8 +696,7 @@ QNN_API int qnn_moe_route(const void* x, int x_dt, const void* w_router, int w_d
     const size_t smem_rows = (size_t)DOT_ROWS * (2 * E + extra + n_groups) * sizeof(float);
     if (T >= ROUTE_FROM && x_dt == QNN_DT_BF16 && w_dt == QNN_DT_BF16 && E + extra <= 32 && W % 8 == 0 && smem_rows <= 24 * 1024 &&
         (((uintptr_t)x | (uintptr_t)w_router) & 15) == 0) {
-        launch_pdl(E + extra <= 16 ? moe_route_rows_kernel<1> : moe_route_rows_kernel<2>, dim3((T + DOT_ROWS - 1) / DOT_ROWS),
-                   dim3(DOT_ROWS * 32), smem_rows, st, (const bf16*)x, (const bf16*)w_router, T, W, E, top, score_fn, renorm, correction,
+        launch_pdl(moe_route_rows_kernel, dim3((T + DOT_ROWS - 1) / DOT_ROWS), dim3(DOT_ROWS * 32), smem_rows, st, (const bf16*)x, (const bf16*)w_router, T, W, E, top, score_fn, renorm, correction,
                    out_scale, sel_e, sel_w, extra, extra_out, n_groups, keep_groups);
         QNN_LAUNCH_CHECK();
     }

@@ -10,7 +10,7 @@
 //   qnn_gate_heads           the same with the gate's logits x . w_h formed in the kernel
 //   qnn_small_linear_f32     x w^T with float32 sums and float32 results, for the few outputs that feed
 //                            float32 math (gates, decay logits)
-#include "mma_split.cuh"
+#include "row_dots.cuh"
 #include "rows.cuh"
 
 using namespace qnn;
@@ -162,47 +162,63 @@ __global__ void small_linear_warp_kernel(const TX* __restrict__ x, const TW* __r
 // Short rows: a thread per output; a block owns 8 rows x 32 outputs and reads their inner elements through shared
 // memory (the weight rows of neighbouring outputs lie K elements apart: read directly, every load of a warp
 // would touch 32 lines).
-// With many rows a block owns 32 of them and a thread four: a weight's element then serves four sums and a row's elements come four
-// at a time (one row per thread reads shared memory twice for every product).  The order of a sum is the same.  A block then takes about
-// three times as long, so that it pays from where the blocks of 8 rows are more than four per SM (measured, 8 / 32 rows a block, us:
-// 576 of them, 128 rows, 1152 outputs of 64, 5.5 / 6.1; 612, 136 rows, 8.5 / 6.9; 512, 2048 rows, 64 outputs of 128, 9.6 / 10.9; 640, 640
-// rows, 256 outputs of 64, 8.7 / 6.9; 9216, 2048 rows, 1152 outputs of 64, 52 / 30; few outputs of 64, 1024 rows, 3.0 / 4.9).
-constexpr int SL_ROWS = 8, SL_OUTS = 32, SL_MAXK = 128, SL_MANY_BLOCKS = 4 * 148;
-template <typename TX, typename TW>
-__global__ void __launch_bounds__(SL_ROWS * SL_OUTS)
-small_linear_rows_kernel(const TX* __restrict__ x, const TW* __restrict__ w, float* __restrict__ out, int T, int N, int K,
-                         const void* __restrict__ bias, int bias_dt, float inv_tau) {
-    constexpr int R = 4;
-    __shared__ __align__(16) float xs[SL_ROWS * R][SL_MAXK];
-    __shared__ float ws[SL_OUTS][SL_MAXK + 1];
-    pdl_wait();
-    const int t0 = blockIdx.y * SL_ROWS * R, n0 = blockIdx.x * SL_OUTS, Kp = (K + 3) / 4 * 4;
-    for (int idx = threadIdx.x; idx < SL_ROWS * R * Kp; idx += blockDim.x) {
-        const int r = idx / Kp, kk = idx - r * Kp;
-        xs[r][kk] = t0 + r < T && kk < K ? to_f(x[(size_t)(t0 + r) * K + kk]) : 0.f;
-    }
-    for (int idx = threadIdx.x; idx < SL_OUTS * Kp; idx += blockDim.x) {
-        const int c = idx / Kp, kk = idx - c * Kp;
-        ws[c][kk] = n0 + c < N && kk < K ? to_f(w[(size_t)(n0 + c) * K + kk]) : 0.f;
-    }
-    __syncthreads();
-    const int r = threadIdx.x / SL_OUTS, c = threadIdx.x % SL_OUTS;
-    float d[R] = {};
-    for (int kk = 0; kk < Kp; kk += 4) {
-        const float w4[4] = {ws[c][kk], ws[c][kk + 1], ws[c][kk + 2], ws[c][kk + 3]};
+// With many rows a block owns 64 of them and 64 outputs and a thread 4 x 4, so that two 16-byte reads of shared memory serve 16 products.
+// The order of a sum, and so its bits, are the same.  A block then takes longer, so that it pays from where the blocks of 8 rows are more
+// than four per SM (us, 8 / 64 rows a block: 576 of them, 128 rows, 1152 outputs of 64 with a decay, 5.8 / 6.8; 864, 192 rows, 9.4 / 6.8;
+// 512, 512 rows, 256 outputs, 5.8 / 6.8; 768, 768 rows, 9.5 / 6.8; 2048 rows, 1152 outputs 56 / 15.8; few outputs of 64, 1024 rows, 4.0 / 6.7).
+constexpr int SL_ROWS = 8, SL_OUTS = 32, SL_MAXK = 128, SL_MANY_BLOCKS = 4 * 148, SL_TILE = 64, SL_STEP = 32;
+template <typename T>
+__device__ __forceinline__ void stage_tile(const T* __restrict__ src, int row0, int rows, int K, int k0, int kc, bool eights, float (*dst)[SL_TILE + 4]) {
+    if (eights) {                                             // lane = row, so that the eight transposed writes of a lane do not conflict
+        const int r = threadIdx.x % SL_TILE, k = threadIdx.x / SL_TILE * 8;
+        float v[8] = {};
+        if (r < rows && k < kc) {
+            constexpr int V = Vec16<T>::N;
 #pragma unroll
-        for (int u = 0; u < R; ++u) {
-            const float4 v = *reinterpret_cast<const float4*>(&xs[r + u * SL_ROWS][kk]);
-            d[u] += v.x * w4[0];
-            d[u] += v.y * w4[1];
-            d[u] += v.z * w4[2];
-            d[u] += v.w * w4[3];
+            for (int j = 0; j < 8; j += V) { Vec16<T> u; u.load(src + (size_t)(row0 + r) * K + k0 + k + j); u.unpack(v + j); }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dst[k + j][r] = v[j];
+    } else {
+        for (int i = threadIdx.x; i < SL_TILE * SL_STEP; i += blockDim.x) {
+            const int r = i / SL_STEP, k = i % SL_STEP;
+            dst[k][r] = r < rows && k < kc ? to_f(src[(size_t)(row0 + r) * K + k0 + k]) : 0.f;
         }
     }
+}
+template <typename TX, typename TW>
+__global__ void __launch_bounds__(SL_TILE * SL_STEP / 8)
+small_linear_tile_kernel(const TX* __restrict__ x, const TW* __restrict__ w, float* __restrict__ out, int T, int N, int K,
+                         const void* __restrict__ bias, int bias_dt, float inv_tau) {
+    __shared__ __align__(16) float xs[SL_STEP][SL_TILE + 4], ws[SL_STEP][SL_TILE + 4];
+    pdl_wait();
+    const int t0 = blockIdx.x * SL_TILE, n0 = blockIdx.y * SL_TILE;
+    const int r0 = threadIdx.x / 16 * 4, c0 = threadIdx.x % 16 * 4;
+    const bool eights = K % 8 == 0 && ((((uintptr_t)x | (uintptr_t)w) & 15) == 0);
+    float d[4][4] = {};
+    for (int k0 = 0; k0 < K; k0 += SL_STEP) {
+        const int kc = min(SL_STEP, K - k0);
+        stage_tile(x, t0, min(SL_TILE, T - t0), K, k0, kc, eights, xs);
+        stage_tile(w, n0, min(SL_TILE, N - n0), K, k0, kc, eights, ws);
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < kc; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(&xs[k][r0]), b = *reinterpret_cast<const float4*>(&ws[k][c0]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int u = 0; u < R; ++u) {
-        const int t = t0 + r + u * SL_ROWS;
-        if (t < T && n0 + c < N) out[(size_t)t * N + n0 + c] = finish(d[u], bias, bias_dt, inv_tau, n0 + c);
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) d[r][c] = fmaf(av[r], bv[c], d[r][c]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        if (t0 + r0 + r >= T) return;
+        float* at = out + (size_t)(t0 + r0 + r) * N + n0 + c0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (n0 + c0 + c < N) at[c] = finish(d[r][c], bias, bias_dt, inv_tau, n0 + c0 + c);
     }
 }
 template <typename TX, typename TW>
@@ -228,59 +244,21 @@ small_linear_thread_kernel(const TX* __restrict__ x, const TW* __restrict__ w, f
     out[(size_t)(t0 + r) * N + n0 + c] = finish(d, bias, bias_dt, inv_tau, n0 + c);
 }
 
-// Both on the tensor cores, for bfloat16 rows and weights and many rows (sums as in row_dots).  Long rows and up to 32 outputs: 8 rows a
-// block.  Short rows: a block does 64 rows of 64 outputs, a warp 16 outputs of 32 rows.  us, the forms above / now: 2809 rows of 1536, 24
-// outputs 22.3 / 6.2, 640 rows 6.8 / 5.3, 256 rows 4.5 / 5.2; 2048 rows of 64, 1152 outputs with a decay 33.4 / 12.3, 640 rows 14.8 / 6.7.
-constexpr int SL_DOTS_FROM = 512, SL_TILE = 64;
-template <int MT>
+// Long rows and up to 32 outputs, bfloat16, many rows: 8 of them a block, the same bits (see row_dots).  us, a warp per output / now: rows of
+// 1536, 24 outputs, 256 rows 4.5 / 6.0, 512 rows 6.0 / 6.0, 1024 rows 9.7 / 6.1, 2048 rows 17.0 / 8.6; of 2304, 32 outputs, 512 rows 9.3 / 9.4, 2048
+// rows 29 / 15.
+constexpr int SL_DOTS_FROM = 512, SL_DOTS_OUTS = 32;
 __global__ void __launch_bounds__(256)
 small_linear_dots_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, float* __restrict__ out, int T, int N, int K,
                          const void* __restrict__ bias, int bias_dt, float inv_tau) {
-    __shared__ __align__(16) double part[8 * MT * 16 * DOT_ROWS];
-    __shared__ float dots[DOT_ROWS][MT * 16];
+    __shared__ float dots[DOT_ROWS][SL_DOTS_OUTS];
     pdl_wait();
     const int t0 = blockIdx.x * DOT_ROWS, rows = min(DOT_ROWS, T - t0);
-    row_dots<MT>(x + (size_t)t0 * K, K, rows, w, N, K, 8, part, &dots[0][0], MT * 16);
+    row_dots(x + (size_t)t0 * K, K, rows, w, N, K, &dots[0][0], SL_DOTS_OUTS);
     for (int i = threadIdx.x; i < rows * N; i += blockDim.x) {
         const int r = i / N, n = i - r * N;
         out[(size_t)t0 * N + i] = finish(dots[r][n], bias, bias_dt, inv_tau, n);
     }
-}
-__global__ void __launch_bounds__(256)
-small_linear_short_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, float* __restrict__ out, int T, int N, int K,
-                          const void* __restrict__ bias, int bias_dt, float inv_tau) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const int n0 = blockIdx.x * SL_TILE + (warp & 3) * 16 + g, t0 = blockIdx.y * SL_TILE + (warp >> 2) * 32;
-    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-    double acc[4][4];
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[m][e] = 0.0;
-    pdl_wait();
-    for (int k = q * 8; k - q * 8 < K; k += 32) {
-        const bool in = k < K;
-        const uint4 lo = in && n0 < N ? *reinterpret_cast<const uint4*>(w + (size_t)n0 * K + k) : none;
-        const uint4 hi = in && n0 + 8 < N ? *reinterpret_cast<const uint4*>(w + (size_t)(n0 + 8) * K + k) : none;
-        const uint32_t first[4] = {lo.x, hi.x, lo.y, hi.y}, second[4] = {lo.z, hi.z, lo.w, hi.w};
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int t = t0 + m * 8 + g;
-            const uint4 b = in && t < T ? *reinterpret_cast<const uint4*>(x + (size_t)t * K + k) : none;
-            float f[4], s[4];
-            mma_first(f, first, b.x, b.y);
-            mma_first(s, second, b.z, b.w);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[m][e] += (double)f[e] + (double)s[e];
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 4; ++m)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int t = t0 + m * 8 + 2 * q + (e & 1), n = n0 + (e >> 1) * 8;
-            if (t < T && n < N) out[(size_t)t * N + n] = finish((float)acc[m][e], bias, bias_dt, inv_tau, n);
-        }
 }
 
 // out[t, h, :] = o[t, h, :] * scale * sigmoid(x[t, :] . w[h, :]) (out may be o; without w: sigmoid(x[t, h])): the gate per head formed (float32) and
@@ -334,20 +312,20 @@ __global__ void gate_heads_kernel(const TX* __restrict__ x, long long ldx, const
         store_from_f(out, o_dt, ob + i, load_as_f(o, o_dt, base + i) * gate[i / D]);
 }
 
-// The same for the many rows of a prompt, 8 per block, the logits on the tensor cores (see row_dots).  us, a block per row / now: 2048 rows of
-// 2304, 9 heads of 128 12.8 / 7.2, 1024 rows 7.6 / 6.1, 512 rows 6.0 / 6.4.
-constexpr int GATE_FROM = 1024, GATE_WARPS = 8;
-template <int MT>
+// The same, bit for bit, for the many rows of a prompt, 8 per block (see row_dots).  us, a block per row / now, rows of 2304, 9 heads: of 256, 768
+// rows 7.2 / 8.4, 1024 rows 7.8 / 7.6, 2048 rows 14.3 / 11.3; of 128, 1024 rows 7.7 / 6.6, 2048 rows 12.5 / 9.9.
+constexpr int GATE_FROM = 1024, GATE_WARPS = 8, GATE_HEADS = 32;
 __global__ void __launch_bounds__(GATE_WARPS * 32)
 gate_heads_rows_kernel(const bf16* __restrict__ x, long long ldx, const bf16* __restrict__ w, int W, const void* o, int o_dt, void* out,
                        long long ldo, float scale, int T, int H, int D) {
-    __shared__ __align__(16) double part[GATE_WARPS * MT * 16 * DOT_ROWS];
-    __shared__ float gate[DOT_ROWS][MT * 16];
+    __shared__ float gate[DOT_ROWS][GATE_HEADS];
     pdl_wait();
     const int t0 = blockIdx.x * DOT_ROWS, rows = min(DOT_ROWS, T - t0), pieces = H * D / 8;
-    row_dots<MT>(x + (size_t)t0 * ldx, ldx, rows, w, H, W, GATE_WARPS, part, &gate[0][0], MT * 16);
-    for (int i = threadIdx.x; i < DOT_ROWS * MT * 16; i += blockDim.x)
-        if (i % (MT * 16) < H) (&gate[0][0])[i] = scale * (1.f / (1.f + expf(-(&gate[0][0])[i])));
+    row_dots(x + (size_t)t0 * ldx, ldx, rows, w, H, W, &gate[0][0], GATE_HEADS);
+    for (int i = threadIdx.x; i < rows * H; i += blockDim.x) {
+        float& g = gate[i / H][i % H];
+        g = scale * (1.f / (1.f + expf(-g)));
+    }
     __syncthreads();
 #pragma unroll 4
     for (int i = threadIdx.x; i < rows * pieces; i += GATE_WARPS * 32) {
@@ -421,26 +399,21 @@ QNN_API int qnn_small_linear_f32(const void* x, int x_dt, const void* w, int w_d
     if (K <= 0 || (bias != nullptr && !(tau > 0.f))) return QNN_ERR_ARGUMENT;
     const float inv_tau = bias != nullptr ? 1.f / tau : 0.f;
     const size_t total = (size_t)T * N;
-    const bool many = (long long)((T + SL_ROWS - 1) / SL_ROWS) * ((N + SL_OUTS - 1) / SL_OUTS) > SL_MANY_BLOCKS;
-    if (x_dt == QNN_DT_BF16 && w_dt == QNN_DT_BF16 && K % 8 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
-        if (T >= SL_DOTS_FROM && K > SL_MAXK && N <= 32) {
-            launch_pdl(N <= 16 ? small_linear_dots_kernel<1> : small_linear_dots_kernel<2>, dim3((T + DOT_ROWS - 1) / DOT_ROWS), dim3(256), 0, st,
-                       (const bf16*)x, (const bf16*)w, out, T, N, K, bias, bias_dt, inv_tau);
-            QNN_LAUNCH_CHECK();
-        }
-        if (T >= 256 && K <= SL_MAXK && many && (T + SL_TILE - 1) / SL_TILE <= 65535) {
-            launch_pdl(small_linear_short_kernel, dim3((N + SL_TILE - 1) / SL_TILE, (T + SL_TILE - 1) / SL_TILE), dim3(256), 0, st,
-                       (const bf16*)x, (const bf16*)w, out, T, N, K, bias, bias_dt, inv_tau);
-            QNN_LAUNCH_CHECK();
-        }
+    const bool many = (long long)((T + SL_ROWS - 1) / SL_ROWS) * ((N + SL_OUTS - 1) / SL_OUTS) > SL_MANY_BLOCKS &&
+                      (N + SL_TILE - 1) / SL_TILE <= 65535;          // columns of tiles: the grid's second extent
+    if (x_dt == QNN_DT_BF16 && w_dt == QNN_DT_BF16 && T >= SL_DOTS_FROM && K > SL_MAXK && N <= SL_DOTS_OUTS && K % 8 == 0 &&
+        (((uintptr_t)x | (uintptr_t)w) & 15) == 0) {
+        launch_pdl(small_linear_dots_kernel, dim3((T + DOT_ROWS - 1) / DOT_ROWS), dim3(256), 0, st, (const bf16*)x, (const bf16*)w, out, T, N, K,
+                   bias, bias_dt, inv_tau);
+        QNN_LAUNCH_CHECK();
     }
 #define QNN_SL(TX, TW)                                                                                               \
     if (K > SL_MAXK)                                                                                                 \
         launch_pdl(small_linear_warp_kernel<TX, TW>, dim3((unsigned)((total + 7) / 8)), dim3(256), 0, st,            \
                    (const TX*)x, (const TW*)w, out, N, K, total, bias, bias_dt, inv_tau);                            \
     else if (many)                                                                                                   \
-        launch_pdl(small_linear_rows_kernel<TX, TW>, dim3((N + SL_OUTS - 1) / SL_OUTS, (T + 4 * SL_ROWS - 1) / (4 * SL_ROWS)), \
-                   dim3(SL_ROWS * SL_OUTS), 0, st, (const TX*)x, (const TW*)w, out, T, N, K, bias, bias_dt, inv_tau); \
+        launch_pdl(small_linear_tile_kernel<TX, TW>, dim3((T + SL_TILE - 1) / SL_TILE, (N + SL_TILE - 1) / SL_TILE), \
+                   dim3(SL_TILE * SL_STEP / 8), 0, st, (const TX*)x, (const TW*)w, out, T, N, K, bias, bias_dt, inv_tau); \
     else                                                                                                             \
         launch_pdl(small_linear_thread_kernel<TX, TW>, dim3((N + SL_OUTS - 1) / SL_OUTS, (T + SL_ROWS - 1) / SL_ROWS), \
                    dim3(SL_ROWS * SL_OUTS), 0, st, (const TX*)x, (const TW*)w, out, T, N, K, bias, bias_dt, inv_tau);
@@ -458,10 +431,9 @@ QNN_API int qnn_gate_heads(const void* x, int x_dt, long long ldx, const void* w
     if (T <= 0) return 0;
     if (W <= 0 || H <= 0 || D <= 0 || ldx < W || ldo < (long long)H * D || (size_t)H * sizeof(float) > 48 * 1024) return QNN_ERR_ARGUMENT;
     const int es = o_dt == QNN_DT_BF16 ? 2 : 4;
-    if (T >= GATE_FROM && w != nullptr && x_dt == QNN_DT_BF16 && w_dt == QNN_DT_BF16 && H <= 32 && W % 8 == 0 && ldx % 8 == 0 && D % 8 == 0 &&
+    if (T >= GATE_FROM && w != nullptr && x_dt == QNN_DT_BF16 && w_dt == QNN_DT_BF16 && H <= GATE_HEADS && W % 8 == 0 && ldx % 8 == 0 && D % 8 == 0 &&
         (ldo * es) % 16 == 0 && (((uintptr_t)x | (uintptr_t)w | (uintptr_t)o | (uintptr_t)out) & 15) == 0) {
-        launch_pdl(H <= 16 ? gate_heads_rows_kernel<1> : gate_heads_rows_kernel<2>, dim3((T + DOT_ROWS - 1) / DOT_ROWS), dim3(GATE_WARPS * 32),
-                   0, st, (const bf16*)x, ldx, (const bf16*)w, W, o, o_dt, out, ldo, scale, T, H, D);
+        launch_pdl(gate_heads_rows_kernel, dim3((T + DOT_ROWS - 1) / DOT_ROWS), dim3(GATE_WARPS * 32), 0, st, (const bf16*)x, ldx, (const bf16*)w, W, o, o_dt, out, ldo, scale, T, H, D);
         QNN_LAUNCH_CHECK();
     }
     const dim3 grid(T), block(row_threads(H * D));

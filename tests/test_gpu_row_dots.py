@@ -1,5 +1,6 @@
-"""Gates per head and router logits of a prompt's many rows (tensor cores, 8 rows a block) beside those of few rows: both as far from
-64 bits as float32 sums are, whatever the width, the outputs and the rows left over."""
+"""Gates per head, router logits and products with few outputs of a prompt's many rows (8 or 64 rows a block) beside those of few rows:
+as far from 64 bits as float32 sums are, whatever the width, the outputs and the rows left over, and the same bits however many rows a
+step has."""
 import pytest
 import torch
 
@@ -78,3 +79,49 @@ def test_small_linear(T, K, N, decay):
     got = ops.small_linear_f32(x, w, **kw)
     few = torch.cat([ops.small_linear_f32(x[lo:lo + 100].contiguous(), w, **kw) for lo in range(0, T, 100)])
     assert off(got, want) < 2e-7 and off(got, want) < 1.1 * off(few, want) + 1e-8
+
+
+def pieces(T):
+    """A step's rows as other steps might bring them: one alone, a few, the rest in hundreds."""
+    cuts = [0, 1, 2, 9] + list(range(100, T, 100)) + [T]
+    return list(zip(cuts[:-1], cuts[1:]))
+
+
+@pytest.mark.parametrize("T", [255, MANY, MANY + 1, MANY + 7, 2050])
+@pytest.mark.parametrize("W,E,extra", [(8, 4, 0), (264, 20, 1), (1536, 32, 0), (2304, 16, 0), (2304, 31, 1), (1536, 36, 0)])
+def test_route_does_not_depend_on_the_rows_beside(T, W, E, extra):
+    torch.manual_seed(T + W + E)
+    x, w = torch.randn((T, W), device=DEV).bfloat16(), (torch.randn((E + extra, W), device=DEV) * 2 * W ** -0.5).bfloat16()
+    kinds = [dict(score="sigmoid"), dict(score="softmax", renormalize=True)]
+    if E % 4 == 0 and E > 4:
+        kinds.append(dict(score="sigmoid", renormalize=True, correction=torch.randn(E, device=DEV), scale=2.5, groups=(4, 2)))
+    for kw in kinds:
+        kw.update({"extra": extra} if extra else {})
+        whole = ops.moe_route(x, w, 2, **kw)
+        parts = [ops.moe_route(x[lo:hi].contiguous(), w, 2, **kw) for lo, hi in pieces(T)]
+        for i, res in enumerate(whole):
+            assert torch.equal(torch.cat([p[i] for p in parts]), res), (kw, i)
+
+
+@pytest.mark.parametrize("T", [1023, 1024, 1025, 2050])
+@pytest.mark.parametrize("W,H,D", [(8, 1, 8), (264, 9, 256), (1536, 31, 8), (2304, 32, 16), (2304, 33, 16)])
+def test_gates_do_not_depend_on_the_rows_beside(T, W, H, D):
+    torch.manual_seed(T + W + H)
+    x, w = torch.randn((T, W), device=DEV).bfloat16(), (torch.randn((H, W), device=DEV) * W ** -0.5).bfloat16()
+    o = torch.randn((T, H * D), device=DEV).bfloat16()
+    parts = [ops.gate_heads(o[lo:hi].clone(), x[lo:hi].contiguous(), w, H, 0.7) for lo, hi in pieces(T)]
+    assert torch.equal(torch.cat(parts), ops.gate_heads(o.clone(), x, w, H, 0.7))
+
+
+@pytest.mark.parametrize("K,N,Ts", [(136, 1, (511, 512, 513, 519)), (1536, 24, (511, 512, 513, 519)), (2304, 32, (512, 2050)), (1536, 33, (513,)),
+                                    (8, 700, (63, 64, 65, 255, 700)), (64, 1152, (127, 137, 256, 700)), (33, 577, (257, 700)), (128, 640, (256, 1500)),
+                                    (100, 65, (2050,))])
+@pytest.mark.parametrize("dtypes", [("bfloat16", "bfloat16"), ("bfloat16", "float32"), ("float32", "float32")])
+@pytest.mark.parametrize("decay", [False, True])
+def test_small_linear_does_not_depend_on_the_rows_beside(K, N, Ts, dtypes, decay):
+    for T in Ts:
+        torch.manual_seed(T + K + N)
+        x, w = torch.randn((T, K), device=DEV).to(getattr(torch, dtypes[0])), (torch.randn((N, K), device=DEV) * K ** -0.5).to(getattr(torch, dtypes[1]))
+        kw = dict(decay_bias=torch.randn(N, device=DEV), tau=8.0) if decay else {}
+        parts = [ops.small_linear_f32(x[lo:hi].contiguous(), w, **kw) for lo, hi in pieces(T)]
+        assert torch.equal(torch.cat(parts), ops.small_linear_f32(x, w, **kw)), T
