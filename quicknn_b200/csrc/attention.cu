@@ -447,7 +447,7 @@ extern "C" int qnn_attn_decode_mma_split(const void* q, long long q_stride, cons
                                          const int* page_table, int max_pages, int page_size, int ring,
                                          const int* slots, const int* slot_len, int B, int nq, int nkv, int hd,
                                          float scale, float cap, int window, float* part_o, float* part_ml,
-                                         int n_splits, void* out, long long out_stride, int* combined,
+                                         int n_splits, int uneven, void* out, long long out_stride, int* combined,
                                          const float* slopes, const float* sinks, cudaStream_t st);
 
 // threads of the combine kernel's block: a group of hd/4 threads for every key range, up to 1024; and the
@@ -470,7 +470,7 @@ template <typename T>
 static int decode_launch(const void* q, long long q_stride, const void* k_pool, const void* v_pool,
                          const int* page_table, int max_pages, int page_size, int ring, const int* slots,
                          const int* slot_len, int B, int nq, int nkv, int hd, float scale, float cap, int window,
-                         float* part_o, float* part_ml, int n_splits, void* out, long long out_stride,
+                         float* part_o, float* part_ml, int n_splits, int uneven, void* out, long long out_stride,
                          const float* slopes, const float* sinks, cudaStream_t st) {
     if (nkv <= 0 || nq % nkv) return QNN_ERR_ARGUMENT;
     const Geometry geo = geometry<T>(hd, nq / nkv);
@@ -490,7 +490,7 @@ static int decode_launch(const void* q, long long q_stride, const void* k_pool, 
         int combined = 0;
         const int rc = qnn_attn_decode_mma_split(q, q_stride, k_pool, v_pool, page_table, max_pages, page_size, ring,
                                                  slots, slot_len, B, nq, nkv, hd, scale, cap, window, part_o, part_ml,
-                                                 n_splits, out, out_stride, &combined, slopes, sinks, st);
+                                                 n_splits, uneven, out, out_stride, &combined, slopes, sinks, st);
         if (rc == 0 && combined) return 0;            // merged inside the kernel's clusters
         if (rc == 0) launched = true;
         else if (rc != QNN_ERR_UNSUPPORTED) return rc;
@@ -543,17 +543,18 @@ QNN_API int qnn_attn_supports(int dtype, int nq, int nkv, int hd) {
     return dtype == QNN_DT_BF16 ? supports<bf16>(nq, nkv, hd) : supports<float>(nq, nkv, hd);
 }
 
-// Scratch: part_o needs B*nq*n_splits*hd floats, part_ml B*nq*n_splits*2 floats.
+// Scratch: part_o needs B*nq*n_splits*hd floats, part_ml B*nq*n_splits*2 floats.  uneven: 1 where the sequences' lengths are known to differ
+// much (a matter of speed only, see qnn_attn_decode_mma_split).
 QNN_API int qnn_attn_decode(const void* q, long long q_stride, int dtype, const void* k_pool, const void* v_pool,
                             const int* page_table, int max_pages, int page_size, int ring, const int* slots,
                             const int* slot_len, int B, int nq, int nkv, int hd, float scale, float cap, int window,
-                            float* part_o, float* part_ml, int n_splits, void* out, long long out_stride,
+                            float* part_o, float* part_ml, int n_splits, int uneven, void* out, long long out_stride,
                             const float* slopes, const float* sinks, cudaStream_t st) {
     if (B <= 0) return 0;
     if (n_splits < 1 || n_splits > 65535 || B > 65535) return QNN_ERR_ARGUMENT;
     if (dtype == QNN_DT_BF16)
         return decode_launch<bf16>(q, q_stride, k_pool, v_pool, page_table, max_pages, page_size, ring, slots, slot_len,
-                                   B, nq, nkv, hd, scale, cap, window, part_o, part_ml, n_splits, out, out_stride, slopes, sinks, st);
+                                   B, nq, nkv, hd, scale, cap, window, part_o, part_ml, n_splits, uneven, out, out_stride, slopes, sinks, st);
     return decode_launch<float>(q, q_stride, k_pool, v_pool, page_table, max_pages, page_size, ring, slots, slot_len, B,
-                                nq, nkv, hd, scale, cap, window, part_o, part_ml, n_splits, out, out_stride, slopes, sinks, st);
+                                nq, nkv, hd, scale, cap, window, part_o, part_ml, n_splits, uneven, out, out_stride, slopes, sinks, st);
 }

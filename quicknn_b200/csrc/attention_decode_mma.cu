@@ -364,11 +364,16 @@ attn_decode_mma_kernel(const bf16* __restrict__ q, size_t q_stride, const bf16* 
 // plain grid followed by the combine kernel; clusters of 2 and 4 measured equal or slightly faster.
 constexpr int CLUSTER_MAX = 4;
 
-// Stages ST of the cp.async pipeline: 3.  A grid of more CTAs than the device holds at once takes 2 at head size 256: a third of the
+// Stages ST of the cp.async pipeline: 3.  At head size 256 a grid of more CTAs than the device holds at once may take 2: a third of the
 // shared memory less, so three CTAs share an SM instead of two and one's start (slot, length, page row, first tile) and merge hide
 // behind the others' keys.  Decode steps of Gemma 2 2B, us, 3 / 2 stages: 64 sequences of 512 to 2048 tokens 3512 / 3233, 32 of
-// them 2561 / 2465, 64 of 1200 3286 / 3285; where all CTAs fit at once the deeper ring is the better one (8 of 6900 tokens 2013 / 2202).
-// A tile's sums do not depend on it.
+// them 2561 / 2465; where all CTAs fit at once the deeper ring is the better one (8 of 6900 tokens 2013 / 2202).
+// CTAs of one length run in rounds, and a round of three per SM takes up to 3/2 of one of two: then 2 stages only where the rounds so
+// weighed are less than 5/4 of what they are with 3.  The attention alone, 4 kv heads, 4000 tokens each, us, 3 / 2 stages: 75 sequences (300
+// CTAs) 338 / 216, 111 (444) 330 / 274, 128 (512, two rounds either way: stays with 3) 335 / 414, 64 in two ranges (512) 174 / 209, 48 in
+// three (576) 119 / 155, 75 in two (600) 316 / 284.  CTAs of `uneven` lengths fill the device whatever their number: 56 sequences of up to 2000
+// tokens in two ranges (448) under a window of 512 29 / 20, 28 of up to 2000 in four (448) 39 / 31.
+// A tile's sums do not depend on the stages; whether key ranges merge in clusters may (see merge_in_clusters), and with it their rounding.
 template <int HD, int MMA_WARPS, int MMA_STAGES>
 size_t smem_bytes(int max_pages) {
     size_t smem = (size_t)MMA_WARPS * MMA_STAGES * 2 * TILE * HD * 2;
@@ -438,17 +443,16 @@ int ctas_at_once(size_t smem) {
     return known;
 }
 
-// Whether a grid of `clusters` clusters of `size` CTAs merges its key ranges inside the clusters.  Yes if
-// they all fit the device at once, or if the device holds nearly as many CTAs in clusters of this size as
-// it holds plain ones (a grid of several rounds loses little then).  Measured at head size 256, 24
-// sequences x 4 kv heads x 3 ranges at context 8192: 96 clusters of 3 do not fit at once where 288 plain
-// CTAs do, and a step of 6 layers took 1.58 ms against 1.08 ms with the combine kernel.
+// Whether a grid of `clusters` clusters of `size` CTAs merges its key ranges inside the clusters: where they all fit the
+// device at once (or all but 1 in 20 of a grid that fits it as plain CTAs).  Measured at head size 256, 24 sequences x 4 kv heads x 3 ranges at context 8192: 96 clusters of 3 do not
+// fit at once where 288 plain CTAs do, and a step of 6 layers took 1.58 ms against 1.08 ms with the combine kernel.  In a grid of
+// several rounds a cluster's places come free together, so it waits where plain CTAs would start (attention alone, 4 kv heads, us, clusters /
+// combine kernel, two stages: 112 sequences of 1000 tokens in 3 ranges 97 / 89, of 4000 301 / 294; three stages, as a geometric mean of
+// lengths: one range 1.22, two 1.13, four 1.07 times the combine kernel's time).
 template <int HD, int MMA_WARPS, int ST>
 bool merge_in_clusters(size_t smem, int size, long long clusters) {
-    const int at_once = clusters_at_once<HD, MMA_WARPS, ST>(smem, size);
-    if (at_once <= 0) return false;
-    if (clusters <= at_once) return true;
-    return (long long)at_once * size * 100 >= (long long)ctas_at_once<HD, MMA_WARPS, ST>(smem) * 95;
+    const long long at_once = clusters_at_once<HD, MMA_WARPS, ST>(smem, size), plain = ctas_at_once<HD, MMA_WARPS, ST>(smem);
+    return clusters <= at_once || (at_once > 0 && clusters * size <= plain && at_once * size * 100 >= plain * 95);
 }
 
 template <int HD, int MMA_WARPS, int ST>
@@ -492,19 +496,30 @@ int launch_staged(const void* q, long long q_stride, const void* k_pool, const v
     return (int)cudaGetLastError();
 }
 
+// Stages for a grid of `ctas`, of which the device holds at3 at once with 3 stages and at2 with 2 (see smem_bytes).
+int stages_for(long long ctas, int at3, int at2, bool uneven) {
+    if (at3 <= 0 || at2 <= 0 || ctas <= at3) return 3;
+    if (uneven) return 2;
+    const long long r3 = (ctas + at3 - 1) / at3 * at3, r2 = (ctas + at2 - 1) / at2 * at2;
+    return r2 * 4 < r3 * 5 ? 2 : 3;
+}
+
 template <int HD, int MMA_WARPS>
 int launch(const void* q, long long q_stride, const void* k_pool, const void* v_pool, const int* page_table,
            int max_pages, int page_size, int ring, const int* slots, const int* slot_len, int B, int nq, int nkv,
-           float scale, float cap, int window, float* part_o, float* part_ml, int n_splits, void* out,
+           float scale, float cap, int window, float* part_o, float* part_ml, int n_splits, int uneven, void* out,
            long long out_stride, int* combined, const float* slopes, const float* sinks, cudaStream_t st) {
 #define QNN_STAGED(ST) launch_staged<HD, MMA_WARPS, ST>(q, q_stride, k_pool, v_pool, page_table, max_pages, page_size, ring, slots,     \
                                                         slot_len, B, nq, nkv, scale, cap, window, part_o, part_ml, n_splits, out, \
                                                         out_stride, combined, slopes, sinks, st)
     if constexpr (HD == 256 && MMA_WARPS == 2) {
-        const size_t smem = smem_bytes<HD, MMA_WARPS, 3>(max_pages);
+        const size_t smem3 = smem_bytes<HD, MMA_WARPS, 3>(max_pages), smem2 = smem_bytes<HD, MMA_WARPS, 2>(max_pages);
         if (const int rc = allow_memory<HD, MMA_WARPS, 3>()) return rc;
+        if (const int rc = allow_memory<HD, MMA_WARPS, 2>()) return rc;
         const long long ctas = (long long)n_splits * nkv * ((nq / nkv + 7) / 8) * B;
-        if (smem <= 220 * 1024 && ctas > ctas_at_once<HD, MMA_WARPS, 3>(smem)) return QNN_STAGED(2);
+        if (smem3 <= 220 * 1024 &&
+            stages_for(ctas, ctas_at_once<HD, MMA_WARPS, 3>(smem3), ctas_at_once<HD, MMA_WARPS, 2>(smem2), uneven) == 2)
+            return QNN_STAGED(2);
     }
     return QNN_STAGED(3);
 #undef QNN_STAGED
@@ -512,25 +527,29 @@ int launch(const void* q, long long q_stride, const void* k_pool, const void* v_
 
 }  // namespace
 
+// The stages that qnn_attn_decode_mma_split takes at head size 256 for so many CTAs on a device that holds at3 / at2 of them at once.
+QNN_API int qnn_attn_decode_stages(long long ctas, int at3, int at2, int uneven) { return stages_for(ctas, at3, at2, uneven); }
+
 // Decode attention for bfloat16 on the tensor cores.  Returns QNN_ERR_UNSUPPORTED for sizes it
 // does not take (the caller then uses the generic kernel).  On success *combined says whether
 // `out` ([B, out_stride] bfloat16, may be null) already holds the result (up to 4 splits, merged
 // inside a cluster) or the caller still has to run the combine pass over part_o / part_ml.
 // slots, slot_len and page_table are read before the kernel waits for the kernel launched in front of it
 // on the stream (programmatic dependent launch): that kernel must not be the one that writes them.  Copies
-// from the host and kernels further back are complete by then.
+// from the host and kernels further back are complete by then.  uneven: the sequences' lengths differ by a tenth or more (a matter
+// of speed only, see stages_for).
 extern "C" int qnn_attn_decode_mma_split(const void* q, long long q_stride, const void* k_pool, const void* v_pool,
                                          const int* page_table, int max_pages, int page_size, int ring,
                                          const int* slots, const int* slot_len, int B, int nq, int nkv, int hd,
                                          float scale, float cap, int window, float* part_o, float* part_ml,
-                                         int n_splits, void* out, long long out_stride, int* combined,
+                                         int n_splits, int uneven, void* out, long long out_stride, int* combined,
                                          const float* slopes, const float* sinks, cudaStream_t st) {
     if (nkv <= 0 || nq % nkv) return QNN_ERR_ARGUMENT;
     if (page_size < TILE || (page_size & (page_size - 1))) return QNN_ERR_UNSUPPORTED;
     if (ring > 0 && (ring % page_size)) return QNN_ERR_UNSUPPORTED;
     if ((q_stride * 2) % 4 || ((uintptr_t)q & 3)) return QNN_ERR_UNSUPPORTED;
 #define QNN_MMA_ARGS q, q_stride, k_pool, v_pool, page_table, max_pages, page_size, ring, slots, slot_len, B, nq, nkv, \
-                     scale, cap, window, part_o, part_ml, n_splits, out, out_stride, combined, slopes, sinks, st
+                     scale, cap, window, part_o, part_ml, n_splits, uneven, out, out_stride, combined, slopes, sinks, st
     static int warps = 0;
     if (warps == 0) {
         const char* e = getenv("QNN_MMA_WARPS");

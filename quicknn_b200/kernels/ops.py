@@ -814,8 +814,9 @@ def attn_decode(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, k_poo
                 v_pool: torch.Tensor, page_table: torch.Tensor, page_size: int, ring: int,
                 slots: torch.Tensor, slot_len: torch.Tensor, scale: float, cap: Optional[float],
                 window: Optional[int], n_splits: int, part_o: torch.Tensor, part_ml: torch.Tensor,
-                slopes: Optional[torch.Tensor] = None, sinks: Optional[torch.Tensor] = None):
+                slopes: Optional[torch.Tensor] = None, sinks: Optional[torch.Tensor] = None, uneven: bool = False):
     """One query row per sequence against the paged cache.  q = the first nq*hd columns of qkv.
+    ``uneven``: the sequences' lengths are known to differ much (grids beyond the device are then laid out for that).
     ``slots``, ``slot_len`` and ``page_table`` must be complete before the kernel that runs just before
     this one on the stream starts (host copies and earlier kernels are): the tensor-core kernel reads
     them while that kernel may still run."""
@@ -835,7 +836,7 @@ def attn_decode(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, k_poo
     _lib.check(L.qnn_attn_decode(
         _p(qkv), ld, dt_code(qkv), _p(k_pool), _p(v_pool), _p(page_table), page_table.shape[1],
         page_size, ring, _p(slots), _p(slot_len), B, n_heads, n_kv, head_dim, float(scale), float(cap or 0.0),
-        int(window or 0), _p(part_o), _p(part_ml), n_splits, _p(out), out.shape[1], _p(slopes), _p(sinks), _stream()), "attn_decode", 2)
+        int(window or 0), _p(part_o), _p(part_ml), n_splits, int(uneven), _p(out), out.shape[1], _p(slopes), _p(sinks), _stream()), "attn_decode", 2)
     return out
 
 

@@ -234,8 +234,19 @@ class AttentionMixer(Mixer):
                 best, best_time = s, t
         return best
 
+    def _uneven(self, step) -> bool:
+        """Whether the keys that a decode step's sequences walk differ much from one to the next (under a window that nearly all of them
+        have outgrown they do not)."""
+        spread = step.spread or 1.0
+        return spread > 1.0 and not (self.window and step.longest >= 4 * self.window * spread)
+
     def schedule(self, step) -> tuple:
-        return (self.decode_splits(step),) if step.mode == "decode" else ()
+        if step.mode != "decode":
+            return ()
+        splits = self.decode_splits(step)
+        blocks = splits * step.n_seqs * self.n_kv * ((self.n_heads // self.n_kv + 7) // 8)
+        # the kernel's layout depends on the lengths at head size 256 and beyond one round of blocks
+        return (splits, self._uneven(step)) if self.head_dim == 256 and blocks > self._resident else (splits,)
 
     def scratch_need(self, step) -> int:
         """Partial (maximum, sum, output) of every key range: float32, [rows, heads, ranges, head_dim + 2]."""
@@ -380,5 +391,5 @@ class AttentionMixer(Mixer):
             a = ops.attn_decode(qkv, self.n_heads, self.n_kv, self.head_dim, line.k, line.v, line.page_table,
                                 line.page_size, line.ring, step.slots, line.slot_len, self.scale, self.softcap,
                                 self.window, splits, part[:n * self.head_dim], part[n * self.head_dim:n * (self.head_dim + 2)],
-                                slopes=self.slopes, sinks=self.sinks)
+                                slopes=self.slopes, sinks=self.sinks, uneven=self._uneven(step))
         return a

@@ -87,3 +87,26 @@ def test_rows_cut_off_a_prompt_product_only_where_a_round_of_tiles_is_saved():
     assert [down(m) for m in (2048, 2049, 2112, 2113, 2304, 4096, 4097, 6145, 257, 100)] == [0, 1, 64, 0, 0, 0, 1, 1, 0, 0]
     for n_out, k, epi in ((4096, 2304, ops.EPI_NONE), (2304, 2048, ops.EPI_NONE), (9216, 2304, ops.EPI_GATED)):
         assert all(ops._rows_for_the_small_kernel(m, n_out, k, epi, cpu) == 0 for m in (2049, 4097, 6145, 8193))
+
+
+def test_stages_of_decode_attention():
+    """296 blocks at once with three stages, 444 with two.  Blocks of one length run in rounds: two rounds of 444 in the place of two of
+    296 took up to 1.3 times as long.  Unequal lengths fill the device whatever the number."""
+    from quicknn_b200.kernels.lib import load
+    stages = load().qnn_attn_decode_stages
+    sizes = (1, 296, 297, 444, 445, 512, 576, 592, 593, 888, 889, 1024, 1184, 1344, 3072)
+    assert {n: stages(n, 296, 444, 0) for n in sizes} == {
+        1: 3, 296: 3, 297: 2, 444: 2, 445: 3, 512: 3, 576: 3, 592: 3, 593: 2, 888: 2, 889: 2, 1024: 2, 1184: 2, 1344: 2, 3072: 2}
+    assert {n: stages(n, 296, 444, 1) for n in sizes} == {n: 2 if n > 296 else 3 for n in sizes}
+    assert stages(500, 0, 444, 1) == 3 and stages(500, 296, 0, 1) == 3     # a device that could not say
+
+
+def test_a_decode_graph_knows_whether_its_lengths_are_uneven_where_the_kernel_asks():
+    m = mixer()
+    m.decode_splits = lambda step: 4
+    assert m.schedule(step(18, 2048, 1.6)) == (4,)                          # one round of blocks
+    assert m.schedule(step(28, 2048, 1.6)) == (4, True) and m.schedule(step(28, 2048, 1.0)) == (4, False)
+    assert mixer(head_dim=128).schedule(step(128, 2048, 1.6)) == (mixer(head_dim=128).decode_splits(step(128, 2048, 1.6)),)
+    w = mixer(window=256)
+    w.decode_splits = m.decode_splits
+    assert w.schedule(step(28, 1024, 1.6)) == (4, True) and w.schedule(step(28, 2048, 1.6)) == (4, False)      # nearly all beyond the window
