@@ -161,23 +161,26 @@ __global__ void head_prep_kernel(const T* src, long long lds, void* dst, int dst
 // lane; the partner of a half-split pair lies rot/16 lanes away and comes by shuffle.  Element types are read at run time (rows and
 // pools of bfloat16 or float32).  Bound by instructions and by the chain load -> sum -> store of a head where a step has many rows, so
 // what is the same for every head of a token (a lane's angles, the norms' weights) is held in registers, and the first heads' rows are
-// asked for before the angles are formed.  us, a warp per head / now: 8 + 4 heads of 128, 8 rows 7.7 / 4.0, 2809 rows 25.8 / 17.5;
-// 12 + 12 heads of 64, 2048 rows 39.0 / 11.8; 8 + 4 heads of 256, 2048 rows 27.8 / 19.5.  (64 registers; with the 91 that the compiler takes
-// by itself 18.6, 13.8 and 20.6.)
-// WHOLE_W: the norms' weights are read in pieces of eight (16-byte aligned, norm_dim a multiple of 8); else one by one.
+// asked for before the angles are formed.  us, a warp per head / now, with norms: 8 + 4 heads of 128, 8 rows 6.6 / 3.1, 2048 rows 19.6 / 9.5;
+// 12 + 12 heads of 64, 2048 rows 35.8 / 9.1; 8 + 4 heads of 256, 2048 rows 20.2 / 13.5.  At most 64 registers (with the 91 that the compiler
+// took by itself 5 to 15 % slower), and only those that a form needs: in one form for all, with weights and eight angles, neighbouring pairs
+// without norms were slower than a warp per head (8 + 4 heads of 256, 4096 rows 13.6 / 17.4, now 11.6; 4 + 1 heads 9.6 / 12.9, now 8.4).
+// NORM: NORM_NONE; NORM_EIGHTS, weights read in pieces of eight (16-byte aligned, norm_dim a multiple of 8); NORM_SINGLE, one by one.
+// INTER: the rotation's pairs are neighbours, so a lane holds four angles and not eight.
+enum { NORM_NONE, NORM_EIGHTS, NORM_SINGLE };
 __device__ __forceinline__ float group_sum(float v, int lph) {
     for (int o = lph >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-template <bool WHOLE_W>
+template <int NORM, bool INTER>
 __global__ void __launch_bounds__(256, 4) head_prep_vec_kernel(const void* src, int s_dt, long long lds, void* dst, int d_dt, long long ldd, int nq,
-                                     int nk, int nv, int hd, int norm_dim, int rot, int interleaved,
+                                     int nk, int nv, int hd, int norm_dim, int rot,
                                      const void* __restrict__ bias, int b_dt, const void* __restrict__ wq,
                                      const void* __restrict__ wk, int w_dt, float eps, const float* __restrict__ inv_freq,
                                      const int* __restrict__ tok_pos, const int* __restrict__ tok_slot, void* k_pool,
                                      void* v_pool, const int* __restrict__ page_table, int max_pages, int page_size,
                                      int ring, const int* __restrict__ slot_len, int write_cache, int flags, int lph) {
-    const int norm_whole = flags & QNN_PREP_WHOLE;
+    const bool norm_whole = NORM != NORM_NONE && (flags & QNN_PREP_WHOLE);
     const bool norm_last = flags & QNN_PREP_NORM_LAST, plain = flags & QNN_PREP_PLAIN_NORM;
     const bool v_is_k = flags & QNN_PREP_VALUES_ARE_KEYS;
     extern __shared__ float sm[];                   // [rot/2] (cos, sin) pairs, then [nq + nk] sums
@@ -208,7 +211,7 @@ __global__ void __launch_bounds__(256, 4) head_prep_vec_kernel(const void* src, 
     float wqv[8], wkv[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) wqv[e] = wkv[e] = 1.f;
-    if (WHOLE_W && !norm_whole && col < norm_dim) {
+    if (NORM == NORM_EIGHTS && !norm_whole && col < norm_dim) {
         if (wq != nullptr) load8_as_f(wq, w_dt, col, wqv);
         if (wk != nullptr) load8_as_f(wk, w_dt, col, wkv);
     }
@@ -248,22 +251,22 @@ __global__ void __launch_bounds__(256, 4) head_prep_vec_kernel(const void* src, 
     } else {
         __syncthreads();
     }
-    // this lane's angles: of pair (col + e) / 2, or of column c and its partner (the lower one's sine with a minus)
+    // this lane's angles: of the four pairs, or of column c and its partner (the lower one's sine with a minus)
     const bool low = col < rh, turns = col < rot;
-    const int partner = interleaved || !turns ? lane : (low ? lane + rh / 8 : lane - rh / 8);
-    float cs[8], sn[8];
+    const int partner = INTER || !turns ? lane : (low ? lane + rh / 8 : lane - rh / 8);
+    constexpr int ANGLES = INTER ? 4 : 8;
+    float cs[ANGLES], sn[ANGLES];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int e = 0; e < ANGLES; ++e) {
         cs[e] = 1.f;
         sn[e] = 0.f;
-        const int c = interleaved ? (col + e) >> 1 : (low ? col + e : col + e - rh);
-        if (col + e < rot) {
+        const int c = INTER ? col / 2 + e : (low ? col + e : col + e - rh);
+        if (INTER ? c < rh : turns) {
             const float2 a = angles[c];
             cs[e] = a.x;
-            sn[e] = interleaved || !low ? a.y : -a.y;
+            sn[e] = INTER || !low ? a.y : -a.y;
         }
     }
-    const bool any_norm = wq != nullptr || wk != nullptr || (plain && norm_dim > 0);
     for (int h0 = warp * hpw; h0 < heads; h0 += nwarp * hpw) {
         const int h = h0 + sub;
         if (h0 != warp * hpw) load_head(h, v);
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(256, 4) head_prep_vec_kernel(const void* src, 
             ss = group_sum(ss, lph);
             if (!normed) return;
             const float inv = norm_whole ? (is_k ? inv_k : inv_q) : rsqrtf(ss / (float)norm_dim + eps);
-            if (WHOLE_W) {
+            if (NORM == NORM_EIGHTS) {
                 float wv[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) wv[e] = is_k ? wkv[e] : wqv[e];
@@ -300,15 +303,15 @@ __global__ void __launch_bounds__(256, 4) head_prep_vec_kernel(const void* src, 
                     if (col + e < norm_dim) v[e] = v[e] * inv * (w != nullptr ? load_as_f(w, w_dt, w0 + col + e) : 1.f);
             }
         };
-        if (any_norm && !norm_last) norm();
+        if (NORM != NORM_NONE && !norm_last) norm();
         if (rot > 0) {
-            if (interleaved) {
+            if constexpr (INTER) {
 #pragma unroll
                 for (int e = 0; e < 8; e += 2) {
                     const float a = v[e], b = v[e + 1];
                     if (col + e < rot) {
-                        v[e] = a * cs[e] - b * sn[e];
-                        v[e + 1] = b * cs[e] + a * sn[e];
+                        v[e] = a * cs[e / 2] - b * sn[e / 2];
+                        v[e + 1] = b * cs[e / 2] + a * sn[e / 2];
                     }
                 }
             } else {
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(256, 4) head_prep_vec_kernel(const void* src, 
                 }
             }
         }
-        if (any_norm && norm_last) norm();
+        if (NORM != NORM_NONE && norm_last) norm();
         if (store) {
             store8_from_f(dst, d_dt, out_row + c0 + col, v);
             if (is_k && wr) store8_from_f(k_pool, d_dt, cache_base + (size_t)(h - nq) * head_stride + col, v);
@@ -385,10 +388,14 @@ QNN_API int qnn_head_prep(const void* src, int dtype, long long lds, void* dst, 
         while (lph * 8 < hd) lph *= 2;
         const int full = (heads * lph + 31) / 32;       // warps that hold every head at once
         if (full < warps) warps = full < 1 ? 1 : full;
-        const bool whole_w = norm_dim % 8 == 0 && (((uintptr_t)wq | (uintptr_t)wk) & 15) == 0;
-        launch_pdl(whole_w ? head_prep_vec_kernel<true> : head_prep_vec_kernel<false>, dim3(T), dim3(warps * 32),
+        const bool normed = wq != nullptr || wk != nullptr || ((flags & QNN_PREP_PLAIN_NORM) && norm_dim > 0);
+        const bool eights = norm_dim % 8 == 0 && (((uintptr_t)wq | (uintptr_t)wk) & 15) == 0;
+        auto kernel = interleaved ? head_prep_vec_kernel<NORM_SINGLE, true> : head_prep_vec_kernel<NORM_SINGLE, false>;
+        if (!normed) kernel = interleaved ? head_prep_vec_kernel<NORM_NONE, true> : head_prep_vec_kernel<NORM_NONE, false>;
+        else if (eights) kernel = interleaved ? head_prep_vec_kernel<NORM_EIGHTS, true> : head_prep_vec_kernel<NORM_EIGHTS, false>;
+        launch_pdl(kernel, dim3(T), dim3(warps * 32),
                    ((size_t)rot + heads) * sizeof(float), st, src, dtype, lds, dst, dst_dt, ldd, nq, nk, nv, hd, norm_dim, rot,
-                   interleaved, bias, b_dt, wq, wk, w_dt, eps, inv_freq, tok_pos, tok_slot, k_pool, v_pool, page_table, max_pages,
+                   bias, b_dt, wq, wk, w_dt, eps, inv_freq, tok_pos, tok_slot, k_pool, v_pool, page_table, max_pages,
                    page_size, ring, slot_len, write_cache, flags, lph);
         QNN_LAUNCH_CHECK();
     }
