@@ -26,7 +26,10 @@
 // tile's walk over K, and a slab takes 0.16 us at 64 columns, 0.18 at 128, 0.24 at 192 and 0.30 at 256 (at 256 the tensor cores' time,
 // below that of fetching: the 16 KB of A stay).  Measured (us, 256 columns / 128 / as chosen): of 2304 x 9216 256 rows 46.4 / 28.5 / 26.3 (64), 640
 // rows 46.5 / 29.5 / 28.6 (96), 1280 rows 50.7 / 51.4 / 41.4 (192), 2809 rows 93.0 / 87.4 / 83.5 (192); of 4096 x 2304 640 rows 17.8 /
-// 17.1 / 15.3 (192), 1280 rows 27.8 / 23.2 / 21.2 (160); of 1536 x 6144 2048 rows 36.4 / 35.1 / 28.9 (192).  An element's
+// 17.1 / 15.3 (192), 1280 rows 27.8 / 23.2 / 21.2 (160); of 1536 x 6144 2048 rows 36.4 / 35.1 / 28.9 (192).  With a short inner size the
+// writing of a tile takes longer than its walk and hides the next one's, 2 us at 64 columns, 2.4 at 128, 3.7 at 256, and 3.5 already at 160: widths
+// that are no multiple of 128 write pieces of rows that are shorter.  So the rule counts both (us, 256 columns / by the walk alone / as chosen:
+// 8192 rows of 2048 x 512 20.7 / 22.2 / 20.7, of 2048 x 768 23.1 / 24.9 / 23.1, 4096 rows of 4096 x 256 17.3 / 20.0 / 17.3).  An element's
 // sum runs over K in the same order whatever the tile, so the results are the same bit for bit.  (Sharing a tile's K among
 // clusters of two or four pairs, summed through distributed shared memory in a fixed order, took 22 and 30 us for 256 and 640 rows of
 // 2304 x 9216.  It is not in: it moves results by rounding, and with them ids that a model samples, where these are to stay the same.
@@ -63,7 +66,8 @@ struct Tile {
 };
 constexpr int STAGING_BYTES = BM * 128 * 2;          // the epilogue's 128 rows x 128 columns of bfloat16
 constexpr int GEMM_THREADS = 192;
-constexpr int SLAB_NS[7] = {160, 167, 175, 205, 235, 268, 300};      // time of a slab in tiles of 64, 96, .. 256 columns
+constexpr int SLAB_NS[7] = {160, 167, 175, 205, 235, 268, 300};             // time of a slab in tiles of 64, 96, .. 256 columns
+constexpr int WRITE_NS[7] = {2000, 2400, 2400, 3500, 3600, 3700, 3700};      // of writing such a tile
 
 
 // `bar` is a shared::cluster address: the leader's barrier, whichever CTA of the pair loads
@@ -329,22 +333,26 @@ gemm_tcgen05_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
 typedef void (*Kernel)(CUtensorMap, CUtensorMap, bf16*, int, int, int, int, ActConsts, int*);
 
-// Columns of a plain product's tile: what takes the fewest rounds of tiles times the time of a slab.
-int plain_tile_cols(long long M, long long N, int sm_count) {
+// Columns of a plain product's tile: the least time, of a round of tiles the longer of walking K and writing, of the last both;
+// a narrower one where that is 2 % less (8192 rows of 6144 x 1536, a tie: 256 columns 102 us, 192 105).
+int plain_tile_cols(long long M, long long N, long long K, int sm_count) {
     const long long m_tiles = (M + 2 * BM - 1) / (2 * BM), pairs = sm_count / 2 > 0 ? sm_count / 2 : 1;
     long long best = 0;
     int cols = 256;
     for (int c = 256; c >= 64; c -= 32) {
-        const long long t = (m_tiles * ((N + c - 1) / c) + pairs - 1) / pairs * SLAB_NS[c / 32 - 2];
-        if (c == 256 || t < best) best = t, cols = c;
+        const long long rounds = (m_tiles * ((N + c - 1) / c) + pairs - 1) / pairs;
+        const long long walk = (K + BK - 1) / BK * SLAB_NS[c / 32 - 2], write = WRITE_NS[c / 32 - 2];
+        const long long t = (rounds - 1) * (walk > write ? walk : write) + walk + write;
+        if (c == 256 || t * 50 < best * 49) best = t, cols = c;
     }
     return cols;
 }
 
 }  // namespace
 
-// The columns that qnn_gemm_tcgen05_2cta chooses for a plain product of this size on a device of so many SMs.
-QNN_API int qnn_gemm_tcgen05_2cta_cols(int M, int N, int sm_count) { return plain_tile_cols(M, N, sm_count); }
+// The columns that qnn_gemm_tcgen05_2cta chooses for a plain product of this size on a device of so many SMs; ..._cols: of a long K.
+QNN_API int qnn_gemm_tcgen05_2cta_width(int M, int N, int K, int sm_count) { return plain_tile_cols(M, N, K, sm_count); }
+QNN_API int qnn_gemm_tcgen05_2cta_cols(int M, int N, int sm_count) { return plain_tile_cols(M, N, 1 << 24, sm_count); }
 
 // The product of qnn_gemm_tcgen05 (same arguments, same meaning of `status`) computed by pairs of CTAs.
 // Returns QNN_ERR_UNSUPPORTED when the device cannot hold a pair (the caller then uses the single-CTA
@@ -365,7 +373,7 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
             sm_count = 148;
     }
     const long long m_tiles = (M + 2 * BM - 1) / (2 * BM);
-    const int cols = epi == EPI_GATED ? 128 : (tile_cols != 0 ? tile_cols : plain_tile_cols(M, N, sm_count));
+    const int cols = epi == EPI_GATED ? 128 : (tile_cols != 0 ? tile_cols : plain_tile_cols(M, N, K, sm_count));
     const long long ntiles = m_tiles * ((Nout + cols - 1) / cols);
     if (ntiles > 0x3fffffffLL) return QNN_ERR_UNSUPPORTED;
     CUtensorMap map_a, map_b;

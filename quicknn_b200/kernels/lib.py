@@ -41,6 +41,7 @@ _SIGNATURES: Dict[str, list] = {
     "qnn_gemm_tcgen05": [c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_vp, c_vp],
     "qnn_gemm_tcgen05_2cta": [c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_vp, c_vp],
     "qnn_gemm_tcgen05_2cta_cols": [c_int, c_int, c_int],
+    "qnn_gemm_tcgen05_2cta_width": [c_int, c_int, c_int, c_int],
     "qnn_gemm_skinny_tcgen05": [c_vp, c_vp, c_vp, c_int, c_int, c_int, c_int, c_float, c_int, c_vp, c_vp],
     "qnn_gemm_skinny_tcgen05_argmax": [c_vp, c_vp, c_vp, c_int, c_int, c_int, c_float, c_vp, c_vp, c_vp],
     "qnn_attn_decode_stages": [c_ll, c_int, c_int, c_int],

@@ -456,14 +456,14 @@ def _sm_count(device) -> int:
 def _rows_for_the_small_kernel(M: int, n_out: int, K: int, epilogue: int, device) -> int:
     """How many of the last rows of a whole-prompt product go to the kernel for few rows instead (0: none).
 
-    The prompt kernel works in 256 x 256 tiles (256 x 128 outputs when gated), a pair of SMs per tile, so its time
-    goes up by a round of tiles when the tile count passes a multiple of the pairs.  Measured for the down product
-    (2304 x 9216): 2048 rows (72 tiles on 74 pairs) 58 us, 2049 rows 92 us, 4096 / 4097 rows 114 / 140 us, 6144 /
-    6145 rows 175 / 212 us: a round that only a few tiles open costs about 0.6 of a tile's time.  The kernel for few
-    rows takes the weights' bytes once more plus 5 us up to 32 rows and 9 us up to 64 (2049 rows: 66 us together, 4097:
-    123, 6145: 179); with more rows it costs what the round does (2200 rows in two launches: 90 against 92 us), and
-    for the matrices with a short inner size the round is cheap, so only up to 64 rows are cut off, and only where
-    the round costs well more than they do."""
+    The prompt kernel works in tiles of 256 rows and up to 256 columns (128 outputs when gated), a pair of SMs per tile, so its
+    time goes up when the count of tiles passes a multiple of the pairs, by less than a round of the widest since it then
+    takes narrower ones.  Measured for the down product (2304 x 9216): 2048 rows (72 tiles on 74 pairs) 56 us, 2049 rows 68 in one
+    launch and 63 with the last row cut off, 2112 rows 68 and 67, 4096 rows 113, 4097 rows 128 and 119.  The kernel for few
+    rows takes the weights' bytes once more plus 5 us up to 32 rows and 9 us up to 64; beyond that it costs what the tiles do, and
+    for the matrices with a short inner size a round is cheap, so only up to 64 rows are cut off, and only where a round (counted
+    below at 256 columns and 0.6 of a tile's time, from when the tiles had one width; the choice was measured again with all) costs well
+    more than they do."""
     if not GEMM_2CTA or M <= 256:
         return 0
     tail = M % 256

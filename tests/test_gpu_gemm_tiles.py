@@ -49,3 +49,20 @@ def test_chosen_widths(cols):
         got = ops.gemm_tcgen05(x, w, out=out[:M - 3])
         assert torch.equal(got, ops.gemm_tcgen05(x, w, tile_cols=256)) and (out[M - 3] == 7.0).all(), (M, N)
     ops.raise_on_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("K", [72, 776, 2312])
+@pytest.mark.parametrize("cols", range(64, 257, 32))
+def test_chosen_widths_by_inner_size(cols, K):
+    """The same with the inner size that the choice counts."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    width = load().qnn_gemm_tcgen05_2cta_width
+    sizes = [(M, N) for M in range(200, 4400, 300) for N in range(8, 4400, 8) if width(M - 3, N, K, sms) == cols]
+    assert sizes or K < 2312
+    for M, N in {sizes[0], sizes[len(sizes) // 2], sizes[-1]} if sizes else ():
+        torch.manual_seed(M + N)
+        x, w = torch.randn((M - 3, K), device=DEV).bfloat16(), (torch.randn((N, K), device=DEV) * 0.05).bfloat16()
+        out = torch.full((M - 2, N), 7.0, dtype=torch.bfloat16, device=DEV)
+        got = ops.gemm_tcgen05(x, w, out=out[:M - 3])
+        assert torch.equal(got, ops.gemm_tcgen05(x, w, tile_cols=256)) and (out[M - 3] == 7.0).all(), (M, N)
+    ops.raise_on_status(torch.device(DEV))

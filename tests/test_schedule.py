@@ -110,3 +110,16 @@ def test_a_decode_graph_knows_whether_its_lengths_are_uneven_where_the_kernel_as
     w = mixer(window=256)
     w.decode_splits = m.decode_splits
     assert w.schedule(step(28, 1024, 1.6)) == (4, True) and w.schedule(step(28, 2048, 1.6)) == (4, False)      # nearly all beyond the window
+
+
+def test_width_of_product_tiles_counts_the_writing_where_the_inner_size_is_short():
+    from quicknn_b200.kernels.lib import load
+    width, long_k = load().qnn_gemm_tcgen05_2cta_width, load().qnn_gemm_tcgen05_2cta_cols
+    # widths that are no multiple of 128 write slowly: by the walk alone these took 192 columns and 4 to 15 % longer than with 256
+    for M, N, K in ((8192, 2048, 512), (8192, 2048, 768), (8192, 3072, 512), (4096, 4096, 256)):
+        assert long_k(M, N, 148) == 192 and width(M, N, K, 148) in (128, 256), (M, N, K)
+    # measured best where the walk is long
+    for (M, N, K), cols in {(256, 2304, 9216): 64, (640, 2304, 9216): 96, (1280, 2304, 9216): 192, (640, 4096, 2304): 192, (1280, 4096, 2304): 160,
+                            (2048, 1536, 6144): 192, (2048, 2304, 9216): 256, (2048, 4096, 2304): 256}.items():
+        assert width(M, N, K, 148) == cols, (M, N, K)
+    assert all(width(M, N, K, 148) % 32 == 0 and 64 <= width(M, N, K, 148) <= 256 for M in (1, 129, 5000, 10 ** 6) for N in (8, 1000, 300000) for K in (8, 65, 70000))
