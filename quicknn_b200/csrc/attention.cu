@@ -503,12 +503,8 @@ static int decode_launch(const void* q, long long q_stride, const void* k_pool, 
 #define QNN_TILED(CPLV, GTV, TTV)                                                                          \
     if (!launched && geo.cpl == CPLV && geo.gt == GTV && tt == TTV) {                                        \
         auto kern = attn_decode_tiled_kernel<T, CPLV, GTV, TTV>;                                            \
-        static bool configured = false;                                                                     \
-        if (!configured) {                                                                                  \
-            cudaError_t ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); \
-            if (ce != cudaSuccess) return (int)ce;                                                          \
-            configured = true;                                                                              \
-        }                                                                                                   \
+        static qnn::OncePerDevice asked;                                                                    \
+        if (const int rc = qnn::allow_shared(asked, kern, 100 * 1024)) return rc;                           \
         qnn::launch_pdl(kern, dim3(grid), dim3(DEC_WARPS * 32), smem_tiled, st, QNN_DEC_ARGS);                                       \
         launched = true;                                                                                    \
     }

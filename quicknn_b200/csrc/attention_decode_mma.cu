@@ -384,63 +384,49 @@ size_t smem_bytes(int max_pages) {
 
 template <int HD, int MMA_WARPS, int ST>
 int allow_memory() {                                 // before the device is asked what it holds, too
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(attn_decode_mma_kernel<HD, MMA_WARPS, ST>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
-    return 0;
+    static OncePerDevice asked;
+    return allow_shared(asked, attn_decode_mma_kernel<HD, MMA_WARPS, ST>, 220 * 1024);
 }
 
-// How many clusters of `size` CTAs of this kernel the device holds at once (asked once per size; 0: none, or
-// clusters are switched off).  Clusters are placed inside a GPC, so fewer CTAs may fit than as a plain grid.
+// How many clusters of `size` CTAs of this kernel the current device holds at once (0: none, or clusters are switched off).
+// Clusters are placed inside a GPC, so fewer CTAs may fit than as a plain grid.
 template <int HD, int MMA_WARPS, int ST>
 int clusters_at_once(size_t smem, int size) {
-    static int known[CLUSTER_MAX + 1] = {-1, -1, -1, -1, -1};
+    static KnownPerDevice known[CLUSTER_MAX + 1];
     if (size < 1 || size > CLUSTER_MAX) return 0;
-    if (known[size] < 0) {
+    return known[size].get(current_device(), (uint32_t)smem, [&] {
         const char* e = getenv("QNN_ATTN_CLUSTER");
-        known[size] = 0;
-        if (!(e && e[0] == '0')) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(size, 1, 1);
-            cfg.blockDim = dim3(MMA_WARPS * 32);
-            cfg.dynamicSmemBytes = smem;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = size;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, attn_decode_mma_kernel<HD, MMA_WARPS, ST>, &cfg) == cudaSuccess && n > 0)
-                known[size] = n;
-            else
-                (void)cudaGetLastError();
-        }
-    }
-    return known[size];
+        if (e && e[0] == '0') return 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(size, 1, 1);
+        cfg.blockDim = dim3(MMA_WARPS * 32);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = size;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, attn_decode_mma_kernel<HD, MMA_WARPS, ST>, &cfg) == cudaSuccess && n > 0) return n;
+        (void)cudaGetLastError();
+        return 0;
+    });
 }
 
-// CTAs of this kernel that the device holds at once as a plain grid (asked once).
+// CTAs of this kernel that the current device holds at once as a plain grid.
 template <int HD, int MMA_WARPS, int ST>
 int ctas_at_once(size_t smem) {
-    static int known = -1;
-    if (known < 0) {
-        int per_sm = 0, dev = 0, sms = 0;
-        known = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_mma_kernel<HD, MMA_WARPS, ST>,
-                                                          MMA_WARPS * 32, smem) == cudaSuccess &&
-            cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
-            known = per_sm * sms;
-        else
-            (void)cudaGetLastError();
-    }
-    return known;
+    static KnownPerDevice known;
+    return known.get(current_device(), (uint32_t)smem, [&] {
+        int per_sm = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_mma_kernel<HD, MMA_WARPS, ST>, MMA_WARPS * 32, smem) ==
+            cudaSuccess)
+            return per_sm * device_sms();
+        (void)cudaGetLastError();
+        return 0;
+    });
 }
 
 // Whether a grid of `clusters` clusters of `size` CTAs merges its key ranges inside the clusters: where they all fit the

@@ -233,12 +233,8 @@ int launch(const void* q, const void* k, const void* v, long long row_stride, vo
            int window, const float* slopes, const float* sinks, cudaStream_t st) {
     auto kern = attn_prefill_mma_kernel<HD, BN>;
     const size_t smem = (size_t)(BM + 4 * BN) * HD * 2;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = qnn::allow_shared(asked, kern, smem)) return rc;
     dim3 grid(nq, B, (max_len + BM - 1) / BM);
     qnn::launch_pdl(kern, dim3(grid), dim3(PF_WARPS * 32), smem, st, (const bf16*)q, (const bf16*)k, (const bf16*)v, (size_t)row_stride,
                                             (bf16*)out, (size_t)out_stride, seq_row0, seq_len, nq, nkv, scale, cap,

@@ -809,24 +809,14 @@ int launch_attn(const Cache& cache, const void* qkv, long long ld, long long tot
     static_assert(layout <= 227 * 1024, "a block's shared memory");
     const size_t smem = layout + 1024 < 227 * 1024 ? layout + 1024 : 227 * 1024;           // with room to align it, where there is
     auto kern = attn_prefill_tcgen05_kernel<HD, FIXED, PAGED>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static OncePerDevice asked;
+    if (const int err = allow_shared(asked, kern, smem)) return err;
     // query tiles of a sequence, of which only the last q_tiles (0: all) hold wanted rows
     const int all_tiles = (max_len + BM - 1) / BM, ntq = q_tiles > 0 && q_tiles < all_tiles ? q_tiles : all_tiles;
-    static int sm_count = 0;
-    if (sm_count == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-            sm_count = 148;
-    }
+    const int sm_count = device_sms();
     // Few CTAs with long key walks: pairs of CTAs share a query tile's keys (see the head of this file).  A pair
     // pays for the cluster launch and the hand-over; the policy and its measurements are below.
-    static int split_ok = -1;                      // the device holds a pair of these CTAs (asked once)
+    static KnownPerDevice holds_a_pair;             // of these CTAs
     const long long singles = (long long)ntq * B * nq;
     const int reach = window > 0 ? (max_len < window + BM - 1 ? max_len : window + BM - 1) : max_len;
     const int key_tiles = (reach + BN - 1) / BN;   // of the heaviest query tile
@@ -857,16 +847,17 @@ int launch_attn(const Cache& cache, const void* qkv, long long ld, long long tot
     attr[1].val.clusterDim.y = 1;
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    if (want_split && split_ok < 0) {
+    const bool pairs = want_split && holds_a_pair.get(current_device(), 0, [&] {
         cfg.gridDim = dim3(2, 1, 1);
         cfg.attrs = attr + 1;
         cfg.numAttrs = 1;
         int n = 0;
-        split_ok = (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) ? 1 : 0;
-        if (!split_ok) (void)cudaGetLastError();
+        const int ok = (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) ? 1 : 0;
+        if (!ok) (void)cudaGetLastError();
         cfg.attrs = attr;
-    }
-    const int split = (want_split && split_ok == 1) ? levels : 0;
+        return ok;
+    }) == 1;
+    const int split = pairs ? levels : 0;
     cfg.gridDim = dim3((unsigned)(split ? 2 * nq : nq), B, ntq);
     const long long ctas = (long long)cfg.gridDim.x * B * ntq;
     const bool pdl = qnn::pdl_enabled() && ctas <= qnn::pdl_max_grid();

@@ -204,12 +204,8 @@ template <int BM, int BN, int WM, int WN, int STAGES>
 int launch_mma(const Args& a, int blocks, cudaStream_t st) {
     auto kern = block_linear_mma_kernel<BM, BN, WM, WN, STAGES>;
     constexpr size_t smem = (size_t)STAGES * (BM + BN) * 128;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = allow_shared(asked, kern, smem)) return rc;
     const dim3 grid((a.N + BN - 1) / BN, (a.T + BM - 1) / BM, blocks);
     launch_pdl(kern, grid, dim3(WM * WN * 32), smem, st, a);
     return (int)cudaGetLastError();

@@ -221,6 +221,20 @@ inline long long pdl_max_grid() {
     return v;
 }
 
+inline int current_device() {
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess) (void)cudaGetLastError();
+    return device;
+}
+inline int device_sms() {
+    static KnownPerDevice known;
+    const int device = current_device();
+    return known.get(device, 0, [&] {
+        int n = 0;
+        return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
+    });
+}
+
 // lets `kernel` have up to `bytes` of dynamic shared memory on the current device; `asked`: a static of the kernel's launcher
 template <typename... KArgs>
 inline int allow_shared(OncePerDevice& asked, void (*kernel)(KArgs...), size_t bytes) {

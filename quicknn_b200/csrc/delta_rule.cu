@@ -887,20 +887,11 @@ delta_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __r
 
 constexpr int MAX_SMEM = 227 * 1024;
 
-int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
-    }
-    return n;
-}
-
 // Shared memory that a scan's blocks ask for.  A block walks its sequence by itself, so a scan takes as long as its slowest block:
 // several on one SM while others are idle (the kernel in front still fills them when blocks are handed out) would set the pace.
 // Up to four rounds of blocks ask for so much that no SM takes more than its share.
 size_t spread(long long blocks, size_t need) {
-    const long long share = (blocks + sm_count() - 1) / sm_count();
+    const long long share = (blocks + device_sms() - 1) / device_sms();
     if (share > 4) return need;
     const size_t least = (size_t)(228 * 1024) / (size_t)(share + 1);
     return need > least ? need : least;
@@ -912,11 +903,8 @@ int scan_tc(const void* q, const void* k, const void* v, long long ld, const voi
             cudaStream_t st) {
     const dim3 grid((vdim + 15) / 16, H, B);
     const size_t smem = spread((long long)grid.x * H * B, TcStage<KS>::TOTAL);
-    static bool set = false;
-    if (!set) {
-        cudaFuncSetAttribute(delta_scan_tc_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
-        set = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = allow_shared(asked, delta_scan_tc_kernel<KS>, MAX_SMEM)) return rc;
     launch_pdl(delta_scan_tc_kernel<KS>, grid, dim3(TC_THREADS), smem, st, (const bf16*)q, (const bf16*)k, (const bf16*)v, ld,
                (const unsigned char*)rec, seq_row0, seq_len, slots, state, slot_stride, out, ldo, H, G, dim, vdim);
     QNN_LAUNCH_CHECK();
@@ -929,11 +917,8 @@ int scan_as(const void* q, const void* k, const void* v, long long ld, const flo
     using Buf = ScanBuf<RPT, CPT>;
     const dim3 grid((vdim + Buf::COLS - 1) / Buf::COLS, H, B);
     const size_t smem = spread((long long)grid.x * H * B, Buf::bytes(RPT <= 16 ? 2 : 1));
-    static bool set = false;
-    if (!set) {
-        cudaFuncSetAttribute(delta_scan_kernel<T, RPT, CPT, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
-        set = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = allow_shared(asked, delta_scan_kernel<T, RPT, CPT, VEC>, MAX_SMEM)) return rc;
     launch_pdl(delta_scan_kernel<T, RPT, CPT, VEC>, grid, dim3(SCAN_THREADS), smem, st,
                (const T*)q, (const T*)k, (const T*)v, ld, inv, ldi, q_scale, rec, seq_row0, seq_len, slots, state, slot_stride, out,
                ldo, H, G, dim, vdim);
@@ -957,11 +942,8 @@ QNN_API int qnn_delta_chunks(const void* q, const void* k, long long ld, int dty
         if (dtype != QNN_DT_BF16 || dim % 8 || ld % 8 || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)rec) & 15)) return QNN_ERR_ARGUMENT;
         const int dpad = (dim + 15) & ~15;
         const size_t smem = (size_t)4 * (2 * CK * (dpad * 2 + 16) + 3 * CK * (CK + 1) * 4);
-        static bool set = false;
-        if (!set) {
-            cudaFuncSetAttribute(delta_chunks_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
-            set = true;
-        }
+        static OncePerDevice asked;
+        if (const int rc = allow_shared(asked, delta_chunks_tc_kernel, MAX_SMEM)) return rc;
         launch_pdl(delta_chunks_tc_kernel, dim3((unsigned)((longest + 4 * CK - 1) / (4 * CK)), G, B), dim3(128), smem, st,
                    (const bf16*)q, (const bf16*)k, ld, inv, ldi, pre, ldp, rate, bias, q_scale, seq_row0, seq_len,
                    (unsigned char*)rec, H, G, dim);

@@ -324,12 +324,8 @@ int launch(const CUtensorMap& map_x, const CUtensorMap& map_w, void* C, int M, i
            float cap, int act, int* status, unsigned tiles, cudaStream_t st, int* err = nullptr) {
     auto kern = gemm_skinny_tcgen05_kernel<EPI>;
     const size_t smem = (size_t)stages * (W_BYTES + NM * BK * 2) + (KS > 1 ? (size_t)BW * ((NM < RECV_COLS ? NM : RECV_COLS) + 4) * 4 : 0) + sizeof(Barriers) + 1024;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = qnn::allow_shared(asked, kern, 227 * 1024)) return rc;
     int tmem_cols = 32;
     while (tmem_cols < NM) tmem_cols *= 2;
     cudaLaunchConfig_t cfg = {};
@@ -371,13 +367,7 @@ static int skinny_tcgen05(const void* A, const void* B, void* C, int M, int N, i
     const long long tiles = (Nout + rows - 1) / rows;
     if (tiles > 0x3fffffffLL) return QNN_ERR_UNSUPPORTED;
     // split K over a cluster when the tiles alone do not fill the GPU; every CTA keeps >= 2 slabs
-    static int sm_count = 0;
-    if (sm_count == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-            sm_count = 148;
-    }
+    const int sm_count = qnn::device_sms();
     const int nk = (K + 63) / 64;
     int KS = 1;
     while (KS < 8 && tiles * KS * 2 <= sm_count && nk / (KS * 2) >= 2) KS *= 2;      // the doubled grid still fits one round
@@ -412,9 +402,10 @@ static int skinny_tcgen05(const void* A, const void* B, void* C, int M, int N, i
         // lost at the 9B and 27B sizes; at 64 rows, where a stage is a third larger, the deep ring is 1 % better)
         stages = depth(113);
     } else if (KS > 1) {
-        static int fits[4][MAX_STAGES + 1];                // clusters of 2^i CTAs that the device holds, by depth (0: not asked)
-        int ki = KS == 2 ? 1 : (KS == 4 ? 2 : 3);
-        if (fits[ki][stages] == 0) {
+        static OncePerDevice asked;
+        static KnownPerDevice fits[4][MAX_STAGES + 1];     // clusters of 2^i CTAs that the device holds, by depth
+        const int ki = KS == 2 ? 1 : (KS == 4 ? 2 : 3);
+        const int held = fits[ki][stages].get(current_device(), 0, [&] {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(KS * 64);
             cfg.blockDim = dim3(THREADS);
@@ -427,14 +418,14 @@ static int skinny_tcgen05(const void* A, const void* B, void* C, int M, int N, i
             cfg.attrs = attr;
             cfg.numAttrs = 1;
             int n = 0;
-            (void)cudaFuncSetAttribute(gemm_skinny_tcgen05_kernel<EPI_NONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            (void)allow_shared(asked, gemm_skinny_tcgen05_kernel<EPI_NONE>, 227 * 1024);
             if (cudaOccupancyMaxActiveClusters(&n, gemm_skinny_tcgen05_kernel<EPI_NONE>, &cfg) != cudaSuccess || n <= 0) {
                 (void)cudaGetLastError();
                 n = -1;
             }
-            fits[ki][stages] = n;
-        }
-        if (fits[ki][stages] < tiles) stages = depth(113);
+            return n;
+        });
+        if (held < tiles) stages = depth(113);
     }
     if (stages > MAX_STAGES || (long long)stages * stage_bytes + recv_bytes + (long long)sizeof(Barriers) + 1024 > 227 * 1024)
         return QNN_ERR_UNSUPPORTED;

@@ -249,35 +249,21 @@ QNN_API int qnn_gemm_tcgen05(const void* A, const void* B, void* C, int M, int N
     if (rc) return rc;
     const int Nout = epi == EPI_GATED ? N / 2 : N;
     const int cols = epi == EPI_GATED ? BN / 2 : BN;
-    static int sm_count = 0;
-    if (sm_count == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-            sm_count = 148;
-    }
+    const int sm_count = qnn::device_sms();
     const long long ntiles = (long long)((M + BM - 1) / BM) * ((Nout + cols - 1) / cols);
     if (ntiles > 0x7fffffffLL) return QNN_ERR_UNSUPPORTED;
     dim3 grid((unsigned)(ntiles < sm_count ? ntiles : sm_count));
     const size_t smem = (size_t)STAGES * STAGE_BYTES + sizeof(Barriers) + 1024;
     if (epi == EPI_GATED) {
         auto kern = gemm_tcgen05_kernel<EPI_GATED>;
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-            configured = true;
-        }
+        static OncePerDevice asked;
+        if (const int rc = qnn::allow_shared(asked, kern, smem)) return rc;
         cudaError_t e = qnn::launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, map_a, map_b, (bf16*)C, M, N, K, act, ActConsts{act_a, act_b}, status);
         return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
     auto kern = gemm_tcgen05_kernel<EPI_NONE>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = qnn::allow_shared(asked, kern, smem)) return rc;
     cudaError_t e = qnn::launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, map_a, map_b, (bf16*)C, M, N, K, act, ActConsts{act_a, act_b}, status);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

@@ -365,13 +365,7 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
     if (tile_cols != 0 && (epi != EPI_NONE || (tile_cols != 64 && tile_cols != 128 && tile_cols != 256))) return QNN_ERR_ARGUMENT;
     if (epi == EPI_GATED && (N & 1)) return QNN_ERR_ARGUMENT;
     const int Nout = epi == EPI_GATED ? N / 2 : N;
-    static int sm_count = 0;
-    if (sm_count == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-            sm_count = 148;
-    }
+    const int sm_count = device_sms();
     const long long m_tiles = (M + 2 * BM - 1) / (2 * BM);
     const int cols = epi == EPI_GATED ? 128 : (tile_cols != 0 ? tile_cols : plain_tile_cols(M, N, K, sm_count));
     const long long ntiles = m_tiles * ((Nout + cols - 1) / cols);
@@ -390,8 +384,8 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
     const int which = epi == EPI_GATED ? 0 : cols / 32 - 1;
     const Kernel kern = forms[which].kernel;
     const size_t smem = (size_t)forms[which].ring_bytes + STAGING_BYTES + sizeof(Barriers) + 1024;
-    static bool configured[8] = {};
-    static int max_pairs = 0;
+    static OncePerDevice asked[8];
+    static KnownPerDevice known[8];
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = smem;
@@ -404,22 +398,17 @@ QNN_API int qnn_gemm_tcgen05_2cta(const void* A, const void* B, void* C, int M, 
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    if (!configured[which]) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured[which] = true;
-    }
-    if (max_pairs == 0) {        // pairs of this kernel that the device holds at once (asked once)
+    if (const int err = allow_shared(asked[which], kern, smem)) return err;
+    const int max_pairs = known[which].get(current_device(), 0, [&] {        // of this kernel that the device holds at once
         cfg.gridDim = dim3(2 * (sm_count / 2));
         cfg.numAttrs = 1;
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
             (void)cudaGetLastError();
-            max_pairs = -1;
-        } else {
-            max_pairs = n < sm_count / 2 ? n : sm_count / 2;
+            return -1;
         }
-    }
+        return n < sm_count / 2 ? n : sm_count / 2;
+    });
     if (max_pairs < 0) return QNN_ERR_UNSUPPORTED;
     const int pairs = ntiles < max_pairs ? (int)ntiles : max_pairs;
     cfg.gridDim = dim3(2 * pairs);

@@ -465,12 +465,9 @@ int scan_launch(const void* q, const void* k, const void* v, long long ld, const
         using C = GlaChunk<RPTV, CPTV>;                                                                              \
         const dim3 grid((vdim + C::COLS - 1) / C::COLS, H, seg_len > 0 ? B * nseg : B);                              \
         const size_t smem = (size_t)C::FLOATS * sizeof(float) * (RPTV <= 16 ? 2 : 1);                                \
-        static bool set = false;                                                                                     \
-        if (smem > 48 * 1024 && !set) {                                                                              \
-            cudaFuncSetAttribute(gla_scan_kernel<T, RPTV, CPTV>, cudaFuncAttributeMaxDynamicSharedMemorySize,        \
-                                 (int)smem);                                                                         \
-            set = true;                                                                                              \
-        }                                                                                                            \
+        static OncePerDevice asked;                                                                                  \
+        if (smem > 48 * 1024)                                                                                        \
+            if (const int rc = allow_shared(asked, gla_scan_kernel<T, RPTV, CPTV>, smem)) return rc;                 \
         launch_pdl(gla_scan_kernel<T, RPTV, CPTV>, grid, dim3(GLA_THREADS), smem, st, (const T*)q, (const T*)k,     \
                    (const T*)v, ld, decay, ldd, q_scale, seq_row0, seq_len, slots, state, out, ldo, H, dim, vdim,    \
                    seg_len, nseg, x.decay_per_head, x.kw, x.ldw, x.ones_col, stride, x.key_from_decay, x.max_rows); \

@@ -301,48 +301,30 @@ QNN_API int qnn_moe_tcgen05(const void* rows, const void* w, void* out, int n_en
     if (rc) return rc;
     const int Nout = epi == EPI_GATED ? N / 2 : N;
     const int cols = epi == EPI_GATED ? BN / 2 : BN;
-    static int sm_count = 0;
-    if (sm_count == 0) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-            sm_count = 148;
-    }
+    const int sm_count = qnn::device_sms();
     const long long ntiles = (long long)max_row_tiles * ((Nout + cols - 1) / cols);
     if (ntiles > 0x7fffffffLL) return QNN_ERR_UNSUPPORTED;
     dim3 grid((unsigned)(ntiles < sm_count ? ntiles : sm_count));
     const size_t smem = (size_t)STAGES * STAGE_BYTES + sizeof(Barriers) + 1024;
     if (epi == EPI_GATED) {
         auto kern = moe_tcgen05_kernel<EPI_GATED>;
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-            configured = true;
-        }
+        static OncePerDevice asked;
+        if (const int rc = qnn::allow_shared(asked, kern, smem)) return rc;
         cudaError_t e = qnn::launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, map_a, map_b, out, N, K, offsets, perm,
                                         sel_w, tiles, n_row_tiles, scale_output, limit, alpha, status);
         return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
     if (epi == EPI_ACT) {
         auto kern = moe_tcgen05_kernel<EPI_ACT>;
-        static bool configured = false;
-        if (!configured) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-            configured = true;
-        }
+        static OncePerDevice asked;
+        if (const int rc = qnn::allow_shared(asked, kern, smem)) return rc;
         cudaError_t e = qnn::launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, map_a, map_b, out, N, K, offsets, perm,
                                         sel_w, tiles, n_row_tiles, scale_output, limit, alpha, status);
         return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
     }
     auto kern = moe_tcgen05_kernel<EPI_NONE>;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = qnn::allow_shared(asked, kern, smem)) return rc;
     cudaError_t e = qnn::launch_pdl(kern, grid, dim3(GEMM_THREADS), smem, st, map_a, map_b, out, N, K, offsets, perm, sel_w,
                                     tiles, n_row_tiles, scale_output, limit, alpha, status);
     return e != cudaSuccess ? (int)e : (int)cudaGetLastError();

@@ -19,4 +19,18 @@ struct OncePerDevice {
     }
 };
 
+// What a launcher asks about a device (how many of its blocks fit at once): the last answer, with what it was asked for.
+struct KnownPerDevice {
+    std::atomic<uint64_t> last[64] = {};                         // 0: nothing yet; else key + 1 above the answer
+    template <typename Ask>
+    int get(int device, uint32_t key, Ask ask) {
+        if (device < 0 || device >= 64) return ask();
+        const uint64_t have = last[device].load(std::memory_order_relaxed), mine = ((uint64_t)key + 1) << 32;
+        if (have >> 32 == mine >> 32) return (int)(uint32_t)have;
+        const int answer = ask();
+        last[device].store(mine | (uint32_t)answer, std::memory_order_relaxed);
+        return answer;
+    }
+};
+
 }  // namespace qnn

@@ -266,11 +266,9 @@ QNN_API int qnn_add_layernorm(float* resid, const void* y, int y_dt, const void*
         QNN_LAUNCH_CHECK();
     }
     const size_t smem = (size_t)H * sizeof(float);
-    static bool set = false;
-    if (smem > 40 * 1024 && !set) {      // beside the static shared memory
-        cudaFuncSetAttribute(add_layernorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        set = true;
-    }
+    static OncePerDevice asked;
+    if (smem > 40 * 1024)                 // beside the static shared memory
+        if (const int rc = allow_shared(asked, add_layernorm_kernel, 160 * 1024)) return rc;
     launch_pdl(add_layernorm_kernel, dim3(T), dim3(row_threads(H)), smem, st, resid, y, y_dt, bias, b_dt, w, w_dt, eps, copy,
                copy_dt, H);
     QNN_LAUNCH_CHECK();
@@ -285,11 +283,9 @@ QNN_API int qnn_mean_rmsnorm(const void* const* ys, const void* const* ws, int n
     Branches br;
     if (int rc = fill(br, ys, ws, n)) return rc;
     const size_t smem = (size_t)H * sizeof(float);
-    static bool set = false;
-    if (smem > 40 * 1024 && !set) {      // beside the static shared memory
-        cudaFuncSetAttribute(mean_rmsnorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        set = true;
-    }
+    static OncePerDevice asked;
+    if (smem > 40 * 1024)                 // beside the static shared memory
+        if (const int rc = allow_shared(asked, mean_rmsnorm_kernel, 160 * 1024)) return rc;
     launch_pdl(mean_rmsnorm_kernel, dim3(T), dim3(row_threads(H)), smem, st, br, y_dt, w_dt, eps, out, out_dt, H);
     QNN_LAUNCH_CHECK();
 }
@@ -308,11 +304,9 @@ QNN_API int qnn_add_mean_layernorm(float* resid, const void* const* ys, const vo
         QNN_LAUNCH_CHECK();
     }
     const size_t smem = (size_t)H * sizeof(float);
-    static bool set = false;
-    if (smem > 40 * 1024 && !set) {      // beside the static shared memory
-        cudaFuncSetAttribute(add_mean_layernorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-        set = true;
-    }
+    static OncePerDevice asked;
+    if (smem > 40 * 1024)                 // beside the static shared memory
+        if (const int rc = allow_shared(asked, add_mean_layernorm_kernel, 160 * 1024)) return rc;
     launch_pdl(add_mean_layernorm_kernel, dim3(T), dim3(row_threads(H)), smem, st, resid, br, y_dt, bw_dt, eps_branch, w,
                w_dt, eps, copy, copy_dt, H);
     QNN_LAUNCH_CHECK();

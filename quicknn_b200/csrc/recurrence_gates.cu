@@ -217,12 +217,8 @@ QNN_API int qnn_recurrence_gates(const void* u, long long ldu, const void* w, co
     p.u = (const bf16*)u; p.w = (const bf16*)w; p.rb = rb; p.ib = ib; p.decay = decay; p.z = z; p.state = state;
     p.scratch = scratch; p.seq_row0 = seq_row0; p.seq_len = seq_len; p.slots = slots; p.ldu = ldu; p.ldz = ldz;
     p.slot_stride = slot_stride; p.C = C; p.part = part; p.nseg = nseg; p.tiles = (part + CH - 1) / CH;
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(recurrence_gates_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
+    static OncePerDevice asked;
+    if (const int rc = allow_shared(asked, recurrence_gates_kernel, SMEM)) return rc;
     launch_pdl(recurrence_gates_kernel, dim3((unsigned)(p.tiles * (C / part)), (unsigned)y, n_seqs), dim3(THREADS), SMEM, st, p);
     QNN_LAUNCH_CHECK();
 }

@@ -258,15 +258,10 @@ QNN_API int qnn_recurrent_step(const void* p, long long ldp, int y_col, int x_co
     s.taps = taps; s.scale = scale;
     const size_t smem = (size_t)((part + BK - 1) / BK) * ROWS * ROWB + (size_t)STAGES * W_STAGE;
     const dim3 grid((part + CH - 1) / CH, (B + ROWS - 1) / ROWS, C / part);
-    static bool configured = false;
-    if (!configured) {
-        const int most = (MAX_PART / BK) * ROWS * ROWB + STAGES * W_STAGE;
-        cudaError_t e = cudaFuncSetAttribute(recurrent_step_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(recurrent_step_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e != cudaSuccess) return (int)e;
-        configured = true;
-    }
-    if (taps == 4 && ((uintptr_t)conv & 15) == 0) launch_pdl(recurrent_step_kernel<4>, grid, dim3(THREADS), smem, st, s);
-    else launch_pdl(recurrent_step_kernel<0>, grid, dim3(THREADS), smem, st, s);
+    static OncePerDevice asked_four, asked_any;
+    const bool four = taps == 4 && ((uintptr_t)conv & 15) == 0;
+    const auto kernel = four ? recurrent_step_kernel<4> : recurrent_step_kernel<0>;
+    if (const int rc = allow_shared(four ? asked_four : asked_any, kernel, (MAX_PART / BK) * ROWS * ROWB + STAGES * W_STAGE)) return rc;
+    launch_pdl(kernel, grid, dim3(THREADS), smem, st, s);
     QNN_LAUNCH_CHECK();
 }
