@@ -307,8 +307,7 @@ _status = {}
 
 def status_words(device) -> torch.Tensor:
     """Two int32 words per device that kernels set and the host reads together: [0] the status of
-    the tcgen05 kernels' bounded waits (1 loads, 2 tensor-core issue, 4 epilogue), [1] the
-    non-finite flag of ``check_finite``."""
+    the tcgen05 kernels (see ``wait_status_message``), [1] the non-finite flag of ``check_finite``."""
     device = torch.device(device)
     t = _status.get(device)
     if t is None:
@@ -328,8 +327,16 @@ def finite_flag(device) -> torch.Tensor:
 
 
 def wait_status_message(v: int) -> str:
-    return (f"a tcgen05 kernel gave up waiting (status {v}: 1 loads, 2 tensor-core issue, 4 epilogue); "
-            f"its result is not valid")
+    """What the status of the tcgen05 kernels says: bits of the waits that ran out (products: 1 loads, 2 tensor-core issue, 4
+    epilogue; prompt attention: 2 keys and values, 4 scores, 8 weights, 16 ring, 32 queries, 64 product, 128 the other half of a
+    pair), and 256 for shared memory that does not start where the prompt attention needs it."""
+    said = []
+    if v & 255 or not v & 256:
+        said.append(f"gave up waiting (status {v & 255}; products: 1 loads, 2 tensor-core issue, 4 epilogue; prompt attention: 2 keys and "
+                    f"values, 4 scores, 8 weights, 16 ring, 32 queries, 64 product, 128 the other half of a pair)")
+    if v & 256:
+        said.append("found its shared memory at an address that leaves no room for its operands (status 256)")
+    return f"a tcgen05 kernel {' and '.join(said)}; its result is not valid"
 
 
 def raise_on_status(device) -> None:

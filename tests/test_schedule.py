@@ -123,3 +123,11 @@ def test_width_of_product_tiles_counts_the_writing_where_the_inner_size_is_short
                             (2048, 1536, 6144): 192, (2048, 2304, 9216): 256, (2048, 4096, 2304): 256}.items():
         assert width(M, N, K, 148) == cols, (M, N, K)
     assert all(width(M, N, K, 148) % 32 == 0 and 64 <= width(M, N, K, 148) <= 256 for M in (1, 129, 5000, 10 ** 6) for N in (8, 1000, 300000) for K in (8, 65, 70000))
+
+
+def test_a_kernel_that_ran_nothing_is_not_reported_as_one_that_gave_up_waiting():
+    from quicknn_b200.kernels.ops import wait_status_message
+    assert "gave up waiting (status 5;" in wait_status_message(5) and "shared memory" not in wait_status_message(5)
+    assert "shared memory" in wait_status_message(256) and "waiting" not in wait_status_message(256)
+    both = wait_status_message(256 | 32)
+    assert "gave up waiting (status 32;" in both and "shared memory" in both
