@@ -789,7 +789,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
 
 
-struct Cache { const void *k_pool, *v_pool; long long rows; const int *table, *slots; int max_pages; };   // k_pool null: packed rows
+struct Cache { const void* k_pool; void* v_pool; long long rows; const int *table, *slots; int max_pages; };   // k_pool null: packed rows
 
 template <int HD, bool FIXED, bool PAGED>
 int launch_attn(const Cache& cache, const void* qkv, long long ld, long long total_rows, void* out, long long out_stride, const int* seq_row0,
@@ -804,7 +804,7 @@ int launch_attn(const Cache& cache, const void* qkv, long long ld, long long tot
     rc = PAGED ? make_map(&map_v, cache.v_pool, cache.rows, HD, BN) : make_map(&map_v, qkv, total_rows, width, BN);
     if (rc) return rc;
     if (!PAGED) map_k = map_v;
-    const Pages pages = {(bf16*)cache.v_pool, cache.table, cache.slots, cache.max_pages};
+    const Pages pages = {static_cast<bf16*>(cache.v_pool), cache.table, cache.slots, cache.max_pages};
     constexpr size_t layout = (size_t)k_stages(HD) * 2 * BN * HD * 2 + (size_t)v_stages(HD) * BN * HD * 2 + 2 * P_BYTES + sizeof(Barriers);
     static_assert(layout <= 227 * 1024, "a block's shared memory");
     const size_t smem = layout + 1024 < 227 * 1024 ? layout + 1024 : 227 * 1024;           // with room to align it, where there is
@@ -923,12 +923,12 @@ QNN_API int qnn_attn_prefill_tcgen05(const void* qkv, long long ld, long long to
 // Attention of a step that continues sequences, over the paged cache, which holds every key and value by now, this step's included
 // (no ring that has wrapped): sequence b's new rows are rows seq_row0[b] .. of qkv and of out, at positions start[b] .. length[b] - 1; no
 // sequence brings more than most_new of them, none is longer than `longest`.  Pools: [pool_pages, nkv, 64, hd]; page_table: [slots, max_pages].
-// The value cells behind a sequence in its last page are cleared.  What it saves is the copy of whole sequences out of the pages into
+// v_pool is written too: the value cells behind a sequence in its last page are cleared.  What it saves is the copy of whole sequences out of the pages into
 // packed rows and of the wanted rows out of the result.
 QNN_API int qnn_attn_extend_tcgen05(const void* qkv, long long ld, long long total_rows, void* out, long long out_stride, const int* seq_row0,
                                     const int* length, const int* start, int most_new, int B, int longest, int nq, int nkv, int hd,
                                     float scale, float cap, int window, int* status, const float* slopes, const float* sinks,
-                                    const void* k_pool, const void* v_pool, long long pool_pages, const int* page_table, int max_pages,
+                                    const void* k_pool, void* v_pool, long long pool_pages, const int* page_table, int max_pages,
                                     const int* slots, cudaStream_t st) {
     if (start == nullptr || k_pool == nullptr || v_pool == nullptr || page_table == nullptr || slots == nullptr || most_new <= 0)
         return QNN_ERR_ARGUMENT;

@@ -188,7 +188,7 @@ class OpTimer:
 
     SKIP = {"status_words", "finite_flag", "raise_on_status", "check_gemm_status", "wait_status_message", "dt_code",
             "attention_refusal", "linear_refusal", "sample_scratch_bytes", "head_candidates", "head_argmax_fusable",
-            "qkv_rope_cache_fusable", "cache_append", "gemm_tcgen05", "gemm_skinny_tcgen05", "activation_"}
+            "qkv_rope_cache_fusable", "extends_in_pages", "cache_append", "gemm_tcgen05", "gemm_skinny_tcgen05", "activation_"}
 
     def __init__(self, engine, hbm_gbs: float, tflops: float, context: int = 0):
         self.engine, self.hbm, self.tflops, self.context = engine, hbm_gbs * 1e9, tflops * 1e12, context
@@ -242,6 +242,9 @@ class OpTimer:
             flops = 4.0 * T * H * dim * vs
             of_values = (kw.get("values") if kw.get("values") is not None else proj).element_size()
             byts = float(T * (2 * H * dim * proj.element_size() + H * vdim * of_values) + T * H * vs * 4 + 2 * n_seqs * H * dim * vs * 4)
+        elif name == "attn_extend_paged":            # every key and value of the step's sequences, once
+            nkv, hd, whole = a[2], a[3], a[8]
+            byts = float(_nbytes(a[0]) + _nbytes(out) + 2 * whole.total * nkv * hd * a[0].element_size())
         elif name == "attn_prefill_paged":
             qkv, nq, nkv, hd, window = a[0], a[1], a[2], a[3], a[13]
             T = qkv.shape[0]

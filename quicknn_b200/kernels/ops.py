@@ -790,17 +790,18 @@ def attn_extend(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, k_poo
 
 
 def extends_in_pages(qkv: torch.Tensor, head_dim: int, line, whole) -> bool:
-    """Whether attn_extend_paged takes a step that continues sequences: many bfloat16 rows, and a cache line that holds every position
-    (no ring, or none that has wrapped) in pages of 64."""
+    """Whether attn_extend_paged takes a step that continues sequences: bfloat16 rows on 16 bytes, and a cache line that holds every
+    position (no ring, or none that has wrapped) in pages of 64."""
     return (whole is not None and ATTN_TCGEN05 and EXTEND_PAGED and qkv.dtype == torch.bfloat16 and head_dim in (64, 128, 256)
-            and whole.most_new >= EXTEND_TENSOR_CORE_FROM and line.writes and line.has_values and line.k.dtype == torch.bfloat16
+            and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0 and whole.most_new >= EXTEND_TENSOR_CORE_FROM and line.writes and line.has_values and line.k.dtype == torch.bfloat16
             and line.page_size == 64 and (not line.ring or whole.longest <= line.ring))
 
 
 def attn_extend_paged(qkv: torch.Tensor, n_heads: int, n_kv: int, head_dim: int, line, scale: float, cap: Optional[float],
                       window: Optional[int], whole, slopes: Optional[torch.Tensor] = None, sinks: Optional[torch.Tensor] = None):
     """``attn_extend`` where this step's keys and values are in the cache line already (and ``extends_in_pages`` holds): the
-    tensor-core prompt kernel reads the pages themselves."""
+    tensor-core prompt kernel reads the pages themselves.  The line's value cells behind a sequence, in its last page, are set to
+    zero: their weights are zero, but zero times an Inf or NaN that an earlier sequence left there is not."""
     ld = _rows(qkv, "qkv", torch.bfloat16)
     _check_per_head(slopes, sinks, n_heads)
     for n, t in (("k_pool", line.k), ("v_pool", line.v)):
