@@ -7,7 +7,7 @@
 // mma.m16n8k16:
 //     S^T[16 keys x 8 heads]  = K[16 keys x hd]   * Q^T[hd x 8 heads]        (A = K,   B = Q^T)
 //     O^T[hd x 8 heads]      += V^T[hd x 16 keys] * P^T[16 keys x 8 heads]   (A = V^T, B = P^T)
-// K and V tiles of 16 keys travel global -> shared memory by cp.async in a 3-stage pipeline per
+// K and V tiles of 16 keys travel global -> shared memory by cp.async in a pipeline of 3 stages (2: see stages_for) per
 // warp (rows XOR-swizzled by 16-byte chunk so that ldmatrix does not conflict); K fragments come
 // from ldmatrix, V^T fragments from ldmatrix.trans; Q^T stays in registers for the whole kernel;
 // P^T is rearranged from the accumulator layout of S^T with eight shuffles.  Softmax state

@@ -25,8 +25,9 @@
 //                       lies in [-cap, cap], so exp(score) can neither overflow nor vanish in float32:
 //                       p = exp(cap tanh(s / cap)) against the fixed reference 0, the same softmax (it is invariant
 //                       under the shift) with nothing carried from tile to tile but a row's sum.
-// Both groups' arithmetic runs on pairs of scores (f32x2 instructions: the same rounding, half the issue slots), which
-// the softmax is bound by.  us before / after both groups and pairs, no softcap: 8 heads of 256, one prompt of 2048 43.2 /
+// Both groups' arithmetic runs on pairs of scores (f32x2 instructions: the same rounding; one prompt of 2048 with a softcap,
+// 8 heads of 256: 8.6 -> 6.5 million instructions, of them on the FMA pipe 4.1 -> 2.6, and the softmax is bound by both).
+// us before / after both groups and pairs, no softcap: 8 heads of 256, one prompt of 2048 43.2 /
 // 37.4, four of 1024 34.1 / 30.6; 8 heads of 128, 1777 + 731 + 301 tokens 37.1 / 29.7; with a softcap (pairs alone, the same
 // bits): 35.6 / 34.9, 31.7 / 29.2, 29.2 / 27.5; 1500 tokens under a window of 300 18.2 / 15.5.
 // What set the pace, in the order in which it was found (clock64 around the waits of each role): the softmax chain of

@@ -180,7 +180,7 @@ __global__ void moe_route_kernel(const TX* __restrict__ x, const TW* __restrict_
 
 // The same, bit for bit, for the many rows of a prompt: 8 rows per block (see row_dots), then a warp per row.  us, a block per row / now:
 // 16 experts of rows of 2304, 256 rows 6.4 / 6.3, 512 rows 7.5 / 6.4, 2048 rows 18.1 / 9.2, 4096 rows 29.9 / 17.1; 32 experts of 1536, 256 rows
-// 7.9 / 7.7, 2048 rows 22.2 / 11.3; below 256 rows a block per row is as fast.  Bound by the issue of loads, unpacking and products.
+// 8.1 / 7.8, 2048 rows 22.2 / 11.3; below 256 rows a block per row is as fast.
 constexpr int ROUTE_FROM = 256;
 __global__ void __launch_bounds__(DOT_ROWS * 32)
 moe_route_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wr, int T, int W, int E, int top, int score_fn, int renorm,

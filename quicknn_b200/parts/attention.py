@@ -180,7 +180,8 @@ class AttentionMixer(Mixer):
         if why:
             raise ValueError(f"attention mixer: {why}")
         # blocks of the decode attention kernel that the device holds at once: its shared memory is
-        # 384 bytes per element of a head, so two fit on an SM at head size 256, four at 128, eight at 64
+        # 384 bytes per element of a head, so two fit on an SM at head size 256, four at 128, eight at 64.  (Beyond that many the
+        # kernel may take a third less at head size 256, so that three fit; the estimates of decode_splits leave that out.)
         dev = torch.device(device)
         sms = torch.cuda.get_device_properties(dev).multi_processor_count if dev.type == "cuda" else 148
         self._resident = sms * max(1, min(8, 512 // max(1, self.head_dim)))
@@ -208,7 +209,8 @@ class AttentionMixer(Mixer):
         2: 1.32, 3: 1.08, 4: 1.34, 5: 1.20, 6: 1.11, 8: 1.18 (one round of 288 blocks, then 2, 2, 2 and 3 rounds);
         batch 28: 2: 1.34, 3: 1.60, 5: 1.23, 6: 1.39; batch 12: 4: 0.91, 5: 0.85, 6: 0.81, 8: 0.94; batch 64 one
         range 9.48 ms (26 layers) against two 9.69 and eight 8.42; batch 64 with prompts of 512 to 2048 tokens one
-        range 4.20 ms, four 4.03, six 3.90, nine 4.12 (the longest sequence no longer sets the pace).  Results
+        range 4.20 ms, four 4.03, six 3.90, nine 4.12 (the longest sequence no longer sets the pace).  (All measured with two
+        blocks an SM; grids beyond ``_resident`` blocks may now run three, see the kernel's stages.)  Results
         differ between these choices by rounding only: ranges are summed in a fixed order."""
         fixed = step.tuning.get("decode_splits")
         if fixed:
