@@ -589,9 +589,9 @@ def test_attention_decode(ops, dtype, nq, nkv, hd, window, cap, splits):
 
 @pytest.mark.parametrize("splits", [2, 3, 4])
 def test_attention_decode_with_more_clusters_than_the_device_holds(ops, splits):
-    """30 sequences x 4 kv heads at head size 256: 120 clusters of 3 CTAs do not fit the device at once, so the
-    key ranges go through the scratch and the merge kernel; with 2 and 4 ranges they merge inside the clusters.
-    The same numbers either way."""
+    """30 sequences x 4 kv heads at head size 256: the 240 CTAs of 2 ranges fit the device at once, the 360 and 480 of 3 and 4 do
+    not (one round of two stages, two rounds of three), and where their clusters do not all fit either the key ranges go through
+    the scratch and the merge kernel.  The same numbers either way."""
     rng = np.random.default_rng(splits)
     nq, nkv, hd, B = 8, 4, 256, 30
     lens = [int(n) for n in rng.integers(1, 190, B)]
